@@ -1,0 +1,53 @@
+"""GPU parity of the persistent decode kernel (decode_fused.cu) against the oracle, at the sizes where it can go wrong: one to
+eight groups of 128 along C, one and several tiles per CTA, fewer CTAs than SMs, query heads per kv head, contexts that end just
+before, on and behind a pass of 128 keys and a split of the keys, vocabularies that leave CTAs different row counts, both cache
+types, and a step count beyond one launch (64 steps)."""
+import numpy as np
+import pytest
+
+from webllm_b200 import Gpu, QwenGpt, synthetic
+
+from test_gpu_qwen import _dense_from_gptq, _ocfg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("C,H,KVH,I,V,prompt,kv", [
+    (128, 2, 1, 128, 64, 5, "f32"),
+    (256, 4, 4, 384, 511, 126, "f16"),
+    (640, 10, 2, 1280, 1000, 230, "f32"),
+    (1024, 16, 4, 2816, 3001, 255, "f16"),
+    (896, 14, 2, 4864, 2048, 1020, "f16"),
+])
+def test_fused_decode_matches_oracle(built_lib, oracle, C, H, KVH, I, V, prompt, kv):
+    cfg = synthetic.QwenShape(V, 2, H, KVH, C, I)
+    G = synthetic.random_qwen_gptq(cfg, seed=C + prompt, std=0.05)
+    ids = np.random.default_rng(prompt).integers(0, V, prompt).astype(np.uint32)
+    steps, max_t = 70, prompt + 80
+    ref = oracle.CachedForward(_ocfg(oracle, cfg), _dense_from_gptq(oracle, G), max_t=max_t, kv_f16=kv == "f16",
+                               threads=oracle.max_threads())
+    tok = first = oracle.sample_greedy(ref.prefill(ids))
+    want = []
+    for _ in range(steps):
+        row = ref.decode_step(tok)
+        tok = oracle.sample_greedy(row)
+        want.append(tok)
+    rms = float(np.sqrt(np.mean(row.astype(np.float64) ** 2)))
+    with Gpu(0, weight_bytes=256 << 20, act_bytes=256 << 20) as gpu:
+        model = QwenGpt(gpu, cfg, max_t=max_t, kv_dtype=kv)
+        model.upload_gptq_model(G, fuse=True)
+        model.set_exact(True)
+        model.prefill(ids, last_only=True)
+        gpu.synchronize()
+        before = gpu.launch_count
+        got = model.decode_greedy(first, steps).tolist()
+        assert gpu.launch_count - before == 4  # the weights laid out (two launches), then 64 and 6 steps
+        assert got == want
+        assert oracle.check_tolerance(model.last_logits(), row, 5e-4 * rms, 5e-4).ok
+        # the same steps one at a time
+        model.reset_cache()
+        model.prefill(ids, last_only=True)
+        for t in [first] + want[:3]:
+            row = model.read_tensor(model.decode_step(t))
+        assert int(row.argmax()) == want[3]
+        model.close()

@@ -1,0 +1,1248 @@
+// Whole decode steps in one persistent kernel: embedding, all layers, final norm, tied lm_head, greedy argmax, token after
+// token, with no kernel boundary in between.
+//
+// What bounds it. A token of a 0.5B-class model streams 458 MB (0.07 ms of HBM), but as one kernel per operation the step is
+// a chain of 125 dependent launches of ~3.9 us each (0.49 ms): every hand-over pays the end of one grid, the start of the
+// next, and the first weight request behind it. Here one CTA per SM stays resident for the step and
+//   * weights never wait for anything: at set-up they are laid out per CTA and layer as one contiguous block, and bulk copies
+//     keep two to three blocks in flight, across phase, layer and token boundaries;
+//   * activations are handed over WITHOUT a barrier: every f32 value is stored together with the step's epoch in one 64-bit
+//     word, and a reader polls the very words that it needs. A hand-over is one store and one load through L2, about
+//     0.9 us from all CTAs to all, against a store, a fence, an atomic and a second round trip for a grid barrier. All layers
+//     use the same words, with an epoch of their own: while each layer had its own, a poll's first try missed L2 (the weights
+//     had pushed the words out since the step before) and came back from HBM a microsecond later, empty. Writing them over is
+//     safe because a CTA gets to write a vector of layer l + 1 only through down of l, which needs the gate|up of every CTA of
+//     l, which comes after that CTA's last read of q|k|v, attention and o of l; down and gate|up of l are guarded the same way
+//     by gate|up of l + 1 and by q|k|v of l + 1;
+//   * every CTA keeps the residual stream itself, so the norms need no hand-over of their own.
+// A layer is five such hand-overs: q|k|v, attention, o, gate|up (with silu * up at the producer), down.
+// Measured on the 0.5B shapes: 0.49 -> 0.30 ms per token at short contexts (0.33 at 400 keys), of which about 0.13 are the CTA's
+// own arithmetic and latencies, 0.03 lm_head beyond what its first slots hide, and the rest hand-overs.
+//
+// Arithmetic. A CTA owns whole output columns in tiles of 8. One m16n8k16 MMA multiplies 256 weights: rows 0-7 of the weight
+// operand are half of the positions of a tile's 8 columns, rows 8-15 the other half, and the activation operand holds the first
+// half in columns 0 (fp16 value) and 1 (fp16 remainder) and the second in columns 2 and 3, so f32 activations keep
+// ~22 bits as in the int4 GEMV; weights are exact integers q - z, f32 accumulation, one f32 scale per 128-row group.
+//
+// All CTAs have to be resident at once, hence the cooperative launch. Every poll is bounded in time; one that gives up sets
+// the context's status word and lets all later polls of its CTA through, so the kernel drains its copies and ends.
+#include <algorithm>
+
+#include "qwen_internal.cuh"
+
+namespace wb {
+namespace fd {
+
+constexpr int kThreads = 256, kWarps = 8;
+constexpr int kUnitBytes = 576;   // 8 columns x 128 rows: 512 of nibbles, then scale * 2^24 and scale * zero point of every column
+constexpr int kSplitMax = 8;      // CTAs that share the keys of one head
+constexpr int kPartWords = 66;    // one split's partial attention result: 64 sums, max, sum of weights
+constexpr int kLmRows = 32;       // lm_head rows per slot of the weight ring
+constexpr int kMaxC = 1024;       // hidden size: four values per thread, four 16-byte pieces of an lm_head row per lane
+constexpr int kMaxI = 8192;
+constexpr int kSlotsMax = 3;
+constexpr int kStatusHandover = 41, kStatusRing = 42;
+
+typedef unsigned long long u64;
+
+// Shared memory: Head | ring of weight slots | planes [4][pitch] | red | attention floats | x [C] f32 | small words
+struct Smem {
+    int ring, planes, red, att, xs, sums, small, total;
+};
+struct Params {
+    const char *blobs;      // [layer][cta] blocks of blob_stride bytes
+    const float *aux;       // per layer: input norm [C], post norm [C], q|k|v bias [C + 2 KV]
+    const float *final_norm;
+    const __half *embed;
+    const float *cs_table;
+    char *k_cache, *v_cache;
+    u64 *ll;                // hand-over words of a layer (ll_layer), then two sets of 2 per CTA for the argmax candidates
+    float *logits;
+    uint32_t *history;      // nullable; pinned host memory
+    int *status;
+    size_t kv_layer_bytes, ll_layer;
+    uint32_t epoch, first_token;
+    int n_cta, n_layer, C, H, KVH, I, V, KV, pos0, n_steps, slots, slot_bytes, blob_stride;
+    float eps;
+    Smem sm;
+};
+
+// The MLP's activations are staged kBatch fours per thread at a time.
+constexpr int kBatch = 5;
+__host__ __device__ inline int padded(int I) { return (I + kBatch * 4 * kThreads - 1) / (kBatch * 4 * kThreads) * (kBatch * 4 * kThreads); }
+
+// Tiles of 8 columns are dealt round robin; the offset moves where the dealing starts, so that the CTAs with one tile more of
+// gate|up are not those with a tile of down.
+struct Deal {
+    int tiles, off;
+};
+__host__ __device__ inline int deal_count(const Deal &d, int cta, int n)
+{
+    const int first = (cta - d.off % n + n) % n;
+    return first < d.tiles ? (d.tiles - first + n - 1) / n : 0;
+}
+__host__ __device__ inline int deal_tile(const Deal &d, int cta, int n, int i) { return (cta - d.off % n + n) % n + i * n; }
+__host__ __device__ inline Deal deal_qkv(int C, int KV) { return {(C + 2 * KV) / 8, 0}; }
+__host__ __device__ inline Deal deal_o(int C, int n) { return {C / 8, n - (C / 8) % n}; }
+__host__ __device__ inline Deal deal_gu(int I) { return {I / 8, 0}; }  // pairs of a gate and an up tile
+__host__ __device__ inline Deal deal_down(int C, int n) { return {C / 8, n - (C / 8) % n}; }
+
+// ---------------------------------------------------------------------------------------------------- device helpers
+__device__ __forceinline__ uint32_t s32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint64_t *b, uint32_t n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s32(b)), "r"(n) : "memory"); }
+__device__ __forceinline__ void mbar_expect(uint64_t *b, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(s32(b)), "r"(bytes) : "memory");
+}
+// Bounded: a copy always completes, so running out means a broken device; the code is recorded and the caller carries on.
+__device__ __forceinline__ void mbar_wait(uint64_t *b, uint32_t parity, int *status)
+{
+    const uint32_t a = s32(b);
+#pragma unroll 1
+    for (uint32_t it = 0; it < (1u << 26); it++) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(a), "r"(parity)
+                     : "memory");
+        if (ok) return;
+    }
+    *(volatile int *)status = kStatusRing;
+}
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(s32(dst)), "l"(src),
+                 "r"(bytes), "r"(s32(bar))
+                 : "memory");
+}
+
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// ---- hand-over words: value in the low half, epoch in the high half ----
+__device__ __forceinline__ void ll_put(u64 *p, float v, uint32_t ep)
+{
+    const u64 w = ((u64)ep << 32) | __float_as_uint(v);
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+__device__ __forceinline__ ulonglong2 ll_load2(const u64 *p)
+{
+    ulonglong2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool ll_ok(const ulonglong2 &v, uint32_t ep) { return (uint32_t)(v.x >> 32) == ep && (uint32_t)(v.y >> 32) == ep; }
+__device__ __forceinline__ float2 ll_vals(const ulonglong2 &v) { return make_float2(__uint_as_float((uint32_t)v.x), __uint_as_float((uint32_t)v.y)); }
+
+// The first bytes of shared memory.
+struct Head {
+    uint64_t full[kSlotsMax + 1];  // ring barriers
+    int *status;
+    volatile int gave_up;
+    volatile uint32_t token;
+    int fill_i, fill_slot, fill_left;  // the feeder's: next fill of the ring (its index in the step, its slot), steps left
+};
+// Waiting for words. Everything that a warp waits for is loaded and checked together (a thread that took its words one after the
+// other would pay a round trip for each: none of them was there yet when it came), only what is missing is loaded again, and the
+// warp leaves the loop as one. Bounded: a poll is a round trip to L2 (at least 0.15 us), so kPolls of them are seconds; a CTA
+// that has given up once lets its later polls through after a few rounds. Full warps only.
+constexpr uint32_t kPolls = 1u << 24;
+__device__ __forceinline__ bool ll_done(bool ok, uint32_t it, Head *hd)
+{
+    if (__all_sync(0xffffffffu, ok)) return true;
+    if ((it & 255) != 0 || (it < kPolls && !hd->gave_up)) return false;
+    if (!hd->gave_up) hd->gave_up = 1, *(volatile int *)hd->status = kStatusHandover;
+    return true;
+}
+// v[i] = the pair of words at p + i * stride (16-byte aligned)
+template <int N>
+__device__ __forceinline__ void ll_get(ulonglong2 (&v)[N], const u64 *p, int stride, uint32_t ep, Head *hd)
+{
+#pragma unroll
+    for (int i = 0; i < N; i++) v[i] = ll_load2(p + i * stride);
+#pragma unroll 1
+    for (uint32_t it = 1;; it++) {
+        bool ok = true;
+#pragma unroll
+        for (int i = 0; i < N; i++) ok = ok && ll_ok(v[i], ep);
+        if (ll_done(ok, it, hd)) break;
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            if (!ll_ok(v[i], ep)) v[i] = ll_load2(p + i * stride);
+    }
+}
+__device__ __forceinline__ float2 ll_get2(const u64 *p, uint32_t ep, Head *hd)
+{
+    ulonglong2 v[1];
+    ll_get(v, p, 0, ep, hd);
+    return ll_vals(v[0]);
+}
+// The MLP's activations are the one long vector that many CTAs read (4864 values by 112 CTAs), and its bytes are what its
+// hand-over takes, so they travel as 32-bit words with the epoch's parity in the lowest mantissa bit (every word is written in
+// every step). The error, 2^-24 of the value, is below that of the fp16 pairs that it is staged as.
+__device__ __forceinline__ void act_put(uint32_t *p, float v, uint32_t ep)
+{
+    const uint32_t w = ((__float_as_uint(v) + (__float_as_uint(v) & 1u)) & ~1u) | (ep & 1u);
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(w) : "memory");
+}
+__device__ __forceinline__ uint4 act_load4(const uint32_t *p)
+{
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool act_ok(const uint4 &v, uint32_t ep) { return ((ep & 1u) ? (v.x & v.y & v.z & v.w & 1u) : ((~(v.x | v.y | v.z | v.w)) & 1u)) != 0; }
+__device__ __forceinline__ float4 act_vals(const uint4 &v)
+{
+    return make_float4(__uint_as_float(v.x & ~1u), __uint_as_float(v.y & ~1u), __uint_as_float(v.z & ~1u), __uint_as_float(v.w & ~1u));
+}
+
+__device__ __forceinline__ float warp_sum(float v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// ---- staging: f32 values -> the four planes of the activation operand ----
+// Plane 0/1: fp16 value / remainder of the positions 0, 1, 4, 5 of every 8, plane 2/3 of 2, 3, 6, 7. The weights' nibbles are laid
+// out to match (lay_out_kernel), so that four neighbouring values are four 32-bit stores. Inside a group of 128 positions the
+// 8-byte pieces (one per plane and packed row) are ordered by row % 4, then row / 4: what a lane needs for the four k-steps of a
+// unit is 32 bytes in a row.
+__host__ __device__ inline int plane_pitch(int K) { return K + 16; }  // bytes, K a multiple of 128: conflict-free 16-byte reads
+__device__ __forceinline__ uint32_t half2_bits(__half2 h) { return *reinterpret_cast<const uint32_t *>(&h); }
+__device__ __forceinline__ void stage4(char *planes, int pitch, int k, float4 v)  // positions k (a multiple of 4) to k + 3
+{
+    char *at = planes + (k & ~127) + ((k & 24) << 2) + ((k & 96) >> 2) + (k & 4);
+    const __half2 e = __floats2half2_rn(v.x, v.y), o = __floats2half2_rn(v.z, v.w);
+    const float2 fe = __half22float2(e), fo = __half22float2(o);
+    *reinterpret_cast<uint32_t *>(at) = half2_bits(e);
+    *reinterpret_cast<uint32_t *>(at + pitch) = half2_bits(__floats2half2_rn(v.x - fe.x, v.y - fe.y));
+    *reinterpret_cast<uint32_t *>(at + 2 * pitch) = half2_bits(o);
+    *reinterpret_cast<uint32_t *>(at + 3 * pitch) = half2_bits(__floats2half2_rn(v.z - fo.x, v.w - fo.y));
+}
+
+// A nibble masked in place is the fp16 subnormal q * 2^-24 (or 16 q * 2^-24), which the MMA multiplies exactly; the zero point
+// comes off through the group's activation sum (as in gemv_core.cuh).
+__device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y));
+}
+__device__ __forceinline__ void mma_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y), "f"(0.f));
+}
+// Units are worked on B at a time without a branch between them, so that their chains (load, mask, four MMAs, one shuffle)
+// overlap: five units of a warp take 500 cycles together, and 1340 with a condition around each. Results of units that are not
+// there are computed from whatever lies behind and not stored. Five is what divides the long projections of the 0.5B model
+// (ten tiles of gate|up and five groups of down per warp).
+constexpr int kBurst = 5;
+struct Unit {  // weights in registers, requested before the activations are there
+    uint4 q;
+    float2 s;
+    __device__ __forceinline__ void load(const char *ub, int lane)
+    {
+        q = *reinterpret_cast<const uint4 *>(ub + lane * 16);
+        s = *reinterpret_cast<const float2 *>(ub + 512 + (lane >> 2) * 8);
+    }
+};
+// This lane's part of a group's staged activations: the four k-steps of its plane.
+struct Acts {
+    uint2 b[4];
+    // (lanes 16 to 31 hold columns of the product that nobody reads)
+    __device__ __forceinline__ void load(const char *xu)
+    {
+        const uint4 p = *reinterpret_cast<const uint4 *>(xu), q = *reinterpret_cast<const uint4 *>(xu + 16);
+        b[0] = make_uint2(p.x, p.y), b[1] = make_uint2(p.z, p.w), b[2] = make_uint2(q.x, q.y), b[3] = make_uint2(q.z, q.w);
+    }
+    // Sum of the positions whose products this lane holds (lane % 4 = 0: the first half, 1: the second), by the same instruction
+    // with a weight operand of ones: no reduction over the warp that staged them.
+    __device__ __forceinline__ float sum() const
+    {
+        constexpr uint32_t kOnes = 0x3c003c00u;
+        float d[4];
+        mma_first(d, kOnes, kOnes, kOnes, kOnes, b[0]);
+#pragma unroll
+        for (int i = 1; i < 4; i++) mma(d, kOnes, kOnes, kOnes, kOnes, b[i]);
+        return d[0] + d[1];
+    }
+};
+// Product of the two before the halves are added: lanes 4c and 4c + 1 hold column c's.
+__device__ __forceinline__ float unit_half(const Unit &u, const Acts &x, float sum, int lane)
+{
+    const uint32_t qv[4] = {u.q.x, u.q.y, u.q.z, u.q.w};
+    float d[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t w8 = qv[i] >> 8;
+        if (i == 0) mma_first(d, qv[i] & 0x000f000fu, qv[i] & 0x00f000f0u, w8 & 0x000f000fu, w8 & 0x00f000f0u, x.b[i]);
+        else mma(d, qv[i] & 0x000f000fu, qv[i] & 0x00f000f0u, w8 & 0x000f000fu, w8 & 0x00f000f0u, x.b[i]);
+    }
+    const float v = (lane & 1) == 0 ? d[0] + d[1] : (d[2] + d[3]) * 0.0625f;
+    return fmaf(u.s.x, v, -u.s.y * sum);
+}
+__device__ __forceinline__ float halves(float v) { return v + __shfl_xor_sync(0xffffffffu, v, 1); }
+
+// ---------------------------------------------------------------------------------------------------- attention
+// One CTA per (head, split of the keys), 16 keys per warp and pass, on the tensor cores: K rows (as they lie in the cache: a lane
+// takes 16 consecutive dims of two keys) are the 16-row operand, the rotated query the column operand (fp16 value and remainder);
+// then V transposed by ldmatrix is the row operand and the softmax weights (value and remainder) the column operand. An f32
+// cache goes through as fp16 value and remainder too, so nothing is rounded beyond ~22 bits. Rows are requested before the query
+// is waited for (they were written in earlier steps), so the cache's latency is hidden. Each warp keeps its own online softmax;
+// the warps' states are combined once at the end. With one multiply per lane and dim instead, the scores and sums of 128
+// keys took 0.8 us of the layer.
+constexpr int kPassKeys = kWarps * 16;
+constexpr int kSplitKeys = 2 * kPassKeys;  // a head gets one more CTA per so many keys: a pass costs less than merging one more split
+
+// shared memory, in floats: query value and remainder (fp16) [64], new k [64], new v [64], max [8], sum [8], sums [8][64]
+constexpr int kAttFloats = 3 * 64 + 2 * kWarps + kWarps * 64;
+
+__device__ __forceinline__ uint32_t pack2(float a, float b) { return half2_bits(__floats2half2_rn(a, b)); }
+__device__ __forceinline__ uint32_t pack2_rest(float a, float b, uint32_t hi)
+{
+    const float2 h = __half22float2(*reinterpret_cast<const __half2 *>(&hi));
+    return pack2(a - h.x, b - h.y);
+}
+
+template <typename KV>
+struct KeyTile;
+template <>
+struct KeyTile<__half> {  // keys g and g + 8 of the warp's 16: dims 16 t to 16 t + 15 as eight fp16 pairs each
+    static constexpr int kParts = 1;
+    uint32_t k[2][1][8];
+    __device__ __forceinline__ void load(int r, const __half *row)
+    {
+        const uint4 a = __ldcg(reinterpret_cast<const uint4 *>(row)), b = __ldcg(reinterpret_cast<const uint4 *>(row) + 1);
+        k[r][0][0] = a.x, k[r][0][1] = a.y, k[r][0][2] = a.z, k[r][0][3] = a.w, k[r][0][4] = b.x, k[r][0][5] = b.y, k[r][0][6] = b.z, k[r][0][7] = b.w;
+    }
+    __device__ __forceinline__ void load_new(int r, const float *row)  // (already rounded to fp16)
+    {
+#pragma unroll
+        for (int i = 0; i < 8; i++) k[r][0][i] = pack2(row[2 * i], row[2 * i + 1]);
+    }
+};
+template <>
+struct KeyTile<float> {
+    static constexpr int kParts = 2;  // value and remainder
+    uint32_t k[2][2][8];
+    __device__ __forceinline__ void load(int r, const float *row)
+    {
+        float4 f[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) f[i] = __ldcg(reinterpret_cast<const float4 *>(row) + i);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            k[r][0][2 * i] = pack2(f[i].x, f[i].y), k[r][0][2 * i + 1] = pack2(f[i].z, f[i].w);
+            k[r][1][2 * i] = pack2_rest(f[i].x, f[i].y, k[r][0][2 * i]), k[r][1][2 * i + 1] = pack2_rest(f[i].z, f[i].w, k[r][0][2 * i + 1]);
+        }
+    }
+    __device__ __forceinline__ void load_new(int r, const float *row)
+    {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            k[r][0][i] = pack2(row[2 * i], row[2 * i + 1]);
+            k[r][1][i] = pack2_rest(row[2 * i], row[2 * i + 1], k[r][0][i]);
+        }
+    }
+};
+
+// The warp's V rows as a tile [16 keys][64 dims] of fp16 in shared memory, 16-byte pieces swizzled by key % 8 for ldmatrix.
+__device__ __forceinline__ uint32_t v_at(int key, int piece) { return (uint32_t)(key * 128 + ((piece ^ (key & 7)) << 4)); }
+template <typename KV>
+struct ValueTile;
+template <>
+struct ValueTile<__half> {
+    __device__ __forceinline__ void load(char *tile, const __half *base, int ld, int keys, int lane)
+    {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int key = i * 4 + (lane >> 3), piece = lane & 7;
+            char *dst = tile + v_at(key, piece);
+            if (key < keys)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s32(dst)), "l"(base + (size_t)key * ld + piece * 8) : "memory");
+            else
+                *reinterpret_cast<uint4 *>(dst) = make_uint4(0u, 0u, 0u, 0u);  // (weight 0, but no stray NaN)
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    __device__ __forceinline__ void arrive(char *, int) { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+    __device__ __forceinline__ void put_new(char *tile, int key, const float *v, int lane)
+    {
+        *reinterpret_cast<uint32_t *>(tile + v_at(key, lane >> 2) + (lane & 3) * 4) = pack2(v[2 * lane], v[2 * lane + 1]);
+    }
+    __device__ __forceinline__ void rest(char *, int) {}
+};
+template <>
+struct ValueTile<float> {
+    float4 f[8];  // key 2 i + lane / 16, dims 4 (lane % 16) to + 3
+    __device__ __forceinline__ void load(char *, const float *base, int ld, int keys, int lane)
+    {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int key = 2 * i + (lane >> 4);
+            f[i] = key < keys ? __ldcg(reinterpret_cast<const float4 *>(base + (size_t)key * ld) + (lane & 15)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    __device__ __forceinline__ void put_new(char *, int key, const float *v, int lane)
+    {
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (key == 2 * i + (lane >> 4)) f[i] = *reinterpret_cast<const float4 *>(v + 4 * (lane & 15));
+    }
+    __device__ __forceinline__ char *at(char *tile, int i, int lane) { return tile + v_at(2 * i + (lane >> 4), (lane & 15) >> 1) + (lane & 1) * 8; }
+    __device__ __forceinline__ void arrive(char *tile, int lane)  // the values
+    {
+#pragma unroll
+        for (int i = 0; i < 8; i++) *reinterpret_cast<uint2 *>(at(tile, i, lane)) = make_uint2(pack2(f[i].x, f[i].y), pack2(f[i].z, f[i].w));
+    }
+    __device__ __forceinline__ void rest(char *tile, int lane)  // the remainders in their place
+    {
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            *reinterpret_cast<uint2 *>(at(tile, i, lane)) =
+                make_uint2(pack2_rest(f[i].x, f[i].y, pack2(f[i].x, f[i].y)), pack2_rest(f[i].z, f[i].w, pack2(f[i].z, f[i].w)));
+    }
+};
+
+// kbase / vbase: the split's first key; nk: its keys, the last of them the new one (in sm) if own_new
+template <typename KV>
+struct Attend {
+    KeyTile<KV> kt;
+    ValueTile<KV> vt;
+
+    __device__ __forceinline__ void load(const KV *kbase, const KV *vbase, int ld, int first, int nk_mem, char *tile, int lane)
+    {
+        const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const int key = first + g + 8 * r;
+            if (key < nk_mem) kt.load(r, kbase + (size_t)key * ld + t * 16);
+        }
+        vt.load(tile, vbase + (size_t)first * ld, ld, nk_mem - first, lane);
+    }
+    // one: the only split of its head: the result is final
+    __device__ __forceinline__ void run(const KV *kbase, const KV *vbase, int ld, int nk, bool own_new, float *sm, char *tile, u64 *out, bool one,
+                                        uint32_t ep, int warp, int lane)
+    {
+        float *wm = sm + 192, *wl = wm + kWarps, *wa = wl + kWarps;
+        const int g = lane >> 2, t = lane & 3, nk_mem = own_new ? nk - 1 : nk;
+        uint2 q[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            q[j] = make_uint2(0u, 0u);
+            if (g < 2) q[j] = *reinterpret_cast<const uint2 *>(reinterpret_cast<const char *>(sm) + g * 128 + (t * 16 + 4 * j) * 2);
+        }
+        float acc[4][4] = {}, m = -INFINITY, l = 0.f;
+#pragma unroll 1
+        for (int first = warp * 16; first < nk; first += kPassKeys) {
+            if (first != warp * 16) load(kbase, vbase, ld, first, nk_mem, tile, lane);
+            if (own_new && nk_mem - first >= 0 && nk_mem - first < 16) {  // the new key is one of these
+                const int at = nk_mem - first;
+                if (g == at) kt.load_new(0, sm + 64 + t * 16);
+                if (g + 8 == at) kt.load_new(1, sm + 64 + t * 16);
+                if (sizeof(KV) == 4) vt.put_new(tile, at, sm + 128, lane);
+                vt.arrive(tile, lane);
+                if (sizeof(KV) == 2) {
+                    __syncwarp();
+                    vt.put_new(tile, at, sm + 128, lane);
+                }
+            } else {
+                vt.arrive(tile, lane);
+            }
+            float d[2][4] = {};
+#pragma unroll
+            for (int part = 0; part < KeyTile<KV>::kParts; part++)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    mma(d[j & 1], kt.k[0][part][2 * j], kt.k[1][part][2 * j], kt.k[0][part][2 * j + 1], kt.k[1][part][2 * j + 1], q[j]);
+            // lanes t = 0: scores of keys g and g + 8
+            float s0 = (d[0][0] + d[1][0]) + (d[0][1] + d[1][1]), s1 = (d[0][2] + d[1][2]) + (d[0][3] + d[1][3]);
+            if (t != 0 || first + g >= nk) s0 = -INFINITY;
+            if (t != 0 || first + g + 8 >= nk) s1 = -INFINITY;
+            float mn = fmaxf(s0, s1);
+#pragma unroll
+            for (int o = 4; o <= 16; o <<= 1) mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+            mn = fmaxf(m, __shfl_sync(0xffffffffu, mn, 0));
+            const float corr = expf(m - mn), p0 = expf(s0 - mn), p1 = expf(s1 - mn);
+            m = mn, l = l * corr + (p0 + p1);
+            // weights of keys 2t, 2t + 1 and 2t + 8, 2t + 9: values for column 0, remainders for column 1
+            const float w0 = __shfl_sync(0xffffffffu, p0, 8 * t), w1 = __shfl_sync(0xffffffffu, p0, 8 * t + 4);
+            const float w2 = __shfl_sync(0xffffffffu, p1, 8 * t), w3 = __shfl_sync(0xffffffffu, p1, 8 * t + 4);
+            uint2 b = make_uint2(pack2(w0, w1), pack2(w2, w3));
+            if (g == 1) b = make_uint2(pack2_rest(w0, w1, b.x), pack2_rest(w2, w3, b.y));
+            if (g > 1) b = make_uint2(0u, 0u);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] *= corr;
+            __syncwarp();  // the tile's pieces are there for the whole warp
+#pragma unroll
+            for (int part = 0; part < KeyTile<KV>::kParts; part++) {
+                if (part == 1) {
+                    __syncwarp();
+                    vt.rest(tile, lane);
+                    __syncwarp();
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    uint32_t a[4];
+                    const uint32_t addr = s32(tile) + v_at((lane & 7) + ((lane >> 4) << 3), 2 * i + ((lane >> 3) & 1));
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
+                                 : "r"(addr)
+                                 : "memory");
+                    mma(acc[i], a[0], a[1], a[2], a[3], b);
+                }
+            }
+            __syncwarp();  // before a next pass writes the tile
+        }
+#pragma unroll
+        for (int o = 4; o <= 16; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        if (t == 0) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) wa[warp * 64 + i * 16 + g] = acc[i][0] + acc[i][1], wa[warp * 64 + i * 16 + g + 8] = acc[i][2] + acc[i][3];
+            if (g == 0) wm[warp] = m, wl[warp] = l;
+        }
+        __syncthreads();
+        if (warp < 3) {  // warps 0 and 1: 32 sums each; warp 2: max and sum of weights
+            const float mw = wm[lane & (kWarps - 1)], lw = wl[lane & (kWarps - 1)];
+            float M = mw;
+#pragma unroll
+            for (int o = kWarps / 2; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+            const float ew = mw == -INFINITY ? 0.f : expf(mw - M);
+            float den = lw * ew, r = 0.f;
+#pragma unroll
+            for (int o = kWarps / 2; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+            if (warp < 2) {
+#pragma unroll
+                for (int i = 0; i < kWarps; i++) r = fmaf(wa[i * 64 + warp * 32 + lane], __shfl_sync(0xffffffffu, ew, i), r);
+                ll_put(out + warp * 32 + lane, one ? r / den : r, ep);
+            } else if (lane < 2) {
+                ll_put(out + 64 + lane, lane == 0 ? M : den, ep);
+            }
+        }
+    }
+};
+
+// ---------------------------------------------------------------------------------------------------- the kernel
+inline Smem smem_layout(int slots, int slot_bytes, int C, int I, int red_units)
+{
+    Smem s;
+    // (the V tiles of the attention lie behind the planes of C)
+    const int planes = 4 * plane_pitch(padded(I)), tiles = 4 * plane_pitch(C) + kWarps * 2048;
+    s.ring = 128;
+    s.planes = s.ring + slots * slot_bytes;
+    s.red = s.planes + (planes > tiles ? planes : tiles);
+    s.att = s.red + red_units * 32;
+    s.xs = s.att + kAttFloats * 4;
+    s.sums = s.xs + C * 4;
+    s.small = s.sums + (padded(I) / 128 * 4 + 15) / 16 * 16;
+    s.total = s.small + 2 * kWarps * 4;
+    return s;
+}
+inline int max_units(int C, int I, int KV, int n)
+{
+    const int G = C / 128, GI = I / 128;
+    const int a = (((C + 2 * KV) / 8 + n - 1) / n) * G, b = ((C / 8 + n - 1) / n) * G;
+    const int c = ((I / 8 + n - 1) / n) * 2 * G, d = ((C / 8 + n - 1) / n) * GI;
+    const int m1 = a > b ? a : b, m2 = c > d ? c : d;
+    return m1 > m2 ? m1 : m2;
+}
+
+template <typename KV>
+__global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params p)
+{
+    extern __shared__ __align__(128) char smem[];
+    const int cta = blockIdx.x, n = gridDim.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int C = p.C, I = p.I, KVd = p.KV, QKV = C + 2 * KVd, G = C / 128, GI = I / 128, L = p.n_layer;
+    const Deal dq = deal_qkv(C, KVd), dow = deal_o(C, n), dg = deal_gu(I), dd = deal_down(C, n);
+    const int nq = deal_count(dq, cta, n), no = deal_count(dow, cta, n), ng = deal_count(dg, cta, n), nd = deal_count(dd, cta, n);
+    const int fq = deal_tile(dq, cta, n, 0), fo = deal_tile(dow, cta, n, 0), fg = deal_tile(dg, cta, n, 0), fdn = deal_tile(dd, cta, n, 0);
+    const int uq = nq * G, uo = no * G, ug = ng * 2 * G, ud = nd * GI;
+    const Smem &so = p.sm;
+    char *planes = smem + so.planes;
+    float *red = reinterpret_cast<float *>(smem + so.red), *att = reinterpret_cast<float *>(smem + so.att);
+    float *xs = reinterpret_cast<float *>(smem + so.xs), *sums = reinterpret_cast<float *>(smem + so.sums);
+    float *ssq = reinterpret_cast<float *>(smem + so.small);  // [16]
+    int *widx = reinterpret_cast<int *>(ssq + kWarps);        // [16]
+    Head *hd = reinterpret_cast<Head *>(smem);
+    uint64_t *full = hd->full;
+    char *ring = smem + so.ring;
+    const int rem = p.V % n, row0 = p.V / n * cta + min(cta, rem), row1 = row0 + p.V / n + (cta < rem);
+    const int lm_fills = (row1 - row0 + kLmRows - 1) / kLmRows;
+
+    if (tid == 0) {
+        for (int i = 0; i < p.slots; i++) mbar_init(&full[i], 1);
+        hd->gave_up = 0, hd->status = p.status;
+        hd->fill_i = 0, hd->fill_slot = 0, hd->fill_left = p.n_steps;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+
+    // The ring of weight slots: the fills of a step are its layers' blocks, then the lm_head rows, and the next step's follow.
+    // One thread of the last warp (the one with the least other work) refills a slot as soon as a barrier has told it that every
+    // warp is done with it.
+    const bool feeder = tid == kThreads - 32;
+    const uint32_t block_bytes = (uint32_t)(uq + uo + ug + ud) * kUnitBytes;
+    auto fill = [&]() {
+        if (hd->fill_left == 0) return;
+        const int i = hd->fill_i, at = hd->fill_slot;
+        const char *src;
+        uint32_t bytes;
+        if (i < L) {
+            src = p.blobs + ((size_t)i * n + cta) * p.blob_stride, bytes = block_bytes;
+        } else {
+            const int r = row0 + (i - L) * kLmRows;
+            src = reinterpret_cast<const char *>(p.embed + (size_t)r * C), bytes = (uint32_t)min(kLmRows, row1 - r) * C * 2;
+        }
+        mbar_expect(&full[at], bytes);
+        if (bytes) bulk_load(ring + at * p.slot_bytes, src, bytes, &full[at]);
+        hd->fill_slot = at + 1 == p.slots ? 0 : at + 1;
+        if (i + 1 == L + lm_fills) hd->fill_i = 0, hd->fill_left--;
+        else hd->fill_i = i + 1;
+    };
+    if (feeder)
+#pragma unroll 1
+        for (int i = 0; i < p.slots; i++) fill();
+    int slot = 0;
+    uint32_t par = 0;
+    auto next_slot = [&]() {
+        if (++slot == p.slots) slot = 0, par ^= 1;
+    };
+
+    const int H = p.H, hpk = H / p.KVH;
+    const int pitch_c = plane_pitch(C), pitch_i = plane_pitch(padded(I)), c4 = 4 * tid;
+    const bool has4 = c4 < C;
+    const float inv_c = 1.f / (float)C;
+    const int w_o = QKV, w_act = w_o + C, w_down = w_act + I / 2, w_att = w_down + C;  // words of a layer; q | k | v first
+    u64 *const ll = p.ll, *const cand = ll + p.ll_layer;
+    uint32_t *const act = reinterpret_cast<uint32_t *>(ll + w_act);
+    uint32_t token = p.first_token;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);  // this thread's part of the residual stream
+    // Projections from C: a warp stays with one group of 128 rows (its activations are loaded once) and takes the CTA's tiles in
+    // turn; where there are fewer groups than half the warps, several warps share a group's tiles.
+    const int wpg = kWarps / G, grp = warp % G, sub = warp / G;
+    const int t_first = sub < wpg ? sub : 1 << 16;  // (no tiles for the warps that are left over)
+    const char *xp_c = planes + ((lane >> 2) & 3) * pitch_c + (lane & 3) * 32 + grp * 128, *xp_i = planes + ((lane >> 2) & 3) * pitch_i + (lane & 3) * 32;
+    const int part = lane & 3, red_at = part * 8 + (lane >> 2);
+    float *red_c = red + grp * 8 + (lane >> 2), *red_i = red + (lane >> 2);
+    char *tile = planes + 4 * pitch_c + warp * 2048;
+
+    // rmsnorm of the residual stream (rmsNormRef, src/reference/qwen-ref.ts:12-29)
+    auto norm = [&](float4 w) {
+        const float ss = warp_sum(fmaf(x.x, x.x, x.y * x.y) + fmaf(x.z, x.z, x.w * x.w));
+        if (lane == 0) ssq[warp] = ss;
+        __syncthreads();
+        const float4 a = reinterpret_cast<const float4 *>(ssq)[0], b = reinterpret_cast<const float4 *>(ssq)[1];
+        const float rstd = rsqrtf((((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) * inv_c + p.eps);
+        return make_float4(x.x * rstd * w.x, x.y * rstd * w.y, x.z * rstd * w.z, x.w * rstd * w.w);
+    };
+    auto load4 = [&](const float *a) { return has4 ? __ldg(reinterpret_cast<const float4 *>(a) + tid) : make_float4(0.f, 0.f, 0.f, 0.f); };
+    auto add_residual = [&](const u64 *a, uint32_t ep) {
+        if (!has4) return;
+        ulonglong2 v[2];
+        ll_get(v, a + c4, 2, ep, hd);
+        const float2 f = ll_vals(v[0]), g = ll_vals(v[1]);
+        x.x += f.x, x.y += f.y, x.z += g.x, x.w += g.y;
+    };
+    Unit u[kBurst];
+    const int tile_step = wpg * G * kUnitBytes;
+    auto load_tiles = [&](const char *w, int i) {  // this warp's tiles from i on (the block's end is not the ring's: no bounds)
+        w += (i * G + grp) * kUnitBytes;
+#pragma unroll
+        for (int j = 0; j < kBurst; j++) u[j].load(w + j * tile_step, lane);
+    };
+    auto load_one = [&](const char *w) { u[0].load(w + (t_first * G + grp) * kUnitBytes, lane); };
+    auto run_tiles = [&](const char *w, int tiles) {  // from load_tiles
+        Acts xa;
+        xa.load(xp_c);
+        const float sum = xa.sum();
+#pragma unroll 1
+        for (int i = t_first; i < tiles; i += kBurst * wpg) {
+            float v[kBurst];
+#pragma unroll
+            for (int j = 0; j < kBurst; j++) v[j] = unit_half(u[j], xa, sum, lane);
+            if (i + kBurst * wpg < tiles) load_tiles(w, i + kBurst * wpg);
+#pragma unroll
+            for (int j = 0; j < kBurst; j++) v[j] = halves(v[j]);
+#pragma unroll
+            for (int j = 0; j < kBurst; j++)
+                if (part == 0 && i + j * wpg < tiles) red_c[(i + j * wpg) * G * 8] = v[j];
+        }
+    };
+    auto run_short = [&](const char *w, int tiles) {  // a projection of few tiles per CTA, from load_one
+        Acts xa;
+        xa.load(xp_c);
+        const float sum = xa.sum();
+#pragma unroll 1
+        for (int i = t_first; i < tiles; i += wpg) {
+            if (i > t_first) u[0].load(w + (i * G + grp) * kUnitBytes, lane);
+            const float v = halves(unit_half(u[0], xa, sum, lane));
+            if (part == 0) red_c[i * G * 8] = v;
+        }
+    };
+    // sum over the groups of one tile: four lanes per column; r: the tile's results
+    auto column_sum_c = [&](const float *r) {  // up to 8 groups (C <= 1024)
+        float a = part < G ? r[red_at] : 0.f;
+        if (part + 4 < G) a += r[red_at + 32];
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        return a + __shfl_xor_sync(0xffffffffu, a, 2);
+    };
+    auto column_sum_i = [&](const float *r) {
+        float a = 0.f, b = 0.f;
+        r += red_at;
+        int g = part;
+#pragma unroll 2
+        for (; g + 4 < GI; g += 8, r += 64) a += r[0], b += r[32];
+        if (g < GI) a += r[0];
+        a += b;
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        return a + __shfl_xor_sync(0xffffffffu, a, 2);
+    };
+
+    if (feeder) mbar_wait(&full[0], 0, p.status);
+    __syncthreads();
+#pragma unroll 1
+    for (int s = 0; s < p.n_steps; s++) {
+        uint32_t ep = p.epoch + (uint32_t)(s * L);  // of this step's first layer; one more per layer
+        const int pos = p.pos0 + s, n_keys = pos + 1;
+        const int S = max(1, min(min(kSplitMax, n / H), (n_keys + kSplitKeys - 1) / kSplitKeys));
+        const int chunk = (n_keys + S - 1) / S;
+        const bool is_att = cta < H * S;
+        const int h = is_att ? cta / S : 0, sp = cta - h * S, kvh = h / hpk;
+        const int k0 = sp * chunk, k1 = min(n_keys, k0 + chunk), nk = max(0, k1 - k0);
+        const bool own_new = is_att && nk > 0 && k1 == n_keys;
+
+        if (has4) {
+            const uint2 e = __ldg(reinterpret_cast<const uint2 *>(p.embed + (size_t)min(token, (uint32_t)p.V - 1u) * C) + tid);
+            const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&e.x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&e.y));
+            x = make_float4(a.x, a.y, b.x, b.y);
+        }
+#pragma unroll 1
+        for (int l = 0; l < L; l++, ep++) {
+            // (the block of this layer has arrived: the feeder waited for it before the barrier that ended the layer before)
+            const char *wb = ring + slot * p.slot_bytes;
+            const float *aux = p.aux + l * (2 * C + QKV);
+
+            // -- q | k | v
+            if (sub < wpg) load_one(wb);
+            float4 nw = load4(aux);
+            const float bias = warp < nq ? __ldg(aux + 2 * C + (fq + warp * n) * 8 + (lane >> 2)) : 0.f;
+            // the rest of the layer's constants comes from HBM too (the weight stream pushes it out of L2): one CTA asks L2 for
+            // the next layer's norm weights and biases, and the attention CTAs request their cache rows here
+            if (l + 1 < L && cta == l % n)
+                for (int i = tid * 32; i < 2 * C + QKV; i += kThreads * 32) prefetch_l2(aux + 2 * C + QKV + i);
+            Attend<KV> at;
+            const KV *kc = reinterpret_cast<const KV *>(p.k_cache + (size_t)l * p.kv_layer_bytes) + (size_t)k0 * KVd + kvh * 64;
+            const KV *vc = reinterpret_cast<const KV *>(p.v_cache + (size_t)l * p.kv_layer_bytes) + (size_t)k0 * KVd + kvh * 64;
+            if (is_att) at.load(kc, vc, KVd, warp * 16, own_new ? nk - 1 : nk, tile, lane);
+            if (l > 0) add_residual(ll + w_down, ep - 1);
+            float4 y = norm(nw);
+            if (has4) stage4(planes, pitch_c, c4, y);
+            __syncthreads();
+            run_short(wb, nq);
+            wb += uq * kUnitBytes;
+            if (nq > 0) __syncthreads();
+            if (warp < nq) {
+                const float a = column_sum_c(red + warp * G * 8) + bias;
+                if (part == 0) ll_put(ll + (fq + warp * n) * 8 + (lane >> 2), a, ep);
+            }
+
+            // -- attention: rotary embedding of q and the new k (ropeHalfRef, src/reference/qwen-ref.ts:35-64), cache append
+            if (is_att) {
+                if (warp < 3 && (warp == 0 || own_new)) {
+                    // a lane reads the pair (2i, 2i + 1), the rotation needs (i, i + 32)
+                    const float2 cs = __ldg(reinterpret_cast<const float2 *>(p.cs_table) + (size_t)pos * 32 + lane);
+                    const float2 a = ll_get2(ll + (warp == 0 ? h * 64 : warp == 1 ? C + kvh * 64 : C + KVd + kvh * 64) + 2 * lane, ep, hd);
+                    float *dst = att + warp * 64;
+                    *reinterpret_cast<float2 *>(dst + 2 * lane) = a;
+                    __syncwarp();
+                    float r0 = dst[lane], r1 = dst[lane + 32];
+                    __syncwarp();
+                    if (warp < 2) {
+                        const float t0 = r0 * cs.x - r1 * cs.y, t1 = r0 * cs.y + r1 * cs.x;
+                        r0 = t0, r1 = t1;
+                    }
+                    if (warp == 0) {
+                        r0 *= 0.125f, r1 *= 0.125f;  // 1 / sqrt(64)
+                        __half *qh = reinterpret_cast<__half *>(dst);
+                        const __half h0 = __float2half_rn(r0), h1 = __float2half_rn(r1);
+                        qh[lane] = h0, qh[lane + 32] = h1;
+                        qh[64 + lane] = __float2half_rn(r0 - __half2float(h0)), qh[96 + lane] = __float2half_rn(r1 - __half2float(h1));
+                    } else {
+                        const KV c0 = (KV)r0, c1 = (KV)r1;  // as a later step will read them
+                        if (h == kvh * hpk) {
+                            KV *cd = reinterpret_cast<KV *>((warp == 1 ? p.k_cache : p.v_cache) + (size_t)l * p.kv_layer_bytes) + (size_t)pos * KVd + kvh * 64;
+                            cd[lane] = c0, cd[lane + 32] = c1;
+                        }
+                        dst[lane] = (float)c0, dst[lane + 32] = (float)c1;
+                    }
+                }
+                __syncthreads();
+                at.run(kc, vc, KVd, nk, own_new, att, tile, ll + w_att + (h * S + sp) * kPartWords, S == 1, ep, warp, lane);
+            }
+
+            // -- o: merge the splits of every head while staging
+            if (no > 0) {
+                if (sub < wpg) load_one(wb);
+                if (has4) {
+                    const u64 *src = ll + w_att + (c4 >> 6) * S * kPartWords, *mine = src + (c4 & 63);
+                    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (S == 1) {
+                        ulonglong2 w[2];
+                        ll_get(w, mine, 2, ep, hd);
+                        const float2 f = ll_vals(w[0]), g = ll_vals(w[1]);
+                        a = make_float4(f.x, f.y, g.x, g.y);
+                    } else {
+                        // every 8 lanes hold the max and sum of all splits of their head; the values are added up over the splits,
+                        // four of them (and the maxima) in flight at a time
+                        float e = 0.f, den = 1.f;
+#pragma unroll 1
+                        for (int i0 = 0; i0 < S; i0 += 4, mine += 4 * kPartWords) {
+                            const int cnt = min(4, S - i0), ms = min(lane & 7, S - 1);
+                            ulonglong2 v0[4], v1[4], vm;
+#pragma unroll
+                            for (int j = 0; j < 4; j++) v0[j] = v1[j] = make_ulonglong2(0, 0);
+                            vm = make_ulonglong2(0, 0);
+#pragma unroll 1
+                            for (uint32_t it = 1;; it++) {
+                                if (!ll_ok(vm, ep)) vm = ll_load2(src + ms * kPartWords + 64);
+#pragma unroll
+                                for (int j = 0; j < 4; j++)
+                                    if (j < cnt) {
+                                        if (!ll_ok(v0[j], ep)) v0[j] = ll_load2(mine + j * kPartWords);
+                                        if (!ll_ok(v1[j], ep)) v1[j] = ll_load2(mine + j * kPartWords + 2);
+                                    }
+                                bool ok = ll_ok(vm, ep);
+#pragma unroll
+                                for (int j = 0; j < 4; j++) ok = ok && (j >= cnt || (ll_ok(v0[j], ep) && ll_ok(v1[j], ep)));
+                                if (ll_done(ok, it, hd)) break;
+                            }
+                            if (i0 == 0) {
+                                float2 ml = ll_vals(vm);
+                                if ((lane & 7) >= S) ml = make_float2(-INFINITY, 0.f);
+                                float M = ml.x;
+#pragma unroll
+                                for (int o = 1; o <= 4; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+                                e = ml.y > 0.f ? expf(ml.x - M) : 0.f;  // (an empty split has sum 0)
+                                den = ml.y * e;
+#pragma unroll
+                                for (int o = 1; o <= 4; o <<= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+                            }
+#pragma unroll
+                            for (int j = 0; j < 4; j++) {
+                                const float ej = __shfl_sync(0xffffffffu, e, (lane & 24) + i0 + j);
+                                if (j < cnt) {
+                                    const float2 f = ll_vals(v0[j]), g = ll_vals(v1[j]);
+                                    a.x = fmaf(f.x, ej, a.x), a.y = fmaf(f.y, ej, a.y), a.z = fmaf(g.x, ej, a.z), a.w = fmaf(g.y, ej, a.w);
+                                }
+                            }
+                        }
+                        const float inv = 1.f / den;
+                        a.x *= inv, a.y *= inv, a.z *= inv, a.w *= inv;
+                    }
+                    stage4(planes, pitch_c, c4, a);
+                }
+                __syncthreads();
+                run_short(wb, no);
+                wb += uo * kUnitBytes;
+                __syncthreads();
+                if (warp < no) {
+                    const float a = column_sum_c(red + warp * G * 8);
+                    if (part == 0) ll_put(ll + w_o + (fo + warp * n) * 8 + (lane >> 2), a, ep);
+                }
+            }
+
+            // -- gate | up, silu * up
+            if (sub < wpg) load_tiles(wb, t_first);
+            nw = load4(aux + C);
+            add_residual(ll + w_o, ep);
+            y = norm(nw);
+            if (has4) stage4(planes, pitch_c, c4, y);
+            __syncthreads();
+            run_tiles(wb, 2 * ng);
+            wb += ug * kUnitBytes;
+            if (nd == 0) {
+                next_slot();
+                if (feeder && l + 1 < L) mbar_wait(&full[slot], par, p.status);
+            }
+            __syncthreads();
+#pragma unroll 1
+            for (int i = warp; i < ng; i += kWarps) {
+                const float *r = red + i * 2 * G * 8;
+                const float gate = column_sum_c(r), up = column_sum_c(r + G * 8);
+                if (part == 0) act_put(act + (fg + i * n) * 8 + (lane >> 2), gate / (1.f + expf(-gate)) * up, ep);
+            }
+
+            // -- down
+            if (nd > 0) {
+                auto load_groups = [&](const char *w) {
+#pragma unroll
+                    for (int j = 0; j < kBurst; j++) u[j].load(w + (warp + j * kWarps) * kUnitBytes, lane);
+                };
+                load_groups(wb);
+#pragma unroll 1
+                for (int k = c4; k < I; k += kBatch * 4 * kThreads) {
+                    // (fours beyond I are those at its end once more, staged behind everything that is used)
+                    uint4 w[kBatch];
+                    const uint32_t *src[kBatch];
+#pragma unroll
+                    for (int i = 0; i < kBatch; i++) src[i] = act + min(k + i * 4 * kThreads, I - 128 + 4 * lane);
+#pragma unroll
+                    for (int i = 0; i < kBatch; i++) w[i] = act_load4(src[i]);
+#pragma unroll 1
+                    for (uint32_t it = 1;; it++) {
+                        bool ok = true;
+#pragma unroll
+                        for (int i = 0; i < kBatch; i++) ok = ok && act_ok(w[i], ep);
+                        if (ll_done(ok, it, hd)) break;
+#pragma unroll
+                        for (int i = 0; i < kBatch; i++)
+                            if (!act_ok(w[i], ep)) w[i] = act_load4(src[i]);
+                    }
+                    // a warp's 128 values are one group: its sum, all of the batch's reductions side by side
+                    float g[kBatch];
+#pragma unroll
+                    for (int i = 0; i < kBatch; i++) {
+                        const float4 f = act_vals(w[i]);
+                        stage4(planes, pitch_i, k + i * 4 * kThreads, f);
+                        g[i] = (f.x + f.y) + (f.z + f.w);
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                        for (int i = 0; i < kBatch; i++) g[i] += __shfl_xor_sync(0xffffffffu, g[i], o);
+                    if (lane == 0)
+#pragma unroll
+                        for (int i = 0; i < kBatch; i++) sums[(k >> 7) + i * kWarps] = g[i];
+                }
+                __syncthreads();
+#pragma unroll 1
+                for (int t = 0; t < nd; t++) {
+#pragma unroll 1
+                    for (int i = warp; i < GI; i += kBurst * kWarps) {
+                        if (t > 0 || i > warp) load_groups(wb + (t * GI + i - warp) * kUnitBytes);
+                        float v[kBurst];
+                        Acts xa[kBurst];
+#pragma unroll
+                        for (int j = 0; j < kBurst; j++) xa[j].load(xp_i + (i + j * kWarps) * 128);
+#pragma unroll
+                        for (int j = 0; j < kBurst; j++) {
+                            const float g = sums[i + j * kWarps];  // comes off once, in the lane of the first half
+                            v[j] = unit_half(u[j], xa[j], (lane & 1) == 0 ? g : 0.f, lane);
+                        }
+#pragma unroll
+                        for (int j = 0; j < kBurst; j++) v[j] = halves(v[j]);
+#pragma unroll
+                        for (int j = 0; j < kBurst; j++)
+                            if (part == 0 && i + j * kWarps < GI) red_i[(t * GI + i + j * kWarps) * 8] = v[j];
+                    }
+                }
+                next_slot();
+                if (feeder && l + 1 < L) mbar_wait(&full[slot], par, p.status);
+                __syncthreads();
+                if (warp < nd) {
+                    const float a = column_sum_i(red + warp * GI * 8);
+                    if (part == 0) ll_put(ll + w_down + (fdn + warp * n) * 8 + (lane >> 2), a, ep);
+                }
+            }
+            if (feeder) fill();  // every warp is past the barrier behind its last unit
+        }
+
+        // -- final norm, tied lm_head (f32 activations, fp16 rows), argmax
+        const float4 w_final = load4(p.final_norm);
+        add_residual(ll + w_down, --ep);  // the last layer's epoch is the step's
+        const float4 y = norm(w_final);
+        if (has4) *reinterpret_cast<float4 *>(xs + c4) = y;
+        __syncthreads();
+        const bool last = s + 1 == p.n_steps;
+        float best = -INFINITY;
+        int best_i = 0x7fffffff;
+        {
+            // Four rows of the slot per warp, without a branch between them; a lane holds 16-byte pieces 32 apart of every row. The
+            // four sums are added up over the lanes together: halves of the warp take two rows each, quarters one.
+            static_assert(kLmRows == 4 * kWarps, "four rows per warp");
+            float xr[4][8];
+            int at[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                at[q] = min(q * 256 + lane * 8, C - 8);
+#pragma unroll
+                for (int j = 0; j < 8; j++) xr[q][j] = q * 256 + lane * 8 < C ? xs[at[q] + j] : 0.f;
+            }
+            const int my = (lane >> 4) * 2 + ((lane >> 3) & 1);  // the row of the four whose sum ends up here
+#pragma unroll 1
+            for (int j = 0; j < lm_fills; j++) {
+                mbar_wait(&full[slot], par, p.status);
+                const __half *rows = reinterpret_cast<const __half *>(ring + slot * p.slot_bytes) + (size_t)warp * 4 * C;
+                float a[4] = {}, b[4] = {};
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    uint4 w[4];
+#pragma unroll
+                    for (int r = 0; r < 4; r++) w[r] = *reinterpret_cast<const uint4 *>(rows + r * C + at[q]);
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        const __half2 *h2 = reinterpret_cast<const __half2 *>(&w[r]);
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const float2 wf = __half22float2(h2[k]);
+                            a[r] = fmaf(wf.x, xr[q][2 * k], a[r]), b[r] = fmaf(wf.y, xr[q][2 * k + 1], b[r]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < 4; r++) a[r] += b[r];
+                const bool up = lane & 16, up2 = lane & 8;
+                const float k0 = (up ? a[2] : a[0]) + __shfl_xor_sync(0xffffffffu, up ? a[0] : a[2], 16);
+                const float k1 = (up ? a[3] : a[1]) + __shfl_xor_sync(0xffffffffu, up ? a[1] : a[3], 16);
+                float v = (up2 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, up2 ? k0 : k1, 8);
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                const int row = row0 + j * kLmRows + warp * 4 + my;
+                const bool in = row < row1;
+                if (in && (v > best || (v == best && row < best_i))) best = v, best_i = row;
+                if (last && in && (lane & 7) == 0) p.logits[row] = v;
+                __syncthreads();
+                if (feeder) fill();
+                next_slot();
+            }
+            // the warp's best row in every lane
+#pragma unroll
+            for (int o = 8; o <= 16; o <<= 1) {
+                const float v = __shfl_xor_sync(0xffffffffu, best, o);
+                const int i = __shfl_xor_sync(0xffffffffu, best_i, o);
+                if (v > best || (v == best && i < best_i)) best = v, best_i = i;
+            }
+        }
+        if (feeder && !last) mbar_wait(&full[slot], par, p.status);  // the next step's first block
+        if (last && p.history == nullptr) break;  // only the logits were asked for
+        // every CTA's best row, then every CTA picks the best of those (first strict maximum: the lowest index wins a tie)
+        if (lane == 0) ssq[warp] = best, widx[warp] = best_i;
+        __threadfence();  // the cache rows of this step, before the words that let other CTAs go on to the next
+        __syncthreads();
+        u64 *cd = cand + (size_t)(s & 1) * 2 * n;  // two sets: a CTA may be a step ahead of one that still reads its candidates
+        auto better = [&](float v, int i) {
+            if (v > best || (v == best && i < best_i)) best = v, best_i = i;
+        };
+        if (warp == 0) {
+            best = lane < kWarps ? ssq[lane] : -INFINITY, best_i = lane < kWarps ? widx[lane] : 0x7fffffff;
+#pragma unroll
+            for (int o = kWarps / 2; o > 0; o >>= 1) better(__shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, best_i, o));
+            if (lane == 0) ll_put(cd + 2 * cta, best, ep), ll_put(cd + 2 * cta + 1, __int_as_float(best_i), ep);
+        }
+        __syncthreads();
+        if (last && cta != 0) break;
+        best = -INFINITY, best_i = 0x7fffffff;
+        if (warp * 32 < n) {
+            const float2 c = ll_get2(cd + 2 * min(tid, n - 1), ep, hd);
+            best = c.x, best_i = __float_as_int(c.y);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) better(__shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, best_i, o));
+        if (lane == 0) ssq[warp] = best, widx[warp] = best_i;
+        __syncthreads();
+        if (tid == 0) {
+            for (int i = 1; i < kWarps; i++) better(ssq[i], widx[i]);
+            const uint32_t t = best_i == 0x7fffffff ? 0u : (uint32_t)best_i;  // all-NaN logits: JS returns index 0
+            hd->token = t;
+            if (cta == 0) p.history[s] = t;
+        }
+        __syncthreads();
+        token = hd->token;
+        __threadfence();
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------- set-up
+struct Source {
+    const uint32_t *qw[4], *qz[4];  // qkv, o, gate_up, down; qz nullable
+    const __half *sc[4];
+    const float *in_norm, *post_norm, *bias;
+};
+
+// One warp per unit (8 columns x 128 rows): checkpoint layout -> the CTA's block.
+__global__ void __launch_bounds__(256) lay_out_kernel(const Source *__restrict__ src, char *__restrict__ blobs, int C, int I, int KV, int n,
+                                                      int blob_stride)
+{
+    const int QKV = C + 2 * KV, G = C / 128, GI = I / 128, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int uq = QKV / 8 * G, uo = C / 8 * G, ug = I / 8 * 2 * G, ud = C / 8 * GI;
+    int u = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (u >= uq + uo + ug + ud) return;
+    const Source &s = src[blockIdx.y];
+    int proj, N, groups, tile, group, col0, at;  // at: unit index inside the CTA's block
+    Deal d;
+    const Deal dq = deal_qkv(C, KV), dow = deal_o(C, n), dg = deal_gu(I), dd = deal_down(C, n);
+    if (u < uq) proj = 0, N = QKV, groups = G, d = dq;
+    else if ((u -= uq) < uo) proj = 1, N = C, groups = G, d = dow;
+    else if ((u -= uo) < ug) proj = 2, N = 2 * I, groups = G, d = dg;
+    else u -= ug, proj = 3, N = C, groups = GI, d = dd;
+    group = u % groups, tile = u / groups;
+    int half = 0;
+    if (proj == 2) half = tile & 1, tile >>= 1;
+    col0 = half * I + tile * 8;
+    const int cta = (tile % n + d.off) % n, local = tile / n;
+    at = (proj == 2 ? local * 2 + half : local) * groups + group;
+    if (proj > 0) at += deal_count(dq, cta, n) * G;
+    if (proj > 1) at += deal_count(dow, cta, n) * G;
+    if (proj > 2) at += deal_count(dg, cta, n) * 2 * G;
+    char *out = blobs + ((size_t)blockIdx.y * n + cta) * blob_stride + (size_t)at * kUnitBytes;
+    // a word's nibbles in the order of stage4's planes: masks 0x000f000f, 0x00f000f0 (shifted by 0 and 8) pick the positions
+    // 0 1 | 2 3 and 4 5 | 6 7
+    auto order = [](uint32_t q) {
+        constexpr int kNibble[8] = {0, 2, 4, 6, 1, 3, 5, 7};  // position held by nibble i
+        uint32_t r = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) r |= ((q >> (4 * kNibble[i])) & 15u) << (4 * i);
+        return r;
+    };
+    uint4 w;
+    const uint32_t *q = s.qw[proj] + (size_t)(group * 16 + t) * N + col0 + g;
+    w.x = order(q[0]), w.y = order(q[(size_t)4 * N]), w.z = order(q[(size_t)8 * N]), w.w = order(q[(size_t)12 * N]);
+    *reinterpret_cast<uint4 *>(out + lane * 16) = w;
+    if (lane < 8) {
+        const int c = col0 + lane;
+        const uint32_t z = s.qz[proj] ? ((s.qz[proj][(size_t)group * ((N + 7) / 8) + (c >> 3)] >> ((c & 7) * 4)) & 15u) + 1u : 8u;
+        const float sc = __half2float(s.sc[proj][(size_t)group * N + c]);
+        *reinterpret_cast<float2 *>(out + 512 + lane * 8) = make_float2(sc * 16777216.f, sc * (float)z);
+    }
+}
+
+__global__ void __launch_bounds__(256) lay_out_aux_kernel(const Source *__restrict__ src, float *__restrict__ aux, int C, int QKV)
+{
+    const Source &s = src[blockIdx.x];
+    float *a = aux + (size_t)blockIdx.x * (2 * C + QKV);
+    for (int i = threadIdx.x; i < C; i += blockDim.x) a[i] = s.in_norm[i], a[C + i] = s.post_norm[i];
+    for (int i = threadIdx.x; i < QKV; i += blockDim.x) a[2 * C + i] = s.bias[i];
+}
+
+}  // namespace fd
+
+// Which models take this kernel: the shapes it is written for (head size 64, fused int4 projections of group 128, a hidden size
+// of four values per thread), and a layer small enough that two of a CTA's blocks fit its shared memory, so that the ring can run
+// ahead of the hand-overs (0.5B: 61 KB per CTA and layer, three slots). Larger models are bound by their weights, not by the
+// hand-overs, and stay on one kernel per projection.
+static bool fused_shape(const wb_qwen *m, int n, int *blob, int *slot, int *slots, int *smem)
+{
+    using namespace fd;
+    const int C = m->C, I = m->I, KV = m->KV;
+    if (m->D != 64 || C % 128 || C > kMaxC || I % 128 || I > kMaxI || m->H > n || n > kThreads || m->V < n) return false;
+    wb_context *ctx = m->ctx;
+    for (const wbq::LayerW &L : m->layers) {
+        if (L.qkv < 0 || L.gate_up < 0) return false;
+        for (int h : {L.qkv, L.o, L.gate_up, L.down}) {
+            const Weight &w = ctx->weights[h];
+            if (w.kind != WeightKind::Gptq || w.group != 128) return false;
+        }
+    }
+    int units = 0;
+    for (int c = 0; c < n; c++)
+        units = std::max(units, deal_count(deal_qkv(C, KV), c, n) * (C / 128) + deal_count(deal_o(C, n), c, n) * (C / 128) +
+                                    deal_count(deal_gu(I), c, n) * 2 * (C / 128) + deal_count(deal_down(C, n), c, n) * (I / 128));
+    if (deal_count(deal_qkv(C, KV), 0, n) > kWarps || (C / 8 + n - 1) / n > kWarps) return false;  // one warp per tile of a sum
+    *blob = (units * kUnitBytes + 127) / 128 * 128;
+    *slot = std::max(*blob, kLmRows * C * 2);
+    for (*slots = kSlotsMax; *slots >= 2; --*slots) {
+        *smem = smem_layout(*slots, *slot, C, I, max_units(C, I, KV, n)).total;
+        if (*smem <= 227 * 1024) return true;
+    }
+    return false;
+}
+
+// One CTA per SM, as long as every CTA has a tile of gate|up: the hand-over words of a layer are written over by the next one, and
+// it is through that projection that every CTA is known to have read what it needs (see the comment at the top).
+static int fused_ctas(const wb_qwen *m) { return std::min(m->ctx->sm_count, m->I / 8); }
+
+static int fused_setup(wb_qwen *m)
+{
+    using namespace fd;
+    m->fused_state = -1;
+    wb_context *ctx = m->ctx;
+    const int n = fused_ctas(m), C = m->C, I = m->I, KV = m->KV, QKV = C + 2 * KV, L = m->cfg.n_layer;
+    int blob, slot, slots, smem;
+    if (!fused_shape(m, n, &blob, &slot, &slots, &smem)) return WB_OK;
+    const size_t ll_layer = (size_t)QKV + 2 * C + I / 2 + (size_t)m->H * kSplitMax * kPartWords;
+    const size_t blob_bytes = align_up((size_t)L * n * blob), aux_bytes = align_up((size_t)L * (2 * C + QKV) * 4);
+    const size_t ll_bytes = align_up((ll_layer + 4 * (size_t)n) * 8), src_bytes = align_up(L * sizeof(Source));
+    char *mem = nullptr;
+    if (cudaMalloc(&mem, blob_bytes + aux_bytes + ll_bytes + src_bytes) != cudaSuccess) {
+        cudaGetLastError();  // no room for the second layout of the weights: the model keeps one kernel per projection
+        return WB_OK;
+    }
+    m->fused_mem = mem;
+    Params p{};
+    p.blobs = mem, p.aux = (const float *)(mem + blob_bytes), p.ll = (u64 *)(mem + blob_bytes + aux_bytes);
+    const char *wb = ctx->arena[WB_ARENA_WEIGHTS].base;
+    auto f32w = [&](int h) { return (const float *)(wb + ctx->weights[h].off_main); };
+    std::vector<Source> src(L);
+    for (int i = 0; i < L; i++) {
+        const wbq::LayerW &W = m->layers[i];
+        const int hs[4] = {W.qkv, W.o, W.gate_up, W.down};
+        for (int j = 0; j < 4; j++) {
+            const Weight &w = ctx->weights[hs[j]];
+            src[i].qw[j] = (const uint32_t *)(wb + w.off_main);
+            src[i].sc[j] = (const __half *)(wb + w.off_scales);
+            src[i].qz[j] = w.has_zeros ? (const uint32_t *)(wb + w.off_zeros) : nullptr;
+        }
+        src[i].in_norm = f32w(W.in_norm), src[i].post_norm = f32w(W.post_norm), src[i].bias = f32w(W.qkvb);
+    }
+    Source *d_src = (Source *)(mem + blob_bytes + aux_bytes + ll_bytes);
+    WB_CUDA(cudaMemcpyAsync(d_src, src.data(), L * sizeof(Source), cudaMemcpyHostToDevice, ctx->stream));
+    WB_CUDA(cudaMemsetAsync(p.ll, 0, ll_bytes, ctx->stream));
+    const int units = (QKV / 8 + C / 8 + I / 4) * (C / 128) + C / 8 * (I / 128);
+    lay_out_kernel<<<dim3((units + 7) / 8, L), 256, 0, ctx->stream>>>(d_src, mem, C, I, KV, n, blob);
+    WB_CUDA(cudaGetLastError());
+    lay_out_aux_kernel<<<L, 256, 0, ctx->stream>>>(d_src, (float *)p.aux, C, QKV);
+    WB_CUDA(cudaGetLastError());
+    ctx->launches += 2;
+    p.final_norm = f32w(m->final_norm), p.embed = (const __half *)f32w(m->embed), p.cs_table = m->cs_table;
+    p.k_cache = m->k_cache, p.v_cache = m->v_cache, p.status = ctx->status_word;
+    const bool kv16 = m->cfg.kv_dtype == WB_F16;
+    p.kv_layer_bytes = (size_t)m->cfg.max_t * KV * (kv16 ? 2 : 4), p.ll_layer = ll_layer;
+    p.n_cta = n, p.n_layer = L, p.C = C, p.H = m->H, p.KVH = m->KVH, p.I = I, p.V = m->V, p.KV = KV;
+    p.sm = smem_layout(slots, slot, C, I, max_units(C, I, KV, n));
+    p.slots = slots, p.slot_bytes = slot, p.blob_stride = blob, p.eps = m->cfg.rms_eps;
+    WB_CUDA(cudaFuncSetAttribute(kv16 ? (const void *)decode_fused_kernel<__half> : (const void *)decode_fused_kernel<float>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    static_assert(sizeof(Params) <= sizeof(m->fused_params), "room for the parameters in the model object");
+    memcpy(m->fused_params, &p, sizeof p);
+    m->fused_smem = smem, m->fused_epoch = 1, m->fused_state = 1;
+    return WB_OK;
+}
+
+int decode_fused_run(wb_qwen *m, uint32_t token, int64_t n_steps, float *logits, uint32_t *history, bool *ran)
+{
+    using namespace fd;
+    *ran = false;
+    if (m->ctx->force_kernel != 0) return WB_OK;  // a forced kernel means one kernel per projection
+    if (m->fused_state == 0) WB_CHECK(fused_setup(m));
+    if (m->fused_state < 0) return WB_OK;
+    wb_context *ctx = m->ctx;
+    Params p;
+    memcpy(&p, m->fused_params, sizeof p);
+    const uint64_t epochs = (uint64_t)n_steps * p.n_layer;
+    if (m->fused_epoch + epochs > 0xfffffff0u) {  // epochs do not wrap: start again on zeroed words
+        WB_CUDA(cudaMemsetAsync(p.ll, 0, (p.ll_layer + 4 * (size_t)p.n_cta) * 8, ctx->stream));
+        m->fused_epoch = 1;
+    }
+    p.epoch = m->fused_epoch, p.first_token = token, p.pos0 = (int)m->cache_len, p.n_steps = (int)n_steps;
+    p.logits = logits, p.history = history;
+    void *args[] = {&p};
+    const void *kern = m->cfg.kv_dtype == WB_F16 ? (const void *)decode_fused_kernel<__half> : (const void *)decode_fused_kernel<float>;
+    WB_CUDA(cudaLaunchCooperativeKernel(kern, dim3(p.n_cta), dim3(kThreads), args, (size_t)m->fused_smem, ctx->stream));
+    m->fused_epoch += (uint32_t)epochs;
+    ctx->launches++;
+    *ran = true;
+    return WB_OK;
+}
+
+void decode_fused_release(wb_qwen *m)
+{
+    if (m->fused_mem) cudaFree(m->fused_mem);
+    m->fused_mem = nullptr, m->fused_state = 0;
+}
+
+}  // namespace wb

@@ -44,5 +44,18 @@ struct wb_qwen {
     cudaStream_t graph_stream = nullptr;
     int graph_exact = -1;
     uint64_t graph_launches = 0;    // kernels in one captured decode step
+    // the persistent decode kernel (decode_fused.cu): its layout of the weights and its hand-over words, made on first use
+    int fused_state = 0;            // 0: not looked at yet, 1: ready, -1: not for this model
+    char *fused_mem = nullptr;
+    int fused_smem = 0;
+    uint32_t fused_epoch = 1;
+    alignas(8) unsigned char fused_params[256];
     uint64_t carve_mark = 0, carve_top = 0;  // weight-arena `used` before and after the model's own allocations
 };
+
+namespace wb {
+// `n_steps` whole decode steps from `token` in one launch; logits of the last step, and (with `history`, pinned host memory) the
+// greedy token of every step. *ran = false: not a model (or not the moment) for that kernel, nothing was enqueued.
+int decode_fused_run(wb_qwen *m, uint32_t token, int64_t n_steps, float *logits, uint32_t *history, bool *ran);
+void decode_fused_release(wb_qwen *m);
+}  // namespace wb

@@ -342,6 +342,7 @@ int wb_qwen_destroy(wb_qwen *m)
     cudaSetDevice(m->ctx->device);
     cudaStreamSynchronize(m->ctx->stream);
     drop_graph(m);
+    decode_fused_release(m);
     // the model's carve is handed back when it still is the top of the weight arena
     ArenaState &wa = m->ctx->arena[WB_ARENA_WEIGHTS];
     if (wa.used == m->carve_top) wa.used = m->carve_mark;
@@ -420,7 +421,16 @@ int wb_qwen_decode_step(wb_qwen *m, uint32_t token, uint64_t *logits_offset)
     if (m->cache_len == 0) return fail(WB_ERR_BAD_ARG, "decodeStep 前请先调用 prefill()");
     if (m->cache_len + 1 > m->cfg.max_t)
         return fail(WB_ERR_BAD_ARG, "上下文长度 %lld 超过 blockSize=%d", (long long)(m->cache_len + 1), m->cfg.max_t);
-    return run_eager(m, &token, 1, 1, 1, m->cache_len, true, true, logits_offset);
+    WB_CHECK(check_tokens(m, &token, 1));
+    WB_CHECK(wb_arena_reset(m->ctx, WB_ARENA_ACT));
+    float *logits = nullptr;
+    WB_CHECK(carve_t(m->ctx, WB_ARENA_ACT, (uint64_t)m->V, &logits));
+    bool ran = false;
+    WB_CHECK(decode_fused_run(m, token, 1, logits, nullptr, &ran));
+    if (!ran) return run_eager(m, &token, 1, 1, 1, m->cache_len, true, true, logits_offset);
+    m->cache_len++;
+    if (logits_offset) *logits_offset = (uint64_t)((char *)logits - m->ctx->arena[WB_ARENA_ACT].base);
+    return WB_OK;
 }
 
 __global__ void set_decode_state_kernel(int *cache_len, int *step, uint32_t *tokens, int len, uint32_t first_token)
@@ -446,6 +456,23 @@ int wb_qwen_decode_greedy(wb_qwen *m, uint32_t first_token, int64_t n_steps, uin
     if (m->cache_len + n_steps > m->cfg.max_t)
         return fail(WB_ERR_BAD_ARG, "上下文长度 %lld 超过 blockSize=%d", (long long)(m->cache_len + n_steps), m->cfg.max_t);
     WB_CHECK(check_tokens(m, &first_token, 1));
+    // One persistent kernel per up to kFusedSteps tokens where the model suits it (about 13 ms: other streams get their turn).
+    constexpr int64_t kFusedSteps = 64;
+    if (n_steps <= (int64_t)m->host_pin_cap) {
+        bool ran = true;
+        for (int64_t s = 0; s < n_steps && ran; s += kFusedSteps) {
+            const int64_t cur = std::min(kFusedSteps, n_steps - s);
+            const uint32_t first = s == 0 ? first_token : m->host_pin[s - 1];
+            WB_CHECK(decode_fused_run(m, first, cur, m->dec.logits, m->host_pin + s, &ran));
+            if (!ran) break;
+            m->cache_len += cur;
+            WB_CHECK(wb_synchronize(ctx));
+        }
+        if (ran) {
+            memcpy(out_tokens, m->host_pin, (size_t)n_steps * 4);
+            return WB_OK;
+        }
+    }
     // the decode state (cache length, step counter, first token) goes to the device as the arguments of one tiny kernel:
     // no staging of pageable host memory on the per-token path
     auto set_state = [&]() -> int {
