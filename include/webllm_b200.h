@@ -284,6 +284,12 @@ WB_API int wb_qwen_decode_step(wb_qwen *model, uint32_t token, uint64_t *logits_
 WB_API int wb_qwen_decode_greedy(wb_qwen *model, uint32_t first_token, int64_t n_steps, uint32_t *out_tokens);
 /* Logits of the last step run by wb_qwen_decode_greedy, [V] f32, copied to the host. */
 WB_API int wb_qwen_last_logits(wb_qwen *model, float *out);
+/* sampleToken (src/infer/sampler.ts:38-78) on a logits row in the activation arena, temperature > 0 and 1 <= top_k <= 1024
+ * (any top_k where the vocabulary has no more than 1024 entries; top_p >= 1 keeps all of them): weights, selection and
+ * order as there, `u` in [0, 1) in place of its random number. *token = -1: the row holds a NaN or an infinite maximum, or
+ * too many equal weights; sample it on the host. Blocks until the token is known. */
+WB_API int wb_sample_token(wb_context *ctx, uint64_t logits_offset, int64_t vocab, float temperature, int64_t top_k,
+                           double top_p, double u, int32_t *token);
 
 /* ---- allocation-free GEMV. No counterpart in the reference (its split-K scratch comes from the arena,
  *      src/model/qwen.ts:584); added for hosts that may not allocate device memory where they run the

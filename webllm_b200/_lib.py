@@ -116,6 +116,7 @@ SIGNATURES = {
     "wb_qwen_decode_step": [_vp, C.c_uint32, C.POINTER(_u64)],
     "wb_qwen_decode_greedy": [_vp, C.c_uint32, _i64, _vp],
     "wb_qwen_last_logits": [_vp, _vp],
+    "wb_sample_token": [_vp, _u64, _i64, C.c_float, _i64, C.c_double, C.c_double, C.POINTER(C.c_int32)],
     "wb_gptq_gemv_static": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i32, _i32, _i32, _vp],
 }
 _RESTYPES = {"wb_last_error": C.c_char_p}

@@ -106,7 +106,7 @@ struct wb_context {
     std::unordered_map<std::string, int> by_name;
     char *workspace = nullptr;       // kWorkspaceBytes of scratch
     unsigned *counters = nullptr;    // kMaxCounters arrival counters, zero between calls
-    int *status_word = nullptr;      // device-side error flag for bounded waits (mapped pinned host memory)
+    int *status_word = nullptr;      // device-side error flag for bounded waits, and a result word (mapped pinned host memory)
     int *status_host = nullptr;
     uint64_t launches = 0;
     int force_kernel = 0, force_split = 0;

@@ -155,8 +155,8 @@ int wb_context_create(int device, wb_context **out)
         WB_CUDA(cudaMalloc(&ctx->workspace, kWorkspaceBytes));
         WB_CUDA(cudaMalloc(&ctx->counters, kMaxCounters * sizeof(unsigned)));
         WB_CUDA(cudaMemset(ctx->counters, 0, kMaxCounters * sizeof(unsigned)));
-        WB_CUDA(cudaHostAlloc(&ctx->status_host, sizeof(int), cudaHostAllocMapped));
-        *ctx->status_host = 0;
+        WB_CUDA(cudaHostAlloc(&ctx->status_host, 2 * sizeof(int), cudaHostAllocMapped));
+        ctx->status_host[0] = ctx->status_host[1] = 0;
         WB_CUDA(cudaHostGetDevicePointer(&ctx->status_word, ctx->status_host, 0));
         cudaDriverEntryPointQueryResult qres;
         WB_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ctx->tmap_encode, cudaEnableDefault, &qres));

@@ -4,7 +4,7 @@ from __future__ import annotations
 import math
 import random
 import time
-from dataclasses import dataclass, field
+from dataclasses import dataclass, field, replace
 
 import numpy as np
 
@@ -38,18 +38,58 @@ def sample_token(logits: np.ndarray, offset: int, vocab_size: int, options: Samp
         return best
     scaled = (row / np.float32(options.temperature)).astype(np.float32)
     weights = np.exp((scaled - scaled.max()).astype(np.float64)).astype(np.float32)
-    total = float(weights.astype(np.float64).sum())
-    order = sorted(range(vocab_size), key=lambda i: -float(weights[i]))  # stable, like Array.prototype.sort
     limit = min(vocab_size, max(1, int(math.floor(options.top_k)))) if options.top_k > 0 else vocab_size
-    kept = order[:limit]
+    if np.isnan(weights).any():
+        return _walk(sorted(range(vocab_size), key=lambda i: -float(weights[i]))[:limit], weights, options)
+    if limit <= 4096:
+        return _walk(_largest(weights, limit).tolist(), weights, options)
+    # the whole vocabulary (or nearly): its largest weights usually decide; a prefix of the order that is long enough gives the
+    # same answer as all of it
+    w64 = weights.astype(np.float64)
+    total, keeps_all = float(w64.sum()), not options.top_p < 1
+    u = (options.rng or random.random)()
+    size = 4096
+    while True:
+        size = min(size, limit)
+        order = _largest(weights, size)
+        w = w64[order]
+        if keeps_all:
+            cut = limit if size == limit else 0
+            kept_sum = math.fsum(w64) if limit == vocab_size else math.fsum(w64[_largest(weights, limit)])
+        else:
+            over = np.flatnonzero(np.cumsum(w / total) >= options.top_p)
+            cut = int(over[0]) + 1 if over.size else (limit if size == limit else 0)
+            kept_sum = math.fsum(w[:cut])
+        if cut or keeps_all:
+            reach = np.flatnonzero(np.cumsum(w[:cut or size]) >= u * kept_sum)
+            if reach.size:
+                return int(order[reach[0]])
+            if cut:
+                return int(order[min(cut, size) - 1])
+        size *= 8
+
+
+def _largest(weights: np.ndarray, k: int) -> np.ndarray:
+    """Indices of the k largest weights, by descending weight and then ascending index (the first k of a stable sort)."""
+    if k < weights.size:
+        least = np.partition(weights, weights.size - k)[weights.size - k]
+        above = np.flatnonzero(weights > least)
+        idx = np.sort(np.concatenate([above, np.flatnonzero(weights == least)[:k - above.size]]))
+    else:
+        idx = np.arange(weights.size)
+    return idx[np.argsort(-weights[idx], kind="stable")]
+
+
+def _walk(kept: list, weights: np.ndarray, options: SamplerOptions) -> int:
+    """The reference's loops over the sorted candidates: the top-p cut, then the draw."""
     if options.top_p < 1:
-        cum, cut = 0.0, kept
+        total = float(weights.astype(np.float64).sum())
+        cum = 0.0
         for i, idx in enumerate(kept):
             cum += float(weights[idx]) / total
             if cum >= options.top_p:
-                cut = kept[:i + 1]
+                kept = kept[:i + 1]
                 break
-        kept = cut
     kept_sum = sum(float(weights[i]) for i in kept)
     r = (options.rng or random.random)() * kept_sum
     acc = 0.0
@@ -75,7 +115,7 @@ def generate_qwen(model: QwenGpt, config, prompt: list, max_new_tokens: int, opt
 
     Greedy decoding without stop tokens runs entirely on the device (``decode_greedy``: argmax and token
     feedback inside a replayed CUDA graph) unless ``on_device=False``; every other option takes the
-    reference's loop: read the logits row back, sample on the host, feed the token."""
+    reference's loop with the draw on the device (a top-k of up to 1024) or, from the row read back, on the host."""
     options = options or SamplerOptions()
     if len(prompt) == 0:
         raise ValueError("generateQwen: prompt 不能为空")
@@ -89,14 +129,24 @@ def generate_qwen(model: QwenGpt, config, prompt: list, max_new_tokens: int, opt
     model.reset_cache()
 
     t0 = time.perf_counter()
-    logits = model.prefill(np.asarray(prompt, np.uint32), last_only=True)
-    row = model.read_tensor_slice(logits, 0, vocab)
+    greedy = not (options.temperature > 0)
+    k = math.floor(options.top_k) if not greedy and options.top_k > 0 else 0
+
+    def sample(logits) -> int:
+        # a short list of candidates is drawn from on the device: the row stays where it is
+        if 1 <= k <= 1024:
+            u = (options.rng or random.random)()
+            token = model.sample(logits, options.temperature, k, options.top_p, u)
+            if token is not None:
+                return token
+            return sample_token(model.read_tensor_slice(logits, 0, vocab), 0, vocab, replace(options, rng=lambda: u))
+        return sample_token(model.read_tensor_slice(logits, 0, vocab), 0, vocab, options)
+
+    nxt = sample(model.prefill(np.asarray(prompt, np.uint32), last_only=True))
     prefill_ms = (time.perf_counter() - t0) * 1e3
 
     t1 = time.perf_counter()
     generated = 0
-    nxt = sample_token(row, 0, vocab, options)
-    greedy = not (options.temperature > 0)
     if on_device is None:
         on_device = greedy and not stop
     if on_device and greedy and not stop and max_new_tokens > 1 and nxt not in stop:
@@ -111,8 +161,6 @@ def generate_qwen(model: QwenGpt, config, prompt: list, max_new_tokens: int, opt
             generated += 1
             if generated >= max_new_tokens:
                 break
-            logits = model.decode_step(nxt)
-            row = model.read_tensor_slice(logits, 0, vocab)
-            nxt = sample_token(row, 0, vocab, options)
+            nxt = sample(model.decode_step(nxt))
     seconds = max(1e-6, time.perf_counter() - t1)
     return QwenGenerateResult(context, len(prompt), generated, generated / seconds, prefill_ms)

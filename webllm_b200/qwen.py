@@ -180,6 +180,15 @@ class QwenGpt:
         L.check(self._lib.wb_qwen_decode_greedy(self._ensure(), int(first_token), n_steps, out.ctypes.data_as(C.c_void_p)))
         return out
 
+    def sample(self, logits: Tensor, temperature: float, top_k: int, top_p: float, u: float) -> int | None:
+        """``sampleToken`` on the last row of ``logits`` where it lies (``wb_sample_token``); None when the row has to be
+        sampled on the host."""
+        tok = C.c_int32()
+        V = self.config.vocab_size
+        L.check(self._lib.wb_sample_token(self.gpu.ctx, logits.offset + (logits.length - V) * 4, V, temperature, top_k, top_p, u,
+                                          C.byref(tok)))
+        return tok.value if tok.value >= 0 else None
+
     def last_logits(self) -> np.ndarray:
         out = np.empty(self.config.vocab_size, np.float32)
         L.check(self._lib.wb_qwen_last_logits(self._ensure(), out.ctypes.data_as(C.c_void_p)))
