@@ -125,6 +125,14 @@ inline char *arena_ptr(wb_context *ctx, int arena, uint64_t off) { return ctx->a
 int check_range(wb_context *ctx, int arena, uint64_t off, uint64_t bytes, const char *what);
 int get_weight(wb_context *ctx, wb_handle h, Weight **out);
 
+// transfer.cu: stream-ordered copies between the device and pageable (or pinned) host memory. To the host: the bytes are
+// there once the stream is synchronised (from 2 MB of pageable memory on: when the call returns). To the device: `host` may still be
+// read until the stream is synchronised.
+int copy_to_host(wb_context *ctx, void *host, const void *dev, size_t bytes);
+int copy_to_device(wb_context *ctx, void *dev, const void *host, size_t bytes);
+void transfer_retain();   // one per context
+void transfer_release();
+
 // kernels' host entry points (one per .cu file)
 int launch_dequant(wb_context *ctx, const Weight &w, void *out, bool f16);
 int launch_f32_to_f16_ref(wb_context *ctx, const float *in, __half *out, int64_t n);

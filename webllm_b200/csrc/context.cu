@@ -147,6 +147,7 @@ int wb_context_create(int device, wb_context **out)
         return fail(WB_ERR_UNSUPPORTED, "device %d is sm_%d%d; this library is built for sm_100a only", device,
                     prop.major, prop.minor);
     wb_context *ctx = new wb_context();
+    transfer_retain();
     ctx->device = device;
     ctx->sm_count = prop.multiProcessorCount;
     const int rc = [&]() -> int {
@@ -184,6 +185,7 @@ int wb_context_destroy(wb_context *ctx)
     if (ctx->counters) cudaFree(ctx->counters);
     if (ctx->status_host) cudaFreeHost(ctx->status_host);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
+    transfer_release();
     delete ctx;
     return WB_OK;
 }
@@ -304,7 +306,7 @@ int wb_upload(wb_context *ctx, int arena, uint64_t offset, const void *host, uin
     WB_CHECK(check_range(ctx, arena, offset, bytes, "wb_upload"));
     if (bytes == 0) return WB_OK;
     if (!host) return fail(WB_ERR_BAD_ARG, "wb_upload: host pointer is NULL");
-    WB_CUDA(cudaMemcpyAsync(arena_ptr(ctx, arena, offset), host, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    WB_CHECK(copy_to_device(ctx, arena_ptr(ctx, arena, offset), host, bytes));
     // The host buffer is borrowed for the call only: pageable copies are already staged when
     // cudaMemcpyAsync returns; pinned ones are not, so wait.
     WB_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -318,7 +320,7 @@ int wb_download(wb_context *ctx, int arena, uint64_t offset, void *host, uint64_
     WB_CHECK(check_range(ctx, arena, offset, bytes, "wb_download"));
     if (bytes == 0) return WB_OK;
     if (!host) return fail(WB_ERR_BAD_ARG, "wb_download: host pointer is NULL");
-    WB_CUDA(cudaMemcpyAsync(host, arena_ptr(ctx, arena, offset), bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    WB_CHECK(copy_to_host(ctx, host, arena_ptr(ctx, arena, offset), bytes));
     return wb_synchronize(ctx);
 }
 
@@ -382,16 +384,17 @@ static int gptq_register_impl(wb_context *ctx, const char *name, const void *qwe
         WB_CHECK(arena_alloc(ctx, WB_ARENA_WEIGHTS, sc_bytes, &w.off_scales));
         if (w.has_zeros) WB_CHECK(arena_alloc(ctx, WB_ARENA_WEIGHTS, qz_bytes, &w.off_zeros));
         char *base = ctx->arena[WB_ARENA_WEIGHTS].base;
-        WB_CUDA(cudaMemcpy2DAsync(base + w.off_main, (size_t)col_count * 4, (const char *)qweight + col_begin * 4,
-                                  (size_t)outF * 4, (size_t)col_count * 4, (size_t)pack_rows, cudaMemcpyHostToDevice,
-                                  ctx->stream));
-        WB_CUDA(cudaMemcpy2DAsync(base + w.off_scales, (size_t)col_count * 2, (const char *)scales + col_begin * 2,
-                                  (size_t)outF * 2, (size_t)col_count * 2, (size_t)groups, cudaMemcpyHostToDevice,
-                                  ctx->stream));
-        if (w.has_zeros)
-            WB_CUDA(cudaMemcpy2DAsync(base + w.off_zeros, (size_t)w.zcols * 4, (const char *)qzeros + col_begin / 8 * 4,
-                                      (size_t)pack_cols * 4, (size_t)w.zcols * 4, (size_t)groups, cudaMemcpyHostToDevice,
-                                      ctx->stream));
+        // rows of `width` elements out of rows of `pitch`
+        auto put = [&](uint64_t off, const void *src, int64_t esz, int64_t first, int64_t width, int64_t pitch, int64_t rows) -> int {
+            const char *from = (const char *)src + first * esz;
+            if (!sliced) return copy_to_device(ctx, base + off, from, (size_t)(rows * width * esz));
+            WB_CUDA(cudaMemcpy2DAsync(base + off, (size_t)(width * esz), from, (size_t)(pitch * esz), (size_t)(width * esz), (size_t)rows,
+                                      cudaMemcpyHostToDevice, ctx->stream));
+            return WB_OK;
+        };
+        WB_CHECK(put(w.off_main, qweight, 4, col_begin, col_count, outF, pack_rows));
+        WB_CHECK(put(w.off_scales, scales, 2, col_begin, col_count, outF, groups));
+        if (w.has_zeros) WB_CHECK(put(w.off_zeros, qzeros, 4, col_begin / 8, w.zcols, pack_cols, groups));
         WB_CUDA(cudaStreamSynchronize(ctx->stream));
         return WB_OK;
     }();
@@ -459,7 +462,7 @@ int wb_f16_write_chunk(wb_context *ctx, wb_handle h, int64_t elem_offset, const 
     __half *dst = (__half *)(ctx->arena[WB_ARENA_WEIGHTS].base + w->off_main) + elem_offset;
     for (int64_t done = 0; done < n; done += piece) {
         int64_t cur = n - done < piece ? n - done : piece;
-        WB_CUDA(cudaMemcpyAsync(ctx->workspace, data + done, (size_t)cur * 4, cudaMemcpyHostToDevice, ctx->stream));
+        WB_CHECK(copy_to_device(ctx, ctx->workspace, data + done, (size_t)cur * 4));
         WB_CHECK(launch_f32_to_f16_ref(ctx, (const float *)ctx->workspace, dst + done, cur));
         WB_CUDA(cudaStreamSynchronize(ctx->stream));
     }
@@ -475,7 +478,7 @@ int wb_f16_write_bits(wb_context *ctx, wb_handle h, int64_t elem_offset, const u
     if (n == 0) return WB_OK;
     if (!bits) return fail(WB_ERR_BAD_ARG, "wb_f16_write_bits: bits is NULL");
     char *dst = ctx->arena[WB_ARENA_WEIGHTS].base + w->off_main + elem_offset * 2;
-    WB_CUDA(cudaMemcpyAsync(dst, bits, (size_t)n * 2, cudaMemcpyHostToDevice, ctx->stream));
+    WB_CHECK(copy_to_device(ctx, dst, bits, (size_t)n * 2));
     WB_CUDA(cudaStreamSynchronize(ctx->stream));
     return WB_OK;
 }
@@ -539,8 +542,7 @@ int wb_read_weight_f16(wb_context *ctx, wb_handle h, int64_t elem_offset, int64_
     WB_NOT_RECORDING(ctx, "wb_read_weight_f16");
     WB_CHECK(dense_f16_target(ctx, h, elem_offset, n, &w));
     if (n == 0) return WB_OK;
-    WB_CUDA(cudaMemcpyAsync(out_bits, ctx->arena[WB_ARENA_WEIGHTS].base + w->off_main + elem_offset * 2,
-                            (size_t)n * 2, cudaMemcpyDeviceToHost, ctx->stream));
+    WB_CHECK(copy_to_host(ctx, out_bits, ctx->arena[WB_ARENA_WEIGHTS].base + w->off_main + elem_offset * 2, (size_t)n * 2));
     WB_CUDA(cudaStreamSynchronize(ctx->stream));
     return WB_OK;
 }

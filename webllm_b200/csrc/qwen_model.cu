@@ -525,7 +525,7 @@ int wb_qwen_last_logits(wb_qwen *m, float *out)
     WB_MODEL(m);
     WB_NOT_RECORDING(m->ctx, "wb_qwen_last_logits");
     if (!out) return fail(WB_ERR_BAD_ARG, "out is NULL");
-    WB_CUDA(cudaMemcpyAsync(out, m->dec.logits, (size_t)m->V * 4, cudaMemcpyDeviceToHost, m->ctx->stream));
+    WB_CHECK(copy_to_host(m->ctx, out, m->dec.logits, (size_t)m->V * 4));
     return wb_synchronize(m->ctx);
 }
 
