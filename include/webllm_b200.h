@@ -68,7 +68,7 @@ typedef struct {
     int32_t split_k;     /* number of K slices (1 = unsplit); the planGemvSplit analogue */
     int32_t grid_x, grid_y, grid_z;
     int32_t block;       /* threads per block */
-    int32_t tile_m, tile_n; /* GEMM_TC: tokens x output columns per CTA; otherwise 0 */
+    int32_t tile_m, tile_n; /* GEMM_TC and GENERIC: tokens x output columns per CTA; otherwise 0 */
     int32_t launches;    /* kernels this call enqueues */
     uint64_t scratch_bytes; /* split-K partial sums / fp16 staging taken from the context workspace */
 } wb_plan;

@@ -250,7 +250,7 @@ cudaError_t launch_prefill(cudaStream_t st, const float *q, const void *kmem, co
 {
     const size_t smem = (size_t)4 * kKeys * (D + 8) * sizeof(__half);
     auto kern = attention_prefill_mma_kernel<KV, D>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (const cudaError_t e = smem_limit_once<attention_prefill_mma_kernel<KV, D>>((int)smem); e != cudaSuccess) return e;
     const dim3 grid((unsigned)((M + kQRows - 1) / kQRows), (unsigned)H);
     return launch_pdl(kern, grid, dim3(128), smem, st, q, (const KV *)kmem, (const KV *)vmem, out, out16, M, H, KVH, past_ptr, past_imm,
                       ldq, kv_ld, 1.0f / sqrtf((float)D));

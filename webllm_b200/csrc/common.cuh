@@ -6,6 +6,7 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <atomic>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -50,6 +51,22 @@ struct TmapSlot {
     bool ok = false;
 };
 
+// The plan of a weight's last calls: planning walks tiles and splits through a cost model (2 to 4 us of host time), and a program
+// calls a weight with the same few row counts again and again.
+struct PlanSlot {
+    int64_t M = 0;
+    int act_dtype = 0, exact = 0, allow_stream = 0;
+    wb_plan plan;
+};
+
+// A tensor map of a call's own tensor (activations, result), kept while pointer and sizes stay the same.
+struct CallMap {
+    const void *base = nullptr;
+    int64_t M = 0;
+    int a = 0, b = 0;
+    TmapSlot map;
+};
+
 struct Weight {
     std::string name;
     WeightKind kind;
@@ -66,6 +83,9 @@ struct Weight {
     uint64_t arena_top = 0;   // `used` of the weight arena right after this registration (what wb_weight_pop checks)
     // tensor maps of the weight operand of the tensor-core GEMM, for 128 and 256 output columns per CTA
     mutable TmapSlot tmap_tc[2];
+    mutable PlanSlot plans[4];
+    mutable int next_plan = 0;
+    mutable CallMap tmap_x, tmap_c;
 };
 
 struct ArenaState {
@@ -218,6 +238,20 @@ inline bool pdl_enabled()
         return !(e && e[0] == '1');
     }();
     return on;
+}
+
+// The dynamic shared memory limit of a kernel, raised to the most that it is ever launched with, once per device: setting it on
+// every call costs as much as a fifth of a launch.
+template <auto *Kernel>
+inline cudaError_t smem_limit_once(int bytes)
+{
+    static std::atomic<bool> set[16] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 16 && set[dev].load(std::memory_order_relaxed)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute((const void *)Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev < 16) set[dev].store(true, std::memory_order_relaxed);
+    return e;
 }
 
 // `cluster_y` > 1 launches thread-block clusters of (1, cluster_y, 1) CTAs (grid.y must be a multiple of it).

@@ -617,6 +617,7 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
 
 __global__ void cast_f32_to_f16_kernel(const float *__restrict__ in, __half *__restrict__ out, int64_t n)
 {
+    pdl_sync();  // `out` may still be read by the GEMM in front
     int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x * 4;
     for (; i + 3 < n; i += stride) {
@@ -963,21 +964,25 @@ int launch_gemm_tc(wb_context *ctx, const Weight &w, const void *A, void *C, con
         const int64_t n = M * w.K;  // K % 64 == 0, so n % 4 == 0
         int blocks = (int)((n / 4 + 255) / 256);
         if (blocks > ctx->sm_count * 8) blocks = ctx->sm_count * 8;
-        tc::cast_f32_to_f16_kernel<<<blocks, 256, 0, ctx->stream>>>((const float *)A, (__half *)ctx->workspace, n);
+        WB_CUDA(launch_pdl(tc::cast_f32_to_f16_kernel, dim3((unsigned)blocks), dim3(256), 0, ctx->stream, (const float *)A, (__half *)ctx->workspace, n));
         ctx->launches++;
-        WB_CUDA(cudaGetLastError());
         a16 = ctx->workspace;
     }
     const int mt = plan.tile_m;
     const bool pair = plan.kernel == WB_KERNEL_GEMM_TC_PAIR;
     const int nh = pair ? 1 : plan.tile_n == 2 * tc::BN ? 2 : 1;  // a CTA of a pair takes 128-column boxes
-    // the activation map depends on the call (pointer, M, tile); the weight map only on the weight and the tile width:
-    // it is encoded once and kept with the weight
-    CUtensorMap mx;
+    // the weight map depends only on the weight and the tile width: it is encoded once and kept with the weight; the maps of
+    // the call's own tensors are kept while the next call's are the same
     TmapSlot &wslot = w.tmap_tc[nh - 1];
     CUtensorMap &mw = *reinterpret_cast<CUtensorMap *>(wslot.bytes);
-    WB_CHECK(make_map_2d(ctx, &mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a16, (uint64_t)w.K, (uint64_t)M, tc::BK,
-                         (uint32_t)(pair ? mt / 2 : mt), true));
+    const int box_x = pair ? mt / 2 : mt;
+    CallMap &cx = w.tmap_x;
+    CUtensorMap &mx = *reinterpret_cast<CUtensorMap *>(cx.map.bytes);
+    if (cx.base != a16 || cx.M != M || cx.a != box_x) {
+        cx.base = nullptr;
+        WB_CHECK(make_map_2d(ctx, &mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a16, (uint64_t)w.K, (uint64_t)M, tc::BK, (uint32_t)box_x, true));
+        cx.base = a16, cx.M = M, cx.a = box_x;
+    }
     tc::Params p;
     p.out = C, p.bias = bias, p.status = ctx->status_word;
     p.M = (int)M, p.N = (int)w.N, p.K = (int)w.K;
@@ -1008,11 +1013,13 @@ int launch_gemm_tc(wb_context *ctx, const Weight &w, const void *A, void *C, con
             // the result (or the K slices' f32 partial sums) leaves the epilogue through shared memory and TMA stores
             // where a work item has few k-blocks: with many, the drain hides under the next item's MMAs anyway and the
             // shared memory serves the 256-token tile better as a sixth pipeline stage
-            CUtensorMap mc;
+            CallMap &cc = w.tmap_c;
+            CUtensorMap &mc = *reinterpret_cast<CUtensorMap *>(cc.map.bytes);
             const bool c16 = S == 1 && out_dtype == WB_F16;
             void *cbase = S > 1 ? (void *)p.partial : C;
             const bool tma_store = (S > 1 || p.n_dst == 0) && w.N % (c16 ? 8 : 4) == 0 && ((uintptr_t)cbase & 15) == 0 && (mt < 256 || p.kb_per_slice <= kPairStageKb);
-            if (tma_store) {
+            if (tma_store && !(cc.base == cbase && cc.M == M && cc.a == S && cc.b == (int)c16)) {
+                cc.base = nullptr;
                 cuuint64_t dims[3] = {(cuuint64_t)w.N, (cuuint64_t)M, (cuuint64_t)S};
                 cuuint64_t strides[2] = {(cuuint64_t)w.N * (c16 ? 2 : 4), (cuuint64_t)w.N * M * (c16 ? 2 : 4)};
                 cuuint32_t box[3] = {(cuuint32_t)tc::BN, c16 ? 64u : 32u, 1u};
@@ -1022,6 +1029,7 @@ int launch_gemm_tc(wb_context *ctx, const Weight &w, const void *A, void *C, con
                                                                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                                                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
                 if (r != CUDA_SUCCESS) return fail(WB_ERR_CUDA, "cuTensorMapEncodeTiled (result) failed with code %d", (int)r);
+                cc.base = cbase, cc.M = M, cc.a = S, cc.b = c16;
             }
             int extra = 0;
             e = launch_gemm_pair(mt, mx, mw, tma_store ? &mc : nullptr, p, plan.grid_x, plan.grid_y, S, ctx->stream, ctx->sm_count,

@@ -545,50 +545,113 @@ __global__ void __launch_bounds__(256) dense_gemv_f16_kernel(const __half *__res
 }
 
 // =====================================================================================================
-// Shape-agnostic kernel: any M, N, K (K % 8 != 0, N % 4 != 0, small groups), GPTQ or dense fp16 weight.
-// One thread per output, k ascending, double accumulator, bias added in double, one rounding on the
-// store: the arithmetic of gemmNTRef (src/reference/qwen-ref.ts:126-145). Correctness path for ragged
-// shapes such as the reference's own (N=53, K=42) and (M=37, N=53, K=41) tests, not a fast path.
+// Shape-agnostic kernel: any M, N, K (K % 8 != 0, N % 4 != 0, small groups), GPTQ or dense fp16 weight, and every M of the
+// fp32-activation mode. k ascending, double accumulator, bias added in double, one rounding on the store: the arithmetic of
+// gemmNTRef (src/reference/qwen-ref.ts:126-145), bit for bit (a product of two f32 values is exact in double, so the fused
+// multiply-add rounds as the separate add does).
+//
+// Bound by the double-precision units (64 multiply-adds per clock and SM). A CTA of 128 threads computes TM rows x 32 columns, a
+// thread TM / 16 rows x 4 columns from operands that are unpacked, widened and staged in shared memory once per 32 k (with one
+// thread per output, as before, every weight was unpacked M times and every access was its own): 145 rows of 1000 -> 1236
+// 132 -> @@ us. 64 rows per CTA unless that leaves SMs without work.
 // =====================================================================================================
-__global__ void __launch_bounds__(128) linear_generic_kernel(const uint32_t *__restrict__ qw,
-                                                             const uint32_t *__restrict__ qz,
-                                                             const __half *__restrict__ sc,
-                                                             const __half *__restrict__ dense,
-                                                             const void *__restrict__ x, void *__restrict__ out,
-                                                             const float *__restrict__ bias, int64_t M, int64_t N,
-                                                             int64_t K, int64_t pack_rows, int64_t group,
-                                                             int64_t zcols, int x_f16, int out_f16, int round_x_f16)
+struct GenericParams {
+    const uint32_t *qw, *qz;
+    const __half *sc, *dense;
+    const void *x;
+    void *out;
+    const float *bias;
+    int64_t M, N, K, pack_rows, group, zcols;
+    int x_f16, out_f16, round_x_f16;
+};
+
+template <int TM>
+__global__ void __launch_bounds__(128) linear_generic_kernel(const GenericParams p)
 {
-    pdl_sync();
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= M * N) return;
-    const int64_t m = idx / N, n = idx - m * N;
-    auto xat = [&](int64_t k) -> float {
-        float v = x_f16 ? __half2float(((const __half *)x)[m * K + k]) : ((const float *)x)[m * K + k];
-        return round_x_f16 ? __half2float(__float2half_rn(v)) : v;
-    };
-    double acc = 0.0;
-    if (dense) {
-        for (int64_t k = 0; k < K; k++) acc += (double)xat(k) * (double)__half2float(dense[n * K + k]);
-    } else {
-        for (int64_t r = 0; r < pack_rows; r++) {
-            const uint32_t word = qw[r * N + n];
-            const int64_t g = (r * 8) / group;
-            const float scale = __half2float(sc[g * N + n]);
-            int zero = 8;
-            if (qz) zero = (int)((qz[g * zcols + (n >> 3)] >> (4 * (n & 7))) & 15u) + 1;
-            for (int j = 0; j < 8; j++) {
-                const int64_t k = r * 8 + j;
-                if (k >= K) break;
-                const float w = (float)((int)((word >> (4 * j)) & 15u) - zero) * scale;
-                acc += (double)xat(k) * (double)w;
+    constexpr int KC = 32, TN = 32, R = TM / 16, XP = TM + 2;
+    __shared__ __align__(16) double xs[KC][XP], ws[KC][TN];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & 7, ty = tid >> 3;
+    const int64_t m0 = (int64_t)blockIdx.y * TM, n0 = (int64_t)blockIdx.x * TN;
+    // staging: this thread's x values are k = k0 + lane of rows warp, warp + 4, ...; its weights 8 k of column tid / 4
+    const int wc = tid >> 2, wr = tid & 3;
+    const int64_t wn = n0 + wc;
+    float xv[TM / 4], wv[8];
+    auto fetch = [&](int64_t k0) {
+        const int64_t k = k0 + lane;
+#pragma unroll
+        for (int i = 0; i < TM / 4; i++) {
+            const int64_t m = m0 + warp + 4 * i;
+            float v = 0.f;
+            if (m < p.M && k < p.K) v = p.x_f16 ? __half2float(((const __half *)p.x)[m * p.K + k]) : ((const float *)p.x)[m * p.K + k];
+            xv[i] = p.round_x_f16 ? __half2float(__float2half_rn(v)) : v;
+        }
+        const int64_t kw = k0 + wr * 8;
+#pragma unroll
+        for (int j = 0; j < 8; j++) wv[j] = 0.f;
+        if (wn < p.N && kw < p.K) {
+            if (p.dense) {
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (kw + j < p.K) wv[j] = __half2float(p.dense[wn * p.K + kw + j]);
+            } else {
+                const int64_t r = kw >> 3, g = kw / p.group;
+                const uint32_t word = p.qw[r * p.N + wn];
+                const float scale = __half2float(p.sc[g * p.N + wn]);
+                const int zero = p.qz ? (int)((p.qz[g * p.zcols + (wn >> 3)] >> (4 * (wn & 7))) & 15u) + 1 : 8;
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (kw + j < p.K) wv[j] = (float)((int)((word >> (4 * j)) & 15u) - zero) * scale;
             }
         }
+    };
+    double acc[R][4];
+#pragma unroll
+    for (int i = 0; i < R; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0.0;
+    pdl_sync();
+    fetch(0);
+    for (int64_t k0 = 0; k0 < p.K; k0 += KC) {
+#pragma unroll
+        for (int i = 0; i < TM / 4; i++) xs[lane][warp + 4 * i] = (double)xv[i];
+#pragma unroll
+        for (int j = 0; j < 8; j++) ws[wr * 8 + j][wc] = (double)wv[j];
+        __syncthreads();
+        if (k0 + KC < p.K) fetch(k0 + KC);  // in flight under the arithmetic
+#pragma unroll 4
+        for (int k = 0; k < KC; k++) {
+            double a[R], b[4];
+#pragma unroll
+            for (int i = 0; i < R; i += 2) {
+                const double2 v = *reinterpret_cast<const double2 *>(&xs[k][ty * R + i]);
+                a[i] = v.x, a[i + 1] = v.y;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j += 2) {
+                const double2 v = *reinterpret_cast<const double2 *>(&ws[k][tx * 4 + j]);
+                b[j] = v.x, b[j + 1] = v.y;
+            }
+#pragma unroll
+            for (int i = 0; i < R; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+        }
+        __syncthreads();
     }
-    if (bias) acc += (double)bias[n];
-    if (out_f16) ((__half *)out)[idx] = __float2half_rn((float)acc);
-    else ((float *)out)[idx] = (float)acc;
+#pragma unroll
+    for (int i = 0; i < R; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int64_t m = m0 + ty * R + i, n = n0 + tx * 4 + j;
+            if (m >= p.M || n >= p.N) continue;
+            double v = acc[i][j];
+            if (p.bias) v += (double)p.bias[n];
+            if (p.out_f16) ((__half *)p.out)[m * p.N + n] = __float2half_rn((float)v);
+            else ((float *)p.out)[m * p.N + n] = (float)v;
+        }
 }
+
+static int generic_tile_m(int64_t M, int64_t N, int sms) { return ((M + 63) / 64) * ((N + 31) / 32) >= sms ? 64 : 32; }
 
 // =====================================================================================================
 // Planner and dispatch
@@ -760,7 +823,7 @@ static void plan_gemv_mma(wb_context *ctx, const Weight &w, int64_t M, int two_h
 }
 
 // allow_stream = false: a decode-size call that fuses a prologue stays on the general GEMV kernel.
-static int plan_linear_ex(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int exact, bool allow_stream, wb_plan *plan)
+static int make_plan(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int exact, bool allow_stream, wb_plan *plan)
 {
     memset(plan, 0, sizeof *plan);
     int kind = ctx->force_kernel;
@@ -816,12 +879,33 @@ static int plan_linear_ex(wb_context *ctx, const Weight &w, int64_t M, int act_d
         plan->kernel = kind;
         plan->split_k = 1;
         plan->block = 128;
-        plan->grid_x = (int)((M * w.N + 127) / 128);
-        plan->grid_y = plan->grid_z = 1;
+        plan->tile_m = generic_tile_m(M, w.N, ctx->sm_count), plan->tile_n = 32;
+        plan->grid_x = (int)((w.N + 31) / 32);
+        plan->grid_y = (int)((M + plan->tile_m - 1) / plan->tile_m);
+        plan->grid_z = 1;
         plan->launches = 1;
         return WB_OK;
     }
     return fail(WB_ERR_BAD_ARG, "unknown kernel kind %d", kind);
+}
+
+static int plan_linear_ex(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int exact, bool allow_stream, wb_plan *plan)
+{
+    // forced kernels, forced splits and column-sharded calls are planned every time
+    const bool keep = ctx->force_kernel == 0 && ctx->force_split == 0 && ctx->place.n_dst == 0;
+    if (keep)
+        for (const PlanSlot &s : w.plans)
+            if (s.M == M && s.act_dtype == act_dtype && s.exact == exact && s.allow_stream == (int)allow_stream) {
+                *plan = s.plan;
+                return WB_OK;
+            }
+    WB_CHECK(make_plan(ctx, w, M, act_dtype, exact, allow_stream, plan));
+    if (keep) {
+        PlanSlot &s = w.plans[w.next_plan];
+        w.next_plan = (w.next_plan + 1) % 4;
+        s.M = M, s.act_dtype = act_dtype, s.exact = exact, s.allow_stream = allow_stream, s.plan = *plan;
+    }
+    return WB_OK;
 }
 
 int plan_linear(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int exact, wb_plan *plan)
@@ -835,7 +919,7 @@ constexpr uint64_t kPrefetchLimit = 32ull << 20;
 template <int MB, bool EXACT, bool DIRECT>
 static cudaError_t launch_gemv_inst(const GemvParams &p, dim3 grid, int block, size_t smem, cudaStream_t st, bool pdl)
 {
-    cudaFuncSetAttribute(gptq_gemv_mma_kernel<MB, EXACT, DIRECT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmemLimit);
+    if (const cudaError_t e = smem_limit_once<gptq_gemv_mma_kernel<MB, EXACT, DIRECT>>(kGemvSmemLimit); e != cudaSuccess) return e;
     return launch_cluster_ex(gptq_gemv_mma_kernel<MB, EXACT, DIRECT>, grid, dim3(block), smem, st, p.cluster ? (unsigned)p.S : 1u, pdl, p);
 }
 
@@ -941,13 +1025,14 @@ int launch_linear(wb_context *ctx, const Weight &w, const void *A, void *C, cons
     case WB_KERNEL_DENSE_GEMV: {
         const __half *W = (const __half *)(base + w.off_main);
         const size_t smem = (size_t)M * w.K * 4;
-        auto go = [&](auto kern) {
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-            return launch_pdl(kern, dim3(plan.grid_x), dim3(256), smem, ctx->stream, W, A, C, bias, (int)M, (int)w.N, (int)w.K,
+        auto go = [&](auto kern, cudaError_t limit) {
+            return limit != cudaSuccess ? limit : launch_pdl(kern, dim3(plan.grid_x), dim3(256), smem, ctx->stream, W, A, C, bias, (int)M, (int)w.N, (int)w.K,
                               (int)(act_dtype == WB_F16), (int)(out_dtype == WB_F16));
         };
-        const cudaError_t e = M == 1 ? go(dense_gemv_f16_kernel<1>) : M == 2 ? go(dense_gemv_f16_kernel<2>)
-                              : M <= 4 ? go(dense_gemv_f16_kernel<4>) : go(dense_gemv_f16_kernel<8>);
+        const cudaError_t e = M == 1   ? go(dense_gemv_f16_kernel<1>, smem_limit_once<dense_gemv_f16_kernel<1>>(160 * 1024))
+                              : M == 2 ? go(dense_gemv_f16_kernel<2>, smem_limit_once<dense_gemv_f16_kernel<2>>(160 * 1024))
+                              : M <= 4 ? go(dense_gemv_f16_kernel<4>, smem_limit_once<dense_gemv_f16_kernel<4>>(160 * 1024))
+                                       : go(dense_gemv_f16_kernel<8>, smem_limit_once<dense_gemv_f16_kernel<8>>(160 * 1024));
         ctx->launches++;
         WB_CUDA(e);
         return WB_OK;
@@ -960,12 +1045,16 @@ int launch_linear(wb_context *ctx, const Weight &w, const void *A, void *C, cons
         // f32 activations are rounded to fp16 for M > 1 unless exact mode is on, as the reference's
         // tiled GEMM does when it stages A (gemm_nt_f16_from_f32.wgsl:58-62); its GEMV keeps f32.
         const int round_x = (act_dtype == WB_F32 && !ex && M > 1) ? 1 : 0;
-        const cudaError_t e = launch_pdl(linear_generic_kernel, dim3(plan.grid_x), dim3(128), 0, ctx->stream,
-            gptq ? (const uint32_t *)(base + w.off_main) : nullptr,
-            (gptq && w.has_zeros) ? (const uint32_t *)(base + w.off_zeros) : nullptr,
-            gptq ? (const __half *)(base + w.off_scales) : nullptr, gptq ? nullptr : (const __half *)(base + w.off_main),
-            A, C, bias, M, w.N, w.K, w.pack_rows, gptq ? w.group : 8, w.zcols, (int)(act_dtype == WB_F16),
-            (int)(out_dtype == WB_F16), round_x);
+        GenericParams g;
+        g.qw = gptq ? (const uint32_t *)(base + w.off_main) : nullptr;
+        g.qz = (gptq && w.has_zeros) ? (const uint32_t *)(base + w.off_zeros) : nullptr;
+        g.sc = gptq ? (const __half *)(base + w.off_scales) : nullptr, g.dense = gptq ? nullptr : (const __half *)(base + w.off_main);
+        g.x = A, g.out = C, g.bias = bias, g.M = M, g.N = w.N, g.K = w.K, g.pack_rows = w.pack_rows;
+        g.group = gptq ? w.group : 8, g.zcols = w.zcols;
+        g.x_f16 = act_dtype == WB_F16, g.out_f16 = out_dtype == WB_F16, g.round_x_f16 = round_x;
+        const dim3 grid((unsigned)plan.grid_x, (unsigned)plan.grid_y);
+        const cudaError_t e = plan.tile_m == 64 ? launch_pdl(linear_generic_kernel<64>, grid, dim3(128), 0, ctx->stream, g)
+                                                : launch_pdl(linear_generic_kernel<32>, grid, dim3(128), 0, ctx->stream, g);
         ctx->launches++;
         WB_CUDA(e);
         return WB_OK;

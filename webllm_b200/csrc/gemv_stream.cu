@@ -315,11 +315,11 @@ int launch_gemv_stream(wb_context *ctx, const Weight &w, const GemvParams &gp, b
     dim3 grid((unsigned)gemv_stream_grid_x(ctx->sm_count, w.N, p.S), (unsigned)p.S);
     cudaError_t e;
     if (has_lo) {
-        cudaFuncSetAttribute(gptq_gemv_stream_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        e = launch_pdl(gptq_gemv_stream_kernel<true>, grid, dim3(256), smem, ctx->stream, p);
+        e = smem_limit_once<gptq_gemv_stream_kernel<true>>(100 * 1024);
+        if (e == cudaSuccess) e = launch_pdl(gptq_gemv_stream_kernel<true>, grid, dim3(256), smem, ctx->stream, p);
     } else {
-        cudaFuncSetAttribute(gptq_gemv_stream_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        e = launch_pdl(gptq_gemv_stream_kernel<false>, grid, dim3(256), smem, ctx->stream, p);
+        e = smem_limit_once<gptq_gemv_stream_kernel<false>>(100 * 1024);
+        if (e == cudaSuccess) e = launch_pdl(gptq_gemv_stream_kernel<false>, grid, dim3(256), smem, ctx->stream, p);
     }
     ctx->launches++;
     WB_CUDA(e);

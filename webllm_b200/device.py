@@ -30,6 +30,7 @@ class Gpu:
             else:
                 L.check(self._lib.wb_arena_create(self._ctx, arena, size))
         self.arena = Arena(self)
+        self._handles: dict[str, int] = {}  # names already looked up
 
     # -- lifetime
     def close(self) -> None:
@@ -134,12 +135,16 @@ class Gpu:
         return h.value
 
     def weight(self, name: str) -> int:
-        h = C.c_int32(-1)
-        L.check(self._lib.wb_weight_lookup(self._ctx, name.encode(), C.byref(h)))
-        return h.value
+        h = self._handles.get(name)
+        if h is None:
+            out = C.c_int32(-1)
+            L.check(self._lib.wb_weight_lookup(self._ctx, name.encode(), C.byref(out)))
+            h = self._handles[name] = out.value
+        return h
 
     def weight_pop(self) -> None:
         L.check(self._lib.wb_weight_pop(self._ctx))
+        self._handles.clear()
 
     def read_weight_f16(self, h: int, elem_offset: int, count: int) -> np.ndarray:
         out = np.empty(count, np.uint16)
@@ -158,9 +163,10 @@ class Gpu:
         L.check(fn(self._ctx, h, out.offset))
 
     def linear(self, weight: int, A: Tensor, Cout: Tensor, bias: int | None, M: int, exact: bool = False) -> None:
-        L.check(self._lib.wb_linear(self._ctx, weight, A.offset, Cout.offset, -1 if bias is None else bias, M,
-                                    L.WB_F32 if A.dtype == "f32" else L.WB_F16,
-                                    L.WB_F32 if Cout.dtype == "f32" else L.WB_F16, 1 if exact else 0))
+        rc = self._lib.wb_linear(self._ctx, weight, A.offset, Cout.offset, -1 if bias is None else bias, M,
+                                 0 if A.dtype == "f32" else 1, 0 if Cout.dtype == "f32" else 1, 1 if exact else 0)  # WB_F32, WB_F16
+        if rc:
+            L.check(rc)
 
     def linear_gather(self, weight: int, A: Tensor, C_full: Tensor, tmp: Tensor, bias: int | None, M: int, n_total: int,
                       col_begin: int, peer_bases: list[int]) -> None:

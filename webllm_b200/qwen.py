@@ -200,10 +200,9 @@ class QwenGpt:
         """``gemm(A, weight, C, bias, M, N, K)``: C = A . W^T (+ bias). N and K are checked against the
         registered weight (the reference trusts the caller)."""
         h = self.gpu.weight(weight)
-        p = self.gpu.plan(h, M, A.dtype)  # raises for a non-matrix weight
-        del p
         hb = None if bias is None else self.gpu.weight(bias)
         if A.length < M * K or Cout.length < M * N:
+            self.gpu.plan(h, M, A.dtype)  # a non-matrix weight is the first thing to say
             raise L.WebllmError(L.WB_ERR_BAD_ARG, f"gemm: tensors too small for M={M} N={N} K={K}")
         self.gpu.linear(h, A, Cout, hb, M, exact=self._exact if exact is None else exact)
 
