@@ -3,14 +3,18 @@
 // (fp16-operand) mode. The scalar kernel in qwen_ops.cu stays the path for the fp32-activation mode, for head sizes
 // other than 64 / 128 and for the uncached forward.
 //
-// One CTA = 4 warps = 64 query rows of one head; a warp owns 16 rows. Keys are walked in blocks of 64: the K and V
-// rows of a block are staged in shared memory as fp16 (cp.async straight from an fp16 cache, double-buffered; an f32
+// One CTA = 64 query rows of one head, two groups of 4 warps: a warp owns 16 rows, group 0 takes the even blocks of 64
+// keys and group 1 the odd ones, and the two states of a row are merged at the end. A late row block walks up to 32
+// blocks at 2048 tokens, and that chain of load, score, softmax, multiply is what the launch lasts; two groups halve
+// it. CTAs start longest first over all heads, so that short ones fill the gaps. 2048 tokens, 14 heads of 64: 54.5 us
+// with one group and heads after each other, 41 us so; tensor pipe 41 % busy, the rest is the softmax between the MMAs.
+// The K and V rows of a block are staged in shared memory as fp16 (cp.async straight from an fp16 cache, double-buffered; an f32
 // cache is converted on the way), S = Q K^T and O += P V run on the warp-level MMA (m16n8k16, fp16 operands, f32
 // accumulate), and the softmax is the online form in f32 registers: per row a running maximum and sum, the
 // accumulator rescaled when the maximum moves. The accumulator fragments of S are, element for element, the A
 // fragments of the P V product, so P never leaves the registers; V is read transposed with ldmatrix.
 // A query row r sees keys [0, past + r]; blocks past a warp's last row are skipped by that warp, and only the blocks
-// that straddle the diagonal pay for the mask. Heavy row blocks (late rows, many keys) are scheduled first.
+// that straddle the diagonal pay for the mask.
 #include "qwen_ops.cuh"
 #include "gemv_core.cuh"
 
@@ -20,6 +24,7 @@ namespace {
 
 constexpr int kQRows = 64;   // query rows per CTA
 constexpr int kKeys = 64;    // keys per block
+constexpr int kGroups = 2;   // groups of 4 warps that share the key blocks of a CTA's rows
 
 __device__ __forceinline__ void cp16(void *dst_smem, const void *src)
 {
@@ -51,19 +56,19 @@ __device__ __forceinline__ float ex2(float x)
 }
 
 // Stages keys [key0, key0 + 64) of one KV head into `dst` ([64][D + 8] halves); rows at or past n_keys become zeros.
-// A thread copies the same pieces of every block (piece u: row (tid + 128 u) / (D / 8), 16 bytes), so the offsets are
-// computed once by the caller: dst_off[u] in halves, src_off[u] in elements of the cache row.
+// A thread copies 16-byte pieces of one column of rows `row`, row + 1024 / D, ... of every block.
 template <typename KV, int D>
-__device__ __forceinline__ void stage_block(__half *dst, const KV *src, int key0, int n_keys, int kv_ld, const int (&dst_off)[D / 16],
-                                            const int (&src_off)[D / 16], const int (&row)[D / 16])
+__device__ __forceinline__ void stage_block(__half *dst, const KV *src, int key0, int n_keys, int kv_ld, int row, int col)
 {
-    const KV *base = src + (int64_t)key0 * kv_ld;
+    constexpr int STEP = 1024 / D;
+    const KV *base = src + (int64_t)(key0 + row) * kv_ld + col;
+    dst += row * (D + 8) + col;
     const bool whole = key0 + kKeys <= n_keys;
 #pragma unroll
     for (int u = 0; u < D / 16; u++) {
-        __half *d = dst + dst_off[u];
-        if (whole || key0 + row[u] < n_keys) {
-            const KV *sp = base + src_off[u];
+        __half *d = dst + u * STEP * (D + 8);
+        if (whole || key0 + row + u * STEP < n_keys) {
+            const KV *sp = base + (int64_t)u * STEP * kv_ld;
             if constexpr (sizeof(KV) == 2) {
                 cp16(d, sp);
             } else {
@@ -79,7 +84,7 @@ __device__ __forceinline__ void stage_block(__half *dst, const KV *src, int key0
 }
 
 template <typename KV, int D>
-__global__ void __launch_bounds__(128, D == 64 ? 4 : 2) attention_prefill_mma_kernel(const float *__restrict__ q, const KV *__restrict__ kmem,
+__global__ void __launch_bounds__(kGroups * 128, D == 64 ? 2 : 1) attention_prefill_mma_kernel(const float *__restrict__ q, const KV *__restrict__ kmem,
                                                                     const KV *__restrict__ vmem, float *__restrict__ out,
                                                                     __half *__restrict__ out16, int M, int H, int KVH,
                                                                     const int *__restrict__ past_ptr, int past_imm, int ldq,
@@ -90,11 +95,12 @@ __global__ void __launch_bounds__(128, D == 64 ? 4 : 2) attention_prefill_mma_ke
     constexpr int KS = D / 16;    // k-steps of Q K^T
     constexpr int DT = D / 8;     // 8-wide tiles of the head dimension
     extern __shared__ uint4 smem_u4[];
-    __half *Ks = reinterpret_cast<__half *>(smem_u4);       // [2][64][LD]
-    __half *Vs = Ks + 2 * kKeys * LD;                        // [2][64][LD]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    const int rb = (int)gridDim.x - 1 - (int)blockIdx.x;     // late (long) row blocks first
-    const int h = blockIdx.y, kvh = h / (H / KVH);
+    const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    __half *Ks = reinterpret_cast<__half *>(smem_u4) + grp * 4 * kKeys * LD;  // [2][64][LD] of this group
+    __half *Vs = Ks + 2 * kKeys * LD;                                         // [2][64][LD]
+    const int rb = (int)gridDim.y - 1 - (int)blockIdx.y;     // late (long) row blocks first
+    const int h = blockIdx.x, kvh = h / (H / KVH);
+    auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory"); };
     const int past = past_ptr ? *past_ptr : past_imm;
     const int r0 = rb * kQRows;
     const int n_keys = past + M;                             // rows of the cache that exist
@@ -102,16 +108,12 @@ __global__ void __launch_bounds__(128, D == 64 ? 4 : 2) attention_prefill_mma_ke
     const int n_blocks = (past + last_row) / kKeys + 1;
     const KV *kbase = kmem + kvh * D, *vbase = vmem + kvh * D;
 
-    // this thread's pieces of a staged block: 64 rows x D / 8 pieces of 16 bytes over 128 threads
-    int st_dst[D / 16], st_src[D / 16], st_row[D / 16];
-#pragma unroll
-    for (int u = 0; u < D / 16; u++) {
-        const int i = tid + 128 * u, r = i / (D / 8), c = (i - r * (D / 8)) * 8;
-        st_row[u] = r, st_dst[u] = r * LD + c, st_src[u] = r * kv_ld + c;
-    }
+    const int st_row = tid / (D / 8), st_col = (tid - st_row * (D / 8)) * 8;  // this thread's pieces of a staged block
     // first block on its way while the Q fragments are loaded
-    stage_block<KV, D>(Ks, kbase, 0, n_keys, kv_ld, st_dst, st_src, st_row);
-    stage_block<KV, D>(Vs, vbase, 0, n_keys, kv_ld, st_dst, st_src, st_row);
+    if (grp < n_blocks) {
+        stage_block<KV, D>(Ks, kbase, grp * kKeys, n_keys, kv_ld, st_row, st_col);
+        stage_block<KV, D>(Vs, vbase, grp * kKeys, n_keys, kv_ld, st_row, st_col);
+    }
     cp_async_commit();
 
     // Q fragments of this warp's 16 rows (rows g and g + 8 of the tile), fp16, kept for the whole kernel
@@ -136,15 +138,15 @@ __global__ void __launch_bounds__(128, D == 64 ? 4 : 2) attention_prefill_mma_ke
     const int warp_last_key = past + min(r0 + warp * 16 + 15, M - 1);  // the last key any row of this warp sees
     const float sl2 = scale * 1.4426950408889634f;                     // scores are kept in units of log2(e)
 
-    for (int kb = 0; kb < n_blocks; kb++) {
-        const int buf = kb & 1;
-        if (kb + 1 < n_blocks) {  // next block into the other buffer (its last readers passed the barrier below)
-            stage_block<KV, D>(Ks + (buf ^ 1) * kKeys * LD, kbase, (kb + 1) * kKeys, n_keys, kv_ld, st_dst, st_src, st_row);
-            stage_block<KV, D>(Vs + (buf ^ 1) * kKeys * LD, vbase, (kb + 1) * kKeys, n_keys, kv_ld, st_dst, st_src, st_row);
+    int buf = 0;
+    for (int kb = grp; kb < n_blocks; kb += kGroups, buf ^= 1) {
+        if (kb + kGroups < n_blocks) {  // next block into the other buffer (its last readers passed the barrier below)
+            stage_block<KV, D>(Ks + (buf ^ 1) * kKeys * LD, kbase, (kb + kGroups) * kKeys, n_keys, kv_ld, st_row, st_col);
+            stage_block<KV, D>(Vs + (buf ^ 1) * kKeys * LD, vbase, (kb + kGroups) * kKeys, n_keys, kv_ld, st_row, st_col);
         }
         cp_async_commit();
         cp_async_wait(1);  // everything but the newest group: block kb has landed
-        __syncthreads();
+        group_sync();
         const int key0 = kb * kKeys;
         if (key0 <= warp_last_key && r0 + warp * 16 < M) {
             const __half *Kb = Ks + buf * kKeys * LD, *Vb = Vs + buf * kKeys * LD;
@@ -221,15 +223,46 @@ __global__ void __launch_bounds__(128, D == 64 ? 4 : 2) attention_prefill_mma_ke
                 }
             }
         }
-        __syncthreads();  // block kb's buffer is refilled by the next iteration's staging
+        group_sync();  // block kb's buffer is refilled by the next iteration's staging
     }
     cp_async_wait(0);
-    // ---- normalise and store (f32)
 #pragma unroll
     for (int r = 0; r < 2; r++) {
         l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
         l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 2);
     }
+    // ---- group 1 hands its state to group 0 through the shared memory of its own blocks: [64][D + 4] sums, [64] maxima, [64] sums
+    {
+        constexpr int OP = D + 4;
+        float *po = reinterpret_cast<float *>(reinterpret_cast<__half *>(smem_u4) + 4 * kKeys * LD), *pm = po + kQRows * OP, *pl = pm + kQRows;
+        const int ra = warp * 16 + g;
+        if (grp == 1) {
+            group_sync();  // every warp of the group has read its last block
+#pragma unroll
+            for (int j = 0; j < DT; j++) {
+                *reinterpret_cast<float2 *>(po + ra * OP + j * 8 + 2 * t) = make_float2(o[j][0], o[j][1]);
+                *reinterpret_cast<float2 *>(po + (ra + 8) * OP + j * 8 + 2 * t) = make_float2(o[j][2], o[j][3]);
+            }
+            if (t == 0) pm[ra] = m_run[0], pm[ra + 8] = m_run[1], pl[ra] = l_run[0], pl[ra + 8] = l_run[1];
+        }
+        __syncthreads();
+        if (grp == 1) return;
+        float own[2], other[2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const float m1 = pm[ra + 8 * r], m = fmaxf(m_run[r], m1), mu = m == -INFINITY ? 0.f : m;
+            own[r] = ex2((m_run[r] - mu) * sl2), other[r] = ex2((m1 - mu) * sl2);
+            l_run[r] = l_run[r] * own[r] + pl[ra + 8 * r] * other[r];
+        }
+#pragma unroll
+        for (int j = 0; j < DT; j++) {
+            const float2 a = *reinterpret_cast<const float2 *>(po + ra * OP + j * 8 + 2 * t);
+            const float2 b = *reinterpret_cast<const float2 *>(po + (ra + 8) * OP + j * 8 + 2 * t);
+            o[j][0] = o[j][0] * own[0] + a.x * other[0], o[j][1] = o[j][1] * own[0] + a.y * other[0];
+            o[j][2] = o[j][2] * own[1] + b.x * other[1], o[j][3] = o[j][3] * own[1] + b.y * other[1];
+        }
+    }
+    // ---- normalise and store (f32)
     const float inv_a = l_run[0] > 0.f ? 1.f / l_run[0] : 0.f, inv_b = l_run[1] > 0.f ? 1.f / l_run[1] : 0.f;
     const int64_t ia = (int64_t)row_a * (H * D) + h * D + 2 * t, ib = (int64_t)row_b * (H * D) + h * D + 2 * t;
 #pragma unroll
@@ -248,11 +281,11 @@ template <typename KV, int D>
 cudaError_t launch_prefill(cudaStream_t st, const float *q, const void *kmem, const void *vmem, float *out, __half *out16, int M, int H,
                            int KVH, const int *past_ptr, int past_imm, int ldq, int kv_ld)
 {
-    const size_t smem = (size_t)4 * kKeys * (D + 8) * sizeof(__half);
+    const size_t smem = (size_t)kGroups * 4 * kKeys * (D + 8) * sizeof(__half);
     auto kern = attention_prefill_mma_kernel<KV, D>;
     if (const cudaError_t e = smem_limit_once<attention_prefill_mma_kernel<KV, D>>((int)smem); e != cudaSuccess) return e;
-    const dim3 grid((unsigned)((M + kQRows - 1) / kQRows), (unsigned)H);
-    return launch_pdl(kern, grid, dim3(128), smem, st, q, (const KV *)kmem, (const KV *)vmem, out, out16, M, H, KVH, past_ptr, past_imm,
+    const dim3 grid((unsigned)H, (unsigned)((M + kQRows - 1) / kQRows));
+    return launch_pdl(kern, grid, dim3(kGroups * 128), smem, st, q, (const KV *)kmem, (const KV *)vmem, out, out16, M, H, KVH, past_ptr, past_imm,
                       ldq, kv_ld, 1.0f / sqrtf((float)D));
 }
 
