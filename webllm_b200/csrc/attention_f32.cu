@@ -1,0 +1,133 @@
+// Causal GQA attention in f32 arithmetic for several query rows: attention_gqa.wgsl / attention_gqa_cache.wgsl (attentionGqaRef,
+// src/reference/qwen-ref.ts:67-116) for the uncached forward, the fp32-activation mode and prompts too short for the fp16
+// tensor-core kernel, head size 64.
+//
+// One CTA = 32 query rows of one head; keys in blocks of 32 staged in shared memory as f32, scores and weighted sums from
+// 4 x 2 and 4 x 4 register tiles, online softmax. One CTA per single row, as the scalar kernel (qwen_ops.cu) has it, reads every
+// key 32 times as often and leaves a warp's lanes one multiply per load. 4 x 101 rows, 14 heads: 57 -> 22 us a layer; what is
+// left is the chain of up to four key blocks in a grid of 224 CTAs.
+#include "qwen_ops.cuh"
+
+namespace wb {
+
+namespace {
+
+constexpr int kD = 64, kRows = 32, kKeys = 32, kThreads = 128;
+constexpr int kQP = kRows + 4, kKP = kKeys + 2, kVP = kD + 4;
+
+__device__ __forceinline__ float4 load4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ float4 load4(const __half *p)
+{
+    const uint2 r = *reinterpret_cast<const uint2 *>(p);
+    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&r.x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&r.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// Rows i of sequence b (row b * T + i of q and out) see keys 0 .. past + i, row b * key_rows + key of kmem / vmem.
+template <typename KV>
+__global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__restrict__ q, const KV *__restrict__ kmem,
+                                                                 const KV *__restrict__ vmem, float *__restrict__ out, int H, int KVH, int T,
+                                                                 const int *__restrict__ past_ptr, int past_imm, int key_rows, int ldq,
+                                                                 int kv_ld, float scale)
+{
+    pdl_sync();
+    __shared__ __align__(16) float Qs[kD][kQP], Ks[kD][kKP], Vs[kKeys][kVP], Ps[kKeys][kQP];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & 15, ty = tid >> 4;
+    const int tile = (int)gridDim.y - 1 - (int)blockIdx.y;  // late (long) tiles first
+    const int i0 = tile * kRows, b = blockIdx.z, h = blockIdx.x, kvh = h / (H / KVH);
+    const int past = past_ptr ? *past_ptr : past_imm;
+    const int n_keys = past + min(i0 + kRows, T);
+    const KV *kb = kmem + (int64_t)b * key_rows * kv_ld + kvh * kD, *vb = vmem + (int64_t)b * key_rows * kv_ld + kvh * kD;
+    const int64_t row0 = (int64_t)b * T + i0;
+    // a lane stages its row (key), a warp every fourth 4 dims
+    for (int d = warp * 4; d < kD; d += 16) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i0 + lane < T) v = load4(q + (row0 + lane) * ldq + h * kD + d);
+        Qs[d][lane] = v.x, Qs[d + 1][lane] = v.y, Qs[d + 2][lane] = v.z, Qs[d + 3][lane] = v.w;
+    }
+    float o[4][4] = {}, m[4], l[4] = {};
+#pragma unroll
+    for (int i = 0; i < 4; i++) m[i] = -INFINITY;
+    for (int key0 = 0; key0 < n_keys; key0 += kKeys) {
+        const bool in = key0 + lane < n_keys;
+        for (int d = warp * 4; d < kD; d += 16) {
+            float4 k = make_float4(0.f, 0.f, 0.f, 0.f), v = k;
+            if (in) k = load4(kb + (int64_t)(key0 + lane) * kv_ld + d), v = load4(vb + (int64_t)(key0 + lane) * kv_ld + d);
+            Ks[d][lane] = k.x, Ks[d + 1][lane] = k.y, Ks[d + 2][lane] = k.z, Ks[d + 3][lane] = k.w;
+            *reinterpret_cast<float4 *>(&Vs[lane][d]) = v;
+        }
+        __syncthreads();
+        float s[4][2] = {};  // rows 4 ty + i, keys 2 tx + j
+#pragma unroll 8
+        for (int d = 0; d < kD; d++) {
+            const float4 a = *reinterpret_cast<const float4 *>(&Qs[d][ty * 4]);
+            const float2 c = *reinterpret_cast<const float2 *>(&Ks[d][tx * 2]);
+            s[0][0] = fmaf(a.x, c.x, s[0][0]), s[0][1] = fmaf(a.x, c.y, s[0][1]);
+            s[1][0] = fmaf(a.y, c.x, s[1][0]), s[1][1] = fmaf(a.y, c.y, s[1][1]);
+            s[2][0] = fmaf(a.z, c.x, s[2][0]), s[2][1] = fmaf(a.z, c.y, s[2][1]);
+            s[3][0] = fmaf(a.w, c.x, s[3][0]), s[3][1] = fmaf(a.w, c.y, s[3][1]);
+        }
+        float p[4][2];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int last = past + i0 + ty * 4 + i;  // the row's last key
+#pragma unroll
+            for (int j = 0; j < 2; j++) s[i][j] = key0 + tx * 2 + j > last ? -INFINITY : s[i][j] * scale;
+            float mx = fmaxf(s[i][0], s[i][1]);
+#pragma unroll
+            for (int w = 8; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
+            const float mn = fmaxf(m[i], mx), c = m[i] == -INFINITY ? 0.f : expf(m[i] - mn);
+            l[i] *= c;
+#pragma unroll
+            for (int j = 0; j < 4; j++) o[i][j] *= c;
+            m[i] = mn;
+#pragma unroll
+            for (int j = 0; j < 2; j++) p[i][j] = s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - mn), l[i] += p[i][j];
+        }
+#pragma unroll
+        for (int j = 0; j < 2; j++) *reinterpret_cast<float4 *>(&Ps[tx * 2 + j][ty * 4]) = make_float4(p[0][j], p[1][j], p[2][j], p[3][j]);
+        __syncwarp();  // a warp's rows are its own
+#pragma unroll 8
+        for (int k = 0; k < kKeys; k++) {
+            const float4 a = *reinterpret_cast<const float4 *>(&Ps[k][ty * 4]), v = *reinterpret_cast<const float4 *>(&Vs[k][tx * 4]);
+            o[0][0] = fmaf(a.x, v.x, o[0][0]), o[0][1] = fmaf(a.x, v.y, o[0][1]), o[0][2] = fmaf(a.x, v.z, o[0][2]), o[0][3] = fmaf(a.x, v.w, o[0][3]);
+            o[1][0] = fmaf(a.y, v.x, o[1][0]), o[1][1] = fmaf(a.y, v.y, o[1][1]), o[1][2] = fmaf(a.y, v.z, o[1][2]), o[1][3] = fmaf(a.y, v.w, o[1][3]);
+            o[2][0] = fmaf(a.z, v.x, o[2][0]), o[2][1] = fmaf(a.z, v.y, o[2][1]), o[2][2] = fmaf(a.z, v.z, o[2][2]), o[2][3] = fmaf(a.z, v.w, o[2][3]);
+            o[3][0] = fmaf(a.w, v.x, o[3][0]), o[3][1] = fmaf(a.w, v.y, o[3][1]), o[3][2] = fmaf(a.w, v.z, o[3][2]), o[3][3] = fmaf(a.w, v.w, o[3][3]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+#pragma unroll
+        for (int w = 8; w > 0; w >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], w);
+        const int r = ty * 4 + i;
+        if (i0 + r >= T) continue;
+        const float inv = 1.f / l[i];
+        *reinterpret_cast<float4 *>(out + (row0 + r) * (H * kD) + h * kD + tx * 4) =
+            make_float4(o[i][0] * inv, o[i][1] * inv, o[i][2] * inv, o[i][3] * inv);
+    }
+}
+
+}  // namespace
+
+// Two rows and more of 16-byte aligned heads of 64 dims (one row keeps the scalar kernel: the decode kernels are for that).
+bool op_attention_f32_supported(int M, int D, int ldq, int kv_ld) { return M > 1 && D == kD && ldq % 4 == 0 && kv_ld % 4 == 0; }
+
+int op_attention_f32(wb_context *ctx, const float *q, const void *kmem, const void *vmem, int kv_f16, float *out, int M, int H, int KVH, int T,
+                     const int *past_ptr, int past_imm, int use_cache, int ldq, int kv_ld)
+{
+    const float scale = 1.0f / sqrtf((float)kD);
+    const dim3 grid((unsigned)H, (unsigned)((T + kRows - 1) / kRows), (unsigned)(M / T));
+    const int key_rows = use_cache ? 0 : T;  // (one sequence with a cache)
+    const cudaError_t e =
+        kv_f16 ? launch_pdl(attention_f32_kernel<__half>, grid, dim3(kThreads), 0, ctx->stream, q, (const __half *)kmem, (const __half *)vmem, out, H,
+                            KVH, T, past_ptr, past_imm, key_rows, ldq, kv_ld, scale)
+               : launch_pdl(attention_f32_kernel<float>, grid, dim3(kThreads), 0, ctx->stream, q, (const float *)kmem, (const float *)vmem, out, H,
+                            KVH, T, past_ptr, past_imm, key_rows, ldq, kv_ld, scale);
+    ctx->launches++;
+    WB_CUDA(e);
+    return WB_OK;
+}
+
+}  // namespace wb
