@@ -81,8 +81,8 @@ struct Weight {
     bool has_zeros = false;
     uint64_t bytes = 0;
     uint64_t arena_top = 0;   // `used` of the weight arena right after this registration (what wb_weight_pop checks)
-    // tensor maps of the weight operand of the tensor-core GEMM, for 128 and 256 output columns per CTA
-    mutable TmapSlot tmap_tc[2];
+    // tensor maps of the weight operand of the tensor-core GEMM, in boxes of 128, 256 and 64 columns
+    mutable TmapSlot tmap_tc[3];
     mutable PlanSlot plans[4];
     mutable int next_plan = 0;
     mutable CallMap tmap_x, tmap_c;
@@ -175,6 +175,8 @@ struct LinearFusion {
 };
 // True when launch_linear would run this weight at M rows of f32 activations through the kernel that fuses.
 bool linear_fusion_supported(wb_context *ctx, const Weight &w, int64_t M);
+// gate | up in one projection with silu(gate) * up as its fp16 result (gemm_pair.cu). *done = false: not a shape for that kernel.
+int launch_gate_up_silu(wb_context *ctx, const Weight &w, const __half *A, __half *act, int64_t M, bool *done);
 int launch_linear(wb_context *ctx, const Weight &w, const void *A, void *C, const float *bias, int64_t M,
                   int act_dtype, int out_dtype, int exact, const LinearFusion *fusion = nullptr);
 

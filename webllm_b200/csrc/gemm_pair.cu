@@ -10,14 +10,14 @@
 //
 // Roles per CTA: a TMA producer warp (own packed-weight box, own half of the activation box), an MMA issuer warp
 // (rank 0 of the pair only; both ranks allocate and free tensor memory), sixteen unpack warps (four sets of one thread
-// per column that take the k-blocks in turn) and four epilogue warps (drain one of the two accumulator sets while the
+// per column that take the k-blocks in turn) and four or eight epilogue warps (drain one of the two accumulator sets while the
 // MMAs of the next item run); which warp id has which role is listed at WARPS_PAIR. The pair walks the work items pair,
 // pair + pairs, ...; an item is (K slice, column tile, token tile); with more than one K slice the items write f32
 // partial sums that the split-K reduce launch adds.
 //   * The weights are constants: the producer requests the packed boxes of the first stages, and the unpack sets unpack
 //     them, before the wait on the previous kernel (programmatic dependent launch); the activation loads and the
 //     epilogue's stores come after it.
-//   * Where a work item is short (K = 896: 14 k-blocks) the result leaves through two 16 KB staging tiles and TMA stores
+//   * Where a work item is short (K = 896: 14 k-blocks) the result leaves through four 8 KB staging tiles and TMA stores
 //     (fp16, f32, or the f32 partial sums of a K slice; STG instantiations); where it is long, from registers, and the
 //     shared memory holds a sixth pipeline stage instead.
 //   * A launch whose last round of work items would leave most pairs idle for a long item cuts those items along K over
@@ -40,23 +40,24 @@ namespace tcp {
 
 using namespace tc;
 
-constexpr int EPI_WARPS = 4;
-// Warp roles as listed at MMA_WARP (gemm_tc.cuh), plus the four epilogue warps 21 .. 24 (a warp reads the tensor-memory
-// lane quarter id % 4).
-constexpr int WARPS_PAIR = WARPS + EPI_WARPS;
-constexpr int THREADS_PAIR = 32 * WARPS_PAIR;
+// Warp roles as listed at MMA_WARP (gemm_tc.cuh), plus the epilogue warps from 21 on, in groups of four (a warp reads the
+// tensor-memory lane quarter id % 4). Short work items, those that leave through staging tiles, have two groups that take the
+// chunks of token rows in turn: at K = 896 an item's MMAs last 5 us, and one group needed 9 us to drain it with silu, since the
+// unpack warps leave it few issue slots (gate | up with silu at 2048 rows: 67 us with one group, 54 us with two; the same GEMM
+// and the separate pass before: 43.7 + 17.8 us). 29 warps of 64 registers.
+constexpr int epi_groups(bool stg) { return stg ? 2 : 1; }
+constexpr int pair_threads(bool stg) { return 32 * (WARPS + 4 * epi_groups(stg)); }
 constexpr int KG = 4;  // unpack sets: 128 threads each, one thread per weight column
-constexpr int STG_ROWS = 64;                 // token rows of an fp16 epilogue staging tile (half as many of f32)
-constexpr int STG_BYTES = STG_ROWS * BN * 2;  // [64 tokens][128 columns] fp16 or [32][128] f32
+constexpr int STG_BYTES = STG_ROWS * BN * 2;  // an epilogue staging tile: [32 tokens][128 columns] fp16 or [16][128] f32
 
-// STG: two epilogue staging tiles are carved out of the shared memory (one pipeline stage fewer for the 256-token tile)
+// STG: two epilogue staging tiles per group are carved out of the shared memory (one pipeline stage fewer for the 256-token tile)
 template <int MT, bool STG>
 struct SmemPair {
     static constexpr int X_BYTES = (MT / 2) * BK * 2;   // this CTA's half of the activation tile
     static constexpr int WD_BYTES = BN * BK * 2;        // unpacked fp16 operand, 128 columns x 64 k
     static constexpr int WP_BYTES = 8 * BN * 4;         // packed box, 8 rows x 128 columns
     static constexpr int STAGE_BYTES = X_BYTES + WD_BYTES + WP_BYTES;  // every piece is a multiple of 1024
-    static constexpr int STG_TOTAL = STG ? 2 * STG_BYTES : 0;
+    static constexpr int STG_TOTAL = STG ? 2 * epi_groups(STG) * STG_BYTES : 0;
     static constexpr int MAX_STAGES = (227 * 1024 - 1280 - STG_TOTAL) / STAGE_BYTES;
     static constexpr int STAGES = MAX_STAGES > 6 ? 6 : MAX_STAGES;
     static constexpr int TOTAL = STAGES * STAGE_BYTES + STG_TOTAL + 1024 /*alignment slack*/ + 256 /*barriers*/;
@@ -116,9 +117,25 @@ struct PairTail {
     float *partial = nullptr;  // [slots][MT][256]
 };
 
+// g / (1 + e^-g) in f32. The fast quotient (within 2 ulp) with one step of iterative refinement: its residual, exact in an fma,
+// divided again. The `/` operator costs a range check and a branch for each of a thread's 128 values, which then run one after
+// the other (75 us -> 67 us at 2048 x 896 -> 2 x 4864). The range is known here: 1 <= d, and below g = -80 d is held
+// at e^80: that quotient is under 1e-32 and 0 in fp16 either way.
+__device__ __forceinline__ float silu(float g)
+{
+    const float d = 1.f + expf(fminf(-g, 80.f));
+    const float q = __fdividef(g, d);
+    return g == INFINITY ? g : q + __fdividef(fmaf(-q, d, g), d);
+}
+
 // GATHER: the result goes to the placement in Params (this GPU's slab and its peers', row pitch ld_out) from registers.
-template <int MT, bool SPLIT, bool STG, bool GATHER = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS_PAIR, 1)
+// SILU: the weight is gate | up (N = 2 I columns) and the result is fp16 silu(gate) * up, [M, I] (siluMulRef,
+// src/reference/qwen-ref.ts:119-123), the input of the down projection. A CTA's 128 weight columns are 64 of gate and the same 64
+// of up, so both factors of a value end up in its own tensor memory; the epilogue warps exchange them through shared memory, half
+// of the rows each way, and compute in f32 what a pass over the f32 result would. At 2048 x 896 -> 2 x 4864 that pass moved
+// 100 MB and took 18 us, and the GEMM itself stored 80 MB instead of 20.
+template <int MT, bool SPLIT, bool STG, bool GATHER = false, bool SILU = false>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(STG), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                  const __grid_constant__ CUtensorMap map_c, const Params p, const int tiles_m, const int tiles_n, const int n_items,
                  const int use_tma_store, const PairTail tail)
@@ -131,7 +148,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     static_assert(USED <= 512 && MT % STG_ROWS == 0 && MT >= 128, "token tile");
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t *stg = smem + STAGES * S::STAGE_BYTES;  // two epilogue staging tiles
+    uint8_t *stg = smem + STAGES * S::STAGE_BYTES;  // two epilogue staging tiles per group
     uint64_t *bars = (uint64_t *)(stg + S::STG_TOTAL);
     uint64_t *full_w = bars, *ready = bars + STAGES, *empty = bars + 2 * STAGES;
     uint64_t *acc_full = bars + 3 * STAGES, *acc_empty = bars + 3 * STAGES + 2;
@@ -152,7 +169,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     auto item_index = [&](int ti) { return is_tail(ti) ? tail.rounds * n_pairs + pair / tail.St : pair + ti * n_pairs; };
     auto item_slice = [&](int ti) { return item_index(ti) / tiles_mn; };
     auto item_m0 = [&](int ti) { return (item_index(ti) % tiles_mn % tiles_m) * MT; };
-    auto item_n0 = [&](int ti) { return (item_index(ti) % tiles_mn / tiles_m) * (2 * BN) + (int)rank * BN; };
+    constexpr int CTA_COLS = SILU ? BN / 2 : BN;  // output columns of a CTA's item
+    auto item_n0 = [&](int ti) { return (item_index(ti) % tiles_mn / tiles_m) * (2 * CTA_COLS) + (int)rank * CTA_COLS; };
+    auto weight_col = [&](int n0, int i) { return SILU && i >= CTA_COLS ? p.N / 2 + n0 + i - CTA_COLS : n0 + i; };  // of accumulator lane i
+    auto load_weights = [&](int s, int n0, int row, uint64_t *bar) {
+        uint8_t *dst = smem + s * S::STAGE_BYTES + S::X_BYTES + S::WD_BYTES;
+        tma_load_2d(dst, &map_w, n0, row, bar);
+        if constexpr (SILU) tma_load_2d(dst + S::WP_BYTES / 2, &map_w, weight_col(n0, CTA_COLS), row, bar);
+    };
     auto item_kb0 = [&](int ti) { return SPLIT ? item_slice(ti) * p.kb_per_slice : is_tail(ti) ? (pair % tail.St) * tail.per : 0; };
     auto item_kbn = [&](int ti) {
         if (!SPLIT && !is_tail(ti)) return KB;
@@ -163,7 +187,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 
     auto xs = [&](int s) { return smem + s * S::STAGE_BYTES; };
     auto wd = [&](int s) { return smem + s * S::STAGE_BYTES + S::X_BYTES; };
-    auto wp = [&](int s) { return (uint32_t *)(smem + s * S::STAGE_BYTES + S::X_BYTES + S::WD_BYTES); };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
@@ -173,7 +196,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 2 * EPI_WARPS);
+            mbar_init(&acc_empty[b], 2 * 4 * epi_groups(STG));
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -201,7 +224,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 const int n0 = item_n0(ti), kb0 = item_kb0(ti), kbn = item_kbn(ti);
                 for (int kb = 0; kb < kbn && pre < STAGES; kb++, pre++) {
                     mbar_expect_tx(&full_w[pre], S::WP_BYTES);
-                    tma_load_2d(wp(pre), &map_w, n0, (kb0 + kb) * 8, &full_w[pre]);
+                    load_weights(pre, n0, (kb0 + kb) * 8, &full_w[pre]);
                 }
             }
             pdl_wait();
@@ -213,7 +236,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     if (!ok) break;
                     if (seq >= pre) {
                         mbar_expect_tx(&full_w[s], S::WP_BYTES);
-                        tma_load_2d(wp(s), &map_w, n0, (kb0 + kb) * 8, &full_w[s]);
+                        load_weights(s, n0, (kb0 + kb) * 8, &full_w[s]);
                     }
                     if (rank == 0) mbar_expect_tx(&ready[s], 2 * S::X_BYTES);
                     tma_load_2d_pairbar(xs(s), &map_x, (kb0 + kb) * BK, m0, cluster_map_shared(&ready[s], 0));
@@ -264,7 +287,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         const int kg = (unpack_idx * 32 + lane) / SET_THREADS;
         const int tn = (unpack_idx * 32 + lane) % SET_THREADS;
         const __half2 sixteenth = __float2half2_rn(0.0625f);
-        const int src_off = S::X_BYTES + S::WD_BYTES + tn * 4;
+        // packed words of this column: rows of 128 (or, in two boxes of gate and up, 64) words
+        const int src_off = S::X_BYTES + S::WD_BYTES + tn * 4 + (SILU && tn >= CTA_COLS ? S::WP_BYTES / 2 - CTA_COLS * 4 : 0);
         int dst_off[8];
 #pragma unroll
         for (int rr = 0; rr < 8; rr++) dst_off[rr] = S::X_BYTES + tn * 128 + ((rr ^ (tn & 7)) << 4);
@@ -279,7 +303,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         int kb0_item = ti < items_cta ? item_kb0(ti) : 0;
         int kabs = kb0_item + kb;  // k-block index in the whole K
         int group = kabs / p.group_blocks;
-        int n = (ti < items_cta ? item_n0(ti) : 0) + tn;
+        int n = weight_col(ti < items_cta ? item_n0(ti) : 0, tn);
         __half next_scale = __float2half_rn(0.f);
         uint32_t next_zeros = 0x77777777u;
         auto request = [&]() {
@@ -312,7 +336,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     if (ti < items_cta) kbn = item_kbn(ti);
                 }
                 if (ti < items_cta) {
-                    if (ti != old_ti) n = item_n0(ti) + tn, kb0_item = item_kb0(ti);
+                    if (ti != old_ti) n = weight_col(item_n0(ti), tn), kb0_item = item_kb0(ti);
                     kabs = kb0_item + kb;
                     group = gshift >= 0 ? kabs >> gshift : kabs / p.group_blocks;
                     if (ti != old_ti || group != old_group) request(), fresh = true;
@@ -324,7 +348,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             const uint32_t *src = (const uint32_t *)(stage + src_off);
 #pragma unroll
             for (int rr = 0; rr < 8; rr++) {
-                uint32_t w = src[rr * BN];
+                uint32_t w = src[rr * CTA_COLS];
                 const uint32_t lo0 = (w & 0x000f000fu) | 0x64006400u;
                 const uint32_t hi0 = (w & 0x00f000f0u) | 0x64006400u;
                 w >>= 8;
@@ -351,7 +375,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
     } else if (warp >= WARPS) {
         // ------------------------------------------------------------------ epilogue: warp w drains TMEM lanes 32 * (w % 4) ..
-        const int q = warp & 3;
+        constexpr int GROUPS = epi_groups(STG);
+        const int q = warp & 3, eg = (warp - WARPS) >> 2;
+        const int epi_tid = (warp - WARPS) * 32 + lane - eg * 128;  // 0 .. 127 within the group, thread 0 issues the stores
         const uint32_t acc_empty0 = cluster_map_shared(&acc_empty[0], 0);
         bool ok = true;
         int stg_sel = 0;
@@ -359,11 +385,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         for (int ti = 0; ti < items_cta && ok; ti++) {
             const int buf = ti & 1, use = ti >> 1;
             ok = mbar_wait_idle(&acc_full[buf], (uint32_t)use & 1u, abort_flag, p.status, 5);
-            // the four warps meet at barriers below: they go on together or not at all
+            // the four warps of a group meet at barriers below: they go on together or not at all
             {
                 uint32_t all;
-                asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                             : "=r"(all) : "r"((uint32_t)ok) : "memory");
+                asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                             : "=r"(all) : "r"((uint32_t)ok), "r"(eg + 1) : "memory");
                 ok = all != 0;
             }
             if (!ok) break;
@@ -386,12 +412,53 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             const int n_warp = n0 + q * 32;
             const int n = n_warp + lane;
             const float bias = (!SPLIT && p.bias && n < p.N) ? p.bias[n] : 0.f;
-            if (is_tail(ti)) {
+            auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(eg + 1) : "memory"); };
+            if constexpr (SILU) {
+                // 32 token rows at a time. Of the CTA's 64 columns warps 0, 1 hold gate and 2, 3 up: gate goes to the exchange
+                // tile for the upper 16 rows, up for the lower 16, then each warp finishes the rows whose other factor it was
+                // given. (A group's barrier after the products also says that the exchange tile has been read.)
+                const int col = (q & 1) * 32 + lane;
+                const bool is_up = q >= 2;
+                uint8_t *mine = stg + eg * 2 * STG_BYTES;
+                float *ex = (float *)mine;  // [32 rows][64 columns]
+                auto rows16 = [&](int c, auto &&f) {
+                    uint32_t r[16];
+                    tmem_ld_32x32b_x16(acc + (uint32_t)c, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; j++) f(j, __uint_as_float(r[j]));
+                };
+                const int give = is_up ? 0 : 16, keep = 16 - give;
+#pragma unroll 1
+                for (int c = eg * STG_ROWS; c < MT; c += GROUPS * STG_ROWS) {
+                    __half *tile = (__half *)(mine + STG_BYTES) + stg_sel * STG_ROWS * 64;  // [32 rows][64 columns], two of them
+                    rows16(c + give, [&](int j, float v) { ex[(give + j) * 64 + col] = v; });
+                    if (epi_tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                    group_sync();
+                    float o[16];  // all at once: a load from ex would not be moved over a store to the tile
+#pragma unroll
+                    for (int j = 0; j < 16; j++) o[j] = ex[(keep + j) * 64 + col];
+                    rows16(c + keep, [&](int j, float v) {
+                        const float g = is_up ? o[j] : v, u = is_up ? v : o[j];
+                        tile[(keep + j) * 64 + col] = __float2half_rn(silu(g) * u);
+                    });
+                    fence_async_smem();
+                    group_sync();
+                    if (epi_tid == 0) {
+                        if (m0 + c < p.M && n0 < p.N / 2)
+                            asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];"
+                                         ::"l"(&map_c), "r"(n0), "r"(m0 + c), "r"(0), "r"(smem_u32(tile))
+                                         : "memory");
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    }
+                    stg_sel ^= 1;
+                }
+            } else if (is_tail(ti)) {
                 // a K slice of a leftover item: the f32 partial tile [MT][256] of this pair, no bias
                 StoreDst dt;
                 dt.dst[0] = tail.partial + (size_t)pair * MT * (2 * BN), dt.n_dst = 1, dt.ld = 2 * BN, dt.col0 = 0;
 #pragma unroll 1
-                for (int c = 0; c < MT; c += 16) {
+                for (int c = eg * 16; c < MT; c += GROUPS * 16) {
                     uint32_t r[16];
                     tmem_ld_32x32b_x16(acc + (uint32_t)c, r);
                     tmem_ld_wait();
@@ -399,7 +466,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 }
             } else if (!STG || !use_tma_store) {
 #pragma unroll 1
-                for (int c = 0; c < MT; c += 16) {
+                for (int c = eg * 16; c < MT; c += GROUPS * 16) {
                     uint32_t r[16];
                     tmem_ld_32x32b_x16(acc + (uint32_t)c, r);
                     tmem_ld_wait();
@@ -408,18 +475,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             } else {
                 // The result leaves through shared memory: a lane holds one output column of 16 token rows, so it writes
                 // 16 words into a [tokens][128 columns] staging tile (no exchange between lanes, no dependent chain), and
-                // one thread hands each finished tile to a TMA store, which also clips the ragged edges. A tile is 16 KB:
-                // 64 token rows of fp16 or 32 of f32 (also the partial sums of a K slice, third map coordinate). Two tiles
-                // alternate; a tile is rewritten once the store that read it has finished reading.
-                const int epi_tid = (warp - WARPS) * 32 + lane;  // 0 .. 127, thread 0 issues the stores
+                // one thread hands each finished tile to a TMA store, which also clips the ragged edges. A tile is 8 KB:
+                // 32 token rows of fp16 or 16 of f32 (also the partial sums of a K slice, third map coordinate). Two tiles
+                // of a group alternate; a tile is rewritten once the store that read it has finished reading.
                 const bool o16 = !SPLIT && out16;
                 const int rows = o16 ? STG_ROWS : STG_ROWS / 2;
                 const int slice = SPLIT ? item_slice(ti) : 0;
 #pragma unroll 1
-                for (int c = 0; c < MT; c += rows) {
+                for (int c = eg * rows; c < MT; c += GROUPS * rows) {
                     if (epi_tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
-                    uint8_t *tile_base = stg + stg_sel * STG_BYTES;
+                    group_sync();
+                    uint8_t *tile_base = stg + (eg * 2 + stg_sel) * STG_BYTES;
 #pragma unroll 1
                     for (int cc = 0; cc < rows; cc += 16) {
                         uint32_t r[16];
@@ -436,7 +502,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         }
                     }
                     fence_async_smem();
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    group_sync();
                     if (epi_tid == 0) {
                         if (m0 + c < p.M && n0 < p.N)
                             asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];"
@@ -453,7 +519,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (lane == 0) mbar_arrive_cluster(acc_empty0 + (uint32_t)buf * 8u);
         }
         // the staging tiles must outlive the stores that read them
-        if (warp == WARPS && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        if (epi_tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
@@ -527,29 +593,30 @@ bool gemm_pair_supports(const Weight &w, int64_t M)
 
 template <int MT>
 static cudaError_t launch_pair_mt(const CUtensorMap &mx, const CUtensorMap &mw, const CUtensorMap *mc, const tc::Params &p, int tiles_m,
-                                  int tiles_n, int S, cudaStream_t st, int sms, const tcp::PairTail &tail)
+                                  int tiles_n, int S, cudaStream_t st, int sms, const tcp::PairTail &tail, bool silu)
 {
-    static bool attr_set[5][16] = {};
+    static bool attr_set[6][16] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     const int n_items = tiles_m * tiles_n * S;
     int pairs = sms / 2;
     if (pairs > n_items) pairs = n_items;
-    auto go = [&](auto kernel, int variant, int smem) -> cudaError_t {
+    auto go = [&](auto kernel, int variant, int smem, bool stg) -> cudaError_t {
         if (!(dev >= 0 && dev < 16 && attr_set[variant][dev])) {
             cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return e;
             if (dev >= 0 && dev < 16) attr_set[variant][dev] = true;
         }
-        return launch_pdl(kernel, dim3((unsigned)(2 * pairs)), dim3(tcp::THREADS_PAIR), (size_t)smem, st, mx, mw, mc ? *mc : mx, p, tiles_m,
+        return launch_pdl(kernel, dim3((unsigned)(2 * pairs)), dim3((unsigned)tcp::pair_threads(stg)), (size_t)smem, st, mx, mw, mc ? *mc : mx, p, tiles_m,
                           tiles_n, n_items, mc ? 1 : 0, tail);
     };
+    if (silu) return go(tcp::gemm_pair_kernel<MT, false, true, false, true>, 5, tcp::SmemPair<MT, true>::TOTAL, true);
     if (S > 1)
-        return mc ? go(tcp::gemm_pair_kernel<MT, true, true>, 3, tcp::SmemPair<MT, true>::TOTAL)
-                  : go(tcp::gemm_pair_kernel<MT, true, false>, 1, tcp::SmemPair<MT, false>::TOTAL);
-    if (p.n_dst > 0) return go(tcp::gemm_pair_kernel<MT, false, false, true>, 4, tcp::SmemPair<MT, false>::TOTAL);
-    if (mc) return go(tcp::gemm_pair_kernel<MT, false, true>, 2, tcp::SmemPair<MT, true>::TOTAL);
-    return go(tcp::gemm_pair_kernel<MT, false, false>, 0, tcp::SmemPair<MT, false>::TOTAL);
+        return mc ? go(tcp::gemm_pair_kernel<MT, true, true>, 3, tcp::SmemPair<MT, true>::TOTAL, true)
+                  : go(tcp::gemm_pair_kernel<MT, true, false>, 1, tcp::SmemPair<MT, false>::TOTAL, false);
+    if (p.n_dst > 0) return go(tcp::gemm_pair_kernel<MT, false, false, true>, 4, tcp::SmemPair<MT, false>::TOTAL, false);
+    if (mc) return go(tcp::gemm_pair_kernel<MT, false, true>, 2, tcp::SmemPair<MT, true>::TOTAL, true);
+    return go(tcp::gemm_pair_kernel<MT, false, false>, 0, tcp::SmemPair<MT, false>::TOTAL, false);
 }
 
 // mc: tensor map of the result or of the K slices' partial sums ([slices, M, N], boxes of 128 columns x 64 fp16 or 32 f32
@@ -558,7 +625,7 @@ static cudaError_t launch_pair_mt(const CUtensorMap &mx, const CUtensorMap &mw, 
 // tail_partial: room for sms / 2 partial tiles [mt][256] f32 (the launch cuts its last round along K where that pays, and
 // then also launches the small kernel that adds the slices; *extra_launches says so), or nullptr to never cut.
 cudaError_t launch_gemm_pair(int mt, const CUtensorMap &mx, const CUtensorMap &mw, const CUtensorMap *mc, const tc::Params &p, int tiles_m,
-                             int tiles_n, int S, cudaStream_t st, int sms, float *tail_partial, int *extra_launches)
+                             int tiles_n, int S, cudaStream_t st, int sms, float *tail_partial, int *extra_launches, bool silu)
 {
     tcp::PairTail tail;
     int rem = 0;
@@ -570,9 +637,9 @@ cudaError_t launch_gemm_pair(int mt, const CUtensorMap &mx, const CUtensorMap &m
     }
     cudaError_t e;
     switch (mt) {
-    case 128: e = launch_pair_mt<128>(mx, mw, mc, p, tiles_m, tiles_n, S, st, sms, tail); break;
-    case 192: e = launch_pair_mt<192>(mx, mw, mc, p, tiles_m, tiles_n, S, st, sms, tail); break;
-    default: e = launch_pair_mt<256>(mx, mw, mc, p, tiles_m, tiles_n, S, st, sms, tail); break;
+    case 128: e = launch_pair_mt<128>(mx, mw, mc, p, tiles_m, tiles_n, S, st, sms, tail, silu); break;
+    case 192: e = launch_pair_mt<192>(mx, mw, mc, p, tiles_m, tiles_n, S, st, sms, tail, silu); break;
+    default: e = launch_pair_mt<256>(mx, mw, mc, p, tiles_m, tiles_n, S, st, sms, tail, silu); break;
     }
     if (e != cudaSuccess || tail.slots == 0) return e;
     *extra_launches = 1;

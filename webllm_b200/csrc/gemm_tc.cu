@@ -731,7 +731,7 @@ static int make_map_2d(wb_context *ctx, CUtensorMap *map, CUtensorMapDataType dt
 // gemm_pair.cu
 bool gemm_pair_supports(const Weight &w, int64_t M);
 cudaError_t launch_gemm_pair(int mt, const CUtensorMap &mx, const CUtensorMap &mw, const CUtensorMap *mc, const tc::Params &p, int tiles_m,
-                             int tiles_n, int S, cudaStream_t st, int sms, float *tail_partial, int *extra_launches);
+                             int tiles_n, int S, cudaStream_t st, int sms, float *tail_partial, int *extra_launches, bool silu);
 bool pair_tail_plan(int64_t n_items, int pairs, int kblocks, int *rounds, int *rem, int *St, int *per);
 
 bool gemm_tc_supports(const Weight &w, int64_t M)
@@ -862,7 +862,7 @@ int plan_gemm_tc(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int
             plan->grid_x = (int)((M + pmt - 1) / pmt);
             plan->grid_y = (int)((w.N + 255) / 256);
             plan->split_k = plan->grid_z = pS;
-            plan->block = 800;
+            plan->block = pmt < 256 || (kblocks + pS - 1) / pS <= kPairStageKb ? 928 : 800;  // staged results: eight epilogue warps
             plan->tile_m = pmt;
             plan->tile_n = 256;
             mt = pmt, nh = 2, S = pS;
@@ -1022,7 +1022,7 @@ int launch_gemm_tc(wb_context *ctx, const Weight &w, const void *A, void *C, con
                 cc.base = nullptr;
                 cuuint64_t dims[3] = {(cuuint64_t)w.N, (cuuint64_t)M, (cuuint64_t)S};
                 cuuint64_t strides[2] = {(cuuint64_t)w.N * (c16 ? 2 : 4), (cuuint64_t)w.N * M * (c16 ? 2 : 4)};
-                cuuint32_t box[3] = {(cuuint32_t)tc::BN, c16 ? 64u : 32u, 1u};
+                cuuint32_t box[3] = {(cuuint32_t)tc::BN, c16 ? (cuuint32_t)tc::STG_ROWS : (cuuint32_t)tc::STG_ROWS / 2, 1u};
                 cuuint32_t estr[3] = {1, 1, 1};
                 CUresult r = ((EncodeTiledFn)ctx->tmap_encode)(&mc, c16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                                                                cbase, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1033,7 +1033,7 @@ int launch_gemm_tc(wb_context *ctx, const Weight &w, const void *A, void *C, con
             }
             int extra = 0;
             e = launch_gemm_pair(mt, mx, mw, tma_store ? &mc : nullptr, p, plan.grid_x, plan.grid_y, S, ctx->stream, ctx->sm_count,
-                                 S == 1 ? p.partial : nullptr, &extra);
+                                 S == 1 ? p.partial : nullptr, &extra, false);
             ctx->launches += (uint64_t)extra;
         } else {
             e = launch_tc_mt<false>(mt, nh, mx, mw, p, grid, ctx->stream, ctx->sm_count);
@@ -1059,6 +1059,51 @@ int launch_gemm_tc(wb_context *ctx, const Weight &w, const void *A, void *C, con
         ctx->launches++;
         WB_CUDA(cudaGetLastError());
     }
+    return WB_OK;
+}
+
+int launch_gate_up_silu(wb_context *ctx, const Weight &w, const __half *A, __half *act, int64_t M, bool *done)
+{
+    *done = false;
+    const int64_t I = w.N / 2;
+    if (w.kind != WeightKind::Gptq || ctx->force_kernel != 0 || ctx->place.n_dst != 0 || I % tc::BN != 0) return WB_OK;
+    wb_plan plan;
+    WB_CHECK(plan_linear(ctx, w, M, WB_F16, 0, &plan));
+    if (plan.kernel != WB_KERNEL_GEMM_TC_PAIR || plan.split_k > 1) return WB_OK;
+    const char *base = ctx->arena[WB_ARENA_WEIGHTS].base;
+    const int mt = plan.tile_m;
+    CallMap &cx = w.tmap_x, &cc = w.tmap_c;
+    CUtensorMap &mx = *reinterpret_cast<CUtensorMap *>(cx.map.bytes), &mc = *reinterpret_cast<CUtensorMap *>(cc.map.bytes);
+    TmapSlot &ws = w.tmap_tc[2];
+    CUtensorMap &mw = *reinterpret_cast<CUtensorMap *>(ws.bytes);
+    if (cx.base != A || cx.M != M || cx.a != mt / 2) {
+        cx.base = nullptr;
+        WB_CHECK(make_map_2d(ctx, &mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, A, (uint64_t)w.K, (uint64_t)M, tc::BK, (uint32_t)(mt / 2), true));
+        cx.base = A, cx.M = M, cx.a = mt / 2;
+    }
+    if (!ws.ok) WB_CHECK(make_map_2d(ctx, &mw, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, base + w.off_main, (uint64_t)w.N, (uint64_t)w.pack_rows, tc::BN / 2, 8, false));
+    ws.ok = true;
+    if (cc.base != act || cc.M != M || cc.a != -1) {
+        cc.base = nullptr;
+        cuuint64_t dims[3] = {(cuuint64_t)I, (cuuint64_t)M, 1}, strides[2] = {(cuuint64_t)I * 2, (cuuint64_t)I * M * 2};
+        cuuint32_t box[3] = {tc::BN / 2, tc::STG_ROWS, 1}, estr[3] = {1, 1, 1};
+        const CUresult r = ((EncodeTiledFn)ctx->tmap_encode)(&mc, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, act, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                                             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return fail(WB_ERR_CUDA, "cuTensorMapEncodeTiled (result) failed with code %d", (int)r);
+        cc.base = act, cc.M = M, cc.a = -1;
+    }
+    tc::Params p;
+    p.out = act, p.bias = nullptr, p.status = ctx->status_word;
+    p.M = (int)M, p.N = (int)w.N, p.K = (int)w.K, p.out_f16 = 1;
+    p.kb_per_slice = (int)(w.K / tc::BK), p.partial = nullptr, p.ld_out = 0, p.col0 = 0, p.n_dst = 0;
+    for (int g = 0; g < kMaxGatherDst; g++) p.dst[g] = nullptr;
+    p.qz = w.has_zeros ? (const uint32_t *)(base + w.off_zeros) : nullptr, p.sc = (const __half *)(base + w.off_scales);
+    p.zcols = (int)w.zcols, p.group_blocks = (int)(w.group / 64);
+    int extra = 0;
+    const cudaError_t e = launch_gemm_pair(mt, mx, mw, &mc, p, plan.grid_x, (int)(I / tc::BN), 1, ctx->stream, ctx->sm_count, nullptr, &extra, true);
+    ctx->launches++;
+    WB_CUDA(e);
+    *done = true;
     return WB_OK;
 }
 

@@ -197,16 +197,24 @@ int forward_impl(wb_qwen *m, const Bufs &b, int64_t M, int64_t B, int64_t T, int
         float *xa = (x == b.x ? b.xa : b.x);
         WB_CHECK(op_rmsnorm(ctx, x, b.proj, xa, f32w(L.post_norm), b.n, (int)M, C, m->cfg.rms_eps, half_in ? b.h16 : nullptr));
         x = xa;
+        const __half *down_in = b.h16;
         if (L.gate_up >= 0) {
-            if (half_in) WB_CHECK(linear_h16(m, L.gate_up, b.h16, b.gu, -1, M));
-            else WB_CHECK(linear(m, L.gate_up, b.n, b.gu, -1, M, L.down));
-            WB_CHECK(op_silu_mul(ctx, b.gu, b.gu + I, b.act, (int)M, I, 2 * I, half_in ? b.h16 : nullptr));
+            // (the fused kernel reads h16, so its own result goes where gate | up would)
+            bool silu_done = false;
+            if (half_in) WB_CHECK(launch_gate_up_silu(ctx, ctx->weights[L.gate_up], b.h16, reinterpret_cast<__half *>(b.gu), M, &silu_done));
+            if (silu_done) {
+                down_in = reinterpret_cast<const __half *>(b.gu);
+            } else {
+                if (half_in) WB_CHECK(linear_h16(m, L.gate_up, b.h16, b.gu, -1, M));
+                else WB_CHECK(linear(m, L.gate_up, b.n, b.gu, -1, M, L.down));
+                WB_CHECK(op_silu_mul(ctx, b.gu, b.gu + I, b.act, (int)M, I, 2 * I, half_in ? b.h16 : nullptr));
+            }
         } else {
             WB_CHECK(linear(m, L.gate, b.n, b.gu, -1, M));
             WB_CHECK(linear(m, L.up, b.n, b.gu + M * I, -1, M));
             WB_CHECK(op_silu_mul(ctx, b.gu, b.gu + M * I, b.act, (int)M, I, I));
         }
-        if (half_in) WB_CHECK(linear_h16(m, L.down, b.h16, b.proj, -1, M));
+        if (half_in) WB_CHECK(linear_h16(m, L.down, down_in, b.proj, -1, M));
         else WB_CHECK(linear(m, L.down, b.act, b.proj, -1, M, i + 1 < m->cfg.n_layer ? m->layers[i + 1].qkv : -1));
         delta = b.proj;
     }
