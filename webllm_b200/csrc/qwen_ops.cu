@@ -199,6 +199,50 @@ __global__ void rope_kv_kernel(float *__restrict__ q, float *__restrict__ k, con
     }
 }
 
+// The same, four neighbouring dims (and their partners half a head away) per thread: D a multiple of 8, rows and pitches 16-byte
+// aligned. Bound by the 18 MB it moves at 2048 x 18 heads; one pair per thread spent its time on index arithmetic: 9.7 -> 6.0 us.
+__device__ __forceinline__ void put4(float *p, const float4 &v) { *reinterpret_cast<float4 *>(p) = v; }
+__device__ __forceinline__ void put4(__half *p, const float4 &v)
+{
+    const __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
+    uint2 o;
+    o.x = *reinterpret_cast<const uint32_t *>(&a), o.y = *reinterpret_cast<const uint32_t *>(&b);
+    *reinterpret_cast<uint2 *>(p) = o;
+}
+template <typename KV>
+__global__ void __launch_bounds__(256) rope_kv_vec4_kernel(float *__restrict__ q, float *__restrict__ k, const float *__restrict__ v,
+                                                           KV *__restrict__ k_cache, KV *__restrict__ v_cache, const float *__restrict__ cs_table,
+                                                           int M, int H, int KVH, int D, int T, const int *__restrict__ pos_offset_ptr,
+                                                           int pos_offset_imm, int ldq, int ldk, int ldv)
+{
+    pdl_sync();
+    const int half = D >> 1, pieces = half >> 2, per_row = (H + 2 * KVH) * pieces;
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= M * per_row) return;
+    const int row = idx / per_row, rem = idx - row * per_row, hh = rem / pieces, i = (rem - hh * pieces) * 4;
+    const int pos_offset = pos_offset_ptr ? *pos_offset_ptr : pos_offset_imm, pos = row % T + pos_offset;
+    const bool is_v = hh >= H + KVH;
+    if (is_v && !v_cache) return;
+    const int head = hh < H ? hh : is_v ? hh - H - KVH : hh - H;
+    float *src = hh < H ? q + (int64_t)row * ldq + head * D : is_v ? const_cast<float *>(v) + (int64_t)row * ldv + head * D : k + (int64_t)row * ldk + head * D;
+    float4 a = *reinterpret_cast<const float4 *>(src + i), b = *reinterpret_cast<const float4 *>(src + i + half);
+    if (!is_v) {
+        const float4 *cs = reinterpret_cast<const float4 *>(cs_table + ((int64_t)pos * half + i) * 2);
+        const float4 c0 = cs[0], c1 = cs[1];  // cos, sin of i, i + 1 and of i + 2, i + 3
+        const float4 x = a, y = b;
+        a.x = x.x * c0.x - y.x * c0.y, b.x = x.x * c0.y + y.x * c0.x;
+        a.y = x.y * c0.z - y.y * c0.w, b.y = x.y * c0.w + y.y * c0.z;
+        a.z = x.z * c1.x - y.z * c1.y, b.z = x.z * c1.y + y.z * c1.x;
+        a.w = x.w * c1.z - y.w * c1.w, b.w = x.w * c1.w + y.w * c1.z;
+    }
+    if (hh < H || (!is_v && !k_cache)) {
+        put4(src + i, a), put4(src + i + half, b);
+    } else {
+        KV *dst = (is_v ? v_cache : k_cache) + ((int64_t)(pos_offset + row) * KVH + head) * D;
+        put4(dst + i, a), put4(dst + i + half, b);
+    }
+}
+
 __device__ __forceinline__ float kv_load(const float *p) { return *p; }
 __device__ __forceinline__ float kv_load(const __half *p) { return __half2float(*p); }
 
@@ -636,6 +680,14 @@ int op_rope_kv(wb_context *ctx, float *q, float *k, const float *v, void *k_cach
                int ldk, int ldv)
 {
     const int64_t n = (int64_t)M * (H + 2 * KVH) * (D / 2);
+    if (D % 8 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && ldv % 4 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0 && n / 4 < (1 << 30)) {
+        const dim3 grid((unsigned)((n / 4 + 255) / 256));
+        WB_CUDA(kv_f16 ? launch_pdl(rope_kv_vec4_kernel<__half>, grid, dim3(256), 0, ctx->stream, q, k, v, (__half *)k_cache, (__half *)v_cache, cs_table, M,
+                                    H, KVH, D, T, pos_ptr, pos_imm, ldq, ldk, ldv)
+                       : launch_pdl(rope_kv_vec4_kernel<float>, grid, dim3(256), 0, ctx->stream, q, k, v, (float *)k_cache, (float *)v_cache, cs_table, M, H,
+                                    KVH, D, T, pos_ptr, pos_imm, ldq, ldk, ldv));
+        LAUNCH_OK(ctx);
+    }
     const unsigned blocks = (unsigned)((n + 255) / 256);
     if (kv_f16)
         WB_CUDA(launch_pdl(rope_kv_kernel<__half>, dim3(blocks), dim3(256), 0, ctx->stream, q, k, v, (__half *)k_cache, (__half *)v_cache, cs_table, M, H,
