@@ -132,6 +132,9 @@ struct wb_context {
     int force_kernel = 0, force_split = 0;
     int prefetch_weight = -1;        // index of the weight the next linear should pull into L2 (-1: none)
     void *tmap_encode = nullptr;     // cuTensorMapEncodeTiled, resolved at context creation
+    bool keep_slices = false;        // the next tensor-core call may leave its K slices unadded (model forward; set per call)
+    const float *slices = nullptr;   // ... and says here that it did: `n_slices` partial sums, [M, N] f32 each
+    int n_slices = 0;
     wb::OutPlace place;              // set for the duration of one wb_linear_gather call (n_dst > 0)
     bool capturing = false;          // a command batch is being recorded (batch.cu)
     uint64_t launches_at_capture = 0;

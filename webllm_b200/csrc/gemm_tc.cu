@@ -1048,6 +1048,10 @@ int launch_gemm_tc(wb_context *ctx, const Weight &w, const void *A, void *C, con
     }
     ctx->launches++;
     WB_CUDA(e);
+    if (S > 1 && ctx->keep_slices && !bias && out_dtype == WB_F32 && ctx->place.n_dst == 0 && w.N % 4 == 0) {
+        ctx->slices = p.partial, ctx->n_slices = S;
+        return WB_OK;
+    }
     if (S > 1) {
         const int64_t MN = M * w.N;
         if (w.N % 4 == 0 && place.ld % 4 == 0 && place.col0 % 4 == 0)

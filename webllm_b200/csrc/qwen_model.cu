@@ -119,6 +119,15 @@ int forward_impl(wb_qwen *m, const Bufs &b, int64_t M, int64_t B, int64_t T, int
 
     WB_CHECK(op_embed(ctx, (const __half *)(wbase + ctx->weights[m->embed].off_main), b.tokens, b.x, (int)M, C, m->V));
     const float *delta = nullptr;  // pending residual contribution, folded into the next rmsnorm
+    int slices = 1;                // ... as so many partial sums, M * C floats apart
+    // o and down feed nothing but the residual add of the next rmsnorm: where they run cut along K, that adds their slices
+    auto to_residual = [&](int rc) -> int {
+        ctx->keep_slices = false;
+        delta = b.proj, slices = 1;
+        if (ctx->slices) delta = ctx->slices, slices = ctx->n_slices, ctx->slices = nullptr;
+        return rc;
+    };
+    const bool may_slice = op_rmsnorm_slices_ok((int)M, C);
     float *x = b.x;                // residual stream before `delta` is added
     // A decode step over fused int4 projections runs five kernels per layer: the norms, silu * up and the rotary
     // embedding + cache append ride inside the projections and the attention kernel (see GemvPrologue).
@@ -161,7 +170,7 @@ int forward_impl(wb_qwen *m, const Bufs &b, int64_t M, int64_t B, int64_t T, int
         // the activations fewer per projection). Only where the fused projections exist (one consumer per producer).
         const bool half_in = !m->exact && b.h16 != nullptr && L.qkv >= 0 && L.gate_up >= 0;
         float *x_in = (delta ? (x == b.x ? b.xa : b.x) : x);
-        WB_CHECK(op_rmsnorm(ctx, x, delta, x_in, f32w(L.in_norm), b.n, (int)M, C, m->cfg.rms_eps, half_in ? b.h16 : nullptr));
+        WB_CHECK(op_rmsnorm(ctx, x, delta, x_in, f32w(L.in_norm), b.n, (int)M, C, m->cfg.rms_eps, half_in ? b.h16 : nullptr, slices, M * C));
         x = x_in;
         if (L.qkv >= 0) {
             if (half_in) WB_CHECK(linear_h16(m, L.qkv, b.h16, b.q, L.qkvb, M));
@@ -191,11 +200,11 @@ int forward_impl(wb_qwen *m, const Bufs &b, int64_t M, int64_t B, int64_t T, int
         } else {
             WB_CHECK(op_attention(ctx, b.q, b.k, b.v, 0, b.att, (int)M, H, KVH, D, (int)T, nullptr, 0, 0, (int)T, b.ldq, b.ldk));
         }
-        if (att_half) WB_CHECK(linear_h16(m, L.o, b.h16, b.proj, -1, M));
-        else WB_CHECK(linear(m, L.o, b.att, b.proj, -1, M, L.gate_up));
+        ctx->keep_slices = may_slice;
+        WB_CHECK(to_residual(att_half ? linear_h16(m, L.o, b.h16, b.proj, -1, M) : linear(m, L.o, b.att, b.proj, -1, M, L.gate_up)));
         // --- MLP sub-layer: xa = x + proj; n = rmsnorm(xa)
         float *xa = (x == b.x ? b.xa : b.x);
-        WB_CHECK(op_rmsnorm(ctx, x, b.proj, xa, f32w(L.post_norm), b.n, (int)M, C, m->cfg.rms_eps, half_in ? b.h16 : nullptr));
+        WB_CHECK(op_rmsnorm(ctx, x, delta, xa, f32w(L.post_norm), b.n, (int)M, C, m->cfg.rms_eps, half_in ? b.h16 : nullptr, slices, M * C));
         x = xa;
         const __half *down_in = b.h16;
         if (L.gate_up >= 0) {
@@ -214,18 +223,18 @@ int forward_impl(wb_qwen *m, const Bufs &b, int64_t M, int64_t B, int64_t T, int
             WB_CHECK(linear(m, L.up, b.n, b.gu + M * I, -1, M));
             WB_CHECK(op_silu_mul(ctx, b.gu, b.gu + M * I, b.act, (int)M, I, I));
         }
-        if (half_in) WB_CHECK(linear_h16(m, L.down, down_in, b.proj, -1, M));
-        else WB_CHECK(linear(m, L.down, b.act, b.proj, -1, M, i + 1 < m->cfg.n_layer ? m->layers[i + 1].qkv : -1));
-        delta = b.proj;
+        ctx->keep_slices = may_slice;
+        WB_CHECK(to_residual(half_in ? linear_h16(m, L.down, down_in, b.proj, -1, M)
+                                     : linear(m, L.down, b.act, b.proj, -1, M, i + 1 < m->cfg.n_layer ? m->layers[i + 1].qkv : -1)));
     }
     // final norm (+ the last residual add), then the tied lm_head
     float *xf = (x == b.x ? b.xa : b.x);
     if (last_only) {
         const int64_t r = M - 1;
-        WB_CHECK(op_rmsnorm(ctx, x + r * C, delta + r * C, xf, f32w(m->final_norm), b.n, 1, C, m->cfg.rms_eps));
+        WB_CHECK(op_rmsnorm(ctx, x + r * C, delta + r * C, xf, f32w(m->final_norm), b.n, 1, C, m->cfg.rms_eps, nullptr, slices, M * C));
         WB_CHECK(linear(m, m->embed, b.n, b.logits, -1, 1));
     } else {
-        WB_CHECK(op_rmsnorm(ctx, x, delta, xf, f32w(m->final_norm), b.n, (int)M, C, m->cfg.rms_eps));
+        WB_CHECK(op_rmsnorm(ctx, x, delta, xf, f32w(m->final_norm), b.n, (int)M, C, m->cfg.rms_eps, nullptr, slices, M * C));
         WB_CHECK(linear(m, m->embed, b.n, b.logits, -1, M));
     }
     return WB_OK;

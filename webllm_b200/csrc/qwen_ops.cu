@@ -61,10 +61,13 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float *__restrict__ 
     }
 }
 
-// The same for D % 4 == 0, D <= 4096: one pass, the row stays in registers (up to four float4 per thread).
+// The same for D % 4 == 0, D <= 4096: one pass, the row stays in registers (up to four float4 per thread). delta may come as
+// `slices` partial sums, slice_stride floats apart (a projection cut along K whose slices nobody has added up yet): added here,
+// in slice order, they cost neither a launch nor a pass of their own (6 us per 2048-token layer).
 __global__ void __launch_bounds__(256) rmsnorm_vec4_kernel(const float *__restrict__ x, const float *__restrict__ delta,
                                                            float *__restrict__ x_out, const float *__restrict__ w,
-                                                           float *__restrict__ y, __half *__restrict__ y16, int D, float eps)
+                                                           float *__restrict__ y, __half *__restrict__ y16, int D, float eps, int slices,
+                                                           int64_t slice_stride)
 {
     pdl_sync();
     __shared__ float red[8];
@@ -79,7 +82,11 @@ __global__ void __launch_bounds__(256) rmsnorm_vec4_kernel(const float *__restri
         if (i < q) {
             v[u] = *reinterpret_cast<const float4 *>(x + base + 4 * i);
             if (delta) {
-                const float4 d = *reinterpret_cast<const float4 *>(delta + base + 4 * i);
+                float4 d = *reinterpret_cast<const float4 *>(delta + base + 4 * i);
+                for (int s = 1; s < slices; s++) {
+                    const float4 e = *reinterpret_cast<const float4 *>(delta + s * slice_stride + base + 4 * i);
+                    d.x += e.x, d.y += e.y, d.z += e.z, d.w += e.w;
+                }
                 v[u].x += d.x, v[u].y += d.y, v[u].z += d.z, v[u].w += d.w;
                 *reinterpret_cast<float4 *>(x_out + base + 4 * i) = v[u];
             }
@@ -645,13 +652,15 @@ int op_embed(wb_context *ctx, const __half *table, const uint32_t *tokens, float
     LAUNCH_OK(ctx);
 }
 
+bool op_rmsnorm_slices_ok(int M, int D) { return M > 1 && D % 4 == 0 && D <= 4096; }
+
 int op_rmsnorm(wb_context *ctx, const float *x, const float *delta, float *x_out, const float *w, float *y, int M, int D, float eps,
-               __half *y16)
+               __half *y16, int slices, int64_t slice_stride)
 {
     // rows kept in registers where they fit; the summation order inside a thread differs from the scalar kernel's
     // (both are f32 sums of D squares: the difference is rounding noise of the statistic)
-    if (M > 1 && D % 4 == 0 && D <= 4096)
-        WB_CUDA(launch_pdl(rmsnorm_vec4_kernel, dim3(M), dim3(256), 0, ctx->stream, x, delta, x_out, w, y, y16, D, eps));
+    if (op_rmsnorm_slices_ok(M, D) || slices > 1)
+        WB_CUDA(launch_pdl(rmsnorm_vec4_kernel, dim3(M), dim3(256), 0, ctx->stream, x, delta, x_out, w, y, y16, D, eps, slices, slice_stride));
     else
         WB_CUDA(launch_pdl(rmsnorm_kernel, dim3(M), dim3(256), 0, ctx->stream, x, delta, x_out, w, y, y16, D, eps));
     LAUNCH_OK(ctx);

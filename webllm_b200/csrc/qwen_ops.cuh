@@ -7,8 +7,10 @@ namespace wb {
 int op_embed(wb_context *ctx, const __half *table, const uint32_t *tokens, float *x, int M, int C, int vocab);
 // y = rmsnorm(x + delta) * w; when delta != nullptr the sum is also stored to x_out (residual stream).
 // y16 != nullptr: y is not written, the result goes to y16 as fp16 (input of a tensor-core GEMM).
+// delta may be `slices` partial sums slice_stride floats apart (where op_rmsnorm_slices_ok, or D % 4 == 0 and D <= 4096 at M = 1).
 int op_rmsnorm(wb_context *ctx, const float *x, const float *delta, float *x_out, const float *w, float *y, int M, int D, float eps,
-               __half *y16 = nullptr);
+               __half *y16 = nullptr, int slices = 1, int64_t slice_stride = 0);
+bool op_rmsnorm_slices_ok(int M, int D);
 int op_add(wb_context *ctx, const float *a, const float *b, float *out, int64_t n);
 int op_silu_mul(wb_context *ctx, const float *gate, const float *up, float *out, int M, int I, int ld, __half *out16 = nullptr);
 // Rotates q in place and k (into the cache when k_cache != nullptr, else in place); copies v to the cache.
