@@ -34,10 +34,10 @@ def test_f32_attention_tiles(built_lib, oracle, small, B, T):
         model.close()
 
 
-WIDE = synthetic.QwenShape(256, 2, 4, 2, 256, 4992)  # 39 column tiles of 128: the last pair has one only
+WIDE = synthetic.QwenShape(256, 1, 14, 2, 896, 4992)  # K = 896: long enough for the CTA-pair kernel at some hundred rows
 
 
-@pytest.mark.parametrize("n", [300, 384, 513])
+@pytest.mark.parametrize("n", [385, 512, 1025])
 def test_gate_up_silu_in_one_kernel(built_lib, oracle, n):
     """Row counts that leave a token tile ragged, fill it and just pass it; against the same model with gate and up on their own."""
     G = synthetic.random_qwen_gptq(WIDE, seed=12, std=0.05)
