@@ -67,6 +67,16 @@ struct CallMap {
     TmapSlot map;
 };
 
+// The calls of the command batch being recorded since the last point that all later ones wait for.
+struct BatchOrder {
+    struct Op {
+        const char *r0, *r1, *w0, *w1;  // bytes read and written
+        cudaGraphNode_t node = nullptr;
+    };
+    std::vector<Op> ops;
+    std::vector<cudaGraphNode_t> base, left;  // nodes to wait for where no call conflicts; the stream's state after the last call
+};
+
 struct Weight {
     std::string name;
     WeightKind kind;
@@ -137,6 +147,7 @@ struct wb_context {
     int n_slices = 0;
     wb::OutPlace place;              // set for the duration of one wb_linear_gather call (n_dst > 0)
     bool capturing = false;          // a command batch is being recorded (batch.cu)
+    wb::BatchOrder order;            // ... and what its linear calls touch
     uint64_t launches_at_capture = 0;
     void *nccl_comm = nullptr;       // ncclComm_t of the column-sharded group (comm.cu); nullptr until wb_comm_init
     int comm_rank = 0, comm_size = 1;
@@ -180,6 +191,10 @@ struct LinearFusion {
 bool linear_fusion_supported(wb_context *ctx, const Weight &w, int64_t M);
 // gate | up in one projection with silu(gate) * up as its fp16 result (gemm_pair.cu). *done = false: not a shape for that kernel.
 int launch_gate_up_silu(wb_context *ctx, const Weight &w, const __half *A, __half *act, int64_t M, bool *done);
+// batch.cu: around the launch of a recorded call that is one kernel without scratch
+int record_before(wb_context *ctx, const void *r0, uint64_t r_bytes, const void *w0, uint64_t w_bytes);
+int record_after(wb_context *ctx);
+bool linear_uses_scratch(const wb_plan &plan, int64_t M);  // the workspace or the counters, which two calls at a time may not
 int launch_linear(wb_context *ctx, const Weight &w, const void *A, void *C, const float *bias, int64_t M,
                   int act_dtype, int out_dtype, int exact, const LinearFusion *fusion = nullptr);
 

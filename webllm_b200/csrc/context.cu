@@ -608,8 +608,19 @@ int wb_linear(wb_context *ctx, wb_handle weight, uint64_t a_offset, uint64_t c_o
                                       (long long)b->N, (long long)w->N);
         bias_ptr = (const float *)(ctx->arena[WB_ARENA_WEIGHTS].base + b->off_main);
     }
-    return launch_linear(ctx, *w, arena_ptr(ctx, WB_ARENA_ACT, a_offset), arena_ptr(ctx, WB_ARENA_ACT, c_offset),
-                         bias_ptr, M, act_dtype, out_dtype, exact);
+    const char *A = (const char *)arena_ptr(ctx, WB_ARENA_ACT, a_offset);
+    char *C = (char *)arena_ptr(ctx, WB_ARENA_ACT, c_offset);
+    if (ctx->capturing && M <= 32) {  // (larger calls fill the chip by themselves)
+        wb_plan plan;
+        WB_CHECK(plan_linear(ctx, *w, M, act_dtype, exact && act_dtype == WB_F32, &plan));
+        if (plan.launches == 1 && !linear_uses_scratch(plan, M)) {
+            WB_CHECK(record_before(ctx, A, (uint64_t)M * w->K * (act_dtype == WB_F16 ? 2 : 4), C, (uint64_t)M * w->N * (out_dtype == WB_F16 ? 2 : 4)));
+            const int rc = launch_linear(ctx, *w, A, C, bias_ptr, M, act_dtype, out_dtype, exact);
+            const int rec = record_after(ctx);
+            return rc != WB_OK ? rc : rec;
+        }
+    }
+    return launch_linear(ctx, *w, A, C, bias_ptr, M, act_dtype, out_dtype, exact);
 }
 
 // `sync` != nullptr: the call also runs the peer barrier (wb_linear_gather_barrier).

@@ -737,6 +737,11 @@ static int gemv_pick_stages(int64_t M, int cps, bool two_halves, int wn, int wk)
 // cluster is portable (<= 8 CTAs) and the merge buffer is small; otherwise through the workspace and arrival counters.
 static bool gemv_cluster_merge(int64_t M, int S) { return S > 1 && S <= 8 && M <= 8; }
 
+bool linear_uses_scratch(const wb_plan &plan, int64_t M)
+{
+    return plan.scratch_bytes != 0 && !(plan.kernel == WB_KERNEL_GEMV_MMA && gemv_cluster_merge(M, plan.split_k));
+}
+
 // `stream`: 0 = the general kernel only, 1 = the streaming kernel where the shape suits it, 2 = the streaming kernel
 // or nothing (plan->kernel stays 0 when it does not take the shape or the forced split).
 static void plan_gemv_mma(wb_context *ctx, const Weight &w, int64_t M, int two_halves, wb_plan *plan, int stream)
