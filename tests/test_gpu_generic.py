@@ -1,5 +1,5 @@
 """The tiled double-precision kernel (fp32-activation mode at many rows, ragged K) against gemmNTRef, bit for bit, at the edges of its
-tiles: rows and columns on and beside 32 and 64, K remainders inside a packed row, a group and a stage, both tile heights."""
+tiles: rows and columns on and beside 32 and 64, K remainders inside a packed row, a group and a stage, both tile widths."""
 import numpy as np
 import pytest
 

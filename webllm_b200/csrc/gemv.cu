@@ -550,10 +550,12 @@ __global__ void __launch_bounds__(256) dense_gemv_f16_kernel(const __half *__res
 // gemmNTRef (src/reference/qwen-ref.ts:126-145), bit for bit (a product of two f32 values is exact in double, so the fused
 // multiply-add rounds as the separate add does).
 //
-// Bound by the double-precision units (64 multiply-adds per clock and SM). A CTA of 128 threads computes TM rows x 32 columns, a
-// thread TM / 16 rows x 4 columns from operands that are unpacked, widened and staged in shared memory once per 32 k (with one
-// thread per output, as before, every weight was unpacked M times and every access was its own): 145 rows of 1000 -> 1236
-// 132 -> @@ us. 64 rows per CTA unless that leaves SMs without work.
+// Bound by the double-precision units and by the shared memory that feeds them. A CTA of 4 warps computes 32 rows x 32 C columns from
+// operands that are unpacked, widened and staged once per 32 k (with one thread per output every weight was unpacked M times).
+// A lane has C columns and 8 rows: the rows' values are the same for the whole warp, one broadcast for two, and the columns lie
+// side by side, so a k costs a warp 4 + 2 C passes over shared memory for 8 C multiply-adds (16 C cycles). Tiles of 2 x 4 outputs
+// with 8 lanes abreast took 20 passes for 8: the shared memory was 80 % busy and the arithmetic 15 %.
+// 145 rows of 1000 -> 1236: 132 us (one thread per output), 85 (2 x 4), 38 now. C = 2 unless smaller tiles spread better.
 // =====================================================================================================
 struct GenericParams {
     const uint32_t *qw, *qz;
@@ -565,84 +567,101 @@ struct GenericParams {
     int x_f16, out_f16, round_x_f16;
 };
 
-template <int TM>
+template <int C>
 __global__ void __launch_bounds__(128) linear_generic_kernel(const GenericParams p)
 {
-    constexpr int KC = 32, TN = 32, R = TM / 16, XP = TM + 2;
-    __shared__ __align__(16) double xs[KC][XP], ws[KC][TN];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & 7, ty = tid >> 3;
+    constexpr int KC = 32, TM = 32, TN = 32 * C, R = 8, XP = TM + 2, BUFS = C == 1 ? 2 : 1;  // (48 KB)
+    __shared__ __align__(16) double xs[BUFS][KC][XP], ws[BUFS][KC][TN];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t m0 = (int64_t)blockIdx.y * TM, n0 = (int64_t)blockIdx.x * TN;
-    // staging: this thread's x values are k = k0 + lane of rows warp, warp + 4, ...; its weights 8 k of column tid / 4
-    const int wc = tid >> 2, wr = tid & 3;
-    const int64_t wn = n0 + wc;
-    float xv[TM / 4], wv[8];
-    auto fetch = [&](int64_t k0) {
-        const int64_t k = k0 + lane;
+    // Staging: this thread's x values are k = k0 + lane of the row pairs warp, warp + 4, ...; its weights words (8 k) tid, tid + 128 of
+    // the stage, columns side by side. In flight under the arithmetic is what memory holds: a conversion would wait for its load.
+    uint32_t xv[8], wv[C][8], wscale[C] = {}, wzero[C] = {};
+    auto fetch = [&](int k0) {
+        const int k = k0 + lane;
 #pragma unroll
-        for (int i = 0; i < TM / 4; i++) {
-            const int64_t m = m0 + warp + 4 * i;
-            float v = 0.f;
-            if (m < p.M && k < p.K) v = p.x_f16 ? __half2float(((const __half *)p.x)[m * p.K + k]) : ((const float *)p.x)[m * p.K + k];
-            xv[i] = p.round_x_f16 ? __half2float(__float2half_rn(v)) : v;
+        for (int i = 0; i < 8; i++) {
+            const int64_t m = m0 + 2 * (warp + 4 * (i >> 1)) + (i & 1);
+            xv[i] = 0;
+            if (m < p.M && k < p.K) {
+                if (p.x_f16) xv[i] = ((const unsigned short *)p.x)[m * p.K + k];
+                else xv[i] = ((const uint32_t *)p.x)[m * p.K + k];
+            }
         }
-        const int64_t kw = k0 + wr * 8;
 #pragma unroll
-        for (int j = 0; j < 8; j++) wv[j] = 0.f;
-        if (wn < p.N && kw < p.K) {
+        for (int c = 0; c < C; c++) {
+            const int idx = tid + 128 * c, kw = k0 + idx / TN * 8;
+            const int64_t n = n0 + idx % TN;
+#pragma unroll
+            for (int j = 0; j < 8; j++) wv[c][j] = 0;
+            if (n >= p.N || kw >= p.K) continue;
             if (p.dense) {
 #pragma unroll
                 for (int j = 0; j < 8; j++)
-                    if (kw + j < p.K) wv[j] = __half2float(p.dense[wn * p.K + kw + j]);
+                    if (kw + j < p.K) wv[c][j] = ((const unsigned short *)p.dense)[n * p.K + kw + j];
             } else {
-                const int64_t r = kw >> 3, g = kw / p.group;
-                const uint32_t word = p.qw[r * p.N + wn];
-                const float scale = __half2float(p.sc[g * p.N + wn]);
-                const int zero = p.qz ? (int)((p.qz[g * p.zcols + (wn >> 3)] >> (4 * (wn & 7))) & 15u) + 1 : 8;
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    if (kw + j < p.K) wv[j] = (float)((int)((word >> (4 * j)) & 15u) - zero) * scale;
+                const int64_t g = (unsigned)kw / (unsigned)p.group;
+                wv[c][0] = p.qw[(int64_t)(kw >> 3) * p.N + n];
+                wscale[c] = ((const unsigned short *)p.sc)[g * p.N + n];
+                wzero[c] = p.qz ? p.qz[g * p.zcols + (n >> 3)] >> (4 * (n & 7)) : 7u;
             }
         }
     };
-    double acc[R][4];
+    auto h2f = [](uint32_t bits) { return __half2float(__ushort_as_half((unsigned short)bits)); };
+    auto x_value = [&](int i) {
+        const float v = p.x_f16 ? h2f(xv[i]) : __uint_as_float(xv[i]);
+        return (double)(p.round_x_f16 ? __half2float(__float2half_rn(v)) : v);
+    };
+    auto w_value = [&](int c, int j, int kw) {
+        if (p.dense) return (double)h2f(wv[c][j]);
+        if (kw + j >= p.K) return 0.0;
+        return (double)((float)((int)((wv[c][0] >> (4 * j)) & 15u) - (int)((wzero[c] & 15u) + 1u)) * h2f(wscale[c]));
+    };
+    double acc[R][C];
 #pragma unroll
     for (int i = 0; i < R; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.0;
+        for (int j = 0; j < C; j++) acc[i][j] = 0.0;
     pdl_sync();
     fetch(0);
-    for (int64_t k0 = 0; k0 < p.K; k0 += KC) {
+    int buf = 0;
+    for (int k0 = 0; k0 < p.K; k0 += KC, buf = (buf + 1) % BUFS) {
+        if (BUFS == 1) __syncthreads();
 #pragma unroll
-        for (int i = 0; i < TM / 4; i++) xs[lane][warp + 4 * i] = (double)xv[i];
+        for (int i = 0; i < 8; i += 2) *reinterpret_cast<double2 *>(&xs[buf][lane][2 * (warp + 2 * i)]) = make_double2(x_value(i), x_value(i + 1));
 #pragma unroll
-        for (int j = 0; j < 8; j++) ws[wr * 8 + j][wc] = (double)wv[j];
-        __syncthreads();
-        if (k0 + KC < p.K) fetch(k0 + KC);  // in flight under the arithmetic
+        for (int c = 0; c < C; c++) {
+            const int idx = tid + 128 * c, wr = idx / TN;
+#pragma unroll
+            for (int j = 0; j < 8; j++) ws[buf][wr * 8 + j][idx % TN] = w_value(c, j, k0 + wr * 8);
+        }
+        __syncthreads();  // (with two buffers every warp has also left the one that the next stage fills)
+        if (k0 + KC < p.K) fetch(k0 + KC);
 #pragma unroll 4
         for (int k = 0; k < KC; k++) {
-            double a[R], b[4];
+            double a[R], b[C];
 #pragma unroll
             for (int i = 0; i < R; i += 2) {
-                const double2 v = *reinterpret_cast<const double2 *>(&xs[k][ty * R + i]);
+                const double2 v = *reinterpret_cast<const double2 *>(&xs[buf][k][warp * R + i]);
                 a[i] = v.x, a[i + 1] = v.y;
             }
-#pragma unroll
-            for (int j = 0; j < 4; j += 2) {
-                const double2 v = *reinterpret_cast<const double2 *>(&ws[k][tx * 4 + j]);
-                b[j] = v.x, b[j + 1] = v.y;
+            if constexpr (C == 2) {
+                const double2 v = *reinterpret_cast<const double2 *>(&ws[buf][k][lane * 2]);
+                b[0] = v.x, b[1] = v.y;
+            } else {
+                b[0] = ws[buf][k][lane];
             }
 #pragma unroll
             for (int i = 0; i < R; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < C; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
         }
-        __syncthreads();
     }
 #pragma unroll
     for (int i = 0; i < R; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int64_t m = m0 + ty * R + i, n = n0 + tx * 4 + j;
+        for (int j = 0; j < C; j++) {
+            const int64_t m = m0 + warp * R + i, n = n0 + lane * C + j;
             if (m >= p.M || n >= p.N) continue;
             double v = acc[i][j];
             if (p.bias) v += (double)p.bias[n];
@@ -651,7 +670,12 @@ __global__ void __launch_bounds__(128) linear_generic_kernel(const GenericParams
         }
 }
 
-static int generic_tile_m(int64_t M, int64_t N, int sms) { return ((M + 63) / 64) * ((N + 31) / 32) >= sms ? 64 : 32; }
+// Columns of a tile, 32 or 64: the passes over shared memory per k of the SM with the most tiles.
+static int generic_tile_n(int64_t M, int64_t N, int sms)
+{
+    auto cost = [&](int cols) { return ((((M + 31) / 32) * ((N + cols - 1) / cols) + sms - 1) / sms) * (cols == 64 ? 8 : 6); };
+    return cost(64) <= cost(32) ? 64 : 32;
+}
 
 // =====================================================================================================
 // Planner and dispatch
@@ -884,8 +908,8 @@ static int make_plan(wb_context *ctx, const Weight &w, int64_t M, int act_dtype,
         plan->kernel = kind;
         plan->split_k = 1;
         plan->block = 128;
-        plan->tile_m = generic_tile_m(M, w.N, ctx->sm_count), plan->tile_n = 32;
-        plan->grid_x = (int)((w.N + 31) / 32);
+        plan->tile_m = 32, plan->tile_n = generic_tile_n(M, w.N, ctx->sm_count);
+        plan->grid_x = (int)((w.N + plan->tile_n - 1) / plan->tile_n);
         plan->grid_y = (int)((M + plan->tile_m - 1) / plan->tile_m);
         plan->grid_z = 1;
         plan->launches = 1;
@@ -1058,8 +1082,8 @@ int launch_linear(wb_context *ctx, const Weight &w, const void *A, void *C, cons
         g.group = gptq ? w.group : 8, g.zcols = w.zcols;
         g.x_f16 = act_dtype == WB_F16, g.out_f16 = out_dtype == WB_F16, g.round_x_f16 = round_x;
         const dim3 grid((unsigned)plan.grid_x, (unsigned)plan.grid_y);
-        const cudaError_t e = plan.tile_m == 64 ? launch_pdl(linear_generic_kernel<64>, grid, dim3(128), 0, ctx->stream, g)
-                                                : launch_pdl(linear_generic_kernel<32>, grid, dim3(128), 0, ctx->stream, g);
+        const cudaError_t e = plan.tile_n == 64 ? launch_pdl(linear_generic_kernel<2>, grid, dim3(128), 0, ctx->stream, g)
+                                                : launch_pdl(linear_generic_kernel<1>, grid, dim3(128), 0, ctx->stream, g);
         ctx->launches++;
         WB_CUDA(e);
         return WB_OK;
