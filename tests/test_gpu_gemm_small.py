@@ -1,0 +1,28 @@
+"""GPU parity of the small-batch int4 GEMM on large matrices (9 to 16 rows): ragged row counts, a last column group that is not full,
+slices that do not divide K, groups of one and several chunks, both column widths and output types."""
+import numpy as np
+import pytest
+
+from helpers import assert_close, oracle_weight, register, run_linear
+from webllm_b200 import synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("K,N,group,zeros", [(1152, 8224, 128, "any"), (8576, 1056, 128, "7or8"), (2560, 3360, 256, "none")])
+@pytest.mark.parametrize("M", [9, 13, 16])
+def test_small_batch_on_a_large_matrix(gpu, oracle, K, N, group, zeros, M):
+    t = synthetic.random_gptq(K, N, group, seed=K + N, zeros=zeros)
+    h = register(gpu, f"gs_{K}_{N}_{M}", t)
+    hb = gpu.f32_upload(f"gsb_{K}_{N}_{M}", np.random.default_rng(N).standard_normal(N).astype(np.float32))
+    bias = np.random.default_rng(N).standard_normal(N).astype(np.float32)
+    x = np.random.default_rng(M).standard_normal((M, K)).astype(np.float32)
+    x16 = x.astype(np.float16)
+    ref = oracle.gemm_nt_ref(x16.astype(np.float32), oracle_weight(oracle, t), M, N, K) + bias
+    p = gpu.plan(h, M, "f32")
+    if p["kernel_name"] == "gemm_tc":
+        assert p["block"] == 256 and p["launches"] == 1
+    for act, xin in (("f16", x16), ("f32", x)):
+        first = run_linear(gpu, h, xin, M, N, hb, act=act, out=act)
+        assert_close(oracle, first, ref, 1e-3, f"{K}x{N} M={M} {act}")
+        assert np.array_equal(first, run_linear(gpu, h, xin, M, N, hb, act=act, out=act))  # slices are added in order
