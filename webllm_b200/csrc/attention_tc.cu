@@ -1,0 +1,315 @@
+// Prefill attention on the 5th-generation tensor cores: causal GQA attention of many query rows against an fp16 KV cache, head
+// size 64 (attention_gqa_cache.wgsl, attentionGqaRef, src/reference/qwen-ref.ts:67-116). Same operands and accumulation as the
+// warp-level kernel of attention_prefill.cu (fp16 q, k, v and softmax weights, f32 sums), which keeps the other cases.
+//
+// One CTA = 128 query rows of one head, in two groups of four warps and a control warp each: group 0 takes the even blocks of 64
+// keys, group 1 the odd ones, and the two states of a row are merged at the end. Per block the control thread of a group issues
+//   S = Q K^T  (tcgen05.mma, both operands K-major tiles in shared memory, 128 x 64 f32 in tensor memory)
+//   O += P V   (P from tensor memory, V as it lies in the cache: keys x dims, an MN-major operand; 128 x 64 f32)
+// and in between a thread of the group owns one row: it reads its 64 scores, takes the maximum, the exponentials (ex2, the unit
+// that bounds the kernel: 16 a cycle per SM) and writes P as fp16 over S. O stays in tensor memory; it is rescaled only where a
+// row's maximum has grown by more than 2^8 since the last time (the weights of the meantime are at most 2^8, and the final division
+// takes the same maximum, so nothing is approximated). K and V boxes come by TMA, two stages each; rows past the last key
+// read as zeros. Two CTAs share an SM (256 tensor-memory columns each): while one group waits for its MMAs another computes.
+// CTAs are started longest first.
+// @@
+#include "gemm_tc.cuh"
+#include "qwen_ops.cuh"
+
+namespace wb {
+
+namespace {
+
+using namespace tc;
+
+constexpr int kD = 64, kRows = 128, kKeys = 64, kGroups = 2;
+constexpr int kThreads = kGroups * 128 + kGroups * 32;
+constexpr int kTile = kKeys * kD * 2;         // a K or V box: 64 rows of 128 bytes
+constexpr int kGroupBytes = 2 * 2 * kTile;    // two stages of K, two of V
+constexpr int kQBytes = kRows * kD * 2;
+constexpr int kSmem = kQBytes + kGroups * kGroupBytes + 2 * kRows * 4 + 256 + 1024 /*alignment slack*/;
+constexpr uint32_t kGroupCols = 128;          // tensor-memory columns of a group: S (P over it) 64, O 64
+static_assert(kRows * kD * 4 == kGroupBytes, "the merge hands O over in a group's stages");
+
+__device__ __forceinline__ float ex2f(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// A from tensor memory (fp16 pairs, two k per column)
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+          "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// An MN-major operand with 64 elements (one 128-byte swizzle atom) along MN: 8 rows of k make an atom of 1024 bytes, the next
+// atom along K follows it. (One atom along MN: the leading offset is not used; both name the same 1024 bytes.)
+__device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t saddr)
+{
+    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (64ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
+attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const float *__restrict__ q,
+                    float *__restrict__ out, __half *__restrict__ out16, int *status, int M, int H, int KVH, int past, int ldq, float scale)
+{
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool control = warp >= kGroups * 4;
+    const int grp = control ? warp - kGroups * 4 : warp >> 2;
+    uint8_t *stages = smem + kQBytes + grp * kGroupBytes;  // K0 K1 V0 V1 of this group
+    float *ml = (float *)(smem + kQBytes + kGroups * kGroupBytes);  // group 1's [128] maxima, [128] sums
+    uint64_t *bars = (uint64_t *)(ml + 2 * kRows);
+    uint64_t *kfull = bars + grp * 6, *vfull = kfull + 2, *s_full = kfull + 4, *p_ready = kfull + 5;
+    uint32_t *tmem_slot = (uint32_t *)(bars + kGroups * 6);
+    volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kGroups * 6; i++) mbar_init(bars + i, i % 6 == 5 ? 4 : 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kGroups * 4) tmem_alloc(tmem_slot, kGroups * kGroupCols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t t_s = *tmem_slot + (uint32_t)grp * kGroupCols, t_o = t_s + 64;
+
+    const int h = blockIdx.x, kvh = h / (H / KVH);
+    const int r0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRows;  // late (long) rows first
+    const int n_blocks = (past + min(r0 + kRows, M) - 1) / kKeys + 1;
+    const int nb = (n_blocks - grp + 1) >> 1;  // blocks of this group
+    pdl_sync();
+
+    auto load_k = [&](int j) {
+        mbar_expect_tx(&kfull[j & 1], kTile);
+        tma_load_2d(stages + (j & 1) * kTile, &map_k, kvh * kD, (2 * j + grp) * kKeys, &kfull[j & 1]);
+    };
+    auto load_v = [&](int j) {
+        mbar_expect_tx(&vfull[j & 1], kTile);
+        tma_load_2d(stages + (2 + (j & 1)) * kTile, &map_v, kvh * kD, (2 * j + grp) * kKeys, &vfull[j & 1]);
+    };
+    if (control) {
+        if (lane == 0)
+            for (int j = 0; j < 2 && j < nb; j++) load_k(j), load_v(j);
+        __syncwarp();
+    } else {
+        // Q as fp16 rows of 128 bytes, 16-byte pieces swizzled as TMA would: two threads a row
+        const int r = threadIdx.x >> 1, half = threadIdx.x & 1;
+        const float *src = q + (int64_t)(r0 + r) * ldq + h * kD + half * 32;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (r0 + r < M) {
+                const float4 a = *reinterpret_cast<const float4 *>(src + c * 8), b = *reinterpret_cast<const float4 *>(src + c * 8 + 4);
+                const __half2 h0 = __floats2half2_rn(a.x, a.y), h1 = __floats2half2_rn(a.z, a.w);
+                const __half2 h2 = __floats2half2_rn(b.x, b.y), h3 = __floats2half2_rn(b.z, b.w);
+                v.x = *reinterpret_cast<const uint32_t *>(&h0), v.y = *reinterpret_cast<const uint32_t *>(&h1);
+                v.z = *reinterpret_cast<const uint32_t *>(&h2), v.w = *reinterpret_cast<const uint32_t *>(&h3);
+            }
+            *reinterpret_cast<uint4 *>(smem + r * 128 + (((half * 4 + c) ^ (r & 7)) << 4)) = v;
+        }
+        fence_async_smem();
+    }
+    __syncthreads();
+
+    float m = -INFINITY, l = 0.f;
+    const int wq = warp & 3;
+    const uint32_t lane_sel = (uint32_t)(wq * 32) << 16;
+    const float sl2 = scale * 1.4426950408889634f;
+    if (control) {
+        if (lane == 0 && nb > 0) {
+            constexpr uint32_t idesc_s = idesc_f16(kRows, kKeys), idesc_o = idesc_f16(kRows, kD) | (1u << 16);
+            const uint64_t dq = smem_desc_sw128(smem_u32(smem));
+            auto scores = [&](int j) {
+                const uint64_t dk = smem_desc_sw128(smem_u32(stages + (j & 1) * kTile));
+#pragma unroll
+                for (int k = 0; k < kD / 16; k++) umma_f16(t_s, dq + 2 * k, dk + 2 * k, idesc_s, k != 0);
+            };
+            bool ok = mbar_wait(&kfull[0], 0, abort_flag, status, 21);
+            if (ok) scores(0), umma_commit(s_full);
+            for (int j = 0; j < nb && ok; j++) {
+                // S_j is complete, and with it O of block j - 1: their K and V stages are free
+                if (!(ok = mbar_wait(s_full, (uint32_t)j & 1u, abort_flag, status, 22))) break;
+                if (j + 2 < nb) load_k(j + 2);
+                if (j >= 1 && j + 1 < nb) load_v(j + 1);
+                if (!(ok = mbar_wait(&vfull[j & 1], (uint32_t)(j >> 1) & 1u, abort_flag, status, 23))) break;
+                if (j + 1 < nb && !(ok = mbar_wait(&kfull[(j + 1) & 1], (uint32_t)((j + 1) >> 1) & 1u, abort_flag, status, 24))) break;
+                if (!(ok = mbar_wait(p_ready, (uint32_t)j & 1u, abort_flag, status, 25))) break;
+                tc_fence_after();
+                const uint64_t dv = smem_desc_mn_sw128(smem_u32(stages + (2 + (j & 1)) * kTile));
+#pragma unroll
+                for (int k = 0; k < kKeys / 16; k++) umma_f16_ts(t_o, t_s + 8 * k, dv + (uint64_t)(k * (2048 >> 4)), idesc_o, (j | k) != 0);
+                if (j + 1 < nb) scores(j + 1);
+                umma_commit(s_full);
+            }
+        }
+        __syncwarp();
+    } else {
+        const int last_key = past + r0 + wq * 32 + lane;  // of this thread's row
+        bool ok = true;
+        for (int j = 0; j < nb; j++) {
+            const int key0 = (2 * j + grp) * kKeys;
+            ok = __all_sync(0xffffffffu, mbar_wait(s_full, (uint32_t)j & 1u, abort_flag, status, 26));
+            if (!ok) break;
+            tc_fence_after();
+            uint32_t s[4][16];
+#pragma unroll
+            for (int c = 0; c < 4; c++) tmem_ld_32x32b_x16(t_s + lane_sel + c * 16, s[c]);
+            tmem_ld_wait();
+            if (key0 + kKeys - 1 > past + r0 + wq * 32) {  // the diagonal is in this block for some row of the warp
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+#pragma unroll
+                    for (int i = 0; i < 16; i++)
+                        if (key0 + c * 16 + i > last_key) s[c][i] = 0xff800000u;  // -infinity
+            }
+            float mx[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                mx[c] = __uint_as_float(s[c][0]);
+#pragma unroll
+                for (int i = 1; i < 16; i++) mx[c] = fmaxf(mx[c], __uint_as_float(s[c][i]));
+            }
+            const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+            if (j == 0) {
+                m = top;
+            } else {
+                const bool grow = (top - m) * sl2 > 8.f;
+                if (__any_sync(0xffffffffu, grow)) {
+                    const float f = grow ? ex2f((m - top) * sl2) : 1.f;
+                    if (grow) m = top, l *= f;
+#pragma unroll 1
+                    for (int c = 0; c < 4; c++) {
+                        uint32_t o[16];
+                        tmem_ld_32x32b_x16(t_o + lane_sel + c * 16, o);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
+                        tmem_st_32x32b_x16(t_o + lane_sel + c * 16, o);
+                    }
+                }
+            }
+            const float base = m == -INFINITY ? 0.f : m * sl2;
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                uint32_t p[16];
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const int e = c * 32 + i * 2;
+                    const float a = ex2f(fmaf(__uint_as_float(s[e >> 4][e & 15]), sl2, -base));
+                    const float b = ex2f(fmaf(__uint_as_float(s[e >> 4][(e & 15) + 1]), sl2, -base));
+                    sum[(i & 1) * 2] += a, sum[(i & 1) * 2 + 1] += b;
+                    const __half2 pr = __floats2half2_rn(a, b);
+                    p[i] = *reinterpret_cast<const uint32_t *>(&pr);
+                }
+                tmem_st_32x32b_x16(t_s + lane_sel + c * 16, p);
+            }
+            l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_ready);
+        }
+        if (ok && nb > 0) {
+            ok = __all_sync(0xffffffffu, mbar_wait(s_full, (uint32_t)nb & 1u, abort_flag, status, 27));
+            tc_fence_after();
+        }
+        if (grp == 1) {  // its state through its own stages, [64 dims][128 rows]
+            float *po = (float *)stages;
+            const int r = wq * 32 + lane;
+#pragma unroll 1
+            for (int c = 0; c < 4; c++) {
+                uint32_t o[16];
+                tmem_ld_32x32b_x16(t_o + lane_sel + c * 16, o);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; i++) po[(c * 16 + i) * kRows + r] = nb > 0 ? __uint_as_float(o[i]) : 0.f;
+            }
+            ml[r] = m, ml[kRows + r] = l;
+        }
+    }
+    __syncthreads();
+    if (!control && grp == 0) {
+        const float *po = (const float *)(stages + kGroupBytes);
+        const int r = wq * 32 + lane;
+        const float m1 = ml[r], l1 = ml[kRows + r], top = fmaxf(m, m1);  // (key 0 is in group 0: top is finite)
+        const float own = ex2f((m - top) * sl2), other = ex2f((m1 - top) * sl2);
+        const float inv = 1.f / (l * own + l1 * other), w0 = own * inv, w1 = other * inv;
+        const int64_t at = (int64_t)(r0 + r) * (H * kD) + h * kD;
+#pragma unroll 1
+        for (int c = 0; c < 4; c++) {
+            uint32_t o[16];
+            tmem_ld_32x32b_x16(t_o + lane_sel + c * 16, o);
+            tmem_ld_wait();
+            float v[16];
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = __uint_as_float(o[i]) * w0 + po[(c * 16 + i) * kRows + r] * w1;
+            if (r0 + r >= M) continue;
+            if (out16) {  // the o projection takes the fp16 value it would round to itself
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const __half2 pr = __floats2half2_rn(v[i], v[(i + 1) & 15]);
+                    o[i] = *reinterpret_cast<const uint32_t *>(&pr);
+                }
+                *reinterpret_cast<uint4 *>(out16 + at + c * 16) = make_uint4(o[0], o[2], o[4], o[6]);
+                *reinterpret_cast<uint4 *>(out16 + at + c * 16 + 8) = make_uint4(o[8], o[10], o[12], o[14]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4 *>(out + at + c * 16 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == kGroups * 4) tmem_dealloc(*tmem_slot, kGroups * kGroupCols);
+}
+
+}  // namespace
+
+bool op_attention_tc_supported(int M, int D, int ldq, int kv_ld, int kv_f16, const void *q)
+{
+    return kv_f16 && D == kD && M >= 64 && ldq % 4 == 0 && kv_ld % 8 == 0 && ((uintptr_t)q & 15) == 0;
+}
+
+int op_attention_tc(wb_context *ctx, const float *q, const void *kmem, const void *vmem, float *out, __half *out16, int M, int H, int KVH,
+                    int past, int ldq, int kv_ld)
+{
+    CUtensorMap maps[2];
+    for (int i = 0; i < 2; i++) {
+        cuuint64_t dims[2] = {(cuuint64_t)KVH * kD, (cuuint64_t)past + M}, strides[1] = {(cuuint64_t)kv_ld * 2};
+        cuuint32_t box[2] = {kD, kKeys}, estr[2] = {1, 1};
+        const CUresult r = ((EncodeTiledFn)ctx->tmap_encode)(&maps[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(i ? vmem : kmem), dims,
+                                                             strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return fail(WB_ERR_CUDA, "cuTensorMapEncodeTiled (KV cache) failed with code %d", (int)r);
+    }
+    if (const cudaError_t e = smem_limit_once<attention_tc_kernel>(kSmem); e != cudaSuccess) WB_CUDA(e);
+    const dim3 grid((unsigned)H, (unsigned)((M + kRows - 1) / kRows));
+    const cudaError_t e = launch_pdl(attention_tc_kernel, grid, dim3(kThreads), (size_t)kSmem, ctx->stream, maps[0], maps[1], q, out, out16,
+                                     ctx->status_word, M, H, KVH, past, ldq, 1.0f / sqrtf((float)kD));
+    ctx->launches++;
+    WB_CUDA(e);
+    return WB_OK;
+}
+
+}  // namespace wb

@@ -709,10 +709,6 @@ __global__ void scatter_cols_kernel(const void *__restrict__ src, const OutPlace
 // host side
 // ----------------------------------------------------------------------------------------------------
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 static int make_map_2d(wb_context *ctx, CUtensorMap *map, CUtensorMapDataType dt, int elem_bytes, const void *base,
                        uint64_t inner, uint64_t outer, uint32_t box_inner, uint32_t box_outer, bool swizzle128)
 {

@@ -188,6 +188,9 @@ int forward_impl(wb_qwen *m, const Bufs &b, int64_t M, int64_t B, int64_t T, int
             if (M == 1 && D % 8 == 0 && D <= 128 && op_attention_decode_smem(D, max_keys, kv16) <= 160 * 1024) {
                 WB_CHECK(op_attention_decode(ctx, b.q, kc, vc, kv16, b.att, m->att_scratch, m->att_counters, H, KVH, D, past_ptr,
                                              (int)past, max_keys, KV));
+            } else if (!m->exact && !past_ptr && op_attention_tc_supported((int)M, D, b.ldq, KV, kv16, b.q)) {
+                att_half = half_in;
+                WB_CHECK(op_attention_tc(ctx, b.q, kc, vc, b.att, att_half ? b.h16 : nullptr, (int)M, H, KVH, (int)past, b.ldq, KV));
             } else if (!m->exact && op_attention_prefill_supported((int)M, H, KVH, D, b.ldq, KV)) {
                 // prefill in the default mode: causal attention on the tensor cores (fp16 operands, like the linears)
                 att_half = half_in;
