@@ -2,17 +2,18 @@
 // size 64 (attention_gqa_cache.wgsl, attentionGqaRef, src/reference/qwen-ref.ts:67-116). Same operands and accumulation as the
 // warp-level kernel of attention_prefill.cu (fp16 q, k, v and softmax weights, f32 sums), which keeps the other cases.
 //
-// One CTA = 128 query rows of one head, in two groups of four warps and a control warp each: group 0 takes the even blocks of 64
-// keys, group 1 the odd ones, and the two states of a row are merged at the end. Per block the control thread of a group issues
+// One CTA = 128 query rows of one head, in four groups of four warps and a control warp each: group i takes every fourth block of 64
+// keys from block i on, and the four states of a row are merged at the end. Per block the control thread of a group issues
 //   S = Q K^T  (tcgen05.mma, both operands K-major tiles in shared memory, 128 x 64 f32 in tensor memory)
 //   O += P V   (P from tensor memory, V as it lies in the cache: keys x dims, an MN-major operand; 128 x 64 f32)
-// and in between a thread of the group owns one row: it reads its 64 scores, takes the maximum, the exponentials (ex2, the unit
-// that bounds the kernel: 16 a cycle per SM) and writes P as fp16 over S. O stays in tensor memory; it is rescaled only where a
-// row's maximum has grown by more than 2^8 since the last time (the weights of the meantime are at most 2^8, and the final division
-// takes the same maximum, so nothing is approximated). K and V boxes come by TMA, two stages each; rows past the last key
-// read as zeros. Two CTAs share an SM (256 tensor-memory columns each): while one group waits for its MMAs another computes.
-// CTAs are started longest first.
-// @@
+// and in between a thread of the group owns one row: it reads its 64 scores, takes the maximum, the exponentials (ex2, 16 a cycle
+// per SM) and writes P as fp16 over S. O stays in tensor memory; it is rescaled only where a row's maximum has grown by more
+// than 2^8 since the last time (the weights of the meantime are at most 2^8, and the final division takes the same maximum, so
+// nothing is approximated). K and V boxes come by TMA, two stages each; rows past the last key read as zeros.
+// Bound by the chain of a block, product - softmax - product, some 3000 cycles when four groups share the SM's exponentials, times
+// the blocks of the longest CTA. So four groups of one row tile rather than two of each of two: half as many blocks in the
+// chain for the same four at a time. CTAs are started longest first. 2048 tokens, 14 heads: 41.6 us (warp-level kernel) -> 31.9 (two
+// groups) -> 29.9; exponentials 33 % of their rate.
 #include "gemm_tc.cuh"
 #include "qwen_ops.cuh"
 
@@ -22,12 +23,12 @@ namespace {
 
 using namespace tc;
 
-constexpr int kD = 64, kRows = 128, kKeys = 64, kGroups = 2;
+constexpr int kD = 64, kRows = 128, kKeys = 64, kGroups = 4;
 constexpr int kThreads = kGroups * 128 + kGroups * 32;
 constexpr int kTile = kKeys * kD * 2;         // a K or V box: 64 rows of 128 bytes
 constexpr int kGroupBytes = 2 * 2 * kTile;    // two stages of K, two of V
 constexpr int kQBytes = kRows * kD * 2;
-constexpr int kSmem = kQBytes + kGroups * kGroupBytes + 2 * kRows * 4 + 256 + 1024 /*alignment slack*/;
+constexpr int kSmem = kQBytes + kGroups * kGroupBytes + kGroups * 2 * kRows * 4 + 256 + 1024 /*alignment slack*/;
 constexpr uint32_t kGroupCols = 128;          // tensor-memory columns of a group: S (P over it) 64, O 64
 static_assert(kRows * kD * 4 == kGroupBytes, "the merge hands O over in a group's stages");
 
@@ -65,7 +66,7 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t saddr)
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (64ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const float *__restrict__ q,
                     float *__restrict__ out, __half *__restrict__ out16, int *status, int M, int H, int KVH, int past, int ldq, float scale)
 {
@@ -75,8 +76,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     const bool control = warp >= kGroups * 4;
     const int grp = control ? warp - kGroups * 4 : warp >> 2;
     uint8_t *stages = smem + kQBytes + grp * kGroupBytes;  // K0 K1 V0 V1 of this group
-    float *ml = (float *)(smem + kQBytes + kGroups * kGroupBytes);  // group 1's [128] maxima, [128] sums
-    uint64_t *bars = (uint64_t *)(ml + 2 * kRows);
+    float *ml = (float *)(smem + kQBytes + kGroups * kGroupBytes);  // of each group [128] maxima, [128] sums
+    uint64_t *bars = (uint64_t *)(ml + kGroups * 2 * kRows);
     uint64_t *kfull = bars + grp * 6, *vfull = kfull + 2, *s_full = kfull + 4, *p_ready = kfull + 5;
     uint32_t *tmem_slot = (uint32_t *)(bars + kGroups * 6);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
@@ -95,27 +96,28 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     const int h = blockIdx.x, kvh = h / (H / KVH);
     const int r0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRows;  // late (long) rows first
     const int n_blocks = (past + min(r0 + kRows, M) - 1) / kKeys + 1;
-    const int nb = (n_blocks - grp + 1) >> 1;  // blocks of this group
+    const int nb = (n_blocks - grp + kGroups - 1) / kGroups;  // blocks of this group
     pdl_sync();
 
     auto load_k = [&](int j) {
         mbar_expect_tx(&kfull[j & 1], kTile);
-        tma_load_2d(stages + (j & 1) * kTile, &map_k, kvh * kD, (2 * j + grp) * kKeys, &kfull[j & 1]);
+        tma_load_2d(stages + (j & 1) * kTile, &map_k, kvh * kD, (kGroups * j + grp) * kKeys, &kfull[j & 1]);
     };
     auto load_v = [&](int j) {
         mbar_expect_tx(&vfull[j & 1], kTile);
-        tma_load_2d(stages + (2 + (j & 1)) * kTile, &map_v, kvh * kD, (2 * j + grp) * kKeys, &vfull[j & 1]);
+        tma_load_2d(stages + (2 + (j & 1)) * kTile, &map_v, kvh * kD, (kGroups * j + grp) * kKeys, &vfull[j & 1]);
     };
     if (control) {
         if (lane == 0)
             for (int j = 0; j < 2 && j < nb; j++) load_k(j), load_v(j);
         __syncwarp();
     } else {
-        // Q as fp16 rows of 128 bytes, 16-byte pieces swizzled as TMA would: two threads a row
-        const int r = threadIdx.x >> 1, half = threadIdx.x & 1;
-        const float *src = q + (int64_t)(r0 + r) * ldq + h * kD + half * 32;
+        // Q as fp16 rows of 128 bytes, 16-byte pieces swizzled as TMA would: a thread of each group per row
+        constexpr int PIECES = 8 / kGroups;
+        const int r = threadIdx.x / kGroups, part = threadIdx.x % kGroups;
+        const float *src = q + (int64_t)(r0 + r) * ldq + h * kD + part * PIECES * 8;
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
+        for (int c = 0; c < PIECES; c++) {
             uint4 v = make_uint4(0, 0, 0, 0);
             if (r0 + r < M) {
                 const float4 a = *reinterpret_cast<const float4 *>(src + c * 8), b = *reinterpret_cast<const float4 *>(src + c * 8 + 4);
@@ -124,7 +126,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                 v.x = *reinterpret_cast<const uint32_t *>(&h0), v.y = *reinterpret_cast<const uint32_t *>(&h1);
                 v.z = *reinterpret_cast<const uint32_t *>(&h2), v.w = *reinterpret_cast<const uint32_t *>(&h3);
             }
-            *reinterpret_cast<uint4 *>(smem + r * 128 + (((half * 4 + c) ^ (r & 7)) << 4)) = v;
+            *reinterpret_cast<uint4 *>(smem + r * 128 + (((part * PIECES + c) ^ (r & 7)) << 4)) = v;
         }
         fence_async_smem();
     }
@@ -166,7 +168,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         const int last_key = past + r0 + wq * 32 + lane;  // of this thread's row
         bool ok = true;
         for (int j = 0; j < nb; j++) {
-            const int key0 = (2 * j + grp) * kKeys;
+            const int key0 = (kGroups * j + grp) * kKeys;
             ok = __all_sync(0xffffffffu, mbar_wait(s_full, (uint32_t)j & 1u, abort_flag, status, 26));
             if (!ok) break;
             tc_fence_after();
@@ -233,48 +235,54 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
             ok = __all_sync(0xffffffffu, mbar_wait(s_full, (uint32_t)nb & 1u, abort_flag, status, 27));
             tc_fence_after();
         }
-        if (grp == 1) {  // its state through its own stages, [64 dims][128 rows]
-            float *po = (float *)stages;
-            const int r = wq * 32 + lane;
-#pragma unroll 1
-            for (int c = 0; c < 4; c++) {
-                uint32_t o[16];
-                tmem_ld_32x32b_x16(t_o + lane_sel + c * 16, o);
-                tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 16; i++) po[(c * 16 + i) * kRows + r] = nb > 0 ? __uint_as_float(o[i]) : 0.f;
-            }
-            ml[r] = m, ml[kRows + r] = l;
-        }
-    }
-    __syncthreads();
-    if (!control && grp == 0) {
-        const float *po = (const float *)(stages + kGroupBytes);
+        // the states of a row meet in shared memory: every group's sums in its own stages, [64 dims][128 rows]
+        float *po = (float *)stages;
         const int r = wq * 32 + lane;
-        const float m1 = ml[r], l1 = ml[kRows + r], top = fmaxf(m, m1);  // (key 0 is in group 0: top is finite)
-        const float own = ex2f((m - top) * sl2), other = ex2f((m1 - top) * sl2);
-        const float inv = 1.f / (l * own + l1 * other), w0 = own * inv, w1 = other * inv;
-        const int64_t at = (int64_t)(r0 + r) * (H * kD) + h * kD;
 #pragma unroll 1
         for (int c = 0; c < 4; c++) {
             uint32_t o[16];
             tmem_ld_32x32b_x16(t_o + lane_sel + c * 16, o);
             tmem_ld_wait();
-            float v[16];
 #pragma unroll
-            for (int i = 0; i < 16; i++) v[i] = __uint_as_float(o[i]) * w0 + po[(c * 16 + i) * kRows + r] * w1;
-            if (r0 + r >= M) continue;
+            for (int i = 0; i < 16; i++) po[(c * 16 + i) * kRows + r] = nb > 0 ? __uint_as_float(o[i]) : 0.f;
+        }
+        ml[grp * 2 * kRows + r] = m, ml[(grp * 2 + 1) * kRows + r] = l;
+    }
+    __syncthreads();
+    if (!control) {  // a group's thread takes 64 / kGroups dims of its row
+        constexpr int DIMS = kD / kGroups;
+        const int r = wq * 32 + lane;
+        float mg[kGroups], w[kGroups], top = -INFINITY, sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < kGroups; i++) mg[i] = ml[i * 2 * kRows + r], top = fmaxf(top, mg[i]);  // (key 0 is in group 0: finite)
+#pragma unroll
+        for (int i = 0; i < kGroups; i++) w[i] = ex2f((mg[i] - top) * sl2), sum += ml[(i * 2 + 1) * kRows + r] * w[i];
+        float v[DIMS];
+#pragma unroll
+        for (int d = 0; d < DIMS; d++) v[d] = 0.f;
+#pragma unroll
+        for (int i = 0; i < kGroups; i++) {
+            const float *po = (const float *)(smem + kQBytes + i * kGroupBytes) + grp * DIMS * kRows + r;
+            const float wi = w[i] / sum;
+#pragma unroll
+            for (int d = 0; d < DIMS; d++) v[d] = fmaf(po[d * kRows], wi, v[d]);
+        }
+        const int64_t at = (int64_t)(r0 + r) * (H * kD) + h * kD + grp * DIMS;
+        if (r0 + r < M) {
             if (out16) {  // the o projection takes the fp16 value it would round to itself
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const __half2 pr = __floats2half2_rn(v[i], v[(i + 1) & 15]);
-                    o[i] = *reinterpret_cast<const uint32_t *>(&pr);
+                for (int d = 0; d < DIMS; d += 8) {
+                    uint32_t o[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const __half2 pr = __floats2half2_rn(v[d + 2 * i], v[d + 2 * i + 1]);
+                        o[i] = *reinterpret_cast<const uint32_t *>(&pr);
+                    }
+                    *reinterpret_cast<uint4 *>(out16 + at + d) = make_uint4(o[0], o[1], o[2], o[3]);
                 }
-                *reinterpret_cast<uint4 *>(out16 + at + c * 16) = make_uint4(o[0], o[2], o[4], o[6]);
-                *reinterpret_cast<uint4 *>(out16 + at + c * 16 + 8) = make_uint4(o[8], o[10], o[12], o[14]);
             } else {
 #pragma unroll
-                for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4 *>(out + at + c * 16 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                for (int d = 0; d < DIMS; d += 4) *reinterpret_cast<float4 *>(out + at + d) = make_float4(v[d], v[d + 1], v[d + 2], v[d + 3]);
             }
         }
     }
