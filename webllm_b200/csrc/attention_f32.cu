@@ -2,18 +2,29 @@
 // src/reference/qwen-ref.ts:67-116) for the uncached forward, the fp32-activation mode and prompts too short for the fp16
 // tensor-core kernel, head size 64.
 //
-// One CTA = 32 query rows of one head; keys in blocks of 32 staged in shared memory as f32, scores and weighted sums from
+// One CTA = 32 query rows of one head; keys in blocks of 32, staged in shared memory as f32, that four groups of four warps take in
+// turn, their states of a row merged at the end; scores and weighted sums from
 // 4 x 2 and 4 x 4 register tiles, online softmax. One CTA per single row, as the scalar kernel (qwen_ops.cu) has it, reads every
-// key 32 times as often and leaves a warp's lanes one multiply per load. 4 x 101 rows, 14 heads: 57 -> 22 us a layer; what is
-// left is the chain of up to four key blocks in a grid of 224 CTAs.
+// key 32 times as often and leaves a warp's lanes one multiply per load. 4 x 101 rows, 14 heads: 57 -> 22 us a layer with
+// one group, whose chain of key blocks it was, 17 with four.
 #include "qwen_ops.cuh"
 
 namespace wb {
 
 namespace {
 
-constexpr int kD = 64, kRows = 32, kKeys = 32, kThreads = 128;
+constexpr int kD = 64, kRows = 32, kKeys = 32, kGroups = 4, kThreads = kGroups * 128;
 constexpr int kQP = kRows + 4, kKP = kKeys + 2, kVP = kD + 4;
+struct GroupSmem {
+    float Ks[kD][kKP];
+    float Vs[kKeys][kVP];  // later the group's sums, [rows][dims]
+    float Ps[kKeys][kQP];
+};
+struct Smem {
+    float Qs[kD][kQP];
+    GroupSmem g[kGroups];
+    float m[kGroups][kRows], l[kGroups][kRows];
+};
 
 __device__ __forceinline__ float4 load4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 __device__ __forceinline__ float4 load4(const __half *p)
@@ -26,13 +37,19 @@ __device__ __forceinline__ float4 load4(const __half *p)
 // Rows i of sequence b (row b * T + i of q and out) see keys 0 .. past + i, row b * key_rows + key of kmem / vmem.
 template <typename KV>
 __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__restrict__ q, const KV *__restrict__ kmem,
-                                                                 const KV *__restrict__ vmem, float *__restrict__ out, int H, int KVH, int T,
+                                                                 const KV *__restrict__ vmem, float *__restrict__ out, __half *__restrict__ out16, int H, int KVH, int T,
                                                                  const int *__restrict__ past_ptr, int past_imm, int key_rows, int ldq,
                                                                  int kv_ld, float scale)
 {
     pdl_sync();
-    __shared__ __align__(16) float Qs[kD][kQP], Ks[kD][kKP], Vs[kKeys][kVP], Ps[kKeys][kQP];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tid & 15, ty = tid >> 4;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
+    const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127, lane = tid & 31, warp = tid >> 5, tx = tid & 15, ty = tid >> 4;
+    auto &Qs = sm.Qs;
+    auto &Ks = sm.g[grp].Ks;
+    auto &Vs = sm.g[grp].Vs;
+    auto &Ps = sm.g[grp].Ps;
+    auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory"); };
     const int tile = (int)gridDim.y - 1 - (int)blockIdx.y;  // late (long) tiles first
     const int i0 = tile * kRows, b = blockIdx.z, h = blockIdx.x, kvh = h / (H / KVH);
     const int past = past_ptr ? *past_ptr : past_imm;
@@ -40,15 +57,16 @@ __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__
     const KV *kb = kmem + (int64_t)b * key_rows * kv_ld + kvh * kD, *vb = vmem + (int64_t)b * key_rows * kv_ld + kvh * kD;
     const int64_t row0 = (int64_t)b * T + i0;
     // a lane stages its row (key), a warp every fourth 4 dims
-    for (int d = warp * 4; d < kD; d += 16) {
+    for (int d = (int)(threadIdx.x >> 5) * 4; d < kD; d += kGroups * 16) {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i0 + lane < T) v = load4(q + (row0 + lane) * ldq + h * kD + d);
         Qs[d][lane] = v.x, Qs[d + 1][lane] = v.y, Qs[d + 2][lane] = v.z, Qs[d + 3][lane] = v.w;
     }
+    __syncthreads();
     float o[4][4] = {}, m[4], l[4] = {};
 #pragma unroll
     for (int i = 0; i < 4; i++) m[i] = -INFINITY;
-    for (int key0 = 0; key0 < n_keys; key0 += kKeys) {
+    for (int key0 = grp * kKeys; key0 < n_keys; key0 += kGroups * kKeys) {
         const bool in = key0 + lane < n_keys;
         for (int d = warp * 4; d < kD; d += 16) {
             float4 k = make_float4(0.f, 0.f, 0.f, 0.f), v = k;
@@ -56,7 +74,7 @@ __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__
             Ks[d][lane] = k.x, Ks[d + 1][lane] = k.y, Ks[d + 2][lane] = k.z, Ks[d + 3][lane] = k.w;
             *reinterpret_cast<float4 *>(&Vs[lane][d]) = v;
         }
-        __syncthreads();
+        group_sync();
         float s[4][2] = {};  // rows 4 ty + i, keys 2 tx + j
 #pragma unroll 8
         for (int d = 0; d < kD; d++) {
@@ -76,7 +94,7 @@ __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__
             float mx = fmaxf(s[i][0], s[i][1]);
 #pragma unroll
             for (int w = 8; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
-            const float mn = fmaxf(m[i], mx), c = m[i] == -INFINITY ? 0.f : expf(m[i] - mn);
+            const float mn = fmaxf(m[i], mx), c = m[i] == -INFINITY ? 0.f : expf(m[i] - mn);  // (a block may hide all its keys from a row)
             l[i] *= c;
 #pragma unroll
             for (int j = 0; j < 4; j++) o[i][j] *= c;
@@ -95,17 +113,39 @@ __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__
             o[2][0] = fmaf(a.z, v.x, o[2][0]), o[2][1] = fmaf(a.z, v.y, o[2][1]), o[2][2] = fmaf(a.z, v.z, o[2][2]), o[2][3] = fmaf(a.z, v.w, o[2][3]);
             o[3][0] = fmaf(a.w, v.x, o[3][0]), o[3][1] = fmaf(a.w, v.y, o[3][1]), o[3][2] = fmaf(a.w, v.z, o[3][2]), o[3][3] = fmaf(a.w, v.w, o[3][3]);
         }
-        __syncthreads();
+        group_sync();
     }
 #pragma unroll
     for (int i = 0; i < 4; i++) {
 #pragma unroll
         for (int w = 8; w > 0; w >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], w);
         const int r = ty * 4 + i;
-        if (i0 + r >= T) continue;
-        const float inv = 1.f / l[i];
-        *reinterpret_cast<float4 *>(out + (row0 + r) * (H * kD) + h * kD + tx * 4) =
-            make_float4(o[i][0] * inv, o[i][1] * inv, o[i][2] * inv, o[i][3] * inv);
+        *reinterpret_cast<float4 *>(&Vs[r][tx * 4]) = make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
+        if (tx == 0) sm.m[grp][r] = m[i], sm.l[grp][r] = l[i];
+    }
+    __syncthreads();
+    // four dims of a row per thread (group 0 has key 0, so the largest maximum is finite)
+    static_assert(kThreads == kRows * kD / 4, "one float4 of the result per thread");
+    const int r = (int)(threadIdx.x >> 4);
+    float mt = sm.m[0][r], lt = 0.f;
+    for (int i = 1; i < kGroups; i++) mt = fmaxf(mt, sm.m[i][r]);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < kGroups; i++) {
+        const float w = expf(sm.m[i][r] - mt);
+        const float4 a = *reinterpret_cast<const float4 *>(&sm.g[i].Vs[r][tx * 4]);
+        lt = fmaf(sm.l[i][r], w, lt);
+        v.x = fmaf(a.x, w, v.x), v.y = fmaf(a.y, w, v.y), v.z = fmaf(a.z, w, v.z), v.w = fmaf(a.w, w, v.w);
+    }
+    if (i0 + r >= T) return;
+    const float inv = 1.f / lt;
+    const int64_t at = (row0 + r) * (H * kD) + h * kD + tx * 4;
+    v.x *= inv, v.y *= inv, v.z *= inv, v.w *= inv;
+    if (out16) {  // the o projection takes the fp16 value it would round to itself
+        const __half2 a = __floats2half2_rn(v.x, v.y), c = __floats2half2_rn(v.z, v.w);
+        *reinterpret_cast<uint2 *>(out16 + at) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&c));
+    } else {
+        *reinterpret_cast<float4 *>(out + at) = v;
     }
 }
 
@@ -115,15 +155,18 @@ __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__
 bool op_attention_f32_supported(int M, int D, int ldq, int kv_ld) { return M > 1 && D == kD && ldq % 4 == 0 && kv_ld % 4 == 0; }
 
 int op_attention_f32(wb_context *ctx, const float *q, const void *kmem, const void *vmem, int kv_f16, float *out, int M, int H, int KVH, int T,
-                     const int *past_ptr, int past_imm, int use_cache, int ldq, int kv_ld)
+                     const int *past_ptr, int past_imm, int use_cache, int ldq, int kv_ld, __half *out16)
 {
     const float scale = 1.0f / sqrtf((float)kD);
     const dim3 grid((unsigned)H, (unsigned)((T + kRows - 1) / kRows), (unsigned)(M / T));
     const int key_rows = use_cache ? 0 : T;  // (one sequence with a cache)
+    if (const cudaError_t e = kv_f16 ? smem_limit_once<attention_f32_kernel<__half>>((int)sizeof(Smem)) : smem_limit_once<attention_f32_kernel<float>>((int)sizeof(Smem));
+        e != cudaSuccess)
+        WB_CUDA(e);
     const cudaError_t e =
-        kv_f16 ? launch_pdl(attention_f32_kernel<__half>, grid, dim3(kThreads), 0, ctx->stream, q, (const __half *)kmem, (const __half *)vmem, out, H,
+        kv_f16 ? launch_pdl(attention_f32_kernel<__half>, grid, dim3(kThreads), sizeof(Smem), ctx->stream, q, (const __half *)kmem, (const __half *)vmem, out, out16, H,
                             KVH, T, past_ptr, past_imm, key_rows, ldq, kv_ld, scale)
-               : launch_pdl(attention_f32_kernel<float>, grid, dim3(kThreads), 0, ctx->stream, q, (const float *)kmem, (const float *)vmem, out, H,
+               : launch_pdl(attention_f32_kernel<float>, grid, dim3(kThreads), sizeof(Smem), ctx->stream, q, (const float *)kmem, (const float *)vmem, out, out16, H,
                             KVH, T, past_ptr, past_imm, key_rows, ldq, kv_ld, scale);
     ctx->launches++;
     WB_CUDA(e);
