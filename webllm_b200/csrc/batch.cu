@@ -45,8 +45,17 @@ int record_before(wb_context *ctx, const void *r0, uint64_t r_bytes, const void 
     if (now != o.left) o.ops.clear(), o.base = now;  // something else was captured: it, and all before it, comes first
     BatchOrder::Op op;
     op.r0 = (const char *)r0, op.r1 = op.r0 + r_bytes, op.w0 = (const char *)w0, op.w1 = op.w0 + w_bytes;
-    for (const BatchOrder::Op &b : o.ops)
-        if (overlap(op.r0, op.r1, b.w0, b.w1) || overlap(op.w0, op.w1, b.r0, b.r1) || overlap(op.w0, op.w1, b.w0, b.w1)) deps.push_back(b.node);
+    // from the last one back, without those that an earlier find already waits for (a plain chain stays one: each call waits for the
+    // call before it and may start its prologue under it)
+    op.before.assign(o.ops.size(), false);
+    for (size_t i = o.ops.size(); i-- > 0;) {
+        BatchOrder::Op &b = o.ops[i];
+        if (op.before[i] || !(overlap(op.r0, op.r1, b.w0, b.w1) || overlap(op.w0, op.w1, b.r0, b.r1) || overlap(op.w0, op.w1, b.w0, b.w1))) continue;
+        deps.push_back(b.node);
+        b.leaf = false, op.before[i] = true;
+        for (size_t k = 0; k < b.before.size(); k++)
+            if (b.before[k]) op.before[k] = true;
+    }
     if (deps.empty()) deps = o.base;
     if (deps.size() > 1) {  // one node to wait for
         cudaGraphNode_t join;
@@ -65,9 +74,10 @@ int record_after(wb_context *ctx)
     WB_CHECK(capture_state(ctx, &graph, &now));
     if (now.size() != 1) return fail(WB_ERR_CUDA, "a recorded call left %d graph nodes", (int)now.size());
     o.ops.back().node = now[0];
-    // whatever is captured by other means waits for all of them
+    // whatever is captured by other means waits for all of them (by way of those that no other call waits for)
     now.clear();
-    for (const BatchOrder::Op &b : o.ops) now.push_back(b.node);
+    for (const BatchOrder::Op &b : o.ops)
+        if (b.leaf) now.push_back(b.node);
     WB_CHECK(set_capture_state(ctx, now));
     return capture_state(ctx, &graph, &o.left);
 }

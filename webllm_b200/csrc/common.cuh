@@ -72,6 +72,8 @@ struct BatchOrder {
     struct Op {
         const char *r0, *r1, *w0, *w1;  // bytes read and written
         cudaGraphNode_t node = nullptr;
+        bool leaf = true;          // no later call waits for it
+        std::vector<bool> before;  // the calls that it waits for, directly or not
     };
     std::vector<Op> ops;
     std::vector<cudaGraphNode_t> base, left;  // nodes to wait for where no call conflicts; the stream's state after the last call

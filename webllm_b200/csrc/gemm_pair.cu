@@ -17,7 +17,7 @@
 //   * The weights are constants: the producer requests the packed boxes of the first stages, and the unpack sets unpack
 //     them, before the wait on the previous kernel (programmatic dependent launch); the activation loads and the
 //     epilogue's stores come after it.
-//   * Where a work item is short (K = 896: 14 k-blocks) the result leaves through four 8 KB staging tiles and TMA stores
+//   * Where a work item is short (K = 896: 14 k-blocks) the result leaves through two 16 KB staging tiles and TMA stores
 //     (fp16, f32, or the f32 partial sums of a K slice; STG instantiations); where it is long, from registers, and the
 //     shared memory holds a sixth pipeline stage instead.
 //   * A launch whose last round of work items would leave most pairs idle for a long item cuts those items along K over
@@ -41,23 +41,23 @@ namespace tcp {
 using namespace tc;
 
 // Warp roles as listed at MMA_WARP (gemm_tc.cuh), plus the epilogue warps from 21 on, in groups of four (a warp reads the
-// tensor-memory lane quarter id % 4). Short work items, those that leave through staging tiles, have two groups that take the
-// chunks of token rows in turn: at K = 896 an item's MMAs last 5 us, and one group needed 9 us to drain it with silu, since the
-// unpack warps leave it few issue slots (gate | up with silu at 2048 rows: 67 us with one group, 54 us with two; the same GEMM
-// and the separate pass before: 43.7 + 17.8 us). 29 warps of 64 registers.
-constexpr int epi_groups(bool stg) { return stg ? 2 : 1; }
-constexpr int pair_threads(bool stg) { return 32 * (WARPS + 4 * epi_groups(stg)); }
+// tensor-memory lane quarter id % 4). With silu there are two groups that take the chunks of token rows in turn: at K = 896 an item's
+// MMAs last 5 us, and one group needed 9 us to drain it, since the unpack warps leave it few issue slots (gate | up with silu at
+// 2048 rows: 67 us with one group, 54 us with two; the GEMM and the separate pass before: 43.7 + 17.8 us; 29 warps of 64
+// registers). A plain result leaves faster than the MMAs come, and one group with larger tiles is 2 to 4 % quicker.
+constexpr int epi_groups(bool silu) { return silu ? 2 : 1; }
+constexpr int pair_threads(bool silu) { return 32 * (WARPS + 4 * epi_groups(silu)); }
 constexpr int KG = 4;  // unpack sets: 128 threads each, one thread per weight column
-constexpr int STG_BYTES = STG_ROWS * BN * 2;  // an epilogue staging tile: [32 tokens][128 columns] fp16 or [16][128] f32
+constexpr int STG_BYTES = STG_ROWS * BN * 2;  // an epilogue staging tile: [64 tokens][128 columns] fp16 or [32][128] f32
 
-// STG: two epilogue staging tiles per group are carved out of the shared memory (one pipeline stage fewer for the 256-token tile)
+// STG: two epilogue staging tiles are carved out of the shared memory (one pipeline stage fewer for the 256-token tile)
 template <int MT, bool STG>
 struct SmemPair {
     static constexpr int X_BYTES = (MT / 2) * BK * 2;   // this CTA's half of the activation tile
     static constexpr int WD_BYTES = BN * BK * 2;        // unpacked fp16 operand, 128 columns x 64 k
     static constexpr int WP_BYTES = 8 * BN * 4;         // packed box, 8 rows x 128 columns
     static constexpr int STAGE_BYTES = X_BYTES + WD_BYTES + WP_BYTES;  // every piece is a multiple of 1024
-    static constexpr int STG_TOTAL = STG ? 2 * epi_groups(STG) * STG_BYTES : 0;
+    static constexpr int STG_TOTAL = STG ? 2 * STG_BYTES : 0;
     static constexpr int MAX_STAGES = (227 * 1024 - 1280 - STG_TOTAL) / STAGE_BYTES;
     static constexpr int STAGES = MAX_STAGES > 6 ? 6 : MAX_STAGES;
     static constexpr int TOTAL = STAGES * STAGE_BYTES + STG_TOTAL + 1024 /*alignment slack*/ + 256 /*barriers*/;
@@ -135,7 +135,7 @@ __device__ __forceinline__ float silu(float g)
 // of the rows each way, and compute in f32 what a pass over the f32 result would. At 2048 x 896 -> 2 x 4864 that pass moved
 // 100 MB and took 18 us, and the GEMM itself stored 80 MB instead of 20.
 template <int MT, bool SPLIT, bool STG, bool GATHER = false, bool SILU = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(STG), 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(SILU), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                  const __grid_constant__ CUtensorMap map_c, const Params p, const int tiles_m, const int tiles_n, const int n_items,
                  const int use_tma_store, const PairTail tail)
@@ -148,7 +148,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     static_assert(USED <= 512 && MT % STG_ROWS == 0 && MT >= 128, "token tile");
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t *stg = smem + STAGES * S::STAGE_BYTES;  // two epilogue staging tiles per group
+    uint8_t *stg = smem + STAGES * S::STAGE_BYTES;  // two epilogue staging tiles
     uint64_t *bars = (uint64_t *)(stg + S::STG_TOTAL);
     uint64_t *full_w = bars, *ready = bars + STAGES, *empty = bars + 2 * STAGES;
     uint64_t *acc_full = bars + 3 * STAGES, *acc_empty = bars + 3 * STAGES + 2;
@@ -196,7 +196,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 2 * 4 * epi_groups(STG));
+            mbar_init(&acc_empty[b], 2 * 4 * epi_groups(SILU));
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -375,7 +375,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
     } else if (warp >= WARPS) {
         // ------------------------------------------------------------------ epilogue: warp w drains TMEM lanes 32 * (w % 4) ..
-        constexpr int GROUPS = epi_groups(STG);
+        constexpr int GROUPS = epi_groups(SILU);
         const int q = warp & 3, eg = (warp - WARPS) >> 2;
         const int epi_tid = (warp - WARPS) * 32 + lane - eg * 128;  // 0 .. 127 within the group, thread 0 issues the stores
         const uint32_t acc_empty0 = cluster_map_shared(&acc_empty[0], 0);
@@ -419,7 +419,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 // given. (A group's barrier after the products also says that the exchange tile has been read.)
                 const int col = (q & 1) * 32 + lane;
                 const bool is_up = q >= 2;
-                uint8_t *mine = stg + eg * 2 * STG_BYTES;
+                uint8_t *mine = stg + eg * STG_BYTES;
                 float *ex = (float *)mine;  // [32 rows][64 columns]
                 auto rows16 = [&](int c, auto &&f) {
                     uint32_t r[16];
@@ -430,8 +430,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 };
                 const int give = is_up ? 0 : 16, keep = 16 - give;
 #pragma unroll 1
-                for (int c = eg * STG_ROWS; c < MT; c += GROUPS * STG_ROWS) {
-                    __half *tile = (__half *)(mine + STG_BYTES) + stg_sel * STG_ROWS * 64;  // [32 rows][64 columns], two of them
+                for (int c = eg * SILU_ROWS; c < MT; c += GROUPS * SILU_ROWS) {
+                    __half *tile = (__half *)(mine + STG_BYTES / 2) + stg_sel * SILU_ROWS * 64;  // [32 rows][64 columns], two of them
                     rows16(c + give, [&](int j, float v) { ex[(give + j) * 64 + col] = v; });
                     if (epi_tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                     group_sync();
@@ -458,7 +458,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 StoreDst dt;
                 dt.dst[0] = tail.partial + (size_t)pair * MT * (2 * BN), dt.n_dst = 1, dt.ld = 2 * BN, dt.col0 = 0;
 #pragma unroll 1
-                for (int c = eg * 16; c < MT; c += GROUPS * 16) {
+                for (int c = 0; c < MT; c += 16) {
                     uint32_t r[16];
                     tmem_ld_32x32b_x16(acc + (uint32_t)c, r);
                     tmem_ld_wait();
@@ -466,7 +466,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 }
             } else if (!STG || !use_tma_store) {
 #pragma unroll 1
-                for (int c = eg * 16; c < MT; c += GROUPS * 16) {
+                for (int c = 0; c < MT; c += 16) {
                     uint32_t r[16];
                     tmem_ld_32x32b_x16(acc + (uint32_t)c, r);
                     tmem_ld_wait();
@@ -475,17 +475,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             } else {
                 // The result leaves through shared memory: a lane holds one output column of 16 token rows, so it writes
                 // 16 words into a [tokens][128 columns] staging tile (no exchange between lanes, no dependent chain), and
-                // one thread hands each finished tile to a TMA store, which also clips the ragged edges. A tile is 8 KB:
-                // 32 token rows of fp16 or 16 of f32 (also the partial sums of a K slice, third map coordinate). Two tiles
-                // of a group alternate; a tile is rewritten once the store that read it has finished reading.
+                // one thread hands each finished tile to a TMA store, which also clips the ragged edges. A tile is 16 KB:
+                // 64 token rows of fp16 or 32 of f32 (also the partial sums of a K slice, third map coordinate). Two tiles
+                // alternate; a tile is rewritten once the store that read it has finished reading.
                 const bool o16 = !SPLIT && out16;
                 const int rows = o16 ? STG_ROWS : STG_ROWS / 2;
                 const int slice = SPLIT ? item_slice(ti) : 0;
 #pragma unroll 1
-                for (int c = eg * rows; c < MT; c += GROUPS * rows) {
+                for (int c = 0; c < MT; c += rows) {
                     if (epi_tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                     group_sync();
-                    uint8_t *tile_base = stg + (eg * 2 + stg_sel) * STG_BYTES;
+                    uint8_t *tile_base = stg + stg_sel * STG_BYTES;
 #pragma unroll 1
                     for (int cc = 0; cc < rows; cc += 16) {
                         uint32_t r[16];
@@ -601,22 +601,22 @@ static cudaError_t launch_pair_mt(const CUtensorMap &mx, const CUtensorMap &mw, 
     const int n_items = tiles_m * tiles_n * S;
     int pairs = sms / 2;
     if (pairs > n_items) pairs = n_items;
-    auto go = [&](auto kernel, int variant, int smem, bool stg) -> cudaError_t {
+    auto go = [&](auto kernel, int variant, int smem) -> cudaError_t {
         if (!(dev >= 0 && dev < 16 && attr_set[variant][dev])) {
             cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return e;
             if (dev >= 0 && dev < 16) attr_set[variant][dev] = true;
         }
-        return launch_pdl(kernel, dim3((unsigned)(2 * pairs)), dim3((unsigned)tcp::pair_threads(stg)), (size_t)smem, st, mx, mw, mc ? *mc : mx, p, tiles_m,
+        return launch_pdl(kernel, dim3((unsigned)(2 * pairs)), dim3((unsigned)tcp::pair_threads(silu)), (size_t)smem, st, mx, mw, mc ? *mc : mx, p, tiles_m,
                           tiles_n, n_items, mc ? 1 : 0, tail);
     };
-    if (silu) return go(tcp::gemm_pair_kernel<MT, false, true, false, true>, 5, tcp::SmemPair<MT, true>::TOTAL, true);
+    if (silu) return go(tcp::gemm_pair_kernel<MT, false, true, false, true>, 5, tcp::SmemPair<MT, true>::TOTAL);
     if (S > 1)
-        return mc ? go(tcp::gemm_pair_kernel<MT, true, true>, 3, tcp::SmemPair<MT, true>::TOTAL, true)
-                  : go(tcp::gemm_pair_kernel<MT, true, false>, 1, tcp::SmemPair<MT, false>::TOTAL, false);
-    if (p.n_dst > 0) return go(tcp::gemm_pair_kernel<MT, false, false, true>, 4, tcp::SmemPair<MT, false>::TOTAL, false);
-    if (mc) return go(tcp::gemm_pair_kernel<MT, false, true>, 2, tcp::SmemPair<MT, true>::TOTAL, true);
-    return go(tcp::gemm_pair_kernel<MT, false, false>, 0, tcp::SmemPair<MT, false>::TOTAL, false);
+        return mc ? go(tcp::gemm_pair_kernel<MT, true, true>, 3, tcp::SmemPair<MT, true>::TOTAL)
+                  : go(tcp::gemm_pair_kernel<MT, true, false>, 1, tcp::SmemPair<MT, false>::TOTAL);
+    if (p.n_dst > 0) return go(tcp::gemm_pair_kernel<MT, false, false, true>, 4, tcp::SmemPair<MT, false>::TOTAL);
+    if (mc) return go(tcp::gemm_pair_kernel<MT, false, true>, 2, tcp::SmemPair<MT, true>::TOTAL);
+    return go(tcp::gemm_pair_kernel<MT, false, false>, 0, tcp::SmemPair<MT, false>::TOTAL);
 }
 
 // mc: tensor map of the result or of the K slices' partial sums ([slices, M, N], boxes of 128 columns x 64 fp16 or 32 f32

@@ -865,7 +865,7 @@ int plan_gemm_tc(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int
             plan->grid_x = (int)((M + pmt - 1) / pmt);
             plan->grid_y = (int)((w.N + 255) / 256);
             plan->split_k = plan->grid_z = pS;
-            plan->block = pmt < 256 || (kblocks + pS - 1) / pS <= kPairStageKb ? 928 : 800;  // staged results: eight epilogue warps
+            plan->block = 800;
             plan->tile_m = pmt;
             plan->tile_n = 256;
             mt = pmt, nh = 2, S = pS;
@@ -1094,7 +1094,7 @@ int launch_gate_up_silu(wb_context *ctx, const Weight &w, const __half *A, __hal
     if (cc.base != act || cc.M != M || cc.a != -1) {
         cc.base = nullptr;
         cuuint64_t dims[3] = {(cuuint64_t)I, (cuuint64_t)M, 1}, strides[2] = {(cuuint64_t)I * 2, (cuuint64_t)I * M * 2};
-        cuuint32_t box[3] = {tc::BN / 2, tc::STG_ROWS, 1}, estr[3] = {1, 1, 1};
+        cuuint32_t box[3] = {tc::BN / 2, tc::SILU_ROWS, 1}, estr[3] = {1, 1, 1};
         const CUresult r = ((EncodeTiledFn)ctx->tmap_encode)(&mc, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, act, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return fail(WB_ERR_CUDA, "cuTensorMapEncodeTiled (result) failed with code %d", (int)r);
