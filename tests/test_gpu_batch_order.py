@@ -19,6 +19,7 @@ def test_recorded_calls_see_their_inputs(built_lib, M):
         t = [gpu.arena.alloc(M * K, [M, K]) for _ in range(6)]
         long = gpu.arena.alloc(M * 4 * K, [M, 4 * K])
         tail = Tensor(long.offset + 3 * M * K * 4, M * K, [M, K])  # the last quarter of `long`
+        many = [gpu.arena.alloc(M * K, [M, K]) for _ in range(11)]
         x = np.random.default_rng(M).standard_normal(M * K).astype(np.float32)
 
         def calls():
@@ -32,11 +33,14 @@ def test_recorded_calls_see_their_inputs(built_lib, M):
             gpu.gptq_dequant(w[0], deq)              # stream order
             gpu.linear(w[0], t[4], t[5], None, M)
             gpu.linear(w[1], t[5], t[4], None, M)
+            for i, y in enumerate(many):             # more than run side by side
+                gpu.linear(w[i % 3], t[5], y, None, M)
+            gpu.linear(w[0], many[0], t[1], None, M)
 
         def result(run):
             gpu.write(t[0], x)
             run()
-            return [gpu.read(v) for v in (*t, long, deq)]
+            return [gpu.read(v) for v in (*t, *many, long, deq)]
 
         ref = result(calls)
         with gpu.batch() as b:

@@ -56,6 +56,17 @@ int record_before(wb_context *ctx, const void *r0, uint64_t r_bytes, const void 
         for (size_t k = 0; k < b.before.size(); k++)
             if (b.before[k]) op.before[k] = true;
     }
+    // At most so many abreast: the graph's branches are streams that the driver sets up at wb_batch_end (a layer 0.6 ms, in sequence
+    // 0.2), and a chip full of decode-size calls gains nothing from more. (Layer at M = 4, abreast 1 / 2 / 4 / all 7, us a submit at
+    // the clocks of an idle chip: 28.7, 20.5, 17.1, 15.7.)
+    constexpr size_t kWidth = 8;
+    if (deps.empty() && o.ops.size() >= kWidth) {
+        const size_t i = o.ops.size() - kWidth;
+        deps.push_back(o.ops[i].node);
+        o.ops[i].leaf = false, op.before[i] = true;
+        for (size_t k = 0; k < o.ops[i].before.size(); k++)
+            if (o.ops[i].before[k]) op.before[k] = true;
+    }
     if (deps.empty()) deps = o.base;
     if (deps.size() > 1) {  // one node to wait for
         cudaGraphNode_t join;

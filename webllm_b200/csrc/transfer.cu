@@ -2,7 +2,7 @@
 // logits, dense weights).
 //
 // A cudaMemcpy of pageable memory goes through the driver's own staging buffer and one thread: 20 GB/s, where the link does 55 and
-// one core's copy 18. Copies of 2 MB and more pass through a ring of pinned slots instead: while the calling thread keeps the
+// one core's copy 18. Copies of 2 MB and more (to the device 8 MB: 2.2 MB up took 157 us either way) pass through a ring of pinned slots instead: while the calling thread keeps the
 // transfers going, three helper threads (six measured no better) copy the pieces between the slots and the caller's memory.
 // 512 KB pieces: smaller ones lose to the gap between two transfers, larger ones to the first and the last piece. Measured on 16
 // cores: 17.4 MB to the host 850 -> 490 us, 64 MB either way 2.8 -> 1.8 ms.
@@ -22,7 +22,7 @@
 namespace wb {
 namespace {
 
-constexpr size_t kPiece = 512 << 10, kHelpersFrom = 2 << 20;
+constexpr size_t kPiece = 512 << 10, kHelpersFrom = 2 << 20, kHelpersUpFrom = 8 << 20;
 constexpr int kSlots = 16, kHelpersMax = 3, kSpins = 20000;  // spins: about a millisecond
 
 struct Job {
@@ -185,7 +185,7 @@ int copy(wb_context *ctx, void *host, void *dev, size_t bytes, bool to_host)
 {
     std::unique_lock<std::mutex> lk(g_ring.use, std::defer_lock);
     cudaPointerAttributes at;
-    if (bytes >= kHelpersFrom && (cudaPointerGetAttributes(&at, host) != cudaSuccess || at.type == cudaMemoryTypeUnregistered) && lk.try_lock()) {
+    if (bytes >= (to_host ? kHelpersFrom : kHelpersUpFrom) && (cudaPointerGetAttributes(&at, host) != cudaSuccess || at.type == cudaMemoryTypeUnregistered) && lk.try_lock()) {
         WB_CHECK(g_ring.prepare(ctx->device));
         Job j;
         j.host = (char *)host, j.bytes = bytes, j.pieces = (int)((bytes + kPiece - 1) / kPiece), j.to_host = to_host;
