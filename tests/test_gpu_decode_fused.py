@@ -51,3 +51,36 @@ def test_fused_decode_matches_oracle(built_lib, oracle, C, H, KVH, I, V, prompt,
             row = model.read_tensor(model.decode_step(t))
         assert int(row.argmax()) == want[3]
         model.close()
+
+
+@pytest.mark.parametrize("kv", ["f16", "f32"])
+@pytest.mark.parametrize("prompt", [3, 140])
+def test_attention_takes_values_beyond_fp16(built_lib, oracle, kv, prompt):
+    """One pair of rotated dims of the query (fp16 cache) or of the cached keys (f32 cache) is about 1e6, and the other side has
+    zeros there, so the scores stay ordinary: f32 arithmetic sees no difference, operands rounded to fp16 are infinite."""
+    cfg = synthetic.QwenShape(300, 2, 4, 2, 256, 1280)
+    G = synthetic.random_qwen_gptq(cfg, seed=prompt, std=0.05)
+    large, zero = ("q", "k") if kv == "f16" else ("k", "q")
+    for layer in G["layers"]:
+        for name, bias in ((large, 1e6), (zero, 0.0)):
+            cols = np.arange(layer[name].out_features) % 32 == 7  # dims 7 and 39 of every head turn together
+            layer[name].scales[:, cols] = 0
+            layer[name + "_bias"][cols] = bias
+    ids = np.random.default_rng(prompt).integers(0, cfg.vocab_size, prompt).astype(np.uint32)
+    ref = oracle.CachedForward(_ocfg(oracle, cfg), _dense_from_gptq(oracle, G), max_t=prompt + 8, kv_f16=kv == "f16",
+                               threads=oracle.max_threads())
+    tok = first = oracle.sample_greedy(ref.prefill(ids))
+    want = []
+    for _ in range(4):
+        row = ref.decode_step(tok)
+        tok = oracle.sample_greedy(row)
+        want.append(tok)
+    rms = float(np.sqrt(np.mean(row.astype(np.float64) ** 2)))
+    with Gpu(0, weight_bytes=64 << 20, act_bytes=64 << 20) as gpu:
+        model = QwenGpt(gpu, cfg, max_t=prompt + 8, kv_dtype=kv)
+        model.upload_gptq_model(G, fuse=True)
+        model.set_exact(True)
+        model.prefill(ids, last_only=True)
+        assert model.decode_greedy(first, 4).tolist() == want
+        assert oracle.check_tolerance(model.last_logits(), row, 5e-4 * rms, 5e-4).ok
+        model.close()
