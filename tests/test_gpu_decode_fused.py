@@ -84,3 +84,24 @@ def test_attention_takes_values_beyond_fp16(built_lib, oracle, kv, prompt):
         assert model.decode_greedy(first, 4).tolist() == want
         assert oracle.check_tolerance(model.last_logits(), row, 5e-4 * rms, 5e-4).ok
         model.close()
+
+
+@pytest.mark.parametrize("what", ["nan", "beyond fp16"])
+def test_mlp_activations_that_are_no_fp16_numbers(built_lib, what):
+    """A NaN in the MLP, or an activation that fp16 cannot hold, comes out as NaN, as it does from the separate projections (their
+    operands are fp16 value and remainder too)."""
+    cfg = synthetic.QwenShape(300, 1, 4, 2, 256, 1280)
+    G = synthetic.random_qwen_gptq(cfg, seed=5, std=0.05)
+    layer = G["layers"][0]
+    if what == "nan":
+        layer["post_norm"][7] = np.nan
+    else:
+        layer["gate"].scales *= np.float16(1e3)
+        layer["up"].scales *= np.float16(1e3)
+    for fuse in (True, False):
+        with Gpu(0, weight_bytes=64 << 20, act_bytes=64 << 20) as gpu:
+            model = QwenGpt(gpu, cfg, max_t=16, kv_dtype="f32")
+            model.upload_gptq_model(G, fuse=fuse)
+            model.prefill(np.arange(3, dtype=np.uint32), last_only=True)
+            assert np.isnan(model.read_tensor(model.decode_step(1))).all(), fuse
+            model.close()

@@ -177,11 +177,14 @@ __device__ __forceinline__ float2 ll_get2(const u64 *p, uint32_t ep, Head *hd)
     return ll_vals(v[0]);
 }
 // The MLP's activations are the one long vector that many CTAs read (4864 values by 112 CTAs), and its bytes are what its
-// hand-over takes, so they travel as 32-bit words with the epoch's parity in the lowest mantissa bit (every word is written in
-// every step). The error, 2^-24 of the value, is below that of the fp16 pairs that it is staged as.
+// hand-over takes, so they travel as 32-bit words with the epoch's parity in the upper exponent bit (every word is written in
+// every step). Scaled by 2^-15 a value below 65536 leaves that bit clear and keeps all of its own bits; from there on the fp16 pair
+// that the reader stages is no number, and neither is it for the word that stands for all of those and for NaN.
+constexpr uint32_t kActParity = 1u << 30, kActTooLarge = kActParity - 1;
 __device__ __forceinline__ void act_put(uint32_t *p, float v, uint32_t ep)
 {
-    const uint32_t w = ((__float_as_uint(v) + (__float_as_uint(v) & 1u)) & ~1u) | (ep & 1u);
+    v *= 1.f / 32768.f;
+    const uint32_t w = (fabsf(v) < 2.f ? __float_as_uint(v) : kActTooLarge) | ((ep & 1u) ? kActParity : 0u);
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(w) : "memory");
 }
 __device__ __forceinline__ uint4 act_load4(const uint32_t *p)
@@ -190,11 +193,12 @@ __device__ __forceinline__ uint4 act_load4(const uint32_t *p)
     asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ bool act_ok(const uint4 &v, uint32_t ep) { return ((ep & 1u) ? (v.x & v.y & v.z & v.w & 1u) : ((~(v.x | v.y | v.z | v.w)) & 1u)) != 0; }
-__device__ __forceinline__ float4 act_vals(const uint4 &v)
+__device__ __forceinline__ bool act_ok(const uint4 &v, uint32_t ep)
 {
-    return make_float4(__uint_as_float(v.x & ~1u), __uint_as_float(v.y & ~1u), __uint_as_float(v.z & ~1u), __uint_as_float(v.w & ~1u));
+    return (((ep & 1u) ? (v.x & v.y & v.z & v.w) : ~(v.x | v.y | v.z | v.w)) & kActParity) != 0;
 }
+__device__ __forceinline__ float act_val(uint32_t w) { return __uint_as_float(w & ~kActParity) * 32768.f; }
+__device__ __forceinline__ float4 act_vals(const uint4 &v) { return make_float4(act_val(v.x), act_val(v.y), act_val(v.z), act_val(v.w)); }
 
 __device__ __forceinline__ float warp_sum(float v)
 {
