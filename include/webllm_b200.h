@@ -262,6 +262,11 @@ typedef struct {
     float rms_eps, rope_theta;
 } wb_qwen_config;
 
+/* The first decode call of a model that the persistent decode kernel takes lays its int4 projections, norms and biases out a
+ * second time, in device memory outside the arenas (0.2 GB for the 0.5B shape; where there is no room the model decodes with one
+ * kernel per projection). wb_upload over registered weights is followed: the next decode call lays them out again. Writes of
+ * the caller's own through device pointers (wb_arena_base, an adopted slab) are not seen there; destroy and create the model
+ * object after them. */
 WB_API int wb_qwen_create(wb_context *ctx, const wb_qwen_config *cfg, wb_qwen **out);
 WB_API int wb_qwen_destroy(wb_qwen *model);
 /* resetCache() */

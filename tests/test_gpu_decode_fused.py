@@ -105,3 +105,43 @@ def test_mlp_activations_that_are_no_fp16_numbers(built_lib, what):
             model.prefill(np.arange(3, dtype=np.uint32), last_only=True)
             assert np.isnan(model.read_tensor(model.decode_step(1))).all(), fuse
             model.close()
+
+
+def test_weights_written_over_after_a_decode(built_lib):
+    """wb_upload over registered weights reaches the next step, although the kernel reads them in a layout of its own: an int4
+    tensor's scales, a norm weight and a bias, each at the end of the range that an upload touches."""
+    import ctypes as C
+
+    from webllm_b200 import _lib as L
+    from webllm_b200.device import Arena
+    cfg = synthetic.QwenShape(300, 2, 4, 2, 256, 1280)
+    before, after = (synthetic.random_qwen_gptq(cfg, seed=s, std=0.05) for s in (8, 9))
+
+    def step(gpu, model):
+        model.reset_cache()
+        model.prefill(np.arange(5, dtype=np.uint32), last_only=True)
+        return model.read_tensor(model.decode_step(1))
+
+    with Gpu(0, weight_bytes=64 << 20, act_bytes=64 << 20) as gpu:
+        model = QwenGpt(gpu, cfg, max_t=16)
+        model.upload_gptq_model(after, fuse=True)
+        image = np.empty(Arena(gpu, L.WB_ARENA_WEIGHTS).used_bytes, np.uint8)
+        L.check(gpu._lib.wb_download(gpu.ctx, L.WB_ARENA_WEIGHTS, 0, image.ctypes.data_as(C.c_void_p), image.nbytes))
+        want = step(gpu, model)
+        model.close()
+    with Gpu(0, weight_bytes=64 << 20, act_bytes=64 << 20) as gpu:
+        model = QwenGpt(gpu, cfg, max_t=16)
+        model.upload_gptq_model(before, fuse=True)
+        first = step(gpu, model)
+        for lo, hi in ((0, image.size // 2), (image.size // 2, image.size)):
+            part = np.ascontiguousarray(image[lo:hi])
+            L.check(gpu._lib.wb_upload(gpu.ctx, L.WB_ARENA_WEIGHTS, lo, part.ctypes.data_as(C.c_void_p), part.nbytes))
+        assert np.array_equal(step(gpu, model), want) and not np.array_equal(first, want)
+        launches = gpu.launch_count
+        step(gpu, model)
+        again = gpu.launch_count - launches
+        L.check(gpu._lib.wb_upload(gpu.ctx, L.WB_ARENA_WEIGHTS, image.size + 256, part.ctypes.data_as(C.c_void_p), 256))  # the cache
+        launches = gpu.launch_count
+        step(gpu, model)
+        assert gpu.launch_count - launches == again  # nothing laid out again for bytes that are no weight's
+        model.close()

@@ -141,6 +141,7 @@ struct wb_context {
     int *status_word = nullptr;      // device-side error flag for bounded waits, and a result word (mapped pinned host memory)
     int *status_host = nullptr;
     uint64_t launches = 0;
+    uint64_t weight_writes = 0;      // uploads over registered weights: a copy of them in another layout is out of date
     int force_kernel = 0, force_split = 0;
     int prefetch_weight = -1;        // index of the weight the next linear should pull into L2 (-1: none)
     void *tmap_encode = nullptr;     // cuTensorMapEncodeTiled, resolved at context creation

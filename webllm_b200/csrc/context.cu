@@ -306,6 +306,12 @@ int wb_upload(wb_context *ctx, int arena, uint64_t offset, const void *host, uin
     WB_CHECK(check_range(ctx, arena, offset, bytes, "wb_upload"));
     if (bytes == 0) return WB_OK;
     if (!host) return fail(WB_ERR_BAD_ARG, "wb_upload: host pointer is NULL");
+    if (arena == WB_ARENA_WEIGHTS)
+        for (const Weight &w : ctx->weights)
+            if (offset < w.arena_top && offset + bytes > w.off_main) {
+                ctx->weight_writes++;
+                break;
+            }
     WB_CHECK(copy_to_device(ctx, arena_ptr(ctx, arena, offset), host, bytes));
     // The host buffer is borrowed for the call only: pageable copies are already staged when
     // cudaMemcpyAsync returns; pinned ones are not, so wait.

@@ -1204,6 +1204,23 @@ static bool fused_shape(const wb_qwen *m, int n, int *blob, int *slot, int *slot
 // it is through that projection that every CTA is known to have read what it needs (see the comment at the top).
 static int fused_ctas(const wb_qwen *m) { return std::min(m->ctx->sm_count, m->I / 8); }
 
+// The weights into the kernel's layout: at set-up, and again after an upload over registered weights.
+static int fused_lay_out(wb_qwen *m, const fd::Params &p)
+{
+    using namespace fd;
+    wb_context *ctx = m->ctx;
+    const int C = p.C, I = p.I, QKV = C + 2 * p.KV, L = p.n_layer;
+    const int units = (QKV / 8 + C / 8 + I / 4) * (C / 128) + C / 8 * (I / 128);
+    const Source *src = (const Source *)m->fused_src;
+    lay_out_kernel<<<dim3((units + 7) / 8, L), 256, 0, ctx->stream>>>(src, const_cast<char *>(p.blobs), C, I, p.KV, p.n_cta, p.blob_stride);
+    WB_CUDA(cudaGetLastError());
+    lay_out_aux_kernel<<<L, 256, 0, ctx->stream>>>(src, const_cast<float *>(p.aux), C, QKV);
+    WB_CUDA(cudaGetLastError());
+    ctx->launches += 2;
+    m->fused_writes = ctx->weight_writes;
+    return WB_OK;
+}
+
 static int fused_setup(wb_qwen *m)
 {
     using namespace fd;
@@ -1240,12 +1257,7 @@ static int fused_setup(wb_qwen *m)
     Source *d_src = (Source *)(mem + blob_bytes + aux_bytes + ll_bytes);
     WB_CUDA(cudaMemcpyAsync(d_src, src.data(), L * sizeof(Source), cudaMemcpyHostToDevice, ctx->stream));
     WB_CUDA(cudaMemsetAsync(p.ll, 0, ll_bytes, ctx->stream));
-    const int units = (QKV / 8 + C / 8 + I / 4) * (C / 128) + C / 8 * (I / 128);
-    lay_out_kernel<<<dim3((units + 7) / 8, L), 256, 0, ctx->stream>>>(d_src, mem, C, I, KV, n, blob);
-    WB_CUDA(cudaGetLastError());
-    lay_out_aux_kernel<<<L, 256, 0, ctx->stream>>>(d_src, (float *)p.aux, C, QKV);
-    WB_CUDA(cudaGetLastError());
-    ctx->launches += 2;
+    m->fused_src = d_src;
     p.final_norm = f32w(m->final_norm), p.embed = (const __half *)f32w(m->embed), p.cs_table = m->cs_table;
     p.k_cache = m->k_cache, p.v_cache = m->v_cache, p.status = ctx->status_word;
     const bool kv16 = m->cfg.kv_dtype == WB_F16;
@@ -1253,6 +1265,7 @@ static int fused_setup(wb_qwen *m)
     p.n_cta = n, p.n_layer = L, p.C = C, p.H = m->H, p.KVH = m->KVH, p.I = I, p.V = m->V, p.KV = KV;
     p.sm = smem_layout(slots, slot, C, I, max_units(C, I, KV, n));
     p.slots = slots, p.slot_bytes = slot, p.blob_stride = blob, p.eps = m->cfg.rms_eps;
+    WB_CHECK(fused_lay_out(m, p));
     WB_CUDA(cudaFuncSetAttribute(kv16 ? (const void *)decode_fused_kernel<__half> : (const void *)decode_fused_kernel<float>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     static_assert(sizeof(Params) <= sizeof(m->fused_params), "room for the parameters in the model object");
@@ -1271,6 +1284,7 @@ int decode_fused_run(wb_qwen *m, uint32_t token, int64_t n_steps, float *logits,
     wb_context *ctx = m->ctx;
     Params p;
     memcpy(&p, m->fused_params, sizeof p);
+    if (m->fused_writes != ctx->weight_writes) WB_CHECK(fused_lay_out(m, p));
     const uint64_t epochs = (uint64_t)n_steps * p.n_layer;
     if (m->fused_epoch + epochs > 0xfffffff0u) {  // epochs do not wrap: start again on zeroed words
         WB_CUDA(cudaMemsetAsync(p.ll, 0, (p.ll_layer + 4 * (size_t)p.n_cta) * 8, ctx->stream));

@@ -47,8 +47,10 @@ struct wb_qwen {
     // the persistent decode kernel (decode_fused.cu): its layout of the weights and its hand-over words, made on first use
     int fused_state = 0;            // 0: not looked at yet, 1: ready, -1: not for this model
     char *fused_mem = nullptr;
+    const void *fused_src = nullptr;  // ... where in it the table of the tensors lies
     int fused_smem = 0;
     uint32_t fused_epoch = 1;
+    uint64_t fused_writes = 0;      // the context's weight_writes when the weights were laid out
     alignas(8) unsigned char fused_params[256];
     uint64_t carve_mark = 0, carve_top = 0;  // weight-arena `used` before and after the model's own allocations
 };
