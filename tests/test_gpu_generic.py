@@ -31,3 +31,14 @@ def test_generic_equals_reference_bits(gpu, oracle, M, N, K, group, zeros):
     bias = np.random.default_rng(N).standard_normal(N).astype(np.float32)
     ref = oracle.gemm_nt_ref(x, oracle_weight(oracle, t), M, N, K, bias, threads=oracle.max_threads())
     assert np.array_equal(got.view(np.uint32), np.asarray(ref, np.float32).reshape(got.shape).view(np.uint32))
+
+
+@pytest.mark.parametrize("M", [65535 * 32, 65535 * 32 + 33])
+def test_more_rows_than_a_second_grid_dimension_holds(gpu, oracle, M):
+    K, N = 4, 3
+    rng = np.random.default_rng(M)
+    W, x = rng.standard_normal((N, K)).astype(np.float16), rng.standard_normal((M, K)).astype(np.float32)
+    h = gpu.f16_alloc(f"rows_{M}", N, K)
+    gpu.f16_write_bits(h, 0, W)
+    got = run_linear(gpu, h, x, M, N, exact=True)
+    assert np.array_equal(got, oracle.gemm_nt_ref(x, W.astype(np.float32), M, N, K))

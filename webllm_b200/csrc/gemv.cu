@@ -670,6 +670,10 @@ __global__ void __launch_bounds__(128) linear_generic_kernel(const GenericParams
         }
 }
 
+// Rows of one launch (tiles of 32 in the grid's second dimension). More are more launches: the tiles in one dimension of the grid, or
+// in its second and third, cost every launch 1 us of its 38.
+constexpr int64_t kGenericRows = 65535 * 32;
+
 // Columns of a tile, 32 or 64: the passes over shared memory per k of the SM with the most tiles.
 static int generic_tile_n(int64_t M, int64_t N, int sms)
 {
@@ -910,9 +914,9 @@ static int make_plan(wb_context *ctx, const Weight &w, int64_t M, int act_dtype,
         plan->block = 128;
         plan->tile_m = 32, plan->tile_n = generic_tile_n(M, w.N, ctx->sm_count);
         plan->grid_x = (int)((w.N + plan->tile_n - 1) / plan->tile_n);
-        plan->grid_y = (int)((M + plan->tile_m - 1) / plan->tile_m);
+        plan->grid_y = (int)((std::min(M, kGenericRows) + plan->tile_m - 1) / plan->tile_m);
         plan->grid_z = 1;
-        plan->launches = 1;
+        plan->launches = (int)((M + kGenericRows - 1) / kGenericRows);
         return WB_OK;
     }
     return fail(WB_ERR_BAD_ARG, "unknown kernel kind %d", kind);
@@ -1081,11 +1085,14 @@ int launch_linear(wb_context *ctx, const Weight &w, const void *A, void *C, cons
         g.x = A, g.out = C, g.bias = bias, g.M = M, g.N = w.N, g.K = w.K, g.pack_rows = w.pack_rows;
         g.group = gptq ? w.group : 8, g.zcols = w.zcols;
         g.x_f16 = act_dtype == WB_F16, g.out_f16 = out_dtype == WB_F16, g.round_x_f16 = round_x;
-        const dim3 grid((unsigned)plan.grid_x, (unsigned)plan.grid_y);
-        const cudaError_t e = plan.tile_n == 64 ? launch_pdl(linear_generic_kernel<2>, grid, dim3(128), 0, ctx->stream, g)
-                                                : launch_pdl(linear_generic_kernel<1>, grid, dim3(128), 0, ctx->stream, g);
-        ctx->launches++;
-        WB_CUDA(e);
+        for (int64_t m = 0; m < M; m += kGenericRows) {
+            g.x = (const char *)A + m * w.K * (g.x_f16 ? 2 : 4), g.out = (char *)C + m * w.N * (g.out_f16 ? 2 : 4), g.M = std::min(M - m, kGenericRows);
+            const dim3 grid((unsigned)plan.grid_x, (unsigned)((g.M + 31) / 32));
+            const cudaError_t e = plan.tile_n == 64 ? launch_pdl(linear_generic_kernel<2>, grid, dim3(128), 0, ctx->stream, g)
+                                                    : launch_pdl(linear_generic_kernel<1>, grid, dim3(128), 0, ctx->stream, g);
+            ctx->launches++;
+            WB_CUDA(e);
+        }
         return WB_OK;
     }
     }
