@@ -75,3 +75,18 @@ def test_tcgen05_prefill_attention(built_lib, oracle, small, n):
         model.close()
     row_err = np.sqrt(np.mean((got - ref).astype(np.float64) ** 2, axis=1)) / rms
     assert oracle.check_tolerance(got, ref, 1e-2 * rms, 2e-2).ok and row_err.max() < 1e-2, (float(row_err.max()), int(row_err.argmax()))
+
+
+def test_more_sequences_than_a_grid_dimension_holds(built_lib, oracle):
+    cfg = synthetic.QwenShape(16, 1, 2, 1, 128, 128)
+    G = synthetic.random_qwen_gptq(cfg, seed=13, std=0.05)
+    pairs = np.array([(i // 16, i % 16) for i in range(256)], np.uint32)
+    ref = oracle.qwen_forward_ref(_ocfg(oracle, cfg), _dense_from_gptq(oracle, G), pairs.ravel(), 256, 2).reshape(256, -1)
+    pick = np.random.default_rng(14).integers(0, 256, 65535 + 40)
+    with Gpu(0, weight_bytes=64 << 20, act_bytes=3 << 30) as gpu:
+        model = QwenGpt(gpu, cfg, max_t=2, kv_dtype="f32")
+        model.upload_gptq_model(G, fuse=True)
+        got = model.read_tensor(model.forward(pairs[pick].ravel(), pick.size, 2)).reshape(pick.size, -1)
+        model.close()
+    rms = float(np.sqrt(np.mean(ref.astype(np.float64) ** 2)))
+    assert np.abs(got - ref[pick]).max() < 2e-2 * rms  # fp16 operands, as in the tests above

@@ -7,6 +7,8 @@
 // 4 x 2 and 4 x 4 register tiles, online softmax. One CTA per single row, as the scalar kernel (qwen_ops.cu) has it, reads every
 // key 32 times as often and leaves a warp's lanes one multiply per load. 4 x 101 rows, 14 heads: 57 -> 22 us a layer with
 // one group, whose chain of key blocks it was, 17 with four.
+#include <algorithm>
+
 #include "qwen_ops.cuh"
 
 namespace wb {
@@ -151,6 +153,9 @@ __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__
 
 }  // namespace
 
+// Sequences of one launch (the grid's third dimension); more are more launches.
+constexpr int kSequences = 65535;
+
 // Two rows and more of 16-byte aligned heads of 64 dims (one row keeps the scalar kernel: the decode kernels are for that).
 bool op_attention_f32_supported(int M, int D, int ldq, int kv_ld) { return M > 1 && D == kD && ldq % 4 == 0 && kv_ld % 4 == 0; }
 
@@ -158,18 +163,25 @@ int op_attention_f32(wb_context *ctx, const float *q, const void *kmem, const vo
                      const int *past_ptr, int past_imm, int use_cache, int ldq, int kv_ld, __half *out16)
 {
     const float scale = 1.0f / sqrtf((float)kD);
-    const dim3 grid((unsigned)H, (unsigned)((T + kRows - 1) / kRows), (unsigned)(M / T));
     const int key_rows = use_cache ? 0 : T;  // (one sequence with a cache)
     if (const cudaError_t e = kv_f16 ? smem_limit_once<attention_f32_kernel<__half>>((int)sizeof(Smem)) : smem_limit_once<attention_f32_kernel<float>>((int)sizeof(Smem));
         e != cudaSuccess)
         WB_CUDA(e);
-    const cudaError_t e =
-        kv_f16 ? launch_pdl(attention_f32_kernel<__half>, grid, dim3(kThreads), sizeof(Smem), ctx->stream, q, (const __half *)kmem, (const __half *)vmem, out, out16, H,
-                            KVH, T, past_ptr, past_imm, key_rows, ldq, kv_ld, scale)
-               : launch_pdl(attention_f32_kernel<float>, grid, dim3(kThreads), sizeof(Smem), ctx->stream, q, (const float *)kmem, (const float *)vmem, out, out16, H,
-                            KVH, T, past_ptr, past_imm, key_rows, ldq, kv_ld, scale);
-    ctx->launches++;
-    WB_CUDA(e);
+    const int B = M / T;
+    for (int b = 0; b < B; b += kSequences) {
+        const dim3 grid((unsigned)H, (unsigned)((T + kRows - 1) / kRows), (unsigned)std::min(B - b, kSequences));
+        const int64_t row = (int64_t)b * T, at = row * H * kD, key = (int64_t)b * key_rows * kv_ld;
+        const float *qb = q + row * ldq;
+        float *ob = out ? out + at : nullptr;
+        __half *o16 = out16 ? out16 + at : nullptr;
+        const cudaError_t e =
+            kv_f16 ? launch_pdl(attention_f32_kernel<__half>, grid, dim3(kThreads), sizeof(Smem), ctx->stream, qb, (const __half *)kmem + key,
+                                (const __half *)vmem + key, ob, o16, H, KVH, T, past_ptr, past_imm, key_rows, ldq, kv_ld, scale)
+                   : launch_pdl(attention_f32_kernel<float>, grid, dim3(kThreads), sizeof(Smem), ctx->stream, qb, (const float *)kmem + key,
+                                (const float *)vmem + key, ob, o16, H, KVH, T, past_ptr, past_imm, key_rows, ldq, kv_ld, scale);
+        ctx->launches++;
+        WB_CUDA(e);
+    }
     return WB_OK;
 }
 
