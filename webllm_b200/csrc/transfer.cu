@@ -41,14 +41,21 @@ public:
     cudaEvent_t event[kSlots] = {};
     int device = -1;
 
-    int prepare(int dev)
+    bool prepare(int dev)  // false: there is no such memory to be had now; the copy goes the plain way
     {
-        if (pinned && device == dev) return WB_OK;
+        if (pinned && device == dev) return true;
         release();
-        WB_CUDA(cudaHostAlloc((void **)&pinned, kSlots * kPiece, cudaHostAllocPortable));
-        for (cudaEvent_t &e : event) WB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        cudaError_t err = cudaHostAlloc((void **)&pinned, kSlots * kPiece, cudaHostAllocPortable);
+        if (err != cudaSuccess) pinned = nullptr;
+        for (cudaEvent_t &e : event)
+            if (err == cudaSuccess && (err = cudaEventCreateWithFlags(&e, cudaEventDisableTiming)) != cudaSuccess) e = nullptr;
+        if (err != cudaSuccess) {
+            cudaGetLastError();
+            release();
+            return false;
+        }
         device = dev;
-        return WB_OK;
+        return true;
     }
     void release()
     {
@@ -185,8 +192,8 @@ int copy(wb_context *ctx, void *host, void *dev, size_t bytes, bool to_host)
 {
     std::unique_lock<std::mutex> lk(g_ring.use, std::defer_lock);
     cudaPointerAttributes at;
-    if (bytes >= (to_host ? kHelpersFrom : kHelpersUpFrom) && (cudaPointerGetAttributes(&at, host) != cudaSuccess || at.type == cudaMemoryTypeUnregistered) && lk.try_lock()) {
-        WB_CHECK(g_ring.prepare(ctx->device));
+    if (bytes >= (to_host ? kHelpersFrom : kHelpersUpFrom) && (cudaPointerGetAttributes(&at, host) != cudaSuccess || at.type == cudaMemoryTypeUnregistered) && lk.try_lock() &&
+        g_ring.prepare(ctx->device)) {
         Job j;
         j.host = (char *)host, j.bytes = bytes, j.pieces = (int)((bytes + kPiece - 1) / kPiece), j.to_host = to_host;
         std::vector<std::atomic<unsigned char>> done((size_t)j.pieces);
