@@ -79,3 +79,9 @@ def harness(tmp_path_factory):
 
 def test_copies_without_a_pinned_ring(harness):
     assert harness(pinned=0, threads=9, release=True) == 2  # one plain copy each way
+
+
+@pytest.mark.parametrize("threads", [0, 1])
+def test_copies_with_fewer_helper_threads(harness, threads):
+    copies = harness(pinned=9, threads=threads, release=True)
+    assert copies == 2 if threads == 0 else copies in (2, 2 * 67)  # (2: a host of few cores has no helpers) pieces of 512 KB

@@ -14,7 +14,10 @@
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
+#include <memory>
 #include <mutex>
+#include <new>
+#include <system_error>
 #include <thread>
 
 #include "common.cuh"
@@ -71,7 +74,10 @@ public:
     {
         if (!helpers) {
             const int n = std::min<int>(kHelpersMax, (int)std::thread::hardware_concurrency() / 2 - 1);
-            for (int i = 0; i < n; i++) threads[helpers++] = std::thread([this] { work(); });
+            try {
+                for (int i = 0; i < n; i++) threads[i] = std::thread([this] { work(); }), helpers++;
+            } catch (const std::system_error &) {  // no more threads for this process: those that there are do
+            }
         }
         if (!helpers) return 0;
         {
@@ -196,9 +202,9 @@ int copy(wb_context *ctx, void *host, void *dev, size_t bytes, bool to_host)
         g_ring.prepare(ctx->device)) {
         Job j;
         j.host = (char *)host, j.bytes = bytes, j.pieces = (int)((bytes + kPiece - 1) / kPiece), j.to_host = to_host;
-        std::vector<std::atomic<unsigned char>> done((size_t)j.pieces);
-        j.done = done.data();
-        if (g_ring.start(&j) > 0) {
+        const std::unique_ptr<std::atomic<unsigned char>[]> done(new (std::nothrow) std::atomic<unsigned char>[(size_t)j.pieces]());
+        j.done = done.get();
+        if (j.done && g_ring.start(&j) > 0) {
             const int rc = run_job(ctx, &j, (char *)dev);
             g_ring.finish(&j);
             if (rc == WB_OK && !to_host) WB_CUDA(cudaStreamSynchronize(ctx->stream));  // the slots are free for the next copy
