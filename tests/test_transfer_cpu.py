@@ -85,3 +85,7 @@ def test_copies_without_a_pinned_ring(harness):
 def test_copies_with_fewer_helper_threads(harness, threads):
     copies = harness(pinned=9, threads=threads, release=True)
     assert copies == 2 if threads == 0 else copies in (2, 2 * 67)  # (2: a host of few cores has no helpers) pieces of 512 KB
+
+
+def test_process_ends_with_a_context_open(harness):
+    harness(pinned=9, threads=9, release=False)
