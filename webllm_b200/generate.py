@@ -113,9 +113,10 @@ def generate_qwen(model: QwenGpt, config, prompt: list, max_new_tokens: int, opt
                   on_device: bool | None = None) -> QwenGenerateResult:
     """``generateQwen``: one prefill, then one decode step per token.
 
-    Greedy decoding without stop tokens runs entirely on the device (``decode_greedy``: argmax and token
-    feedback inside a replayed CUDA graph) unless ``on_device=False``; every other option takes the
-    reference's loop with the draw on the device (a top-k of up to 1024) or, from the row read back, on the host."""
+    Greedy decoding without stop tokens runs entirely on the device (``decode_greedy``: argmax and token feedback inside
+    one persistent kernel, or a replayed CUDA graph for models that it does not take) unless ``on_device=False``; every
+    other option takes the reference's loop with the draw on the device (a top-k of up to 1024) or, from the row read
+    back, on the host."""
     options = options or SamplerOptions()
     if len(prompt) == 0:
         raise ValueError("generateQwen: prompt 不能为空")
@@ -132,21 +133,28 @@ def generate_qwen(model: QwenGpt, config, prompt: list, max_new_tokens: int, opt
     greedy = not (options.temperature > 0)
     k = math.floor(options.top_k) if not greedy and options.top_k > 0 else 0
 
-    def sample(logits) -> int:
-        # a short list of candidates is drawn from on the device: the row stays where it is
-        if 1 <= k <= 1024:
+    on_device_draw = 1 <= k <= 1024  # a short list of candidates is drawn from on the device: the row stays where it is
+
+    def sample(logits, row=None) -> int:
+        if on_device_draw:
             u = (options.rng or random.random)()
             token = model.sample(logits, options.temperature, k, options.top_p, u)
             if token is not None:
                 return token
             return sample_token(model.read_tensor_slice(logits, 0, vocab), 0, vocab, replace(options, rng=lambda: u))
-        return sample_token(model.read_tensor_slice(logits, 0, vocab), 0, vocab, options)
+        return sample_token(model.read_tensor_slice(logits, 0, vocab) if row is None else row, 0, vocab, options)
 
-    nxt = sample(model.prefill(np.asarray(prompt, np.uint32), last_only=True))
+    # prefill_ms ends with the prompt's logits; the first draw is part of the decoding, as in the reference
+    logits, row = model.prefill(np.asarray(prompt, np.uint32), last_only=True), None
+    if on_device_draw:
+        model.gpu.synchronize()
+    else:
+        row = model.read_tensor_slice(logits, 0, vocab)
     prefill_ms = (time.perf_counter() - t0) * 1e3
 
     t1 = time.perf_counter()
     generated = 0
+    nxt = sample(logits, row)
     if on_device is None:
         on_device = greedy and not stop
     if on_device and greedy and not stop and max_new_tokens > 1 and nxt not in stop:
