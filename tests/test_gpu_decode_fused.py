@@ -145,3 +145,41 @@ def test_weights_written_over_after_a_decode(built_lib):
         step(gpu, model)
         assert gpu.launch_count - launches == again  # nothing laid out again for bytes that are no weight's
         model.close()
+
+
+_GIVE_UP_CHILD = """
+import sys
+import numpy as np
+from webllm_b200 import Gpu, QwenGpt, WebllmError, _lib, synthetic
+cfg = synthetic.QwenShape(300, 2, 4, 2, 256, 1280)
+prompt = np.arange(5, dtype=np.uint32)
+with Gpu(0, weight_bytes=64 << 20, act_bytes=64 << 20) as gpu:
+    model = QwenGpt(gpu, cfg, max_t=80)
+    model.upload_gptq_model(synthetic.random_qwen_gptq(cfg, seed=1), fuse=True)
+    want = model.read_tensor(model.prefill(prompt, last_only=True))
+    for steps in (3, 70, 0):
+        try:
+            model.decode_greedy(1, steps) if steps else model.read_tensor(model.decode_step(1))
+            raise SystemExit("the wait did not run out")
+        except WebllmError as e:
+            assert e.status == _lib.WB_ERR_TIMEOUT and f"code {sys.argv[1]}" in str(e), str(e)
+        assert model.cache_len == (5 if steps else 6)  # greedy steps that failed are not in the cache
+    model.reset_cache()
+    assert np.array_equal(model.read_tensor(model.prefill(prompt, last_only=True)), want)
+    model.close()
+print("give-up-ok")
+"""
+
+
+@pytest.mark.parametrize("code", [41])
+def test_waits_give_up_instead_of_hanging(built_lib, code):
+    """41: a hand-over's words never come (the test's setting makes attention wait for an epoch that nobody writes). The kernel
+    ends, the next synchronize reports WB_ERR_TIMEOUT, and the context keeps working. (The setting is read once per process.)"""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+    env = dict(os.environ, WEBLLM_B200_DECODE_GIVE_UP={41: "1"}[code])
+    r = subprocess.run([sys.executable, "-c", _GIVE_UP_CHILD, str(code)], env=env, cwd=str(Path(__file__).resolve().parent.parent),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "give-up-ok" in r.stdout, r.stdout + r.stderr

@@ -481,13 +481,17 @@ int wb_qwen_decode_greedy(wb_qwen *m, uint32_t first_token, int64_t n_steps, uin
     constexpr int64_t kFusedSteps = 64;
     if (n_steps <= (int64_t)m->host_pin_cap) {
         bool ran = true;
+        const int64_t before = m->cache_len;
         for (int64_t s = 0; s < n_steps && ran; s += kFusedSteps) {
             const int64_t cur = std::min(kFusedSteps, n_steps - s);
             const uint32_t first = s == 0 ? first_token : m->host_pin[s - 1];
             WB_CHECK(decode_fused_run(m, first, cur, m->dec.logits, m->host_pin + s, &ran));
             if (!ran) break;
+            if (const int rc = wb_synchronize(ctx)) {
+                m->cache_len = before;
+                return rc;
+            }
             m->cache_len += cur;
-            WB_CHECK(wb_synchronize(ctx));
         }
         if (ran) {
             memcpy(out_tokens, m->host_pin, (size_t)n_steps * 4);
