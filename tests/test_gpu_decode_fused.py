@@ -171,15 +171,15 @@ print("give-up-ok")
 """
 
 
-@pytest.mark.parametrize("code", [41])
+@pytest.mark.parametrize("code", [41, 42])
 def test_waits_give_up_instead_of_hanging(built_lib, code):
-    """41: a hand-over's words never come (the test's setting makes attention wait for an epoch that nobody writes). The kernel
-    ends, the next synchronize reports WB_ERR_TIMEOUT, and the context keeps working. (The setting is read once per process.)"""
+    """41: a hand-over's words never come (the test's setting makes attention wait for an epoch that nobody writes). 42: a wait for
+    a slot of the weight ring runs out (the setting's limit is no poll at all, so the copy is still on its way). The kernel ends, the next synchronize reports WB_ERR_TIMEOUT, and the context keeps working. (The setting is read once per process.)"""
     import os
     import subprocess
     import sys
     from pathlib import Path
-    env = dict(os.environ, WEBLLM_B200_DECODE_GIVE_UP={41: "1"}[code])
+    env = dict(os.environ, WEBLLM_B200_DECODE_GIVE_UP=str(code - 40))
     r = subprocess.run([sys.executable, "-c", _GIVE_UP_CHILD, str(code)], env=env, cwd=str(Path(__file__).resolve().parent.parent),
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "give-up-ok" in r.stdout, r.stdout + r.stderr

@@ -26,6 +26,8 @@
 //
 // All CTAs have to be resident at once, hence the cooperative launch. Every poll is bounded in time; one that gives up sets
 // the context's status word and lets all later polls of its CTA through, so the kernel drains its copies and ends.
+#include <stdlib.h>
+
 #include <algorithm>
 
 #include "qwen_internal.cuh"
@@ -61,7 +63,7 @@ struct Params {
     uint32_t *history;      // nullable; pinned host memory
     int *status;
     size_t kv_layer_bytes, ll_layer;
-    uint32_t epoch, first_token, polls, miss;  // limit of a hand-over's polls; a test's setting, else 0
+    uint32_t epoch, first_token, polls, ring_polls, miss;  // limits of the polls; a test's setting, else 0
     int n_cta, n_layer, C, H, KVH, I, V, KV, pos0, n_steps, slots, slot_bytes, blob_stride;
     float eps;
     Smem sm;
@@ -94,20 +96,19 @@ __device__ __forceinline__ void mbar_expect(uint64_t *b, uint32_t bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(s32(b)), "r"(bytes) : "memory");
 }
-// Bounded: a copy always completes, so running out means a broken device; the code is recorded and the caller carries on.
-__device__ __forceinline__ void mbar_wait(uint64_t *b, uint32_t parity, int *status)
+__device__ __forceinline__ bool mbar_poll(uint64_t *b, uint32_t parity, uint32_t polls)  // false: not in so many polls
 {
     const uint32_t a = s32(b);
 #pragma unroll 1
-    for (uint32_t it = 0; it < (1u << 26); it++) {
+    for (uint32_t it = 0; it < polls; it++) {
         uint32_t ok;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(ok)
                      : "r"(a), "r"(parity)
                      : "memory");
-        if (ok) return;
+        if (ok) return true;
     }
-    *(volatile int *)status = kStatusRing;
+    return false;
 }
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
 {
@@ -141,7 +142,18 @@ struct Head {
     uint32_t polls;
     volatile uint32_t token;
     int fill_i, fill_slot, fill_left;  // the feeder's: next fill of the ring (its index in the step, its slot), steps left
+    uint32_t fills, ring_polls;        // ... fills so far
+    volatile int ring_lost;            // a wait for a slot has given up
 };
+static_assert(sizeof(Head) <= 128, "the ring begins behind it");
+// Waiting for a slot of the ring. Bounded: its copy always completes, and in microseconds, so running out means a broken device. The
+// code is recorded, the slots are not filled again, and the CTA runs through the rest without them (the numbers are lost).
+constexpr uint32_t kRingPolls = 1u << 24;
+__device__ __forceinline__ void ring_wait(Head *hd, int slot, uint32_t parity)
+{
+    if (mbar_poll(&hd->full[slot], parity, hd->ring_polls) || hd->ring_lost) return;
+    hd->ring_lost = 1, hd->ring_polls = 0, *(volatile int *)hd->status = kStatusRing;
+}
 // Waiting for words. Everything that a warp waits for is loaded and checked together (a thread that took its words one after the
 // other would pay a round trip for each: none of them was there yet when it came), only what is missing is loaded again, and the
 // warp leaves the loop as one. Bounded: a poll is a round trip to L2 (at least 0.15 us), so kPolls of them are seconds; a CTA
@@ -617,6 +629,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     if (tid == 0) {
         for (int i = 0; i < p.slots; i++) mbar_init(&full[i], 1);
         hd->gave_up = 0, hd->status = p.status, hd->polls = p.polls;
+        hd->fills = 0, hd->ring_lost = 0, hd->ring_polls = p.ring_polls;
         hd->fill_i = 0, hd->fill_slot = 0, hd->fill_left = p.n_steps;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -628,7 +641,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     const bool feeder = tid == kThreads - 32;
     const uint32_t block_bytes = (uint32_t)(uq + uo + ug + ud) * kUnitBytes;
     auto fill = [&]() {
-        if (hd->fill_left == 0) return;
+        if (hd->fill_left == 0 || hd->ring_lost) return;
         const int i = hd->fill_i, at = hd->fill_slot;
         const char *src;
         uint32_t bytes;
@@ -640,6 +653,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
         }
         mbar_expect(&full[at], bytes);
         if (bytes) bulk_load(ring + at * p.slot_bytes, src, bytes, &full[at]);
+        hd->fills++;
         hd->fill_slot = at + 1 == p.slots ? 0 : at + 1;
         if (i + 1 == L + lm_fills) hd->fill_i = 0, hd->fill_left--;
         else hd->fill_i = i + 1;
@@ -743,7 +757,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
         return a + __shfl_xor_sync(0xffffffffu, a, 2);
     };
 
-    if (feeder) mbar_wait(&full[0], 0, p.status);
+    if (feeder) ring_wait(hd, 0, 0);
     __syncthreads();
 #pragma unroll 1
     for (int s = 0; s < p.n_steps; s++) {
@@ -916,7 +930,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
             wb += ug * kUnitBytes;
             if (nd == 0) {
                 next_slot();
-                if (feeder && l + 1 < L) mbar_wait(&full[slot], par, p.status);
+                if (feeder && l + 1 < L) ring_wait(hd, slot, par);
             }
             __syncthreads();
 #pragma unroll 1
@@ -991,7 +1005,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
                     }
                 }
                 next_slot();
-                if (feeder && l + 1 < L) mbar_wait(&full[slot], par, p.status);
+                if (feeder && l + 1 < L) ring_wait(hd, slot, par);
                 __syncthreads();
                 if (warp < nd) {
                     const float a = column_sum_i(red + warp * GI * 8);
@@ -1025,7 +1039,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
             const int my = (lane >> 4) * 2 + ((lane >> 3) & 1);  // the row of the four whose sum ends up here
 #pragma unroll 1
             for (int j = 0; j < lm_fills; j++) {
-                mbar_wait(&full[slot], par, p.status);
+                ring_wait(hd, slot, par);
                 const __half *rows = reinterpret_cast<const __half *>(ring + slot * p.slot_bytes) + (size_t)warp * 4 * C;
                 float a[4] = {}, b[4] = {};
 #pragma unroll
@@ -1067,7 +1081,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
                 if (v > best || (v == best && i < best_i)) best = v, best_i = i;
             }
         }
-        if (feeder && !last) mbar_wait(&full[slot], par, p.status);  // the next step's first block
+        if (feeder && !last) ring_wait(hd, slot, par);  // the next step's first block
         if (last && p.history == nullptr) break;  // only the logits were asked for
         // every CTA's best row, then every CTA picks the best of those (first strict maximum: the lowest index wins a tie)
         if (lane == 0) ssq[warp] = best, widx[warp] = best_i;
@@ -1104,6 +1118,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
         token = hd->token;
         __threadfence();
     }
+    if (feeder && hd->ring_lost)  // no copy may be under way into memory that the CTA gives back
+        for (uint32_t i = hd->fills - min(hd->fills, (uint32_t)p.slots); i < hd->fills; i++) mbar_poll(&full[i % p.slots], i / p.slots & 1, kRingPolls);
 }
 
 // ---------------------------------------------------------------------------------------------------- set-up
@@ -1294,8 +1310,9 @@ int decode_fused_run(wb_qwen *m, uint32_t token, int64_t n_steps, float *logits,
     p.epoch = m->fused_epoch, p.first_token = token, p.pos0 = (int)m->cache_len, p.n_steps = (int)n_steps;
     p.logits = logits, p.history = history;
     // A test's setting: attention waits for words of an epoch that nobody writes, and not for long.
-    static const bool miss = [] { const char *e = getenv("WEBLLM_B200_DECODE_GIVE_UP"); return e && e[0] == '1'; }();
-    p.miss = miss ? 0x80000000u : 0u, p.polls = miss ? kPollsTest : kPolls;
+    // Or the first wait for a slot of the ring does not wait at all.
+    static const int give_up = [] { const char *e = getenv("WEBLLM_B200_DECODE_GIVE_UP"); return e ? atoi(e) : 0; }();
+    p.miss = give_up == 1 ? 0x80000000u : 0u, p.polls = give_up == 1 ? kPollsTest : kPolls, p.ring_polls = give_up == 2 ? 0u : kRingPolls;
     void *args[] = {&p};
     const void *kern = m->cfg.kv_dtype == WB_F16 ? (const void *)decode_fused_kernel<__half> : (const void *)decode_fused_kernel<float>;
     WB_CUDA(cudaLaunchCooperativeKernel(kern, dim3(p.n_cta), dim3(kThreads), args, (size_t)m->fused_smem, ctx->stream));
