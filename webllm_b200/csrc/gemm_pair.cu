@@ -33,6 +33,7 @@
 //   acc_empty[b] rank 0  both CTAs' epilogue warps have drained set b (remote arrive from rank 1)
 // No load in this file is a cluster-multicast load: every CTA fetches its own boxes.
 #include "gemm_tc.cuh"
+#include "silu.cuh"
 
 namespace wb {
 
@@ -116,17 +117,6 @@ struct PairTail {
     int rounds = 0, slots = 0, St = 1, per = 0;
     float *partial = nullptr;  // [slots][MT][256]
 };
-
-// g / (1 + e^-g) in f32. The fast quotient (within 2 ulp) with one step of iterative refinement: its residual, exact in an fma,
-// divided again. The `/` operator costs a range check and a branch for each of a thread's 128 values, which then run one after
-// the other (75 us -> 67 us at 2048 x 896 -> 2 x 4864). The range is known here: 1 <= d, and below g = -80 d is held
-// at e^80: that quotient is under 1e-32 and 0 in fp16 either way.
-__device__ __forceinline__ float silu(float g)
-{
-    const float d = 1.f + expf(fminf(-g, 80.f));
-    const float q = __fdividef(g, d);
-    return g == INFINITY ? g : q + __fdividef(fmaf(-q, d, g), d);
-}
 
 // GATHER: the result goes to the placement in Params (this GPU's slab and its peers', row pitch ld_out) from registers.
 // SILU: the weight is gate | up (N = 2 I columns) and the result is fp16 silu(gate) * up, [M, I] (siluMulRef,
