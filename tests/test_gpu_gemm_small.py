@@ -26,3 +26,26 @@ def test_small_batch_on_a_large_matrix(gpu, oracle, K, N, group, zeros, M):
         first = run_linear(gpu, h, xin, M, N, hb, act=act, out=act)
         assert_close(oracle, first, ref, 1e-3, f"{K}x{N} M={M} {act}")
         assert np.array_equal(first, run_linear(gpu, h, xin, M, N, hb, act=act, out=act))  # slices are added in order
+
+
+@pytest.mark.parametrize("K,N", [(8576, 1056), (2560, 3360)])
+@pytest.mark.parametrize("split", [0, 1, 2, 20, 64])
+def test_every_number_of_slices(gpu, oracle, K, N, split):
+    """The kernel for certain (its plan has blocks of 256), at the planner's number of slices and at given ones: one, halves, a last
+    slice shorter than the others or of a single chunk."""
+    t = synthetic.random_gptq(K, N, 128, seed=K + N, zeros="any")
+    h = register(gpu, f"gss_{K}_{N}_{split}", t)
+    x = np.random.default_rng(split).standard_normal((11, K)).astype(np.float32)
+    ref = oracle.gemm_nt_ref(x.astype(np.float16).astype(np.float32), oracle_weight(oracle, t), 11, N, K)
+    gpu.plan_override(0, split)
+    try:
+        for act in ("f16", "f32"):
+            p = gpu.plan(h, 11, act)
+            taken = p["block"] == 256 and p["launches"] == 1
+            if split:  # slices that are too long for the shared memory, or would be empty, stay with the tcgen05 kernel
+                per = -(-(K // 128) // min(split, K // 128))
+                assert taken == (-(-(K // 128) // per) == min(split, K // 128) and per <= 25), p
+            assert p["kernel_name"] == "gemm_tc" and (taken or split), p
+            assert_close(oracle, run_linear(gpu, h, x.astype(np.float16) if act == "f16" else x, 11, N, act=act, out=act), ref, 1e-3, f"{K}x{N} {split} {act}")
+    finally:
+        gpu.plan_override(0, 0)
