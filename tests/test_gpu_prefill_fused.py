@@ -77,16 +77,22 @@ def test_tcgen05_prefill_attention(built_lib, oracle, small, n):
     assert oracle.check_tolerance(got, ref, 1e-2 * rms, 2e-2).ok and row_err.max() < 1e-2, (float(row_err.max()), int(row_err.argmax()))
 
 
-def test_more_sequences_than_a_grid_dimension_holds(built_lib, oracle):
-    cfg = synthetic.QwenShape(16, 1, 2, 1, 128, 128)
+@pytest.mark.parametrize("B,T", [(1, 8), (2, 8), (1, 9), (2, 9)])
+def test_f32_attention_where_the_tiles_begin(built_lib, oracle, small, B, T):
+    test_f32_attention_tiles(built_lib, oracle, small, B, T)
+
+
+@pytest.mark.parametrize("T", [2, 9])  # the scalar kernel and the tiles
+def test_more_sequences_than_a_grid_dimension_holds(built_lib, oracle, T):
+    cfg = synthetic.QwenShape(16, 1, 1, 1, 64, 64)
     G = synthetic.random_qwen_gptq(cfg, seed=13, std=0.05)
-    pairs = np.array([(i // 16, i % 16) for i in range(256)], np.uint32)
-    ref = oracle.qwen_forward_ref(_ocfg(oracle, cfg), _dense_from_gptq(oracle, G), pairs.ravel(), 256, 2).reshape(256, -1)
-    pick = np.random.default_rng(14).integers(0, 256, 65535 + 40)
-    with Gpu(0, weight_bytes=64 << 20, act_bytes=3 << 30) as gpu:
-        model = QwenGpt(gpu, cfg, max_t=2, kv_dtype="f32")
+    some = np.random.default_rng(T).integers(0, 16, (64, T)).astype(np.uint32)
+    ref = oracle.qwen_forward_ref(_ocfg(oracle, cfg), _dense_from_gptq(oracle, G), some.ravel(), 64, T).reshape(64, -1)
+    pick = np.random.default_rng(14).integers(0, 64, 65535 + 40)
+    with Gpu(0, weight_bytes=64 << 20, act_bytes=4 << 30) as gpu:
+        model = QwenGpt(gpu, cfg, max_t=T, kv_dtype="f32")
         model.upload_gptq_model(G, fuse=True)
-        got = model.read_tensor(model.forward(pairs[pick].ravel(), pick.size, 2)).reshape(pick.size, -1)
+        got = model.read_tensor(model.forward(some[pick].ravel(), pick.size, T)).reshape(pick.size, -1)
         model.close()
     rms = float(np.sqrt(np.mean(ref.astype(np.float64) ** 2)))
     assert np.abs(got - ref[pick]).max() < 2e-2 * rms  # fp16 operands, as in the tests above

@@ -1,6 +1,6 @@
 // Causal GQA attention in f32 arithmetic for several query rows: attention_gqa.wgsl / attention_gqa_cache.wgsl (attentionGqaRef,
 // src/reference/qwen-ref.ts:67-116) for the uncached forward, the fp32-activation mode and prompts too short for the fp16
-// tensor-core kernel, head size 64.
+// tensor-core kernel, from 9 rows on, head size 64.
 //
 // One CTA = 32 query rows of one head; keys in blocks of 32, staged in shared memory as f32, that four groups of four warps take in
 // turn, their states of a row merged at the end; scores and weighted sums from
@@ -156,8 +156,11 @@ __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__
 // Sequences of one launch (the grid's third dimension); more are more launches.
 constexpr int kSequences = 65535;
 
-// Two rows and more of 16-byte aligned heads of 64 dims (one row keeps the scalar kernel: the decode kernels are for that).
-bool op_attention_f32_supported(int M, int D, int ldq, int kv_ld) { return M > 1 && D == kD && ldq % 4 == 0 && kv_ld % 4 == 0; }
+// Sequences of more than 8 rows, 16-byte aligned heads of 64 dims. A tile has 32 rows and keys whatever the sequence has, and the
+// scalar kernel's work goes with the rows times the keys. Whole layers of 14 heads, us, scalar and tiled, one sequence / 64 / 256:
+// T = 4 29.6, 31.5 / 49.4, 61.0 / 78.8, 122; T = 8 36.9, 37.8 / 60.7, 65.8 / 118, 138 (2 to 16 sequences 0.7 the other way);
+// T = 10 36.3, 34.9 / 69.0, 69.8 / 148, 153; T = 16 38.7, 35.8 / 89.6, 76.9 / 227, 178.
+bool op_attention_f32_supported(int T, int D, int ldq, int kv_ld) { return T > 8 && D == kD && ldq % 4 == 0 && kv_ld % 4 == 0; }
 
 int op_attention_f32(wb_context *ctx, const float *q, const void *kmem, const void *vmem, int kv_f16, float *out, int M, int H, int KVH, int T,
                      const int *past_ptr, int past_imm, int use_cache, int ldq, int kv_ld, __half *out16)

@@ -201,7 +201,7 @@ int forward_impl(wb_qwen *m, const Bufs &b, int64_t M, int64_t B, int64_t T, int
                                       b.ldq, KV));
             }
         } else {
-            att_half = half_in && op_attention_f32_supported((int)M, D, b.ldq, b.ldk);
+            att_half = half_in && op_attention_f32_supported((int)T, D, b.ldq, b.ldk);
             WB_CHECK(op_attention(ctx, b.q, b.k, b.v, 0, b.att, (int)M, H, KVH, D, (int)T, nullptr, 0, 0, (int)T, b.ldq, b.ldk, att_half ? b.h16 : nullptr));
         }
         ctx->keep_slices = may_slice;

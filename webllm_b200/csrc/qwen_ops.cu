@@ -710,7 +710,7 @@ int op_rope_kv(wb_context *ctx, float *q, float *k, const float *v, void *k_cach
 int op_attention(wb_context *ctx, const float *q, const void *kmem, const void *vmem, int kv_f16, float *out, int M, int H,
                  int KVH, int D, int T, const int *past_ptr, int past_imm, int use_cache, int max_keys, int ldq, int kv_ld, __half *out16)
 {
-    if (op_attention_f32_supported(M, D, ldq, kv_ld) && M % T == 0 && (!use_cache || M == T))
+    if (op_attention_f32_supported(T, D, ldq, kv_ld) && M % T == 0 && (!use_cache || M == T))
         return op_attention_f32(ctx, q, kmem, vmem, kv_f16, out, M, H, KVH, T, past_ptr, past_imm, use_cache, ldq, kv_ld, out16);
     if (out16) return fail(WB_ERR_UNSUPPORTED, "fp16 attention output needs the tiled kernel");
     const size_t smem = (size_t)(D + max_keys) * sizeof(float);

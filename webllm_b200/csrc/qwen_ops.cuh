@@ -21,8 +21,8 @@ int op_rope_kv(wb_context *ctx, float *q, float *k, const float *v, void *k_cach
 int op_attention(wb_context *ctx, const float *q, const void *kmem, const void *vmem, int kv_f16, float *out, int M, int H,
                  int KVH, int D, int T, const int *past_ptr, int past_imm, int use_cache, int max_keys, int ldq, int kv_ld,
                  __half *out16 = nullptr);
-// The same in f32 tiles for M > 1 rows, head size 64 (attention_f32.cu); what op_attention itself takes where it can.
-bool op_attention_f32_supported(int M, int D, int ldq, int kv_ld);
+// The same in f32 tiles for sequences of more than 8 rows, head size 64 (attention_f32.cu); what op_attention itself takes where it can.
+bool op_attention_f32_supported(int T, int D, int ldq, int kv_ld);
 int op_attention_f32(wb_context *ctx, const float *q, const void *kmem, const void *vmem, int kv_f16, float *out, int M, int H, int KVH, int T,
                      const int *past_ptr, int past_imm, int use_cache, int ldq, int kv_ld, __half *out16);
 // attention_tc.cu: the same for M >= 64 rows against an fp16 cache, head size 64, on the tcgen05 tensor cores; past is known to the host
