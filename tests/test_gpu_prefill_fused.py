@@ -59,10 +59,11 @@ def test_gate_up_silu_in_one_kernel(built_lib, oracle, n):
     assert err[True] < 1.05 * err[False], err  # no precision given up by the fusion
 
 
-@pytest.mark.parametrize("n", [64, 65, 127, 128, 129, 193, 320])
+@pytest.mark.parametrize("n", [64, 65, 127, 128, 129, 193, 320, 511, 512, 513, 575, 577, 640, 705, 897])
 def test_tcgen05_prefill_attention(built_lib, oracle, small, n):
-    """fp16 cache, from 64 rows on: every row against the reference at row counts beside the tiles of 128 rows and 64 keys (one key
-    group without a block, odd and even numbers of blocks, ragged last ones)."""
+    """fp16 cache; the warp-level kernel below 512 rows, tcgen05 from there on: every row against the reference at row counts beside the
+    tiles of 128 rows and 64 keys (key groups of different numbers of blocks, a first row tile of which two groups have none,
+    ragged last tiles and blocks)."""
     G, Wd = small
     tokens = np.random.default_rng(n).integers(0, SMALL.vocab_size, n).astype(np.uint32)
     ref = oracle.qwen_forward_ref(_ocfg(oracle, SMALL), Wd, tokens, 1, n, threads=oracle.max_threads())

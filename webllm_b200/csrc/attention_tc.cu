@@ -294,9 +294,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
 
 }  // namespace
 
+// From 512 rows on. Below, the chain of a CTA is a block or two long, and its set-up (tensor memory, barriers, the merge of four groups)
+// is more than the warp-level kernel's whole chain. Whole layers, us, warp-level and this: 14 heads, 64 rows 36.0, 37.9; 128 40.5,
+// 43.2; 256 45.6, 47.7; 384 51.3, 51.9; 512 54.9, 54.3; 1024 75.1, 69.6; 2048 103, 92.2. 4 heads even at 576 rows (43.1, 43.7 at 512),
+// 32 heads at about 350 (70.4, 69.1 at 384).
 bool op_attention_tc_supported(int M, int D, int ldq, int kv_ld, int kv_f16, const void *q)
 {
-    return kv_f16 && D == kD && M >= 64 && ldq % 4 == 0 && kv_ld % 8 == 0 && ((uintptr_t)q & 15) == 0;
+    return kv_f16 && D == kD && M >= 512 && ldq % 4 == 0 && kv_ld % 8 == 0 && ((uintptr_t)q & 15) == 0;
 }
 
 int op_attention_tc(wb_context *ctx, const float *q, const void *kmem, const void *vmem, float *out, __half *out16, int M, int H, int KVH,

@@ -25,7 +25,7 @@ int op_attention(wb_context *ctx, const float *q, const void *kmem, const void *
 bool op_attention_f32_supported(int T, int D, int ldq, int kv_ld);
 int op_attention_f32(wb_context *ctx, const float *q, const void *kmem, const void *vmem, int kv_f16, float *out, int M, int H, int KVH, int T,
                      const int *past_ptr, int past_imm, int use_cache, int ldq, int kv_ld, __half *out16);
-// attention_tc.cu: the same for M >= 64 rows against an fp16 cache, head size 64, on the tcgen05 tensor cores; past is known to the host
+// attention_tc.cu: the same for M >= 512 rows against an fp16 cache, head size 64, on the tcgen05 tensor cores; past is known to the host
 bool op_attention_tc_supported(int M, int D, int ldq, int kv_ld, int kv_f16, const void *q);
 int op_attention_tc(wb_context *ctx, const float *q, const void *kmem, const void *vmem, float *out, __half *out16, int M, int H, int KVH,
                     int past, int ldq, int kv_ld);
