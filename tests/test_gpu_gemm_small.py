@@ -49,3 +49,15 @@ def test_every_number_of_slices(gpu, oracle, K, N, split):
             assert_close(oracle, run_linear(gpu, h, x.astype(np.float16) if act == "f16" else x, 11, N, act=act, out=act), ref, 1e-3, f"{K}x{N} {split} {act}")
     finally:
         gpu.plan_override(0, 0)
+
+
+@pytest.mark.parametrize("K,N,small", [(896, 9728, True), (1152, 8224, True), (896, 4864, False), (1152, 8228, False)])
+def test_which_calls_it_takes_on_wide_matrices(gpu, K, N, small):
+    """Short K, wide N, 9 to 16 rows: fp16 activations where the matrix has 8 M weights and whole tiles; f32 activations stay with the
+    GEMV, which keeps their bits."""
+    h = register(gpu, f"gsp_{K}_{N}", synthetic.random_gptq(K, N, 128, seed=N))
+    for M in (8, 9, 12, 13, 16):
+        f16, f32 = gpu.plan(h, M, "f16"), gpu.plan(h, M, "f32")
+        assert (f16["kernel_name"] == "gemm_tc" and f16["block"] == 256) == (small and M > 8), (M, f16)
+        assert (f16["kernel_name"] == "gemv_mma") == (M <= 8 or (M <= 12 and not small)), (M, f16)
+        assert f32["kernel_name"] == "gemv_mma", (M, f32)

@@ -200,6 +200,7 @@ int record_after(wb_context *ctx);
 bool linear_uses_scratch(const wb_plan &plan, int64_t M);  // the workspace or the counters, which two calls at a time may not
 // gemm_small.cu: the small-batch form of the tensor-core GEMM; a plan with this block size is one
 constexpr int kSmallBlock = 256;
+bool gemm_small_takes(wb_context *ctx, const Weight &w, int64_t M);
 bool plan_gemm_small(wb_context *ctx, const Weight &w, int64_t M, wb_plan *plan);
 int launch_gemm_small(wb_context *ctx, const Weight &w, const void *A, void *C, const float *bias, int64_t M, int act_dtype, int out_dtype,
                       const wb_plan &plan);

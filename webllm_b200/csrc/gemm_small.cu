@@ -17,6 +17,8 @@
 // 28.1 -> 24.4, 3584 -> 3584 11.6 -> 8.9; M = 9 alike. It is bound by its fixed parts (staging, the slices' meeting), not by
 // HBM (5.2 us) or the MMAs. A version for 24 and 32 rows was no faster than the tcgen05 kernel (three and four row blocks leave no
 // registers for loads under way), nor were slices as clusters with one CTA of 16 warps an SM.
+#include <stdlib.h>
+
 #include <algorithm>
 
 #include "common.cuh"
@@ -271,11 +273,19 @@ size_t small_smem(int cps, int wk)
 // fp16, M = 9: 9.1 us here, 7.8 there; 3584 -> 512: 7.3 and 7.0).
 constexpr int64_t kFromWeights = 8 << 20;
 
+// WEBLLM_B200_GEMM_SMALL=0 leaves these calls to the tcgen05 kernel (for comparisons).
+bool gemm_small_takes(wb_context *ctx, const Weight &w, int64_t M)
+{
+    static const bool on = [] { const char *e = getenv("WEBLLM_B200_GEMM_SMALL"); return !(e && e[0] == '0'); }();
+    return on && w.kind == WeightKind::Gptq && M >= 1 && M <= 8 * kMB && w.K * w.N >= kFromWeights && w.K % 128 == 0 && w.N % 32 == 0 &&
+           w.group % 128 == 0 && ctx->place.n_dst == 0;
+}
+
 // Slices and columns per CTA by a small cost model in microseconds: rounds of resident CTAs, each a fixed part (launch, staging,
 // reduction) and a warp's chunks, and the traffic of the partial sums. False: not a shape for this kernel.
 bool plan_gemm_small(wb_context *ctx, const Weight &w, int64_t M, wb_plan *plan)
 {
-    if (w.kind != WeightKind::Gptq || M < 1 || M > 8 * kMB || w.K * w.N < kFromWeights || w.K % 128 != 0 || w.N % 32 != 0 || w.group % 128 != 0 || ctx->place.n_dst > 0) return false;
+    if (!gemm_small_takes(ctx, w, M)) return false;
     const int chunks = (int)(w.K / 128);
     double best = 0.;
     int best_s = 0, best_wk = 0;

@@ -835,18 +835,12 @@ static double pick_plan_pair(int64_t M, int64_t N, int kblocks, int sms, int for
     return best;
 }
 
-static bool small_enabled()
-{
-    static const bool on = [] { const char *e = getenv("WEBLLM_B200_GEMM_SMALL"); return !(e && e[0] == '0'); }();
-    return on;
-}
-
 // pair_mode: 0 = one-CTA kernels only, 1 = whichever the cost model prefers, 2 = the CTA-pair kernel or nothing
 // (plan->kernel stays 0 when the shape does not qualify).
 int plan_gemm_tc(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int exact, int pair_mode, wb_plan *plan)
 {
     (void)exact;
-    if (pair_mode == 1 && small_enabled() && plan_gemm_small(ctx, w, M, plan)) return WB_OK;
+    if (pair_mode == 1 && plan_gemm_small(ctx, w, M, plan)) return WB_OK;
     const int kblocks = (int)(w.K / 64);
     int mt, nh, S;
     // microseconds that the stores to the peers of a column-sharded call take at ~700 GB/s per direction
