@@ -252,12 +252,6 @@ __device__ __forceinline__ void mma_first(float (&d)[4], uint32_t a0, uint32_t a
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y), "f"(0.f));
 }
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b)
-{
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y));
-}
 // Units are worked on B at a time without a branch between them, so that their chains (load, mask, four MMAs, one shuffle)
 // overlap: five units of a warp take 500 cycles together, and 1340 with a condition around each. Results of units that are not
 // there are computed from whatever lies behind and not stored. Five is what divides the long projections of the 0.5B model
@@ -310,99 +304,57 @@ __device__ __forceinline__ float unit_half(const Unit &u, const Acts &x, float s
 __device__ __forceinline__ float halves(float v) { return v + __shfl_xor_sync(0xffffffffu, v, 1); }
 
 // ---------------------------------------------------------------------------------------------------- attention
-// One CTA per (head, split of the keys), 16 keys per warp and pass, on the tensor cores: K rows (as they lie in the cache: a lane
-// takes 16 consecutive dims of two keys) are the 16-row operand, the rotated query the column operand; then V transposed by
-// ldmatrix is the row operand and the softmax weights the column operand. Rows are requested before the query is waited for (they
-// were written in earlier steps), so the cache's latency is hidden. Each warp keeps its own online softmax; the warps' states are
-// combined once at the end. With one multiply per lane and dim instead, the scores and sums of 128 keys took 0.8 us of the layer.
+// One CTA per (head, split of the keys), 16 keys per warp and pass. A lane takes 16 consecutive dims of two keys (K rows as they lie
+// in the cache). Rows are requested before the query is waited for (they were written in earlier steps), so the cache's latency is
+// hidden. Each warp keeps its own online softmax; the warps' states are combined once at the end.
 //
-// The arithmetic is that of f32: an f32 operand goes in as three 16-bit parts whose sum is its value, in columns 0 to 2 (the MMA has
-// eight and would leave them idle) or, for an f32 cache, in three passes of the row operand, and products of parts are exact.
-//   * fp16 cache: fp16 parts. The query is scaled by a power of two that puts its largest element at 2^14, the weights by 2^15:
-//     three parts then hold 33 bits of the largest element, and no value is too large for fp16.
-//   * f32 cache: bf16 parts of everything, 24 bits in all and the range of f32.
-// Two fp16 parts kept about 22 bits, lost small softmax weights and made infinities of a query or a cached value above 65504.
-// Measured against 64 bits, attention alone, 5 to 2000 keys: at most as far off as with two parts or as the separate kernels on
-// ordinary values, and 1e-7 to 1e-6 where queries or keys leave the middle of fp16's range (two parts: 1e-5 to 2e-4, or NaN). It
-// takes 0.1 ms of 40 ms for 128 tokens with an fp16 cache, and 14 us a step with an f32 one.
+// fp16 cache: on the tensor cores. K rows are the 16-row operand and the rotated query the column operand; then V transposed by
+// ldmatrix is the row operand and the softmax weights the column operand. The query and the weights keep their f32 bits: they go in
+// as three fp16 parts whose sum is the value, in columns 0 to 2 (the MMA has eight and would leave them idle); products of parts are
+// exact. The query is scaled by a power of two that puts its largest element at 2^14, the weights by 2^15, so the parts hold 33
+// bits of the largest element, and no value is too large for fp16. (Two parts without a scale lost small weights and made
+// infinities of a query above 65504; against 64 bits, attention alone, 5 to 2000 keys, queries or keys away from the middle of fp16's
+// range: 2e-8 to 3e-6 for 1e-5 to 2e-4 or NaN. It takes no longer.)
+// f32 cache: multiply-adds in f32. The operands lie in registers as they came, 32 of them for the scores and 32 for the sums of a
+// warp's 16 keys. A step at 8, 120 and 510 keys: 315, 350, 376 us; with MMAs of two fp16 parts 327, 369, 386 (22 bits, and infinite
+// from 65504 on), of three bf16 parts 345, 388, 403.
 constexpr int kPassKeys = kWarps * 16;
 constexpr int kSplitKeys = 2 * kPassKeys;  // a head gets one more CTA per so many keys: a pass costs less than merging one more split
 
-// shared memory, in floats: new k [64], new v [64], the query's parts (16-bit) [3][64], max [8], sum [8], sums [8][64], the query's
-// scale taken back [4]
+// shared memory, in floats: new k [64], new v [64], the query [64] or its parts (fp16) [3][64], max [8], sum [8], sums [8][64], the
+// query's scale taken back [4]
 constexpr int kAttQ = 128, kAttMax = kAttQ + 96, kAttScale = kAttMax + 2 * kWarps + kWarps * 64;
 constexpr int kAttFloats = kAttScale + 4;
 
-// The next 16-bit parts of two values, taken off them.
-template <typename KV>
-__device__ __forceinline__ uint32_t take2(float &a, float &b);
-template <>
-__device__ __forceinline__ uint32_t take2<__half>(float &a, float &b)
+// The next fp16 parts of two values, taken off them.
+__device__ __forceinline__ uint32_t take2(float &a, float &b)
 {
     const __half2 h = __floats2half2_rn(a, b);
     const float2 f = __half22float2(h);
     a -= f.x, b -= f.y;
     return half2_bits(h);
 }
-template <>
-__device__ __forceinline__ uint32_t take2<float>(float &a, float &b)
-{
-    // bf16, cut off: three times eight bits are the value, and no value is rounded up to infinity
-    const uint32_t x = __float_as_uint(a), y = __float_as_uint(b);
-    a -= __uint_as_float(x & 0xffff0000u), b -= __uint_as_float(y & 0xffff0000u);
-    return __byte_perm(x, y, 0x7632);
-}
-template <typename KV>
-__device__ __forceinline__ void mma_kv(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b)
-{
-    if constexpr (sizeof(KV) == 2) mma(d, a0, a1, a2, a3, b);
-    else mma_bf16(d, a0, a1, a2, a3, b);
-}
 // Biased exponent of the power of two that puts a magnitude (its bits) into [2^14, 2^15); it and its inverse are normal numbers.
 __device__ __forceinline__ uint32_t scale_to_2_14(uint32_t bits) { return (uint32_t)min(max(127 + 14 + 127 - (int)(bits >> 23), 1), 253); }
 
+// The cache rows of a warp's 16 keys, and its sums. Of a key row lane (g, t) = (lane / 4, lane % 4) has dims 16 t to 16 t + 15 of
+// keys g and g + 8; scores() leaves the scores of these two in the lanes t = 0.
 template <typename KV>
-struct KeyTile;
+struct Rows;
 template <>
-struct KeyTile<__half> {  // keys g and g + 8 of the warp's 16: dims 16 t to 16 t + 15 as eight fp16 pairs each
-    static constexpr int kParts = 1;
-    uint32_t k[2][8];
-    __device__ __forceinline__ uint32_t part(int r, int i) { return k[r][i]; }
-    __device__ __forceinline__ void load(int r, const __half *row)
+struct Rows<__half> {
+    uint32_t k[2][8];  // fp16 pairs
+    uint2 q[4];
+    float unscale, acc[4][4];
+
+    // V rows as a tile [16 keys][64 dims] in shared memory, 16-byte pieces swizzled by key % 8 for ldmatrix
+    static __device__ __forceinline__ uint32_t v_at(int key, int piece) { return (uint32_t)(key * 128 + ((piece ^ (key & 7)) << 4)); }
+    __device__ __forceinline__ void load_k(int r, const __half *row)
     {
         const uint4 a = __ldcg(reinterpret_cast<const uint4 *>(row)), b = __ldcg(reinterpret_cast<const uint4 *>(row) + 1);
         k[r][0] = a.x, k[r][1] = a.y, k[r][2] = a.z, k[r][3] = a.w, k[r][4] = b.x, k[r][5] = b.y, k[r][6] = b.z, k[r][7] = b.w;
     }
-    __device__ __forceinline__ void load_new(int r, const float *row)  // (already rounded to fp16)
-    {
-#pragma unroll
-        for (int i = 0; i < 8; i++) k[r][i] = half2_bits(__floats2half2_rn(row[2 * i], row[2 * i + 1]));
-    }
-};
-template <>
-struct KeyTile<float> {
-    static constexpr int kParts = 3;
-    float f[2][16];  // what the parts so far have left
-    __device__ __forceinline__ uint32_t part(int r, int i) { return take2<float>(f[r][2 * i], f[r][2 * i + 1]); }
-    __device__ __forceinline__ void load(int r, const float *row)
-    {
-#pragma unroll
-        for (int i = 0; i < 4; i++) *reinterpret_cast<float4 *>(&f[r][4 * i]) = __ldcg(reinterpret_cast<const float4 *>(row) + i);
-    }
-    __device__ __forceinline__ void load_new(int r, const float *row)
-    {
-#pragma unroll
-        for (int i = 0; i < 16; i++) f[r][i] = row[i];
-    }
-};
-
-// The warp's V rows as a tile [16 keys][64 dims] of 16-bit parts in shared memory, 16-byte pieces swizzled by key % 8 for ldmatrix.
-__device__ __forceinline__ uint32_t v_at(int key, int piece) { return (uint32_t)(key * 128 + ((piece ^ (key & 7)) << 4)); }
-template <typename KV>
-struct ValueTile;
-template <>
-struct ValueTile<__half> {
-    __device__ __forceinline__ void load(char *tile, const __half *base, int ld, int keys, int lane)
+    __device__ __forceinline__ void load_v(char *tile, const __half *base, int ld, int keys, int lane)
     {
 #pragma unroll
         for (int i = 0; i < 4; i++) {
@@ -415,44 +367,159 @@ struct ValueTile<__half> {
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    __device__ __forceinline__ void arrive(char *, int) { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-    __device__ __forceinline__ void put_new(char *tile, int key, const float *v, int lane)
+    __device__ __forceinline__ void arrive() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+    __device__ __forceinline__ void new_k(int r, const float *row)  // (already rounded to fp16)
     {
+#pragma unroll
+        for (int i = 0; i < 8; i++) k[r][i] = half2_bits(__floats2half2_rn(row[2 * i], row[2 * i + 1]));
+    }
+    __device__ __forceinline__ void new_v(char *tile, int key, const float *v, int lane)
+    {
+        __syncwarp();  // (the zeros there are another lane's)
         *reinterpret_cast<uint32_t *>(tile + v_at(key, lane >> 2) + (lane & 3) * 4) = half2_bits(__floats2half2_rn(v[2 * lane], v[2 * lane + 1]));
+    }
+    // One warp: the rotated query's elements lane and lane + 32 into shared memory.
+    static __device__ __forceinline__ void put_q(float *att, float r0, float r1, int lane)
+    {
+        const uint32_t e = scale_to_2_14(__reduce_max_sync(0xffffffffu, max(__float_as_uint(fabsf(r0)), __float_as_uint(fabsf(r1)))));
+        r0 *= __uint_as_float(e << 23), r1 *= __uint_as_float(e << 23);
+        uint16_t *qp = reinterpret_cast<uint16_t *>(att + kAttQ);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const uint32_t w = take2(r0, r1);
+            qp[64 * i + lane] = (uint16_t)w, qp[64 * i + 32 + lane] = (uint16_t)(w >> 16);
+        }
+        if (lane == 0) att[kAttScale] = __uint_as_float((254 - e) << 23);
+    }
+    __device__ __forceinline__ void begin(const float *att, int g, int t)
+    {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            q[j] = make_uint2(0u, 0u);
+            if (g < 3) q[j] = *reinterpret_cast<const uint2 *>(reinterpret_cast<const char *>(att + kAttQ) + g * 128 + (t * 16 + 4 * j) * 2);
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[i][j] = 0.f;
+        }
+        unscale = att[kAttScale];
+    }
+    __device__ __forceinline__ float2 scores()
+    {
+        float d[2][4] = {};
+#pragma unroll
+        for (int j = 0; j < 4; j++) mma(d[j & 1], k[0][2 * j], k[1][2 * j], k[0][2 * j + 1], k[1][2 * j + 1], q[j]);
+        // (column 2 is lane t = 1's first)
+        const float a = d[0][0] + d[1][0], b = d[0][2] + d[1][2];
+        const float a2 = __shfl_xor_sync(0xffffffffu, a, 1), b2 = __shfl_xor_sync(0xffffffffu, b, 1);
+        return make_float2((a + ((d[0][1] + d[1][1]) + a2)) * unscale, (b + ((d[0][3] + d[1][3]) + b2)) * unscale);
+    }
+    __device__ __forceinline__ void add(const char *tile, float p0, float p1, float corr, int g, int t, int lane)
+    {
+        // weights of keys 2t, 2t + 1 and 2t + 8, 2t + 9
+        float w0 = __shfl_sync(0xffffffffu, p0, 8 * t) * 32768.f, w1 = __shfl_sync(0xffffffffu, p0, 8 * t + 4) * 32768.f;
+        float w2 = __shfl_sync(0xffffffffu, p1, 8 * t) * 32768.f, w3 = __shfl_sync(0xffffffffu, p1, 8 * t + 4) * 32768.f;
+        uint2 b = make_uint2(0u, 0u);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const uint32_t lo = take2(w0, w1), hi = take2(w2, w3);
+            if (g == i) b = make_uint2(lo, hi);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[i][j] *= corr;
+        __syncwarp();  // the tile's pieces are there for the whole warp
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            uint32_t a[4];
+            const uint32_t addr = s32(tile) + v_at((lane & 7) + ((lane >> 4) << 3), 2 * i + ((lane >> 3) & 1));
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
+                         : "r"(addr)
+                         : "memory");
+            mma(acc[i], a[0], a[1], a[2], a[3], b);
+        }
+        __syncwarp();  // before a next pass writes the tile
+    }
+    __device__ __forceinline__ void put_sums(float *wa, int g, int t, int)
+    {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float r0 = __shfl_xor_sync(0xffffffffu, acc[i][0], 1), r1 = __shfl_xor_sync(0xffffffffu, acc[i][2], 1);
+            if (t == 0) {
+                wa[i * 16 + g] = (acc[i][0] + (acc[i][1] + r0)) * (1.f / 32768.f);
+                wa[i * 16 + g + 8] = (acc[i][2] + (acc[i][3] + r1)) * (1.f / 32768.f);
+            }
+        }
     }
 };
 template <>
-struct ValueTile<float> {
-    float4 f[8];  // key 2 i + lane / 16, dims 4 (lane % 16) to + 3
-    __device__ __forceinline__ void load(char *, const float *base, int ld, int keys, int lane)
+struct Rows<float> {
+    float k[2][16], q[16];
+    float4 v[8], acc;  // of key 2 i + lane / 16 dims 4 (lane % 16) to + 3
+
+    __device__ __forceinline__ void load_k(int r, const float *row)
+    {
+#pragma unroll
+        for (int i = 0; i < 4; i++) *reinterpret_cast<float4 *>(&k[r][4 * i]) = __ldcg(reinterpret_cast<const float4 *>(row) + i);
+    }
+    __device__ __forceinline__ void load_v(char *, const float *base, int ld, int keys, int lane)
     {
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             const int key = 2 * i + (lane >> 4);
-            f[i] = key < keys ? __ldcg(reinterpret_cast<const float4 *>(base + (size_t)key * ld) + (lane & 15)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[i] = key < keys ? __ldcg(reinterpret_cast<const float4 *>(base + (size_t)key * ld) + (lane & 15)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
-    __device__ __forceinline__ void put_new(char *, int key, const float *v, int lane)
+    __device__ __forceinline__ void arrive() {}
+    __device__ __forceinline__ void new_k(int r, const float *row)
+    {
+#pragma unroll
+        for (int i = 0; i < 4; i++) *reinterpret_cast<float4 *>(&k[r][4 * i]) = reinterpret_cast<const float4 *>(row)[i];
+    }
+    __device__ __forceinline__ void new_v(char *, int key, const float *row, int lane)
     {
 #pragma unroll
         for (int i = 0; i < 8; i++)
-            if (key == 2 * i + (lane >> 4)) f[i] = *reinterpret_cast<const float4 *>(v + 4 * (lane & 15));
+            if (key == 2 * i + (lane >> 4)) v[i] = *reinterpret_cast<const float4 *>(row + 4 * (lane & 15));
     }
-    __device__ __forceinline__ void arrive(char *tile, int lane)  // the next parts
+    static __device__ __forceinline__ void put_q(float *att, float r0, float r1, int lane) { att[kAttQ + lane] = r0, att[kAttQ + lane + 32] = r1; }
+    __device__ __forceinline__ void begin(const float *att, int, int t)
     {
 #pragma unroll
+        for (int i = 0; i < 4; i++) *reinterpret_cast<float4 *>(&q[4 * i]) = reinterpret_cast<const float4 *>(att + kAttQ + t * 16)[i];
+        acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __device__ __forceinline__ float2 scores()
+    {
+        float a[2] = {}, b[2] = {};
+#pragma unroll
+        for (int i = 0; i < 16; i++) a[i & 1] = fmaf(k[0][i], q[i], a[i & 1]), b[i & 1] = fmaf(k[1][i], q[i], b[i & 1]);
+        float2 s = make_float2(a[0] + a[1], b[0] + b[1]);
+#pragma unroll
+        for (int o = 1; o <= 2; o <<= 1) s.x += __shfl_xor_sync(0xffffffffu, s.x, o), s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+        return s;
+    }
+    __device__ __forceinline__ void add(const char *, float p0, float p1, float corr, int, int, int lane)
+    {
+        acc.x *= corr, acc.y *= corr, acc.z *= corr, acc.w *= corr;
+#pragma unroll
         for (int i = 0; i < 8; i++) {
-            const uint32_t lo = take2<float>(f[i].x, f[i].y), hi = take2<float>(f[i].z, f[i].w);
-            *reinterpret_cast<uint2 *>(tile + v_at(2 * i + (lane >> 4), (lane & 15) >> 1) + (lane & 1) * 8) = make_uint2(lo, hi);
+            const float w = __shfl_sync(0xffffffffu, i < 4 ? p0 : p1, 4 * ((2 * i + (lane >> 4)) & 7));
+            acc.x = fmaf(w, v[i].x, acc.x), acc.y = fmaf(w, v[i].y, acc.y), acc.z = fmaf(w, v[i].z, acc.z), acc.w = fmaf(w, v[i].w, acc.w);
         }
+    }
+    __device__ __forceinline__ void put_sums(float *wa, int, int, int lane)
+    {
+        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 16), acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 16);
+        acc.z += __shfl_xor_sync(0xffffffffu, acc.z, 16), acc.w += __shfl_xor_sync(0xffffffffu, acc.w, 16);
+        if (lane < 16) reinterpret_cast<float4 *>(wa)[lane] = acc;
     }
 };
 
 // kbase / vbase: the split's first key; nk: its keys, the last of them the new one (in sm) if own_new
 template <typename KV>
 struct Attend {
-    KeyTile<KV> kt;
-    ValueTile<KV> vt;
+    Rows<KV> rows;
 
     __device__ __forceinline__ void load(const KV *kbase, const KV *vbase, int ld, int first, int nk_mem, char *tile, int lane)
     {
@@ -460,103 +527,42 @@ struct Attend {
 #pragma unroll
         for (int r = 0; r < 2; r++) {
             const int key = first + g + 8 * r;
-            if (key < nk_mem) kt.load(r, kbase + (size_t)key * ld + t * 16);
+            if (key < nk_mem) rows.load_k(r, kbase + (size_t)key * ld + t * 16);
         }
-        vt.load(tile, vbase + (size_t)first * ld, ld, nk_mem - first, lane);
+        rows.load_v(tile, vbase + (size_t)first * ld, ld, nk_mem - first, lane);
     }
     // one: the only split of its head: the result is final
     __device__ __forceinline__ void run(const KV *kbase, const KV *vbase, int ld, int nk, bool own_new, float *sm, char *tile, u64 *out, bool one,
                                         uint32_t ep, int warp, int lane)
     {
         float *wm = sm + kAttMax, *wl = wm + kWarps, *wa = wl + kWarps;
-        constexpr float kWeight = sizeof(KV) == 2 ? 32768.f : 1.f;  // scale of the softmax weights
         const int g = lane >> 2, t = lane & 3, nk_mem = own_new ? nk - 1 : nk;
-        uint2 q[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            q[j] = make_uint2(0u, 0u);
-            if (g < 3) q[j] = *reinterpret_cast<const uint2 *>(reinterpret_cast<const char *>(sm + kAttQ) + g * 128 + (t * 16 + 4 * j) * 2);
-        }
-        const float unscale = sm[kAttScale];
-        float acc[4][4] = {}, m = -INFINITY, l = 0.f;
+        rows.begin(sm, g, t);
+        float m = -INFINITY, l = 0.f;
 #pragma unroll 1
         for (int first = warp * 16; first < nk; first += kPassKeys) {
             if (first != warp * 16) load(kbase, vbase, ld, first, nk_mem, tile, lane);
-            if (own_new && nk_mem - first >= 0 && nk_mem - first < 16) {  // the new key is one of these
-                const int at = nk_mem - first;
-                if (g == at) kt.load_new(0, sm + t * 16);
-                if (g + 8 == at) kt.load_new(1, sm + t * 16);
-                if (sizeof(KV) == 4) vt.put_new(tile, at, sm + 64, lane);
-                vt.arrive(tile, lane);
-                if (sizeof(KV) == 2) {
-                    __syncwarp();
-                    vt.put_new(tile, at, sm + 64, lane);
-                }
-            } else {
-                vt.arrive(tile, lane);
+            rows.arrive();
+            const int at = nk_mem - first;
+            if (own_new && at >= 0 && at < 16) {  // the new key is one of these
+                if (g == at) rows.new_k(0, sm + t * 16);
+                if (g + 8 == at) rows.new_k(1, sm + t * 16);
+                rows.new_v(tile, at, sm + 64, lane);
             }
-            float d[2][4] = {};
-#pragma unroll
-            for (int part = 0; part < KeyTile<KV>::kParts; part++)
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    mma_kv<KV>(d[j & 1], kt.part(0, 2 * j), kt.part(1, 2 * j), kt.part(0, 2 * j + 1), kt.part(1, 2 * j + 1), q[j]);
-            // lanes t = 0: scores of keys g and g + 8; column 2 is lane t = 1's first
-            float s0 = d[0][0] + d[1][0], s1 = d[0][2] + d[1][2];
-            const float r0 = __shfl_xor_sync(0xffffffffu, s0, 1), r1 = __shfl_xor_sync(0xffffffffu, s1, 1);
-            s0 = (s0 + ((d[0][1] + d[1][1]) + r0)) * unscale, s1 = (s1 + ((d[0][3] + d[1][3]) + r1)) * unscale;
-            if (t != 0 || first + g >= nk) s0 = -INFINITY;
-            if (t != 0 || first + g + 8 >= nk) s1 = -INFINITY;
-            float mn = fmaxf(s0, s1);
+            float2 s = rows.scores();
+            if (t != 0 || first + g >= nk) s.x = -INFINITY;
+            if (t != 0 || first + g + 8 >= nk) s.y = -INFINITY;
+            float mn = fmaxf(s.x, s.y);
 #pragma unroll
             for (int o = 4; o <= 16; o <<= 1) mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
             mn = fmaxf(m, __shfl_sync(0xffffffffu, mn, 0));
-            const float corr = expf(m - mn), p0 = expf(s0 - mn), p1 = expf(s1 - mn);
+            const float corr = expf(m - mn), p0 = expf(s.x - mn), p1 = expf(s.y - mn);
             m = mn, l = l * corr + (p0 + p1);
-            // weights of keys 2t, 2t + 1 and 2t + 8, 2t + 9: their parts for columns 0 to 2
-            float w0 = __shfl_sync(0xffffffffu, p0, 8 * t) * kWeight, w1 = __shfl_sync(0xffffffffu, p0, 8 * t + 4) * kWeight;
-            float w2 = __shfl_sync(0xffffffffu, p1, 8 * t) * kWeight, w3 = __shfl_sync(0xffffffffu, p1, 8 * t + 4) * kWeight;
-            uint2 b = make_uint2(0u, 0u);
-#pragma unroll
-            for (int i = 0; i < 3; i++) {
-                const uint32_t lo = take2<KV>(w0, w1), hi = take2<KV>(w2, w3);
-                if (g == i) b = make_uint2(lo, hi);
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] *= corr;
-            __syncwarp();  // the tile's pieces are there for the whole warp
-#pragma unroll
-            for (int part = 0; part < KeyTile<KV>::kParts; part++) {
-                if (part > 0) {
-                    __syncwarp();
-                    vt.arrive(tile, lane);
-                    __syncwarp();
-                }
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    uint32_t a[4];
-                    const uint32_t addr = s32(tile) + v_at((lane & 7) + ((lane >> 4) << 3), 2 * i + ((lane >> 3) & 1));
-                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
-                                 : "r"(addr)
-                                 : "memory");
-                    mma_kv<KV>(acc[i], a[0], a[1], a[2], a[3], b);
-                }
-            }
-            __syncwarp();  // before a next pass writes the tile
+            rows.add(tile, p0, p1, corr, g, t, lane);
         }
 #pragma unroll
         for (int o = 4; o <= 16; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {  // column 2 is lane t = 1's first
-            const float r0 = __shfl_xor_sync(0xffffffffu, acc[i][0], 1), r1 = __shfl_xor_sync(0xffffffffu, acc[i][2], 1);
-            if (t == 0) {
-                wa[warp * 64 + i * 16 + g] = (acc[i][0] + (acc[i][1] + r0)) * (1.f / kWeight);
-                wa[warp * 64 + i * 16 + g + 8] = (acc[i][2] + (acc[i][3] + r1)) * (1.f / kWeight);
-            }
-        }
+        rows.put_sums(wa + warp * 64, g, t, lane);
         if (lane == 0) wm[warp] = m, wl[warp] = l;
         __syncthreads();
         if (warp < 3) {  // warps 0 and 1: 32 sums each; warp 2: max and sum of weights
@@ -822,19 +828,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
                     }
                     if (warp == 0) {
                         r0 *= 0.125f, r1 *= 0.125f;  // 1 / sqrt(64)
-                        float unscale = 1.f;
-                        if (sizeof(KV) == 2) {
-                            const uint32_t top = __reduce_max_sync(0xffffffffu, max(__float_as_uint(fabsf(r0)), __float_as_uint(fabsf(r1))));
-                            const uint32_t e = scale_to_2_14(top);
-                            r0 *= __uint_as_float(e << 23), r1 *= __uint_as_float(e << 23), unscale = __uint_as_float((254 - e) << 23);
-                        }
-                        uint16_t *qp = reinterpret_cast<uint16_t *>(dst);
-#pragma unroll
-                        for (int i = 0; i < 3; i++) {
-                            const uint32_t w = take2<KV>(r0, r1);
-                            qp[64 * i + lane] = (uint16_t)w, qp[64 * i + 32 + lane] = (uint16_t)(w >> 16);
-                        }
-                        if (lane == 0) att[kAttScale] = unscale;
+                        Rows<KV>::put_q(att, r0, r1, lane);
                     } else {
                         const KV c0 = (KV)r0, c1 = (KV)r1;  // as a later step will read them
                         if (h == kvh * hpk) {
