@@ -4,7 +4,7 @@
     python bench.py --case gemv|gemm|decode|read ...          (small fixed workloads for a profiler, see below)
 
 Headline. A step is one decode step (one token) of the 24-layer model: 96 fused int4 linears (q|k|v, o, gate|up,
-down per layer), the fp16 tied lm_head, the steps between them and the on-device argmax, replayed as one CUDA graph.
+down per layer), the fp16 tied lm_head, the steps between them and the on-device argmax, up to 64 steps in one persistent kernel.
 Weights are N(0, 0.02) quantised by round-to-nearest into the GPTQ checkpoint layout, the prompt is 512 random ids
 (synthetic: no checkpoint or dataset is available offline). Every token streams 458 MB of weights, more than the
 126 MB L2, so no explicit L2 flush is needed between steps. The timed region is exactly K steps after the 512-token
@@ -611,7 +611,7 @@ def run_ours(args) -> None:
         gpu.synchronize()
         clock.barrier()
 
-    # ---- device-timed decode: W warm-up steps (captures the graph), then regions of exactly K steps
+    # ---- device-timed decode: W warm-up steps (lays the weights out), then regions of exactly K steps
     tok = refill()
     model.decode_greedy(tok, W)
     launches_per_region, regions = 0, []
@@ -741,7 +741,7 @@ def run_case(args) -> None:
         model.upload_gptq_model(weights, fuse=True)
         prompt = np.random.default_rng(100).integers(0, cfg.vocab_size, args.prompt).astype(np.uint32)
         tok = int(np.argmax(model.read_tensor(model.prefill(prompt, last_only=True))))
-        toks = model.decode_greedy(tok, 1)  # builds the graph
+        toks = model.decode_greedy(tok, 1)  # lays the weights out
         gpu.synchronize()
         t0 = time.perf_counter()
         toks = model.decode_greedy(int(toks[-1]), args.steps)

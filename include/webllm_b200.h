@@ -284,8 +284,9 @@ WB_API int wb_qwen_prefill(wb_qwen *model, const uint32_t *tokens, int64_t n, in
 /* decodeStep(token): logits [1, V]. */
 WB_API int wb_qwen_decode_step(wb_qwen *model, uint32_t token, uint64_t *logits_offset);
 /* Greedy decoding kept on the device: feeds `first_token`, then n_steps times (forward one token, argmax
- * with the reference's first-strict-maximum rule, src/infer/sampler.ts:30-36, append). The step is captured
- * in a CUDA graph on first use and replayed; out_tokens receives the n_steps sampled tokens. Replaces the
+ * with the reference's first-strict-maximum rule, src/infer/sampler.ts:30-36, append). Up to 64
+ * steps are one launch of a persistent kernel; for models that it does not take, the step is captured in a CUDA graph on
+ * first use and replayed. out_tokens receives the n_steps sampled tokens. Replaces the
  * per-token logits readback of generateQwen (src/infer/qwen-generate.ts:66-74). */
 WB_API int wb_qwen_decode_greedy(wb_qwen *model, uint32_t first_token, int64_t n_steps, uint32_t *out_tokens);
 /* Logits of the last step run by wb_qwen_decode_greedy, [V] f32, copied to the host. */

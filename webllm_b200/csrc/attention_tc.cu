@@ -7,8 +7,8 @@
 //   S = Q K^T  (tcgen05.mma, both operands K-major tiles in shared memory, 128 x 64 f32 in tensor memory)
 //   O += P V   (P from tensor memory, V as it lies in the cache: keys x dims, an MN-major operand; 128 x 64 f32)
 // and in between a thread of the group owns one row: it reads its 64 scores, takes the maximum, the exponentials (ex2, 16 a cycle
-// per SM) and writes P as fp16 over S. O stays in tensor memory; it is rescaled only where a row's maximum has grown by more
-// than 2^8 since the last time (the weights of the meantime are at most 2^8, and the final division takes the same maximum, so
+// per SM) and writes P as fp16 over S. O stays in tensor memory; as in FlashAttention-4 it is rescaled only where a row's maximum has
+// grown by more than 2^8 since the last time (the weights of the meantime are at most 2^8, and the final division takes the same maximum, so
 // nothing is approximated). K and V boxes come by TMA, two stages each; rows past the last key read as zeros.
 // Bound by the chain of a block, product - softmax - product, some 3000 cycles when four groups share the SM's exponentials, times
 // the blocks of the longest CTA. So four groups of one row tile rather than two of each of two: half as many blocks in the

@@ -7,7 +7,7 @@
 //   * weights never wait for anything: at set-up they are laid out per CTA and layer as one contiguous block, and bulk copies
 //     keep two to three blocks in flight, across phase, layer and token boundaries;
 //   * activations are handed over WITHOUT a barrier: every f32 value is stored together with the step's epoch in one 64-bit
-//     word, and a reader polls the very words that it needs. A hand-over is one store and one load through L2, about
+//     word (as in NCCL's LL protocol), and a reader polls the very words that it needs. A hand-over is one store and one load through L2, about
 //     0.9 us from all CTAs to all, against a store, a fence, an atomic and a second round trip for a grid barrier. All layers
 //     use the same words, with an epoch of their own: while each layer had its own, a poll's first try missed L2 (the weights
 //     had pushed the words out since the step before) and came back from HBM a microsecond later, empty. Writing them over is
@@ -16,8 +16,9 @@
 //     by gate|up of l + 1 and by q|k|v of l + 1;
 //   * every CTA keeps the residual stream itself, so the norms need no hand-over of their own.
 // A layer is five such hand-overs: q|k|v, attention, o, gate|up (with silu * up at the producer), down.
-// Measured on the 0.5B shapes: 0.49 -> 0.30 ms per token at short contexts (0.33 at 400 keys), of which about 0.13 are the CTA's
-// own arithmetic and latencies, 0.03 lm_head beyond what its first slots hide, and the rest hand-overs.
+// Measured on the 0.5B shapes: 0.49 -> 0.31 ms per token at short contexts (0.34 at 400 keys; 0.315 and 0.40 with an f32 cache), of
+// which about 0.13 are the CTA's own arithmetic and latencies, 0.03 lm_head beyond what its first slots hide, and the rest
+// hand-overs.
 //
 // Arithmetic. A CTA owns whole output columns in tiles of 8. One m16n8k16 MMA multiplies 256 weights: rows 0-7 of the weight
 // operand are half of the positions of a tile's 8 columns, rows 8-15 the other half, and the activation operand holds the first
@@ -1182,8 +1183,11 @@ __global__ void __launch_bounds__(256) lay_out_aux_kernel(const Source *__restri
 
 // Which models take this kernel: the shapes it is written for (head size 64, fused int4 projections of group 128, a hidden size
 // of four values per thread), and a layer small enough that two of a CTA's blocks fit its shared memory, so that the ring can run
-// ahead of the hand-overs (0.5B: 61 KB per CTA and layer, three slots). Larger models are bound by their weights, not by the
-// hand-overs, and stay on one kernel per projection.
+// ahead of the hand-overs (0.5B: 61 KB per CTA and layer, three slots). Other models stay on five kernels a layer, which is not
+// because their weights bound them: a layer takes 22.7 us at hidden size 1152 (head size 64; 1.6 us of HBM time), and at head size
+// 128 29.8 us at 1536 x 8960 (3.7), 39.6 at 2048 x 11008 (6.1) and 86.7 at 3584 x 18944 (18.5). It is that the residual stream, the
+// staging and the attention here are laid out for four values per thread and 64 dims, and that a layer of the larger ones does not
+// fit a CTA's shared memory twice.
 static bool fused_shape(const wb_qwen *m, int n, int *blob, int *slot, int *slots, int *smem)
 {
     using namespace fd;

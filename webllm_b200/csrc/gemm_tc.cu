@@ -1069,6 +1069,10 @@ int launch_gemm_tc(wb_context *ctx, const Weight &w, const void *A, void *C, con
     return WB_OK;
 }
 
+// gate | up with silu as one kernel wherever the plain product runs unsplit on CTA pairs, in the tile that it would have: whole
+// layers, separate and fused, us, K = 896 (I = 4864): 256 rows 60.1, 59.2; 512 75.6, 74.3; 1024 108, 103; 2048 152, 147; K = 2048
+// (11008): 256 rows 109, 106; 1024 229, 217; 2048 454, 430; K = 3584 (18944): 192 rows 157, 152; 1024 545, 529; 2048 1105, 1051. At no
+// size measured (128 to 2048 rows, K = 896, 1536, 2048 and 3584) was it slower.
 int launch_gate_up_silu(wb_context *ctx, const Weight &w, const __half *A, __half *act, int64_t M, bool *done)
 {
     *done = false;
