@@ -61,6 +61,10 @@ CONFIG = {"workload": WORKLOAD,
           "timed_region": "exactly --steps decode steps after the 512-token prompt; repeated until >= 0.5 s is timed, median region",
           "l2": "each step streams 458 MB of weights (> 126 MB L2); no flush needed"}
 
+# dram__bytes_read.sum + dram__bytes_write.sum per step of decode_fused_kernel, from an ncu capture of a launch of two steps of
+# the 24-layer model at 18 keys (956.2 MB). Algorithmic bytes: int4 tensors + fp16 lm_head, 458 171 392 a step.
+NCU_TRAFFIC_BYTES_PER_STEP = 478115384
+
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of gptq_gemv_mma_kernel, mean over the four projections
 # of a layer, from an ncu capture of a 2-layer model of the same shapes (one pass per launch, caches flushed between
 # launches, the L2 prefetch of the next weight switched off); traffic is proportional to the number of layers, so the
@@ -327,8 +331,9 @@ def rotating_linear(gpu, clock, tag, t, M, act="f16", copies=None, reps=10):
 
 # ---------------------------------------------------------------------------------------------------- sections of the line
 def kernel_sections(gpu, clock, cfg, peaks) -> dict:
-    """roofline: the int4 GEMV over the 96 fused linears of one token (command batch, CUDA events on the launching
-    stream); algorithmic bytes = packed weights + scales + zeros + f32 x + f32 y of every launch."""
+    """The 96 fused linears of one token as separate launches of the int4 GEMV, which models that the persistent kernel does not
+    take decode with (command batch, CUDA events on the launching stream); algorithmic bytes = packed weights + scales +
+    zeros + f32 x + f32 y of every launch."""
     peak = peaks["hbm_gbs"]
     gpu.arena.reset()
     C, KV, I = cfg.n_embd, cfg.kv_dim, cfg.intermediate
@@ -656,13 +661,18 @@ def run_ours(args) -> None:
 
     extras = {}
     if rank == 0:
-        line["roofline"] = kernel_sections(gpu, clock, cfg, peaks)
-        # the same question for the whole step (all 125 launches, lm_head included), from the headline's own timing:
-        # weight bytes that one token has to stream / the measured step time
+        # the step is one kernel, up to 64 of them a launch: weight bytes that a token has to stream (int4 tensors and
+        # lm_head) over the headline's own time
         step_bytes = int4_bytes_per_token(cfg) + cfg.vocab_size * cfg.n_embd * 2
         step_gbs = step_bytes / (line["ms_per_step"] * 1e-3) / 1e9
-        line["roofline"]["whole_step"] = {"algorithmic_bytes": step_bytes, "achieved": step_gbs, "unit": "GB/s",
-                                          "frac": step_gbs / peaks["hbm_gbs"], "hbm_floor_ms": step_bytes / peaks["hbm_gbs"] / 1e6}
+        per_launch = K / launches_per_region
+        line["roofline"] = {"bound": "hbm", "kernel": "decode_fused_kernel", "achieved": step_gbs, "peak": peaks["hbm_gbs"],
+                            "unit": "GB/s", "frac": step_gbs / peaks["hbm_gbs"], "peak_source": f"of {peaks['source']}",
+                            "launches_timed": int(launches_per_region), "steps_per_launch": per_launch,
+                            "avg_launch_us": line["ms_per_step"] * 1e3 * per_launch,
+                            "algorithmic_bytes_per_launch": step_bytes * per_launch,
+                            "traffic": NCU_TRAFFIC_BYTES_PER_STEP * per_launch, "hbm_floor_ms_per_step": step_bytes / peaks["hbm_gbs"] / 1e6,
+                            "separate_projections": kernel_sections(gpu, clock, cfg, peaks)}
     if not args.no_extras:
         if rank == 0:
             progress("extras: gemv")
