@@ -61,3 +61,21 @@ def test_which_calls_it_takes_on_wide_matrices(gpu, K, N, small):
         assert (f16["kernel_name"] == "gemm_tc" and f16["block"] == 256) == (small and M > 8), (M, f16)
         assert (f16["kernel_name"] == "gemv_mma") == (M <= 8 or (M <= 12 and not small)), (M, f16)
         assert f32["kernel_name"] == "gemv_mma", (M, f32)
+
+
+@pytest.mark.parametrize("K,N", [(896, 9728), (2560, 3360)])
+def test_column_sharded_calls_on_its_matrices(gpu, oracle, K, N):
+    """A call with a placement has no use of the kernel by itself, but may write the dense piece with it that a scatter launch spreads
+    (short K) or go to the tcgen05 kernel's own placement: the tensor equals the product, the columns beside it are left alone."""
+    t = synthetic.random_gptq(K, N, 128, seed=N, zeros="any")
+    h = register(gpu, f"gsg_{K}_{N}", t)
+    x = np.random.default_rng(K).standard_normal((9, K)).astype(np.float16)
+    ref = oracle.gemm_nt_ref(x.astype(np.float32), oracle_weight(oracle, t), 9, N, K)
+    gpu.arena.reset()
+    A, full, tmp = gpu.arena.alloc(9 * K, [9, K], "f16"), gpu.arena.alloc(9 * (N + 64), [9, N + 64], "f32"), gpu.arena.alloc(9 * N, [9, N], "f32")
+    gpu.write(A, x)
+    gpu.write(full, np.full(9 * (N + 64), -7.0, np.float32))
+    gpu.linear_gather(h, A, full, tmp, None, 9, N + 64, 32, [])
+    got = gpu.read(full).reshape(9, N + 64)
+    assert np.all(got[:, :32] == -7.0) and np.all(got[:, 32 + N:] == -7.0)
+    assert_close(oracle, got[:, 32:32 + N], ref, 1e-3, f"{K}x{N}")
