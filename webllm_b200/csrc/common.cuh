@@ -93,8 +93,8 @@ struct Weight {
     bool has_zeros = false;
     uint64_t bytes = 0;
     uint64_t arena_top = 0;   // `used` of the weight arena right after this registration (what wb_weight_pop checks)
-    // tensor maps of the weight operand of the tensor-core GEMM, in boxes of 128, 256 and 64 columns
-    mutable TmapSlot tmap_tc[3];
+    // tensor maps of the weight operand of the tensor-core GEMM, in boxes of 128, 256 and 64 columns, and of 128 columns by 16 rows
+    mutable TmapSlot tmap_tc[4];
     mutable PlanSlot plans[4];
     mutable int next_plan = 0;
     mutable CallMap tmap_x, tmap_c;
@@ -204,6 +204,11 @@ bool gemm_small_takes(wb_context *ctx, const Weight &w, int64_t M);
 bool plan_gemm_small(wb_context *ctx, const Weight &w, int64_t M, wb_plan *plan);
 int launch_gemm_small(wb_context *ctx, const Weight &w, const void *A, void *C, const float *bias, int64_t M, int act_dtype, int out_dtype,
                       const wb_plan &plan);
+// gemm_thin.cu: the tensor-core GEMM with its weight operand in tensor memory, up to 128 rows; likewise with this block size
+constexpr int kThinBlock = 896;
+inline bool is_thin_plan(const wb_plan &plan) { return plan.kernel == WB_KERNEL_GEMM_TC && plan.block == kThinBlock; }
+bool plan_gemm_thin(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, wb_plan *plan, double *t_out);
+int launch_gemm_thin(wb_context *ctx, const Weight &w, const void *x, bool perm, void *C, const float *bias, int64_t M, int out_dtype, const wb_plan &plan);
 int launch_linear(wb_context *ctx, const Weight &w, const void *A, void *C, const float *bias, int64_t M,
                   int act_dtype, int out_dtype, int exact, const LinearFusion *fusion = nullptr);
 

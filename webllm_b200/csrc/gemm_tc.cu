@@ -615,6 +615,19 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
     if (warp == MMA_WARP) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
+// The same for gemm_thin.cu: the k's of a packed word in the order 0 4 1 5 2 6 3 7. n is a multiple of 8.
+__global__ void cast_f32_to_f16_words_kernel(const float *__restrict__ in, __half *__restrict__ out, int64_t n)
+{
+    pdl_sync();
+    int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x * 8;
+    for (; i < n; i += stride) {
+        const float4 a = *reinterpret_cast<const float4 *>(in + i), b = *reinterpret_cast<const float4 *>(in + i + 4);
+        const __half2 h[4] = {__floats2half2_rn(a.x, b.x), __floats2half2_rn(a.y, b.y), __floats2half2_rn(a.z, b.z), __floats2half2_rn(a.w, b.w)};
+        *reinterpret_cast<uint4 *>(out + i) = *reinterpret_cast<const uint4 *>(h);
+    }
+}
+
 __global__ void cast_f32_to_f16_kernel(const float *__restrict__ in, __half *__restrict__ out, int64_t n)
 {
     pdl_sync();  // `out` may still be read by the GEMM in front
@@ -709,7 +722,7 @@ __global__ void scatter_cols_kernel(const void *__restrict__ src, const OutPlace
 // host side
 // ----------------------------------------------------------------------------------------------------
 
-static int make_map_2d(wb_context *ctx, CUtensorMap *map, CUtensorMapDataType dt, int elem_bytes, const void *base,
+int make_map_2d(wb_context *ctx, CUtensorMap *map, CUtensorMapDataType dt, int elem_bytes, const void *base,
                        uint64_t inner, uint64_t outer, uint32_t box_inner, uint32_t box_outer, bool swizzle128)
 {
     cuuint64_t dims[2] = {inner, outer};
@@ -846,6 +859,14 @@ int plan_gemm_tc(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int
     // microseconds that the stores to the peers of a column-sharded call take at ~700 GB/s per direction
     const double t_remote = ctx->place.n_dst > 1 ? (double)(ctx->place.n_dst - 1) * M * w.N * ctx->place.elem_bytes / 700e3 : 0.;
     const double t_one = pick_plan(M, w.N, kblocks, ctx->sm_count, ctx->force_split, t_remote, &mt, &nh, &S);
+    if (pair_mode == 1) {
+        wb_plan thin = *plan;
+        double t;
+        if (plan_gemm_thin(ctx, w, M, act_dtype, &thin, &t) && t < t_one) {
+            *plan = thin;
+            return WB_OK;
+        }
+    }
     // Stores into peers' slabs stay with the one-CTA kernels: a two-GPU run of the pair kernel with peer destinations
     // (7B-class shards at M = 4096) ended in a launch failure whose cause reading has not shown, so it is not launched so.
     const bool pair_ok = pair_mode > 0 && ctx->place.n_dst <= 1 && gemm_pair_supports(w, M) && ctx->sm_count >= 2;
@@ -956,6 +977,7 @@ int launch_gemm_tc(wb_context *ctx, const Weight &w, const void *A, void *C, con
     (void)exact;
     if (plan.block == kSmallBlock) return launch_gemm_small(ctx, w, A, C, bias, M, act_dtype, out_dtype, plan);
     const char *base = ctx->arena[WB_ARENA_WEIGHTS].base;
+    const bool thin = is_thin_plan(plan);
     const void *a16 = A;
     if (act_dtype == WB_F32) {
         // The reference rounds f32 activations to fp16 when it stages a tile (gemm_nt_f16_from_f32.wgsl:58-62).
@@ -966,11 +988,12 @@ int launch_gemm_tc(wb_context *ctx, const Weight &w, const void *A, void *C, con
         // longer cast more than the start (cast and GEMM, with -> without: 1024 x 3584 32.7 -> 33.2 us, 2048 x 3584 55.8 -> 56.3, but
         // 2048 x 4864 34.7 -> 33.5).
         const bool early = n <= (int64_t)8 << 20;
-        WB_CUDA(launch_cluster_ex(tc::cast_f32_to_f16_kernel, dim3((unsigned)blocks), dim3(256), 0, ctx->stream, 1u, early, (const float *)A,
-                                  (__half *)ctx->workspace, n));
+        WB_CUDA(launch_cluster_ex(thin ? tc::cast_f32_to_f16_words_kernel : tc::cast_f32_to_f16_kernel, dim3((unsigned)blocks), dim3(256), 0, ctx->stream, 1u,
+                                  early, (const float *)A, (__half *)ctx->workspace, n));
         ctx->launches++;
         a16 = ctx->workspace;
     }
+    if (thin) return launch_gemm_thin(ctx, w, a16, act_dtype == WB_F32, C, bias, M, out_dtype, plan);
     const int mt = plan.tile_m;
     const bool pair = plan.kernel == WB_KERNEL_GEMM_TC_PAIR;
     const int nh = pair ? 1 : plan.tile_n == 2 * tc::BN ? 2 : 1;  // a CTA of a pair takes 128-column boxes
