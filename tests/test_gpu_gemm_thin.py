@@ -76,3 +76,24 @@ def test_infinities_and_nan_stay_in_their_rows(gpu, oracle):
     ref = _reference(oracle, t, x[clean], len(clean), N, K).reshape(len(clean), N)
     assert np.isnan(got[7]).all() and not np.isfinite(got[4]).any()
     assert_close(oracle, got[clean].ravel(), ref.ravel(), 1e-3, "rows beside them")
+
+
+@pytest.mark.parametrize("K,N,M", [(896, 1152, 404), (1472, 260, 129), (896, 132, 1000), (3456, 392, 300), (896, 4868, 177), (512, 9604, 256)])
+def test_several_row_tiles(gpu, oracle, K, N, M):
+    """Row tiles of equal size (up to 128 or up to 256 rows), the last one not full, alone and with slices."""
+    t = synthetic.random_gptq(K, N, 64, seed=M, zeros="any")
+    h = register(gpu, f"thm_{K}_{M}", t)
+    bias = np.random.default_rng(N).standard_normal(N).astype(np.float32)
+    hb = gpu.f32_upload(f"thmb_{K}_{M}", bias)
+    x = np.random.default_rng(M).standard_normal((M, K)).astype(np.float32)
+    x16 = x.astype(np.float16)
+    ref = _reference(oracle, t, x16, M, N, K, bias)
+    p = gpu.plan(h, M, "f16")
+    assert p["block"] == BLOCK and p["grid_x"] in (-(-M // 128), -(-M // 256)) and p["grid_x"] * p["tile_m"] >= M, p
+    for split in (0, 1, 3):
+        gpu.plan_override(0, split)
+        try:
+            for act, xin, out in (("f16", x16, "f32"), ("f32", x, "f16")):
+                assert_close(oracle, run_linear(gpu, h, xin, M, N, hb, act=act, out=out), ref, 1e-3, f"{K}x{N} M={M} {act} split {split}")
+        finally:
+            gpu.plan_override(0, 0)

@@ -55,7 +55,7 @@ struct TmapSlot {
 // calls a weight with the same few row counts again and again.
 struct PlanSlot {
     int64_t M = 0;
-    int act_dtype = 0, exact = 0, allow_stream = 0;
+    int act_dtype = 0, exact = 0, allow_stream = 0, keep_slices = 0;
     wb_plan plan;
 };
 

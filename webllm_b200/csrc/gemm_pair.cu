@@ -121,9 +121,10 @@ struct PairTail {
 // GATHER: the result goes to the placement in Params (this GPU's slab and its peers', row pitch ld_out) from registers.
 // SILU: the weight is gate | up (N = 2 I columns) and the result is fp16 silu(gate) * up, [M, I] (siluMulRef,
 // src/reference/qwen-ref.ts:119-123), the input of the down projection. A CTA's 128 weight columns are 64 of gate and the same 64
-// of up, so both factors of a value end up in its own tensor memory; the epilogue warps exchange them through shared memory, half
-// of the rows each way, and compute in f32 what a pass over the f32 result would. At 2048 x 896 -> 2 x 4864 that pass moved
-// 100 MB and took 18 us, and the GEMM itself stored 80 MB instead of 20.
+// of up, dealt so that both factors of a value lie in one warp's quarter of its tensor memory; the epilogue warps exchange
+// them by shuffles and compute in f32 what a pass over the f32 result would. (2048 x 896 -> 2 x 4864: 43.7 us and a pass of 17.8;
+// with the factors exchanged through shared memory, two barriers of four warps per 32 rows, and the result through staging
+// tiles 51.)
 template <int MT, bool SPLIT, bool STG, bool GATHER = false, bool SILU = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(SILU), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
@@ -161,11 +162,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     auto item_m0 = [&](int ti) { return (item_index(ti) % tiles_mn % tiles_m) * MT; };
     constexpr int CTA_COLS = SILU ? BN / 2 : BN;  // output columns of a CTA's item
     auto item_n0 = [&](int ti) { return (item_index(ti) % tiles_mn / tiles_m) * (2 * CTA_COLS) + (int)rank * CTA_COLS; };
-    auto weight_col = [&](int n0, int i) { return SILU && i >= CTA_COLS ? p.N / 2 + n0 + i - CTA_COLS : n0 + i; };  // of accumulator lane i
+    // Column of the weight that accumulator lane i holds. SILU: of every 32 lanes the lower 16 hold gate columns, the upper 16 the same
+    // columns of up.
+    auto weight_col = [&](int n0, int i) { return SILU ? n0 + (i >> 5) * 16 + (i & 15) + (i & 16 ? p.N / 2 : 0) : n0 + i; };
     auto load_weights = [&](int s, int n0, int row, uint64_t *bar) {
         uint8_t *dst = smem + s * S::STAGE_BYTES + S::X_BYTES + S::WD_BYTES;
         tma_load_2d(dst, &map_w, n0, row, bar);
-        if constexpr (SILU) tma_load_2d(dst + S::WP_BYTES / 2, &map_w, weight_col(n0, CTA_COLS), row, bar);
+        if constexpr (SILU) tma_load_2d(dst + S::WP_BYTES / 2, &map_w, p.N / 2 + n0, row, bar);
     };
     auto item_kb0 = [&](int ti) { return SPLIT ? item_slice(ti) * p.kb_per_slice : is_tail(ti) ? (pair % tail.St) * tail.per : 0; };
     auto item_kbn = [&](int ti) {
@@ -278,7 +281,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         const int tn = (unpack_idx * 32 + lane) % SET_THREADS;
         const __half2 sixteenth = __float2half2_rn(0.0625f);
         // packed words of this column: rows of 128 (or, in two boxes of gate and up, 64) words
-        const int src_off = S::X_BYTES + S::WD_BYTES + tn * 4 + (SILU && tn >= CTA_COLS ? S::WP_BYTES / 2 - CTA_COLS * 4 : 0);
+        const int src_off = S::X_BYTES + S::WD_BYTES + (SILU ? ((tn >> 5) * 16 + (tn & 15)) * 4 + (tn & 16 ? S::WP_BYTES / 2 : 0) : tn * 4);
         int dst_off[8];
 #pragma unroll
         for (int rr = 0; rr < 8; rr++) dst_off[rr] = S::X_BYTES + tn * 128 + ((rr ^ (tn & 7)) << 4);
@@ -404,44 +407,41 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             const float bias = (!SPLIT && p.bias && n < p.N) ? p.bias[n] : 0.f;
             auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(eg + 1) : "memory"); };
             if constexpr (SILU) {
-                // 32 token rows at a time. Of the CTA's 64 columns warps 0, 1 hold gate and 2, 3 up: gate goes to the exchange
-                // tile for the upper 16 rows, up for the lower 16, then each warp finishes the rows whose other factor it was
-                // given. (A group's barrier after the products also says that the exchange tile has been read.)
-                const int col = (q & 1) * 32 + lane;
-                const bool is_up = q >= 2;
-                uint8_t *mine = stg + eg * STG_BYTES;
-                float *ex = (float *)mine;  // [32 rows][64 columns]
-                auto rows16 = [&](int c, auto &&f) {
+                // 16 token rows at a time, a warp by itself. Its lower lanes hold gate columns and its upper ones the same columns of
+                // up: each half gives the other what it needs of eight rows, and the results are exchanged among eight lanes
+                // until each holds 16 bytes of one row, as in store_block16_f16.
+                const bool upper = lane & 16, b1 = lane & 1, b2 = lane & 2, b4 = lane & 4;
+                __half *out = (__half *)p.out + n0 + q * 16 + (lane & 8);
+                const int I = p.N / 2;
+#pragma unroll 1
+                for (int c = eg * 16; c < MT; c += GROUPS * 16) {
                     uint32_t r[16];
                     tmem_ld_32x32b_x16(acc + (uint32_t)c, r);
                     tmem_ld_wait();
+                    float o[8];
 #pragma unroll
-                    for (int j = 0; j < 16; j++) f(j, __uint_as_float(r[j]));
-                };
-                const int give = is_up ? 0 : 16, keep = 16 - give;
-#pragma unroll 1
-                for (int c = eg * SILU_ROWS; c < MT; c += GROUPS * SILU_ROWS) {
-                    __half *tile = (__half *)(mine + STG_BYTES / 2) + stg_sel * SILU_ROWS * 64;  // [32 rows][64 columns], two of them
-                    rows16(c + give, [&](int j, float v) { ex[(give + j) * 64 + col] = v; });
-                    if (epi_tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                    group_sync();
-                    float o[16];  // all at once: a load from ex would not be moved over a store to the tile
-#pragma unroll
-                    for (int j = 0; j < 16; j++) o[j] = ex[(keep + j) * 64 + col];
-                    rows16(c + keep, [&](int j, float v) {
-                        const float g = is_up ? o[j] : v, u = is_up ? v : o[j];
-                        tile[(keep + j) * 64 + col] = __float2half_rn(silu(g) * u);
-                    });
-                    fence_async_smem();
-                    group_sync();
-                    if (epi_tid == 0) {
-                        if (m0 + c < p.M && n0 < p.N / 2)
-                            asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];"
-                                         ::"l"(&map_c), "r"(n0), "r"(m0 + c), "r"(0), "r"(smem_u32(tile))
-                                         : "memory");
-                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    for (int j = 0; j < 8; j++) {
+                        const float own = __uint_as_float(upper ? r[8 + j] : r[j]);
+                        const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(upper ? r[j] : r[8 + j]), 16);
+                        o[j] = silu(upper ? got : own) * (upper ? own : got);
                     }
-                    stg_sel ^= 1;
+                    uint32_t h[4];  // h[i]: two columns of row 2 i + b1
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const float got = __shfl_xor_sync(0xffffffffu, b1 ? o[2 * i] : o[2 * i + 1], 1);
+                        const __half2 pr = b1 ? __floats2half2_rn(got, o[2 * i + 1]) : __floats2half2_rn(o[2 * i], got);
+                        h[i] = *(const uint32_t *)&pr;
+                    }
+                    uint2 f[2];  // f[i]: four columns of row 4 i + 2 b2 + b1
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        const uint32_t got = __shfl_xor_sync(0xffffffffu, b2 ? h[2 * i] : h[2 * i + 1], 2);
+                        f[i] = b2 ? make_uint2(got, h[2 * i + 1]) : make_uint2(h[2 * i], got);
+                    }
+                    const uint2 snd = b4 ? f[0] : f[1];
+                    const uint32_t gx = __shfl_xor_sync(0xffffffffu, snd.x, 4), gy = __shfl_xor_sync(0xffffffffu, snd.y, 4);
+                    const int m = m0 + c + (upper ? 8 : 0) + (lane & 7);
+                    if (m < p.M) *(uint4 *)(out + (int64_t)m * I) = b4 ? make_uint4(gx, gy, f[1].x, f[1].y) : make_uint4(f[0].x, f[0].y, gx, gy);
                 }
             } else if (is_tail(ti)) {
                 // a K slice of a leftover item: the f32 partial tile [MT][256] of this pair, no bias
@@ -600,7 +600,7 @@ static cudaError_t launch_pair_mt(const CUtensorMap &mx, const CUtensorMap &mw, 
         return launch_pdl(kernel, dim3((unsigned)(2 * pairs)), dim3((unsigned)tcp::pair_threads(silu)), (size_t)smem, st, mx, mw, mc ? *mc : mx, p, tiles_m,
                           tiles_n, n_items, mc ? 1 : 0, tail);
     };
-    if (silu) return go(tcp::gemm_pair_kernel<MT, false, true, false, true>, 5, tcp::SmemPair<MT, true>::TOTAL);
+    if (silu) return go(tcp::gemm_pair_kernel<MT, false, false, false, true>, 5, tcp::SmemPair<MT, false>::TOTAL);
     if (S > 1)
         return mc ? go(tcp::gemm_pair_kernel<MT, true, true>, 3, tcp::SmemPair<MT, true>::TOTAL)
                   : go(tcp::gemm_pair_kernel<MT, true, false>, 1, tcp::SmemPair<MT, false>::TOTAL);

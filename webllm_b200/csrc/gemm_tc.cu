@@ -859,14 +859,9 @@ int plan_gemm_tc(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int
     // microseconds that the stores to the peers of a column-sharded call take at ~700 GB/s per direction
     const double t_remote = ctx->place.n_dst > 1 ? (double)(ctx->place.n_dst - 1) * M * w.N * ctx->place.elem_bytes / 700e3 : 0.;
     const double t_one = pick_plan(M, w.N, kblocks, ctx->sm_count, ctx->force_split, t_remote, &mt, &nh, &S);
-    if (pair_mode == 1) {
-        wb_plan thin = *plan;
-        double t;
-        if (plan_gemm_thin(ctx, w, M, act_dtype, &thin, &t) && t < t_one) {
-            *plan = thin;
-            return WB_OK;
-        }
-    }
+    wb_plan thin = *plan;
+    double t_thin = 0.;
+    const bool thin_ok = pair_mode == 1 && plan_gemm_thin(ctx, w, M, act_dtype, &thin, &t_thin) && t_thin < t_one;
     // Stores into peers' slabs stay with the one-CTA kernels: a two-GPU run of the pair kernel with peer destinations
     // (7B-class shards at M = 4096) ended in a launch failure whose cause reading has not shown, so it is not launched so.
     const bool pair_ok = pair_mode > 0 && ctx->place.n_dst <= 1 && gemm_pair_supports(w, M) && ctx->sm_count >= 2;
@@ -875,7 +870,7 @@ int plan_gemm_tc(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int
         int pmt, pS;
         double t_pair = pick_plan_pair(M, w.N, kblocks, ctx->sm_count, ctx->force_split, ctx->place.n_dst == 0, &pmt, &pS);
         if (t_remote > 0. && pS == 1 && t_pair < t_remote) t_pair = t_remote;  // the stores to the peers run under the MMAs
-        if (pair_mode == 2 || (t_pair > 0. && t_pair < t_one)) {
+        if (pair_mode == 2 || (t_pair > 0. && t_pair < t_one && !(thin_ok && t_thin < t_pair))) {
             plan->kernel = WB_KERNEL_GEMM_TC_PAIR;
             plan->grid_x = (int)((M + pmt - 1) / pmt);
             plan->grid_y = (int)((w.N + 255) / 256);
@@ -885,6 +880,10 @@ int plan_gemm_tc(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int
             plan->tile_n = 256;
             mt = pmt, nh = 2, S = pS;
         }
+    }
+    if (plan->kernel == 0 && thin_ok) {
+        *plan = thin;
+        return WB_OK;
     }
     if (plan->kernel == 0) {
         plan->kernel = WB_KERNEL_GEMM_TC;
@@ -1106,8 +1105,8 @@ int launch_gate_up_silu(wb_context *ctx, const Weight &w, const __half *A, __hal
     if (plan.kernel != WB_KERNEL_GEMM_TC_PAIR || plan.split_k > 1) return WB_OK;
     const char *base = ctx->arena[WB_ARENA_WEIGHTS].base;
     const int mt = plan.tile_m;
-    CallMap &cx = w.tmap_x, &cc = w.tmap_c;
-    CUtensorMap &mx = *reinterpret_cast<CUtensorMap *>(cx.map.bytes), &mc = *reinterpret_cast<CUtensorMap *>(cc.map.bytes);
+    CallMap &cx = w.tmap_x;
+    CUtensorMap &mx = *reinterpret_cast<CUtensorMap *>(cx.map.bytes);
     TmapSlot &ws = w.tmap_tc[2];
     CUtensorMap &mw = *reinterpret_cast<CUtensorMap *>(ws.bytes);
     if (cx.base != A || cx.M != M || cx.a != mt / 2) {
@@ -1117,15 +1116,6 @@ int launch_gate_up_silu(wb_context *ctx, const Weight &w, const __half *A, __hal
     }
     if (!ws.ok) WB_CHECK(make_map_2d(ctx, &mw, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, base + w.off_main, (uint64_t)w.N, (uint64_t)w.pack_rows, tc::BN / 2, 8, false));
     ws.ok = true;
-    if (cc.base != act || cc.M != M || cc.a != -1) {
-        cc.base = nullptr;
-        cuuint64_t dims[3] = {(cuuint64_t)I, (cuuint64_t)M, 1}, strides[2] = {(cuuint64_t)I * 2, (cuuint64_t)I * M * 2};
-        cuuint32_t box[3] = {tc::BN / 2, tc::SILU_ROWS, 1}, estr[3] = {1, 1, 1};
-        const CUresult r = ((EncodeTiledFn)ctx->tmap_encode)(&mc, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, act, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                                             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return fail(WB_ERR_CUDA, "cuTensorMapEncodeTiled (result) failed with code %d", (int)r);
-        cc.base = act, cc.M = M, cc.a = -1;
-    }
     tc::Params p;
     p.out = act, p.bias = nullptr, p.status = ctx->status_word;
     p.M = (int)M, p.N = (int)w.N, p.K = (int)w.K, p.out_f16 = 1;
@@ -1134,7 +1124,7 @@ int launch_gate_up_silu(wb_context *ctx, const Weight &w, const __half *A, __hal
     p.qz = w.has_zeros ? (const uint32_t *)(base + w.off_zeros) : nullptr, p.sc = (const __half *)(base + w.off_scales);
     p.zcols = (int)w.zcols, p.group_blocks = (int)(w.group / 64);
     int extra = 0;
-    const cudaError_t e = launch_gemm_pair(mt, mx, mw, &mc, p, plan.grid_x, (int)(I / tc::BN), 1, ctx->stream, ctx->sm_count, nullptr, &extra, true);
+    const cudaError_t e = launch_gemm_pair(mt, mx, mw, nullptr, p, plan.grid_x, (int)(I / tc::BN), 1, ctx->stream, ctx->sm_count, nullptr, &extra, true);
     ctx->launches++;
     WB_CUDA(e);
     *done = true;

@@ -21,8 +21,8 @@ namespace tc {
 constexpr int BN = 128;       // output columns per accumulator (UMMA M); a CTA holds NH = 1 or 2 of them
 constexpr int BK = 64;        // k per stage: one 128-byte swizzle atom of fp16
 constexpr int UNPACK_WARPS = 16;
-// token rows of an fp16 epilogue staging tile of the CTA-pair kernel (half as many of f32), and of its form with silu
-constexpr int STG_ROWS = 64, SILU_ROWS = 32;
+// token rows of an fp16 epilogue staging tile of the CTA-pair kernel (half as many of f32)
+constexpr int STG_ROWS = 64;
 // Warp roles, shared by the three kernels. The thread that issues the MMAs paces a kernel with its own instruction
 // latency (a wait, four to eight tcgen05.mma, a commit per k-block), and a warp scheduler serves the warps with the same
 // id % 4: so the scheduler of the issuing warp carries no unpack warp. Warp 1 = MMA issuer, 5 = TMA producer, 9 / 13 / 17

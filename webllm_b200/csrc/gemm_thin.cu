@@ -1,8 +1,9 @@
-// int4 GEMM of a few dozen rows on the 5th-generation tensor cores, the weight operand taken from tensor memory: served batches and
-// short prompts, up to 128 rows. Same contract as gemm_tc.cu: fp16 operands, the weight rounded to fp16 once, f32 accumulation, f32
-// activations rounded to fp16 (gemm_nt_f16_from_f32.wgsl:58-62).
+// int4 GEMM on the 5th-generation tensor cores with the weight operand taken from tensor memory, for products that are one round of tiles
+// of 128 columns x up to 128 rows: served batches, short prompts, and the narrow projections of long ones. Same contract as
+// gemm_tc.cu: fp16 operands, the weight rounded to fp16 once, f32 accumulation, f32 activations rounded to fp16
+// (gemm_nt_f16_from_f32.wgsl:58-62).
 //
-// At these row counts the weights have to be read once and unpacked once, and that is all there is to do. gemm_tc.cu takes 0.25 to
+// With few rows the weights have to be read once and unpacked once, and that is all there is to do. gemm_tc.cu takes 0.25 to
 // 0.33 us for 64 k's of 128 columns whatever the rows: each unpacked weight goes through shared memory twice, and one thread waits,
 // issues and commits for every 64 k's. Here a tile's 128 output columns are the 128 lanes of tensor memory, which is how the checkpoint
 // already lies: thread = output column = lane, a packed word = eight consecutive k's of it.
@@ -21,7 +22,9 @@
 // the order 0 4 1 5 2 6 3 7 that masks yield (13 instead of 16 instructions a word).
 // Measured, gemm_tc.cu -> this, fp16 activations, us at 20 and 128 rows: 3584 -> 18944 20.4 -> 12.2, 23.2 -> 14.9; 18944 -> 3584 23.6 ->
 // 16.1, 27.5 -> 19.2; 3584 -> 3584 9.2 -> 6.8, 11.5 -> 9.5; 3584 -> 512 6.9 -> 4.3, 8.4 -> 7.2; 896 -> 4864 6.9 -> 4.2, 8.6 -> 6.6; 4864 -> 896
-// 7.6 -> 4.9, 9.2 -> 7.8; 896 -> 896 5.2 -> 4.1, 6.5 -> 6.4. Built and slower: weights straight into registers (a use waits for the youngest load),
+// 7.6 -> 4.9, 9.2 -> 7.8; 896 -> 896 5.2 -> 4.1, 6.5 -> 6.4; at 512 and 2048 rows (against the CTA pairs where they were taken): 896 -> 1152
+// 8.7 -> 6.6, 9.2 -> 7.9; 4864 -> 896 12.6 -> 10.5, 25.5 -> 17.4; 3584 -> 3584 at 512 and 1024 22.8 -> 14.3, 27.8 -> 22.6; 3584 -> 18944
+// at 256 29.7 -> 23.3. Built and slower: weights straight into registers (a use waits for the youngest load),
 // cp.async for all of them (130 cycles each to issue), activations rounded by warps of this kernel, the next chunk's words read under
 // this one's arithmetic, two CTAs of half the size per SM, and shares of several tiles per CTA (the code for that alone cost a
 // fifth: the roles' code does not fit the instruction caches side by side).
@@ -42,17 +45,19 @@ constexpr int kSets = 4;                    // sets of unpack warps
 constexpr int kUnpackWarps = 4 * kSets;
 constexpr int kUnpackThreads = 32 * kUnpackWarps;
 constexpr int kBufs = kSets;                // chunks in tensor memory, 64 columns each: one per set
-constexpr int kWordStages = 8, kWordBytes = kK / 8 * BN * 4;  // packed chunks: boxes of [16][128] words
+constexpr int kWordBytes = kK / 8 * BN * 4;  // a packed chunk: a box of [16][128] words
+constexpr int word_stages(bool big) { return big ? 4 : 8; }
 constexpr int kHalfBytes = BN * 2 + BN / 2, kGroupBytes = 2 * kHalfBytes;  // of each half of a chunk: scales [128] fp16, zero words [16]
-constexpr int kActStages = 8;
+constexpr int kActStages = 8;               // at most
+constexpr int act_warps(bool big) { return big ? 1 : 4; }
 constexpr uint32_t kCols = 512, kABase = 256;  // tensor memory: the accumulators, then the weights
 constexpr int kIssueWarp = kUnpackWarps, kIssuers = 4, kWordWarp = kIssueWarp + kIssuers, kWordWarps = 4;
 constexpr int kActWarp = kWordWarp + kWordWarps, kActWarps = 4;
-constexpr int kMaxRows = 128;
+constexpr int kRows = 128, kRowsBig = 256;  // of a tile, in the two forms
 static_assert(kThinBlock == 32 * (kActWarp + kActWarps), "the block size of a plan");
 // A barrier is waited for by parity, so a warp that waits for a phase has to have seen the one before the last: the same warp comes round
 // to the same buffer or stage.
-static_assert(kBufs % kSets == 0 && kBufs % kIssuers == 0 && kWordStages % kSets == 0 && kWordStages % kWordWarps == 0 && kActStages % kActWarps == 0,
+static_assert(kBufs % kSets == 0 && kBufs % kIssuers == 0 && word_stages(true) % kSets == 0 && word_stages(true) % kWordWarps == 0 && kActStages % kActWarps == 0,
               "owners");
 
 struct ThinParams {
@@ -61,12 +66,12 @@ struct ThinParams {
     const float *bias;        // nullable
     void *out;
     int *status;
-    int M, N, nt;             // nt: rows of the activation tile, a multiple of 16
+    int M, N, nt;             // nt: rows of an activation tile, a multiple of 16
     int accs;                 // accumulators, and threads that issue MMAs
     int zcols, chunks;        // chunks = K / 128 rounded up: what lies beyond K reads as zero activations
     int halves;               // K / 64
     uint32_t group_magic;     // h / (group / 64) = umulhi(h, group_magic); 0: group / 64 = 1
-    int per, slices;          // chunks of a CTA; grid (tiles, slices), the slices of a tile a cluster
+    int per, slices;          // chunks of a CTA; grid (column tiles, slices, row tiles), the slices of a tile a cluster
     int out_f16;
     int stages;               // of the activations
 };
@@ -102,14 +107,16 @@ __device__ __forceinline__ uint32_t elect_one()
 __device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<const __half2 *>(&v); }
 __device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<const uint32_t *>(&v); }
 
-// PERM: the activations' k's lie in the order 0 4 1 5 2 6 3 7 of every eight.
-template <bool PERM>
+// PERM: the activations' k's lie in the order 0 4 1 5 2 6 3 7 of every eight. BIG: tiles of 129 to 256 rows: one accumulator and one issuer
+// (eight MMAs of a chunk take 1000 cycles there), and stages of 64 k's of the activations, of which as many as fit, walked in order.
+template <bool PERM, bool BIG>
 __global__ void __launch_bounds__(kThinBlock, 1)
 gemm_thin_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const ThinParams p)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    const int half_bytes = p.nt * 128, stage_bytes = 2 * half_bytes;  // two halves of 64 k each
+    constexpr int kWordStages = word_stages(BIG), kLoaders = act_warps(BIG), kPerChunk = BIG ? 2 : 1;  // stages of activations per chunk
+    const int half_bytes = p.nt * 128, stage_bytes = 2 / kPerChunk * half_bytes;
     uint8_t *words = smem + p.stages * stage_bytes, *groups = words + kWordStages * kWordBytes;
     __shared__ uint64_t ready[kBufs], done[kBufs], full[kActStages], empty[kActStages], acc_full[kIssuers], word_full[kWordStages], word_empty[kWordStages];
     __shared__ uint32_t tmem_slot;
@@ -117,7 +124,7 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     volatile int *abort_flag = &abort_word;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int set = warp >> 2, quarter = warp & 3, col = quarter * 32 + lane;  // an unpacking thread's column of the tile
-    const int n0 = (int)blockIdx.x * BN, rank = (int)blockIdx.y;
+    const int n0 = (int)blockIdx.x * BN, rank = (int)blockIdx.y, m0 = (int)blockIdx.z * p.nt, M = min(p.M - m0, p.nt);  // M: rows of this tile
     const int kb0 = rank * p.per, n_chunks = min(p.per, p.chunks - kb0);
 
     // Weights: a warp's every fourth chunk, a box of words and small copies that arrive at the same barrier. A lane copies four columns'
@@ -178,27 +185,54 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             const uint64_t bd0 = smem_desc_sw128(__shfl_sync(0xffffffffu, smem_u32(smem), 0));
             const uint32_t b_step = (uint32_t)stage_bytes >> 4, b_half = (uint32_t)half_bytes >> 4;
             uint32_t ph = 0;
+            bool full_ok = false, ready_ok = false;
             int s = acc;  // (the number of stages is a multiple of the step)
 #pragma unroll 1
             for (int i = acc; i < n_chunks; i += step) {
                 const int b = i & (kBufs - 1);
-                ok = mbar_wait(&full[s], ph, abort_flag, p.status, 67);
-                if (!ok) break;
-                ok = mbar_wait(&ready[b], (uint32_t)(i / kBufs) & 1u, abort_flag, p.status, 61);
-                if (!ok) break;
-                tc_fence_after();
                 const uint32_t a = tm + kABase + b * 64;
-                const uint64_t bd = bd0 + (uint32_t)s * b_step;
-                if (elected) {
-                    umma_ts(d, a, bd, idesc, i != acc);
+                if constexpr (!BIG) {
+                    ok = mbar_wait(&full[s], ph, abort_flag, p.status, 67);
+                    if (!ok) break;
+                    ok = mbar_wait(&ready[b], (uint32_t)(i / kBufs) & 1u, abort_flag, p.status, 61);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t bd = bd0 + (uint32_t)s * b_step;
+                    if (elected) {
+                        umma_ts(d, a, bd, idesc, i != acc);
 #pragma unroll
-                    for (int k = 1; k < 8; k++) umma_ts(d, a + 8 * k, bd + (k < 4 ? 2 * k : b_half + 2 * (k - 4)), idesc, 1);
-                    umma_commit(&done[b]);
-                    umma_commit(&empty[s]);
-                    if (i + step >= n_chunks) umma_commit(&acc_full[acc]);
+                        for (int k = 1; k < 8; k++) umma_ts(d, a + 8 * k, bd + (k < 4 ? 2 * k : b_half + 2 * (k - 4)), idesc, 1);
+                        umma_commit(&done[b]);
+                        umma_commit(&empty[s]);
+                        if (i + step >= n_chunks) umma_commit(&acc_full[acc]);
+                    }
+                    __syncwarp();
+                    if ((s += step) >= p.stages) s -= p.stages, ph ^= 1;
+                } else {
+                    // a barrier is asked while the MMAs before it are issued: the answer alone takes 200 cycles
+                    if (!ready_ok) ok = mbar_wait(&ready[b], (uint32_t)(i / kBufs) & 1u, abort_flag, p.status, 61);
+#pragma unroll
+                    for (int h = 0; h < 2 && ok; h++) {
+                        if (!full_ok) ok = mbar_wait(&full[s], ph, abort_flag, p.status, 67);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint64_t bd = bd0 + (uint32_t)s * b_step;
+                        uint64_t *emptied = &empty[s];
+                        if (++s == p.stages) s = 0, ph ^= 1;
+                        full_ok = mbar_try(&full[s], ph);
+                        if (h == 1) ready_ok = mbar_try(&ready[(b + 1) & (kBufs - 1)], (uint32_t)((i + 1) / kBufs) & 1u);
+                        if (elected) {
+                            umma_ts(d, a + 32 * h, bd, idesc, (i | h) != 0);
+#pragma unroll
+                            for (int k = 1; k < 4; k++) umma_ts(d, a + 32 * h + 8 * k, bd + 2 * k, idesc, 1);
+                            umma_commit(emptied);
+                            if (h == 1) umma_commit(&done[b]);
+                            if (h == 1 && i + 1 == n_chunks) umma_commit(&acc_full[0]);
+                        }
+                        __syncwarp();
+                    }
+                    if (!ok) break;
                 }
-                __syncwarp();
-                if ((s += step) >= p.stages) s -= p.stages, ph ^= 1;
             }
         }
     } else if (warp >= kWordWarp && warp < kActWarp) {
@@ -214,18 +248,18 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         if (*abort_flag)  // a copy on its way has its time to arrive before the shared memory is given back
             for (int i = 0; i < 256; i++) __nanosleep(1000);
     } else if (warp >= kActWarp) {
-        // ------------------------------------------------------------------ activations: every fourth chunk
-        if (lane == 0) {
+        // ------------------------------------------------------------------ activations
+        if (lane == 0 && warp < kActWarp + kLoaders) {
             pdl_wait();
             int s = warp - kActWarp;
             uint32_t ph = 1;
-            for (int i = warp - kActWarp; i < n_chunks; i += kActWarps) {
+            for (int i = warp - kActWarp; i < n_chunks * kPerChunk; i += kLoaders) {
                 if (!mbar_wait_idle(&empty[s], ph, abort_flag, p.status, 62)) break;
                 mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
                 uint8_t *to = smem + s * stage_bytes;
-                tma_load_2d(to, &map_x, (kb0 + i) * kK, 0, &full[s]);
-                tma_load_2d(to + half_bytes, &map_x, (kb0 + i) * kK + BK, 0, &full[s]);
-                if ((s += kActWarps) >= p.stages) s -= p.stages, ph ^= 1;
+                tma_load_2d(to, &map_x, kb0 * kK + i * (kK / kPerChunk), m0, &full[s]);
+                if constexpr (!BIG) tma_load_2d(to + half_bytes, &map_x, kb0 * kK + i * kK + BK, m0, &full[s]);
+                if ((s += kLoaders) >= p.stages) s -= p.stages, ph ^= 1;
             }
             if (*abort_flag)
                 for (int i = 0; i < 256; i++) __nanosleep(1000);
@@ -321,13 +355,13 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             for (int c = set * 16; c < p.nt; c += 16 * kSets) {
                 uint32_t r[16];
                 result16(c, r);
-                store_block16<false>(d, p.out_f16 != 0, (p.N & 7) == 0, r, bias, c, p.M, n_warp, p.N, lane);
+                store_block16<false>(d, p.out_f16 != 0, (p.N & 7) == 0, r, bias, m0 + c, p.M, n_warp, p.N, lane);
             }
         }
     } else {
         // Every CTA of the cluster adds up its part of the rows, which all of them write into its shared memory in the place of what has
         // been read there (every copy has arrived: the last chunk's results are there).
-        const int rows = (p.M + p.slices - 1) / p.slices;
+        const int rows = (M + p.slices - 1) / p.slices;
         float *sums = reinterpret_cast<float *>(smem);  // [slices][rows][128 columns]
         cluster_barrier();
         if (warp < kUnpackWarps && ok) {
@@ -338,7 +372,7 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 int to = c / rows, row = c - to * rows;
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
-                    if (c + j < p.M) cluster_store_f32(cluster_map_shared(sums + (rank * rows + row) * BN + col, (uint32_t)to), __uint_as_float(r[j]));
+                    if (c + j < M) cluster_store_f32(cluster_map_shared(sums + (rank * rows + row) * BN + col, (uint32_t)to), __uint_as_float(r[j]));
                     if (++row == rows) row = 0, to++;
                 }
             }
@@ -346,9 +380,9 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         __syncwarp();
         cluster_barrier();
         if (warp < kUnpackWarps) {
-            const int here = min(rows, p.M - rank * rows);
+            const int here = min(rows, M - rank * rows);
             for (int i = threadIdx.x; i < here * (BN / 4); i += kUnpackThreads) {
-                const int m = rank * rows + (i >> 5), n4 = n0 + (i & 31) * 4;
+                const int m = m0 + rank * rows + (i >> 5), n4 = n0 + (i & 31) * 4;
                 if (n4 >= p.N) continue;
                 const float4 *src = reinterpret_cast<const float4 *>(sums) + i;
                 float4 v = src[0];
@@ -372,12 +406,21 @@ gemm_thin_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     if (warp == kIssueWarp) tmem_dealloc(tmem, kCols);
 }
 
-int thin_rows(int64_t M) { return (int)((M + 15) / 16 * 16); }
-int thin_stages(int nt) { return nt > 64 ? 4 : kActStages; }
-size_t thin_smem(int nt) { return 1024 + kWordStages * (kWordBytes + kGroupBytes) + (size_t)thin_stages(nt) * nt * 256; }
-static_assert(1024 + kWordStages * (kWordBytes + kGroupBytes) + kActStages * 64 * 256 <= 227 * 1024 && 4 * kMaxRows == kActStages * 64, "shared memory");
-// (the slices meet in at most (M + 8) * 512 bytes, which is less than the words' stages alone)
-static_assert((kMaxRows + 8) * BN * 4 <= kWordStages * kWordBytes + 4 * 16 * 256, "the slices' meeting");
+// Row tiles of at most `most` rows, and the rows of one.
+int64_t thin_tiles(int64_t M, int most) { return (M + most - 1) / most; }
+int thin_rows(int64_t M, int most) { return (int)(((M + thin_tiles(M, most) - 1) / thin_tiles(M, most) + 15) / 16 * 16); }
+constexpr size_t kSmemMost = 227 * 1024 - 512;  // (the barriers are outside)
+constexpr size_t word_bytes(bool big) { return 1024 + (size_t)word_stages(big) * (kWordBytes + kGroupBytes); }
+int thin_stages(int nt)
+{
+    if (nt <= kRows) return nt > 64 ? 4 : kActStages;
+    return (int)std::min<size_t>(kActStages, (kSmemMost - word_bytes(true)) / ((size_t)nt * 128));
+}
+size_t thin_smem(int nt) { return word_bytes(nt > kRows) + (size_t)thin_stages(nt) * nt * (nt > kRows ? 128 : 256); }
+constexpr size_t kSmemThin = word_bytes(false) + kActStages * 64 * 256;  // the most that the form for up to 128 rows takes
+static_assert(kSmemThin <= kSmemMost && 4 * kRows == kActStages * 64, "shared memory");
+// (the slices meet in at most (rows + 8) * 512 bytes, which is less than the stages take)
+static_assert((kRows + 8) * BN * 4 <= word_bytes(false) - 1024 + 4 * 16 * 256 && (kRowsBig + 8) * BN * 4 <= word_bytes(true) - 1024 + 5 * kRowsBig * 128, "the slices' meeting");
 
 // Clusters of S CTAs that are resident at once, as the driver counts them for this device (a cluster stays inside a GPC, and these
 // differ in size). 0: not known, so not taken.
@@ -392,9 +435,9 @@ int thin_clusters(int S, int sms)
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 1, attr.val.clusterDim.y = (unsigned)S, attr.val.clusterDim.z = 1;
-    cfg.gridDim = dim3(1, (unsigned)S), cfg.blockDim = dim3(kThinBlock), cfg.dynamicSmemBytes = thin_smem(64), cfg.attrs = &attr, cfg.numAttrs = 1;
+    cfg.gridDim = dim3(1, (unsigned)S), cfg.blockDim = dim3(kThinBlock), cfg.dynamicSmemBytes = kSmemThin, cfg.attrs = &attr, cfg.numAttrs = 1;
     int n = 0;
-    if (smem_limit_once<gemm_thin_kernel<false>>((int)thin_smem(64)) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_thin_kernel<false>, &cfg) != cudaSuccess)
+    if (smem_limit_once<gemm_thin_kernel<false, false>>((int)kSmemThin) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_thin_kernel<false, false>, &cfg) != cudaSuccess)
         return cudaGetLastError(), 0;
     if (dev < 16) known[dev][S].store(n + 1, std::memory_order_relaxed);
     return n;
@@ -406,7 +449,7 @@ int thin_clusters(int S, int sms)
 bool gemm_thin_takes(wb_context *ctx, const Weight &w, int64_t M)
 {
     static const bool on = [] { const char *e = getenv("WEBLLM_B200_GEMM_THIN"); return !(e && e[0] == '0'); }();
-    return on && w.kind == WeightKind::Gptq && M >= 1 && M <= kMaxRows && w.K % 64 == 0 && w.N % 4 == 0 && w.group % 64 == 0 && ctx->place.n_dst == 0 &&
+    return on && w.kind == WeightKind::Gptq && M >= 1 && w.K % 64 == 0 && w.N % 4 == 0 && w.group % 64 == 0 && ctx->place.n_dst == 0 &&
            w.K * (w.group / BK) < (int64_t)1 << 37;  // (group_magic)
 }
 
@@ -415,22 +458,32 @@ bool plan_gemm_thin(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, 
 {
     if (!gemm_thin_takes(ctx, w, M)) return false;
     const int chunks = (int)((w.K + kK - 1) / kK), sms = ctx->sm_count;
-    const int64_t tiles = (w.N + BN - 1) / BN;
+    const int64_t cols = (w.N + BN - 1) / BN;
     double best = -1.;
-    int best_s = 0;
-    for (int S = 1; S <= 8 && S <= chunks; S++) {
-        if (ctx->force_split > 0 && S != std::min(ctx->force_split, chunks)) continue;
-        const int per = (chunks + S - 1) / S, at_once = thin_clusters(S, sms);
-        if ((chunks + per - 1) / per != S || (S > 1 && tiles > at_once)) continue;
-        const int64_t rounds = S > 1 ? 1 : (tiles + sms - 1) / sms;
-        const double t = 1.6 + 0.022 * M + rounds * per * (0.27 + 0.07 * std::min<double>(1., (double)tiles * S / sms)) + (S > 1 ? 1.3 : 0.);
-        if (best < 0. || t < best) best = t, best_s = S;
+    int best_s = 0, best_rows = 0;
+    for (int most : {kRows, kRowsBig}) {
+        if (M <= kRows && most != kRows) continue;
+        const int nt = thin_rows(M, most);
+        const int64_t rows = thin_tiles(M, most), tiles = cols * rows;
+        if (rows > 1 && tiles > sms) continue;  // every CTA sets itself up and drains: larger products go to persistent ones
+        // Long products of a long K: as a call by itself these stay with the pairs, whose plan cuts K, as it is asked to
+        // (4864 -> 896, 2048 rows: 25.5 us, 17.3 here). A caller that would add the slices itself gets the whole result from here.
+        if (rows > 8 && chunks > 32 && !ctx->keep_slices) continue;
+        for (int S = 1; S <= 8 && S <= chunks; S++) {
+            if (ctx->force_split > 0 && S != std::min(ctx->force_split, chunks)) continue;
+            const int per = (chunks + S - 1) / S, at_once = thin_clusters(S, sms);
+            if ((chunks + per - 1) / per != S || (S > 1 && tiles > at_once)) continue;
+            const int64_t rounds = S > 1 ? 1 : (tiles + sms - 1) / sms;
+            const double chunk = nt > kRows ? 0.66 : 0.27 + 0.07 * std::min<double>(1., (double)tiles * S / sms);
+            const double t = 1.6 + 0.022 * nt + rounds * per * chunk + (S > 1 ? 1.3 : 0.);
+            if (best < 0. || t < best) best = t, best_s = S, best_rows = most;
+        }
     }
     if (best_s == 0) return false;
     const bool cast = act_dtype == WB_F32;
     plan->kernel = WB_KERNEL_GEMM_TC;
-    plan->tile_m = thin_rows(M), plan->tile_n = BN;
-    plan->grid_x = (int)tiles, plan->grid_y = best_s, plan->grid_z = 1;
+    plan->tile_m = thin_rows(M, best_rows), plan->tile_n = BN;
+    plan->grid_x = (int)thin_tiles(M, best_rows), plan->grid_y = (int)cols, plan->grid_z = best_s;  // (the launch has the slices in y, for the clusters)
     plan->split_k = best_s;
     plan->block = kThinBlock;
     plan->launches = cast ? 2 : 1;
@@ -459,7 +512,7 @@ int launch_gemm_thin(wb_context *ctx, const Weight &w, const void *x, bool perm,
     p.qz = w.has_zeros ? (const uint32_t *)(base + w.off_zeros) : nullptr;
     p.sc = (const __half *)(base + w.off_scales);
     p.bias = bias, p.out = C, p.status = ctx->status_word;
-    p.M = (int)M, p.N = (int)w.N, p.nt = nt, p.accs = nt <= 64 ? kIssuers : kIssuers / 2;
+    p.M = (int)M, p.N = (int)w.N, p.nt = nt, p.accs = nt <= 64 ? kIssuers : nt <= kRows ? kIssuers / 2 : 1;
     p.zcols = (int)w.zcols, p.chunks = (int)((w.K + kK - 1) / kK), p.halves = (int)(w.K / BK);
     const uint32_t gb = (uint32_t)(w.group / BK);
     p.group_magic = gb == 1 ? 0u : (uint32_t)((0x100000000ull + gb - 1) / gb);  // exact while halves * gb < 2^32
@@ -467,11 +520,13 @@ int launch_gemm_thin(wb_context *ctx, const Weight &w, const void *x, bool perm,
     p.out_f16 = out_dtype == WB_F16;
     p.stages = thin_stages(nt);
     auto go = [&](auto kern, cudaError_t limit) {
-        return limit != cudaSuccess ? limit : launch_pdl_cluster(kern, dim3((unsigned)plan.grid_x, (unsigned)plan.grid_y), dim3(kThinBlock), thin_smem(nt),
-                                                                 ctx->stream, (unsigned)plan.grid_y, mx, mw, p);
+        return limit != cudaSuccess ? limit : launch_pdl_cluster(kern, dim3((unsigned)plan.grid_y, (unsigned)plan.grid_z, (unsigned)plan.grid_x), dim3(kThinBlock), thin_smem(nt),
+                                                                 ctx->stream, (unsigned)plan.grid_z, mx, mw, p);
     };
-    const cudaError_t e = perm ? go(gemm_thin_kernel<true>, smem_limit_once<gemm_thin_kernel<true>>((int)thin_smem(64)))
-                               : go(gemm_thin_kernel<false>, smem_limit_once<gemm_thin_kernel<false>>((int)thin_smem(64)));
+    const cudaError_t e = nt > kRows ? (perm ? go(gemm_thin_kernel<true, true>, smem_limit_once<gemm_thin_kernel<true, true>>((int)kSmemMost))
+                                             : go(gemm_thin_kernel<false, true>, smem_limit_once<gemm_thin_kernel<false, true>>((int)kSmemMost)))
+                                     : (perm ? go(gemm_thin_kernel<true, false>, smem_limit_once<gemm_thin_kernel<true, false>>((int)kSmemThin))
+                                             : go(gemm_thin_kernel<false, false>, smem_limit_once<gemm_thin_kernel<false, false>>((int)kSmemThin)));
     ctx->launches++;
     WB_CUDA(e);
     return WB_OK;

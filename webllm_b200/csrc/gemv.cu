@@ -933,7 +933,7 @@ static int plan_linear_ex(wb_context *ctx, const Weight &w, int64_t M, int act_d
     const bool keep = ctx->force_kernel == 0 && ctx->force_split == 0 && ctx->place.n_dst == 0;
     if (keep)
         for (const PlanSlot &s : w.plans)
-            if (s.M == M && s.act_dtype == act_dtype && s.exact == exact && s.allow_stream == (int)allow_stream) {
+            if (s.M == M && s.act_dtype == act_dtype && s.exact == exact && s.allow_stream == (int)allow_stream && s.keep_slices == (int)ctx->keep_slices) {
                 *plan = s.plan;
                 return WB_OK;
             }
@@ -941,7 +941,7 @@ static int plan_linear_ex(wb_context *ctx, const Weight &w, int64_t M, int act_d
     if (keep) {
         PlanSlot &s = w.plans[w.next_plan];
         w.next_plan = (w.next_plan + 1) % 4;
-        s.M = M, s.act_dtype = act_dtype, s.exact = exact, s.allow_stream = allow_stream, s.plan = *plan;
+        s.M = M, s.act_dtype = act_dtype, s.exact = exact, s.allow_stream = allow_stream, s.keep_slices = ctx->keep_slices, s.plan = *plan;
     }
     return WB_OK;
 }
