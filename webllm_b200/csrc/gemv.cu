@@ -550,13 +550,15 @@ __global__ void __launch_bounds__(256) dense_gemv_f16_kernel(const __half *__res
 // gemmNTRef (src/reference/qwen-ref.ts:126-145), bit for bit (a product of two f32 values is exact in double, so the fused
 // multiply-add rounds as the separate add does).
 //
-// Bound by the double-precision units and by the shared memory that feeds them. A CTA of 4 warps computes 32 rows x 32 C columns from
-// operands that are unpacked, widened and staged once per 32 k (with one thread per output every weight was unpacked M times).
-// A lane has C columns and 8 rows: the rows' values are the same for the whole warp, one broadcast for two, and the columns lie
-// side by side, so a k costs a warp 4 + 2 C passes over shared memory for 8 C multiply-adds (16 C cycles). Tiles of 2 x 4 outputs
-// with 8 lanes abreast took 20 passes for 8. (100 CTAs on 148 SMs: over the whole chip the double-precision units are 27 % busy and
-// the shared memory 29 %.)
-// 145 rows of 1000 -> 1236: 132 us (one thread per output), 85 (2 x 4), 38 now. C = 2 unless smaller tiles spread better.
+// The multiply-adds are double-precision MMAs (m8n8k4), whose four products per output are a chain of fused multiply-adds in
+// ascending k, rounded each (262144 outputs against that chain, half of them of operands over sixty binades: the same bits; the
+// descending chain differs in a quarter). They are no faster than the scalar instruction (64 a cycle and SM, 57) but need a
+// quarter of the operands: two doubles per lane for 256 multiply-adds. Scalar, a tile of 32 x 64 was bound by the shared memory
+// that fed it, as much as by the arithmetic (145 rows of 1000 -> 1236 38 us; 132 with one thread per output).
+// A CTA of 4 warps computes 8 U rows x 32 columns: a warp 8 columns and all rows, U accumulators. Operands are unpacked, widened and
+// staged once per 32 k, [row or column][k] with a pitch of 36 doubles, which both fragments read without a conflict; two buffers, so
+// that a stage is filled under the arithmetic of the one before. What the arithmetic costs is rounds of tiles per SM, so U is the
+// one that makes the fullest SM's share smallest (generic_rows).
 // =====================================================================================================
 struct GenericParams {
     const uint32_t *qw, *qz;
@@ -568,21 +570,22 @@ struct GenericParams {
     int x_f16, out_f16, round_x_f16;
 };
 
-template <int C>
+template <int U>
 __global__ void __launch_bounds__(128) linear_generic_kernel(const GenericParams p)
 {
-    constexpr int KC = 32, TM = 32, TN = 32 * C, R = 8, XP = TM + 2, BUFS = C == 1 ? 2 : 1;  // (48 KB)
-    __shared__ __align__(16) double xs[BUFS][KC][XP], ws[BUFS][KC][TN];
+    constexpr int KC = 32, TM = 8 * U, TN = 32, PITCH = KC + 4, XV = TM / 4;
+    __shared__ __align__(16) double xs[2][TM][PITCH], ws[2][TN][PITCH];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t m0 = (int64_t)blockIdx.y * TM, n0 = (int64_t)blockIdx.x * TN;
-    // Staging: this thread's x values are k = k0 + lane of the row pairs warp, warp + 4, ...; its weights words (8 k) tid, tid + 128 of
-    // the stage, columns side by side. In flight under the arithmetic is what memory holds: a conversion would wait for its load.
-    uint32_t xv[8], wv[C][8], wscale[C] = {}, wzero[C] = {};
+    // Staging: this thread's x values are k = k0 + lane of rows warp, warp + 4, ...; its weights word (8 k) is word tid / 32 of column
+    // tid % 32. In flight under the arithmetic is what memory holds: a conversion would wait for its load.
+    uint32_t xv[XV], wv[8], wscale = 0, wzero = 0;
+    const int64_t n = n0 + lane;
     auto fetch = [&](int k0) {
-        const int k = k0 + lane;
+        const int k = k0 + lane, kw = k0 + warp * 8;
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int64_t m = m0 + 2 * (warp + 4 * (i >> 1)) + (i & 1);
+        for (int i = 0; i < XV; i++) {
+            const int64_t m = m0 + warp + 4 * i;
             xv[i] = 0;
             if (m < p.M && k < p.K) {
                 if (p.x_f16) xv[i] = ((const unsigned short *)p.x)[m * p.K + k];
@@ -590,22 +593,17 @@ __global__ void __launch_bounds__(128) linear_generic_kernel(const GenericParams
             }
         }
 #pragma unroll
-        for (int c = 0; c < C; c++) {
-            const int idx = tid + 128 * c, kw = k0 + idx / TN * 8;
-            const int64_t n = n0 + idx % TN;
+        for (int j = 0; j < 8; j++) wv[j] = 0;
+        if (n >= p.N || kw >= p.K) return;
+        if (p.dense) {
 #pragma unroll
-            for (int j = 0; j < 8; j++) wv[c][j] = 0;
-            if (n >= p.N || kw >= p.K) continue;
-            if (p.dense) {
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    if (kw + j < p.K) wv[c][j] = ((const unsigned short *)p.dense)[n * p.K + kw + j];
-            } else {
-                const int64_t g = (unsigned)kw / (unsigned)p.group;
-                wv[c][0] = p.qw[(int64_t)(kw >> 3) * p.N + n];
-                wscale[c] = ((const unsigned short *)p.sc)[g * p.N + n];
-                wzero[c] = p.qz ? p.qz[g * p.zcols + (n >> 3)] >> (4 * (n & 7)) : 7u;
-            }
+            for (int j = 0; j < 8; j++)
+                if (kw + j < p.K) wv[j] = ((const unsigned short *)p.dense)[n * p.K + kw + j];
+        } else {
+            const int64_t g = (unsigned)kw / (unsigned)p.group;
+            wv[0] = p.qw[(int64_t)(kw >> 3) * p.N + n];
+            wscale = ((const unsigned short *)p.sc)[g * p.N + n];
+            wzero = p.qz ? p.qz[g * p.zcols + (n >> 3)] >> (4 * (n & 7)) : 7u;
         }
     };
     auto h2f = [](uint32_t bits) { return __half2float(__ushort_as_half((unsigned short)bits)); };
@@ -613,73 +611,63 @@ __global__ void __launch_bounds__(128) linear_generic_kernel(const GenericParams
         const float v = p.x_f16 ? h2f(xv[i]) : __uint_as_float(xv[i]);
         return (double)(p.round_x_f16 ? __half2float(__float2half_rn(v)) : v);
     };
-    auto w_value = [&](int c, int j, int kw) {
-        if (p.dense) return (double)h2f(wv[c][j]);
+    auto w_value = [&](int j, int kw) {
+        if (p.dense) return (double)h2f(wv[j]);
         if (kw + j >= p.K) return 0.0;
-        return (double)((float)((int)((wv[c][0] >> (4 * j)) & 15u) - (int)((wzero[c] & 15u) + 1u)) * h2f(wscale[c]));
+        return (double)((float)((int)((wv[0] >> (4 * j)) & 15u) - (int)((wzero & 15u) + 1u)) * h2f(wscale));
     };
-    double acc[R][C];
+    double acc[U][2];  // row 8 u + lane / 4, columns 2 (lane % 4) and the next
 #pragma unroll
-    for (int i = 0; i < R; i++)
-#pragma unroll
-        for (int j = 0; j < C; j++) acc[i][j] = 0.0;
+    for (int u = 0; u < U; u++) acc[u][0] = acc[u][1] = 0.0;
     pdl_sync();
     fetch(0);
     int buf = 0;
-    for (int k0 = 0; k0 < p.K; k0 += KC, buf = (buf + 1) % BUFS) {
-        if (BUFS == 1) __syncthreads();
+    for (int k0 = 0; k0 < p.K; k0 += KC, buf ^= 1) {
 #pragma unroll
-        for (int i = 0; i < 8; i += 2) *reinterpret_cast<double2 *>(&xs[buf][lane][2 * (warp + 2 * i)]) = make_double2(x_value(i), x_value(i + 1));
+        for (int i = 0; i < XV; i++) xs[buf][warp + 4 * i][lane] = x_value(i);
 #pragma unroll
-        for (int c = 0; c < C; c++) {
-            const int idx = tid + 128 * c, wr = idx / TN;
-#pragma unroll
-            for (int j = 0; j < 8; j++) ws[buf][wr * 8 + j][idx % TN] = w_value(c, j, k0 + wr * 8);
-        }
-        __syncthreads();  // (with two buffers every warp has also left the one that the next stage fills)
+        for (int j = 0; j < 8; j += 2)
+            *reinterpret_cast<double2 *>(&ws[buf][lane][warp * 8 + j]) = make_double2(w_value(j, k0 + warp * 8), w_value(j + 1, k0 + warp * 8));
+        __syncthreads();  // (and every warp has left the buffer that the next stage fills)
         if (k0 + KC < p.K) fetch(k0 + KC);
-#pragma unroll 4
-        for (int k = 0; k < KC; k++) {
-            double a[R], b[C];
+        const double *xf = &xs[buf][lane >> 2][lane & 3], *wf = &ws[buf][warp * 8 + (lane >> 2)][lane & 3];
 #pragma unroll
-            for (int i = 0; i < R; i += 2) {
-                const double2 v = *reinterpret_cast<const double2 *>(&xs[buf][k][warp * R + i]);
-                a[i] = v.x, a[i + 1] = v.y;
-            }
-            if constexpr (C == 2) {
-                const double2 v = *reinterpret_cast<const double2 *>(&ws[buf][k][lane * 2]);
-                b[0] = v.x, b[1] = v.y;
-            } else {
-                b[0] = ws[buf][k][lane];
-            }
+        for (int k = 0; k < KC; k += 4) {
+            const double b = wf[k];
 #pragma unroll
-            for (int i = 0; i < R; i++)
-#pragma unroll
-                for (int j = 0; j < C; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+            for (int u = 0; u < U; u++)
+                asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                    : "+d"(acc[u][0]), "+d"(acc[u][1])
+                    : "d"(xf[u * 8 * PITCH + k]), "d"(b));
         }
     }
 #pragma unroll
-    for (int i = 0; i < R; i++)
+    for (int u = 0; u < U; u++)
 #pragma unroll
-        for (int j = 0; j < C; j++) {
-            const int64_t m = m0 + warp * R + i, n = n0 + lane * C + j;
-            if (m >= p.M || n >= p.N) continue;
-            double v = acc[i][j];
-            if (p.bias) v += (double)p.bias[n];
-            if (p.out_f16) ((__half *)p.out)[m * p.N + n] = __float2half_rn((float)v);
-            else ((float *)p.out)[m * p.N + n] = (float)v;
+        for (int j = 0; j < 2; j++) {
+            const int64_t m = m0 + u * 8 + (lane >> 2), col = n0 + warp * 8 + 2 * (lane & 3) + j;
+            if (m >= p.M || col >= p.N) continue;
+            double v = acc[u][j];
+            if (p.bias) v += (double)p.bias[col];
+            if (p.out_f16) ((__half *)p.out)[m * p.N + col] = __float2half_rn((float)v);
+            else ((float *)p.out)[m * p.N + col] = (float)v;
         }
 }
 
-// Rows of one launch (tiles of 32 in the grid's second dimension). More are more launches: the tiles in one dimension of the grid, or
-// in its second and third, cost every launch 1 us of its 38.
-constexpr int64_t kGenericRows = 65535 * 32;
+// Rows of one launch: the tiles of the grid's second dimension. More are more launches: the tiles in one dimension of the grid, or
+// in its second and third, cost every launch 1 us.
+constexpr int64_t kGenericTiles = 65535;
 
-// Columns of a tile, 32 or 64: the passes over shared memory per k of the SM with the most tiles.
-static int generic_tile_n(int64_t M, int64_t N, int sms)
+// Rows of a tile, 8 to 32: the multiply-adds of the SM with the most tiles, and a part per tile for staging its weights.
+static int generic_rows(int64_t M, int64_t N, int sms)
 {
-    auto cost = [&](int cols) { return ((((M + 31) / 32) * ((N + cols - 1) / cols) + sms - 1) / sms) * (cols == 64 ? 8 : 6); };
-    return cost(64) <= cost(32) ? 64 : 32;
+    int best = 4;
+    int64_t best_cost = 0;
+    for (int u = 4; u >= 1; u--) {
+        const int64_t cost = (((M + 8 * u - 1) / (8 * u)) * ((N + 31) / 32) + sms - 1) / sms * (2 * u + 1);
+        if (u == 4 || cost < best_cost) best = u, best_cost = cost;
+    }
+    return 8 * best;
 }
 
 // =====================================================================================================
@@ -917,11 +905,11 @@ static int make_plan(wb_context *ctx, const Weight &w, int64_t M, int act_dtype,
         plan->kernel = kind;
         plan->split_k = 1;
         plan->block = 128;
-        plan->tile_m = 32, plan->tile_n = generic_tile_n(M, w.N, ctx->sm_count);
+        plan->tile_m = generic_rows(M, w.N, ctx->sm_count), plan->tile_n = 32;
         plan->grid_x = (int)((w.N + plan->tile_n - 1) / plan->tile_n);
-        plan->grid_y = (int)((std::min(M, kGenericRows) + plan->tile_m - 1) / plan->tile_m);
+        plan->grid_y = (int)std::min<int64_t>((M + plan->tile_m - 1) / plan->tile_m, kGenericTiles);
         plan->grid_z = 1;
-        plan->launches = (int)((M + kGenericRows - 1) / kGenericRows);
+        plan->launches = (int)(((M + plan->tile_m - 1) / plan->tile_m + kGenericTiles - 1) / kGenericTiles);
         return WB_OK;
     }
     return fail(WB_ERR_BAD_ARG, "unknown kernel kind %d", kind);
@@ -1090,11 +1078,15 @@ int launch_linear(wb_context *ctx, const Weight &w, const void *A, void *C, cons
         g.x = A, g.out = C, g.bias = bias, g.M = M, g.N = w.N, g.K = w.K, g.pack_rows = w.pack_rows;
         g.group = gptq ? w.group : 8, g.zcols = w.zcols;
         g.x_f16 = act_dtype == WB_F16, g.out_f16 = out_dtype == WB_F16, g.round_x_f16 = round_x;
-        for (int64_t m = 0; m < M; m += kGenericRows) {
-            g.x = (const char *)A + m * w.K * (g.x_f16 ? 2 : 4), g.out = (char *)C + m * w.N * (g.out_f16 ? 2 : 4), g.M = std::min(M - m, kGenericRows);
-            const dim3 grid((unsigned)plan.grid_x, (unsigned)((g.M + 31) / 32));
-            const cudaError_t e = plan.tile_n == 64 ? launch_pdl(linear_generic_kernel<2>, grid, dim3(128), 0, ctx->stream, g)
-                                                    : launch_pdl(linear_generic_kernel<1>, grid, dim3(128), 0, ctx->stream, g);
+        const int64_t rows = kGenericTiles * plan.tile_m;
+        for (int64_t m = 0; m < M; m += rows) {
+            g.x = (const char *)A + m * w.K * (g.x_f16 ? 2 : 4), g.out = (char *)C + m * w.N * (g.out_f16 ? 2 : 4), g.M = std::min(M - m, rows);
+            const dim3 grid((unsigned)plan.grid_x, (unsigned)((g.M + plan.tile_m - 1) / plan.tile_m));
+            auto go = [&](auto kern) { return launch_pdl(kern, grid, dim3(128), 0, ctx->stream, g); };
+            const cudaError_t e = plan.tile_m == 8    ? go(linear_generic_kernel<1>)
+                                  : plan.tile_m == 16 ? go(linear_generic_kernel<2>)
+                                  : plan.tile_m == 24 ? go(linear_generic_kernel<3>)
+                                                      : go(linear_generic_kernel<4>);
             ctx->launches++;
             WB_CUDA(e);
         }
