@@ -4,9 +4,11 @@
 //
 // One CTA = 32 query rows of one head; keys in blocks of 32, staged in shared memory as f32, that four groups of four warps take in
 // turn, their states of a row merged at the end; scores and weighted sums from
-// 4 x 2 and 4 x 4 register tiles, online softmax. One CTA per single row, as the scalar kernel (qwen_ops.cu) has it, reads every
-// key 32 times as often and leaves a warp's lanes one multiply per load. 4 x 101 rows, 14 heads: 57 -> 22 us a layer with
-// one group, whose chain of key blocks it was, 17 with four.
+// 4 x 2 and 4 x 4 register tiles, online softmax. Rows are read as they lie, 256 bytes by 16 lanes, and stay rows in shared memory (a lane per
+// key, 32 lines touched per load, took the L1 8000 cycles an SM); scores are taken four dims at a time from 16-byte pieces. One CTA per single row, as the scalar kernel (qwen_ops.cu) has it, reads every
+// key 32 times as often and leaves a warp's lanes one multiply per load. 4 x 101 rows, 14 heads: 57 -> 22 us with
+// one group, whose chain of key blocks it was, 17 with four, 14 with rows read as they lie. Bound by the multiply-adds and the loads
+// that feed them on the SMs that have two long tiles.
 #include <algorithm>
 
 #include "qwen_ops.cuh"
@@ -16,14 +18,14 @@ namespace wb {
 namespace {
 
 constexpr int kD = 64, kRows = 32, kKeys = 32, kGroups = 4, kThreads = kGroups * 128;
-constexpr int kQP = kRows + 4, kKP = kKeys + 2, kVP = kD + 4;
+constexpr int kPP = kRows + 4, kDP = kD + 4;  // pitches: 16-byte pieces of 8 rows lie in different banks
 struct GroupSmem {
-    float Ks[kD][kKP];
-    float Vs[kKeys][kVP];  // later the group's sums, [rows][dims]
-    float Ps[kKeys][kQP];
+    float Ks[kKeys][kDP];
+    float Vs[kKeys][kDP];  // later the group's sums, [rows][dims]
+    float Ps[kKeys][kPP];
 };
 struct Smem {
-    float Qs[kD][kQP];
+    float Qs[kRows][kDP];
     GroupSmem g[kGroups];
     float m[kGroups][kRows], l[kGroups][kRows];
 };
@@ -38,7 +40,7 @@ __device__ __forceinline__ float4 load4(const __half *p)
 
 // Rows i of sequence b (row b * T + i of q and out) see keys 0 .. past + i, row b * key_rows + key of kmem / vmem.
 template <typename KV>
-__global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__restrict__ q, const KV *__restrict__ kmem,
+__global__ void __launch_bounds__(kThreads, 2) attention_f32_kernel(const float *__restrict__ q, const KV *__restrict__ kmem,
                                                                  const KV *__restrict__ vmem, float *__restrict__ out, __half *__restrict__ out16, int H, int KVH, int T,
                                                                  const int *__restrict__ past_ptr, int past_imm, int key_rows, int ldq,
                                                                  int kv_ld, float scale)
@@ -46,8 +48,7 @@ __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__
     pdl_sync();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
-    const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127, lane = tid & 31, warp = tid >> 5, tx = tid & 15, ty = tid >> 4;
-    auto &Qs = sm.Qs;
+    const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127, tx = tid & 15, ty = tid >> 4;
     auto &Ks = sm.g[grp].Ks;
     auto &Vs = sm.g[grp].Vs;
     auto &Ps = sm.g[grp].Ps;
@@ -58,41 +59,47 @@ __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__
     const int n_keys = past + min(i0 + kRows, T);
     const KV *kb = kmem + (int64_t)b * key_rows * kv_ld + kvh * kD, *vb = vmem + (int64_t)b * key_rows * kv_ld + kvh * kD;
     const int64_t row0 = (int64_t)b * T + i0;
-    // a lane stages its row (key), a warp every fourth 4 dims
-    for (int d = (int)(threadIdx.x >> 5) * 4; d < kD; d += kGroups * 16) {
+    {
+        static_assert(kThreads == kRows * kD / 4, "one 16-byte piece of the query per thread");
+        const int r = (int)(threadIdx.x >> 4);
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (i0 + lane < T) v = load4(q + (row0 + lane) * ldq + h * kD + d);
-        Qs[d][lane] = v.x, Qs[d + 1][lane] = v.y, Qs[d + 2][lane] = v.z, Qs[d + 3][lane] = v.w;
+        if (i0 + r < T) v = load4(q + (row0 + r) * ldq + h * kD + tx * 4);
+        *reinterpret_cast<float4 *>(&sm.Qs[r][tx * 4]) = v;
     }
-    __syncthreads();
     float o[4][4] = {}, m[4], l[4] = {};
 #pragma unroll
     for (int i = 0; i < 4; i++) m[i] = -INFINITY;
+    if (grp * kKeys >= n_keys) asm volatile("bar.arrive %0, %1;" ::"r"(kGroups + 1), "n"(kThreads) : "memory");  // no block: nothing to wait for
     for (int key0 = grp * kKeys; key0 < n_keys; key0 += kGroups * kKeys) {
-        const bool in = key0 + lane < n_keys;
-        for (int d = warp * 4; d < kD; d += 16) {
-            float4 k = make_float4(0.f, 0.f, 0.f, 0.f), v = k;
-            if (in) k = load4(kb + (int64_t)(key0 + lane) * kv_ld + d), v = load4(vb + (int64_t)(key0 + lane) * kv_ld + d);
-            Ks[d][lane] = k.x, Ks[d + 1][lane] = k.y, Ks[d + 2][lane] = k.z, Ks[d + 3][lane] = k.w;
-            *reinterpret_cast<float4 *>(&Vs[lane][d]) = v;
+        float4 k[4], v[4];  // pieces tx of keys ty, ty + 8, ...
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int key = key0 + ty + 8 * i;
+            k[i] = v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (key < n_keys) k[i] = load4(kb + (int64_t)key * kv_ld + tx * 4), v[i] = load4(vb + (int64_t)key * kv_ld + tx * 4);
         }
-        group_sync();
-        float s[4][2] = {};  // rows 4 ty + i, keys 2 tx + j
-#pragma unroll 8
-        for (int d = 0; d < kD; d++) {
-            const float4 a = *reinterpret_cast<const float4 *>(&Qs[d][ty * 4]);
-            const float2 c = *reinterpret_cast<const float2 *>(&Ks[d][tx * 2]);
-            s[0][0] = fmaf(a.x, c.x, s[0][0]), s[0][1] = fmaf(a.x, c.y, s[0][1]);
-            s[1][0] = fmaf(a.y, c.x, s[1][0]), s[1][1] = fmaf(a.y, c.y, s[1][1]);
-            s[2][0] = fmaf(a.z, c.x, s[2][0]), s[2][1] = fmaf(a.z, c.y, s[2][1]);
-            s[3][0] = fmaf(a.w, c.x, s[3][0]), s[3][1] = fmaf(a.w, c.y, s[3][1]);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            *reinterpret_cast<float4 *>(&Ks[ty + 8 * i][tx * 4]) = k[i], *reinterpret_cast<float4 *>(&Vs[ty + 8 * i][tx * 4]) = v[i];
+        if (key0 == grp * kKeys) asm volatile("bar.sync %0, %1;" ::"r"(kGroups + 1), "n"(kThreads) : "memory");  // the query is there too
+        else group_sync();
+        float s[4][2] = {};  // rows 4 ty + i, keys tx + 16 j
+#pragma unroll 2
+        for (int d = 0; d < kD; d += 4) {
+            const float4 c0 = *reinterpret_cast<const float4 *>(&Ks[tx][d]), c1 = *reinterpret_cast<const float4 *>(&Ks[tx + 16][d]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float4 a = *reinterpret_cast<const float4 *>(&sm.Qs[ty * 4 + i][d]);
+                s[i][0] = fmaf(a.w, c0.w, fmaf(a.z, c0.z, fmaf(a.y, c0.y, fmaf(a.x, c0.x, s[i][0]))));
+                s[i][1] = fmaf(a.w, c1.w, fmaf(a.z, c1.z, fmaf(a.y, c1.y, fmaf(a.x, c1.x, s[i][1]))));
+            }
         }
         float p[4][2];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int last = past + i0 + ty * 4 + i;  // the row's last key
 #pragma unroll
-            for (int j = 0; j < 2; j++) s[i][j] = key0 + tx * 2 + j > last ? -INFINITY : s[i][j] * scale;
+            for (int j = 0; j < 2; j++) s[i][j] = key0 + tx + 16 * j > last ? -INFINITY : s[i][j] * scale;
             float mx = fmaxf(s[i][0], s[i][1]);
 #pragma unroll
             for (int w = 8; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
@@ -105,7 +112,7 @@ __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__
             for (int j = 0; j < 2; j++) p[i][j] = s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - mn), l[i] += p[i][j];
         }
 #pragma unroll
-        for (int j = 0; j < 2; j++) *reinterpret_cast<float4 *>(&Ps[tx * 2 + j][ty * 4]) = make_float4(p[0][j], p[1][j], p[2][j], p[3][j]);
+        for (int j = 0; j < 2; j++) *reinterpret_cast<float4 *>(&Ps[tx + 16 * j][ty * 4]) = make_float4(p[0][j], p[1][j], p[2][j], p[3][j]);
         __syncwarp();  // a warp's rows are its own
 #pragma unroll 8
         for (int k = 0; k < kKeys; k++) {
@@ -127,7 +134,6 @@ __global__ void __launch_bounds__(kThreads) attention_f32_kernel(const float *__
     }
     __syncthreads();
     // four dims of a row per thread (group 0 has key 0, so the largest maximum is finite)
-    static_assert(kThreads == kRows * kD / 4, "one float4 of the result per thread");
     const int r = (int)(threadIdx.x >> 4);
     float mt = sm.m[0][r], lt = 0.f;
     for (int i = 1; i < kGroups; i++) mt = fmaxf(mt, sm.m[i][r]);
