@@ -68,7 +68,8 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t saddr)
 
 __global__ void __launch_bounds__(kThreads, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const float *__restrict__ q,
-                    float *__restrict__ out, __half *__restrict__ out16, int *status, int M, int H, int KVH, int past, int ldq, float scale)
+                    const float *__restrict__ cs_table, float *__restrict__ out, __half *__restrict__ out16, int *status, int M, int H, int KVH, int past, int ldq,
+                    float scale)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -112,22 +113,29 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
             for (int j = 0; j < 2 && j < nb; j++) load_k(j), load_v(j);
         __syncwarp();
     } else {
-        // Q as fp16 rows of 128 bytes, 16-byte pieces swizzled as TMA would: a thread of each group per row
-        constexpr int PIECES = 8 / kGroups;
+        // Q as fp16 rows of 128 bytes, 16-byte pieces swizzled as TMA would: a thread of each group per row, with dims 8 part to + 7
+        // and the same of the upper half, which are what the rotary embedding turns together (ropeHalfRef,
+        // src/reference/qwen-ref.ts:35-64; a pass over q by itself took 4 us at 2048 rows)
+        static_assert(kGroups * 8 * 2 == kD, "two pieces per thread");
         const int r = threadIdx.x / kGroups, part = threadIdx.x % kGroups;
-        const float *src = q + (int64_t)(r0 + r) * ldq + h * kD + part * PIECES * 8;
+        const float4 *src = reinterpret_cast<const float4 *>(q + (int64_t)(r0 + r) * ldq + h * kD + part * 8);
+        const float4 *cs = reinterpret_cast<const float4 *>(cs_table + ((int64_t)(past + r0 + r) * (kD / 2) + part * 8) * 2);
+        uint32_t lo[4] = {}, hi[4] = {};
+        if (r0 + r < M) {
 #pragma unroll
-        for (int c = 0; c < PIECES; c++) {
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (r0 + r < M) {
-                const float4 a = *reinterpret_cast<const float4 *>(src + c * 8), b = *reinterpret_cast<const float4 *>(src + c * 8 + 4);
-                const __half2 h0 = __floats2half2_rn(a.x, a.y), h1 = __floats2half2_rn(a.z, a.w);
-                const __half2 h2 = __floats2half2_rn(b.x, b.y), h3 = __floats2half2_rn(b.z, b.w);
-                v.x = *reinterpret_cast<const uint32_t *>(&h0), v.y = *reinterpret_cast<const uint32_t *>(&h1);
-                v.z = *reinterpret_cast<const uint32_t *>(&h2), v.w = *reinterpret_cast<const uint32_t *>(&h3);
+            for (int c = 0; c < 2; c++) {
+                const float4 x = src[c], y = src[c + kD / 8];
+                const float4 c0 = cs[2 * c], c1 = cs[2 * c + 1];  // cos, sin of a dim and the next
+                const __half2 a0 = __floats2half2_rn(x.x * c0.x - y.x * c0.y, x.y * c0.z - y.y * c0.w);
+                const __half2 a1 = __floats2half2_rn(x.z * c1.x - y.z * c1.y, x.w * c1.z - y.w * c1.w);
+                const __half2 b0 = __floats2half2_rn(x.x * c0.y + y.x * c0.x, x.y * c0.w + y.y * c0.z);
+                const __half2 b1 = __floats2half2_rn(x.z * c1.y + y.z * c1.x, x.w * c1.w + y.w * c1.z);
+                lo[2 * c] = *reinterpret_cast<const uint32_t *>(&a0), lo[2 * c + 1] = *reinterpret_cast<const uint32_t *>(&a1);
+                hi[2 * c] = *reinterpret_cast<const uint32_t *>(&b0), hi[2 * c + 1] = *reinterpret_cast<const uint32_t *>(&b1);
             }
-            *reinterpret_cast<uint4 *>(smem + r * 128 + (((part * PIECES + c) ^ (r & 7)) << 4)) = v;
         }
+        *reinterpret_cast<uint4 *>(smem + r * 128 + ((part ^ (r & 7)) << 4)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        *reinterpret_cast<uint4 *>(smem + r * 128 + (((part + kGroups) ^ (r & 7)) << 4)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
         fence_async_smem();
     }
     __syncthreads();
@@ -303,7 +311,7 @@ bool op_attention_tc_supported(int M, int D, int ldq, int kv_ld, int kv_f16, con
     return kv_f16 && D == kD && M >= 512 && ldq % 4 == 0 && kv_ld % 8 == 0 && ((uintptr_t)q & 15) == 0;
 }
 
-int op_attention_tc(wb_context *ctx, const float *q, const void *kmem, const void *vmem, float *out, __half *out16, int M, int H, int KVH,
+int op_attention_tc(wb_context *ctx, const float *q, const float *cs_table, const void *kmem, const void *vmem, float *out, __half *out16, int M, int H, int KVH,
                     int past, int ldq, int kv_ld)
 {
     CUtensorMap maps[2];
@@ -317,7 +325,7 @@ int op_attention_tc(wb_context *ctx, const float *q, const void *kmem, const voi
     }
     if (const cudaError_t e = smem_limit_once<attention_tc_kernel>(kSmem); e != cudaSuccess) WB_CUDA(e);
     const dim3 grid((unsigned)H, (unsigned)((M + kRows - 1) / kRows));
-    const cudaError_t e = launch_pdl(attention_tc_kernel, grid, dim3(kThreads), (size_t)kSmem, ctx->stream, maps[0], maps[1], q, out, out16,
+    const cudaError_t e = launch_pdl(attention_tc_kernel, grid, dim3(kThreads), (size_t)kSmem, ctx->stream, maps[0], maps[1], q, cs_table, out, out16,
                                      ctx->status_word, M, H, KVH, past, ldq, 1.0f / sqrtf((float)kD));
     ctx->launches++;
     WB_CUDA(e);

@@ -180,7 +180,8 @@ int forward_impl(wb_qwen *m, const Bufs &b, int64_t M, int64_t B, int64_t T, int
             WB_CHECK(linear(m, L.k, b.n, b.k, L.kb, M));
             WB_CHECK(linear(m, L.v, b.n, b.v, L.vb, M));
         }
-        WB_CHECK(op_rope_kv(ctx, b.q, b.k, b.v, kc, vc, kv16, m->cs_table, (int)M, H, KVH, D, (int)T, past_ptr, (int)past,
+        const bool att_tc = use_cache && M > 1 && !m->exact && !past_ptr && op_attention_tc_supported((int)M, D, b.ldq, KV, kv16, b.q);
+        WB_CHECK(op_rope_kv(ctx, b.q, b.k, b.v, kc, vc, kv16, m->cs_table, (int)M, att_tc ? 0 : H, KVH, D, (int)T, past_ptr, (int)past,
                             b.ldq, b.ldk, b.ldv));
         bool att_half = false;
         if (use_cache) {
@@ -188,9 +189,9 @@ int forward_impl(wb_qwen *m, const Bufs &b, int64_t M, int64_t B, int64_t T, int
             if (M == 1 && D % 8 == 0 && D <= 128 && op_attention_decode_smem(D, max_keys, kv16) <= 160 * 1024) {
                 WB_CHECK(op_attention_decode(ctx, b.q, kc, vc, kv16, b.att, m->att_scratch, m->att_counters, H, KVH, D, past_ptr,
                                              (int)past, max_keys, KV));
-            } else if (!m->exact && !past_ptr && op_attention_tc_supported((int)M, D, b.ldq, KV, kv16, b.q)) {
+            } else if (att_tc) {
                 att_half = half_in;
-                WB_CHECK(op_attention_tc(ctx, b.q, kc, vc, b.att, att_half ? b.h16 : nullptr, (int)M, H, KVH, (int)past, b.ldq, KV));
+                WB_CHECK(op_attention_tc(ctx, b.q, m->cs_table, kc, vc, b.att, att_half ? b.h16 : nullptr, (int)M, H, KVH, (int)past, b.ldq, KV));
             } else if (!m->exact && op_attention_prefill_supported((int)M, H, KVH, D, b.ldq, KV)) {
                 // prefill in the default mode: causal attention on the tensor cores (fp16 operands, like the linears)
                 att_half = half_in;

@@ -27,7 +27,8 @@ int op_attention_f32(wb_context *ctx, const float *q, const void *kmem, const vo
                      const int *past_ptr, int past_imm, int use_cache, int ldq, int kv_ld, __half *out16);
 // attention_tc.cu: the same for M >= 512 rows against an fp16 cache, head size 64, on the tcgen05 tensor cores; past is known to the host
 bool op_attention_tc_supported(int M, int D, int ldq, int kv_ld, int kv_f16, const void *q);
-int op_attention_tc(wb_context *ctx, const float *q, const void *kmem, const void *vmem, float *out, __half *out16, int M, int H, int KVH,
+// (q before its rotary embedding, which the kernel does as op_rope_kv would)
+int op_attention_tc(wb_context *ctx, const float *q, const float *cs_table, const void *kmem, const void *vmem, float *out, __half *out16, int M, int H, int KVH,
                     int past, int ldq, int kv_ld);
 // The same for M >= 16 rows against the KV cache on the tensor cores (attention_prefill.cu): fp16 operands, f32 softmax
 // and accumulation; head size 64 or 128. Used by the default mode; the fp32-activation mode keeps op_attention.
