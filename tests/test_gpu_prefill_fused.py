@@ -59,6 +59,25 @@ def test_gate_up_silu_in_one_kernel(built_lib, oracle, n):
     assert err[True] < 1.05 * err[False], err  # no precision given up by the fusion
 
 
+@pytest.mark.parametrize("n", [129, 256, 257, 384])
+def test_gate_up_silu_where_the_plain_product_takes_another_kernel(built_lib, oracle, n):
+    """The edges of the row counts at which only the fused form runs on CTA pairs, with the same bounds as above."""
+    G = synthetic.random_qwen_gptq(WIDE, seed=13, std=0.05)
+    tokens = np.random.default_rng(n).integers(0, WIDE.vocab_size, n).astype(np.uint32)
+    ref = oracle.qwen_forward_ref(_ocfg(oracle, WIDE), _dense_from_gptq(oracle, G), tokens, 1, n, threads=oracle.max_threads())
+    rms = float(np.sqrt(np.mean(ref.astype(np.float64) ** 2)))
+    err = {}
+    for fuse in (True, False):
+        with Gpu(0, weight_bytes=64 << 20, act_bytes=256 << 20) as gpu:
+            model = QwenGpt(gpu, WIDE, max_t=n, kv_dtype="f32")
+            model.upload_gptq_model(G, fuse=fuse)
+            got = model.read_tensor(model.forward(tokens, 1, n)).reshape(n, -1)
+            model.close()
+        assert oracle.check_tolerance(got, ref, 1e-2 * rms, 2e-2).ok
+        err[fuse] = float(np.sqrt(np.mean((got - ref).astype(np.float64) ** 2))) / rms
+    assert err[True] < 1.05 * err[False], err
+
+
 @pytest.mark.parametrize("n", [64, 65, 127, 128, 129, 193, 320, 511, 512, 513, 575, 577, 640, 705, 897])
 def test_tcgen05_prefill_attention(built_lib, oracle, small, n):
     """fp16 cache; the warp-level kernel below 512 rows, tcgen05 from there on: every row against the reference at row counts beside the

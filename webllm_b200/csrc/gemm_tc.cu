@@ -1091,10 +1091,12 @@ int launch_gemm_tc(wb_context *ctx, const Weight &w, const void *A, void *C, con
     return WB_OK;
 }
 
-// gate | up with silu as one kernel wherever the plain product runs unsplit on CTA pairs, in the tile that it would have: whole
-// layers, separate and fused, us, K = 896 (I = 4864): 256 rows 60.1, 59.2; 512 75.6, 74.3; 1024 108, 103; 2048 152, 147; K = 2048
+// gate | up with silu as one kernel from 129 rows on wherever the product runs unsplit on CTA pairs (in the tile that it would have there),
+// also where the plain product would rather be one of the other kernels and a launch for silu: whole layers, separate and fused, us, K = 896 (I = 4864): 256 rows 60.1, 59.2; 512 75.6, 74.3; 1024 108, 103; 2048 152, 147; K = 2048
 // (11008): 256 rows 109, 106; 1024 229, 217; 2048 454, 430; K = 3584 (18944): 192 rows 157, 152; 1024 545, 529; 2048 1105, 1051. At no
-// size measured (128 to 2048 rows, K = 896, 1536, 2048 and 3584) was it slower.
+// size measured (128 to 2048 rows, K = 896, 1536, 2048 and 3584) was it slower. Against the persistent one-CTA kernel and silu (257 to
+// 384 rows) or the tensor-memory one and silu (129 to 256), twelve layers of K = 896, us: 144 rows 557, 550; 256 634, 631; 258 698, 674;
+// 300 724, 697; 384 776, 745. Up to 128 rows a tile would be half empty.
 int launch_gate_up_silu(wb_context *ctx, const Weight &w, const __half *A, __half *act, int64_t M, bool *done)
 {
     *done = false;
@@ -1102,6 +1104,11 @@ int launch_gate_up_silu(wb_context *ctx, const Weight &w, const __half *A, __hal
     if (w.kind != WeightKind::Gptq || ctx->force_kernel != 0 || ctx->place.n_dst != 0 || I % tc::BN != 0) return WB_OK;
     wb_plan plan;
     WB_CHECK(plan_linear(ctx, w, M, WB_F16, 0, &plan));
+    if (plan.kernel != WB_KERNEL_GEMM_TC_PAIR) {
+        if (M <= 128 || plan.split_k > 1) return WB_OK;
+        memset(&plan, 0, sizeof plan);
+        WB_CHECK(plan_gemm_tc(ctx, w, M, WB_F16, 0, 2, &plan));
+    }
     if (plan.kernel != WB_KERNEL_GEMM_TC_PAIR || plan.split_k > 1) return WB_OK;
     const char *base = ctx->arena[WB_ARENA_WEIGHTS].base;
     const int mt = plan.tile_m;
