@@ -54,7 +54,7 @@ typedef enum {
     WB_KERNEL_GEMV_MMA = 1,   /* M <= 32: weights streamed once, register unpack, warp-level MMA, split-K. The planner's
                                  choice up to M = 8 (on short-K, wide-N shapes up to 16 with f32 activations and, under 8 M weights, up to
                                  12 with fp16 ones) */
-    WB_KERNEL_GEMM_TC = 2,    /* tcgen05 / TMEM GEMM, TMA-fed, dequant in shared memory; f32 activations are rounded to
+    WB_KERNEL_GEMM_TC = 2,    /* tcgen05 / TMEM GEMM, TMA-fed, dequant in shared or (one round of tiles) tensor memory; f32 activations are rounded to
                                  fp16 first (as the reference's tiled GEMM stages them), never in exact mode */
     WB_KERNEL_GENERIC = 3,    /* shape-agnostic CUDA kernel for ragged sizes (K%8, N%4, group%32 != 0) */
     WB_KERNEL_DENSE_GEMV = 4, /* fp16 [N,K] weight, M <= 8 */

@@ -851,10 +851,11 @@ static int make_plan(wb_context *ctx, const Weight &w, int64_t M, int act_dtype,
     int kind = ctx->force_kernel;
     if (kind == 0) {
         // M <= 8: the GEMV (its one-row-block instance, 2 - 8 us). 9 <= M <= 16: its two-row-block instance costs 6 - 16 us
-        // and grows with M and K, the tensor-core kernel a flat 5 - 8 us (+ 2.3 us for the cast of f32 activations); measured
-        // on the 0.5B and the 7B-class shapes the GEMV still wins there only on short-K, wide-N projections (896 -> 4864: fp16
-        // 6.0 and 7.1 us at M = 9, 6.7 and 7.1 at 12, 7.6 and 7.1 at 16; f32 7.4 and 9.5 at M = 9, 9.7 and 9.5 at 16): up to M = 12
-        // with fp16 activations, up to 16 with f32 ones. Where the small-batch kernel takes the matrix (gemm_small.cu), it is
+        // and grows with M and K, the tensor-core kernels 4 - 8 us (+ 2 us for the cast of f32 activations). On short-K, wide-N
+        // projections the GEMV was even with the one-CTA tensor-core kernel (896 -> 4864: fp16 6.0 and 7.1 us at M = 9, 7.6 and 7.1
+        // at 16; f32 7.4 and 9.5, 9.7 and 9.5): up to M = 12 with fp16 activations, up to 16 with f32 ones. The kernel with its
+        // weights in tensor memory is faster there now (4.2 us), but rounds each weight times its scale to fp16 where the GEMV
+        // scales f32 sums, so these rows stay. Where the small-batch kernel takes the matrix (gemm_small.cu), it is
         // ahead of the GEMV from M = 9 on (fp16, M = 9: 896 -> 9728 7.2 and 5.2 us, 1536 -> 17920 19.2 and 9.3, 2048 -> 22016 30.4
         // and 13.9), so fp16 activations go there; f32 activations stay (20.8 and 9.9 us on 1536 -> 17920): the GEMV keeps
         // their ~22 bits, and every other kernel would round them to fp16.
