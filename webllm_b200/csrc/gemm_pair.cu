@@ -335,7 +335,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     if (ti != old_ti || group != old_group) request(), fresh = true;
                 }
             }
-            ok = mbar_wait(&full_w[s], ph, abort_flag, p.status, 4);
+            ok = mbar_wait_set<STAGES, KG>(&empty[s], &full_w[s], ph, abort_flag, p.status, 4);
             if (!ok) break;
             uint8_t *stage = smem + s * S::STAGE_BYTES;
             const uint32_t *src = (const uint32_t *)(stage + src_off);

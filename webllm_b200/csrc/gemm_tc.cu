@@ -204,7 +204,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                     request_group(group);
                     fresh = true;
                 }
-                ok = mbar_wait(&full[s], ph, abort_flag, p.status, 4);
+                ok = mbar_wait_set<STAGES, KG>(&empty[s], &full[s], ph, abort_flag, p.status, 4);
                 if (!ok) break;
                 uint8_t *stage = smem + s * S::STAGE_BYTES;
                 const uint32_t *src = (const uint32_t *)(stage + src_off);
@@ -478,7 +478,7 @@ gemm_tc_persist_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
                     request();
                     fresh = true;
                 }
-                ok = mbar_wait(&full[s], ph, abort_flag, p.status, 4);
+                ok = mbar_wait_set<STAGES, KG>(&empty[s], &full[s], ph, abort_flag, p.status, 4);
                 if (!ok) break;
                 uint8_t *stage = smem + s * S::STAGE_BYTES;
                 const uint32_t *src = (const uint32_t *)(stage + src_off);

@@ -88,6 +88,23 @@ __device__ __forceinline__ bool mbar_wait_idle(uint64_t *bar, uint32_t parity, v
     return false;
 }
 
+// Wait of an unpack set for the boxes of its next k-block. With SETS sets taking the k-blocks of a ring of STAGES stages in turn, a
+// set that does not come round to the same stages (SETS does not divide STAGES) has not seen the phase before the one it waits for,
+// and the parity of a barrier two phases back is the same: with the boxes of the stage's previous k-block still under way (two sets
+// can be done with later ones by then) the wait would be over at once, the set would unpack what is not there, and its arrivals would
+// be taken for the other set's. So it first waits until that k-block's MMAs are done, which the TMA producer waits for too. That
+// answer can not be taken for another: the MMAs two rounds back are done, since the set has had a k-block whose boxes were asked for
+// after them, and this round's can not be, without the set. Both are asked at once; the first has nearly always come long before.
+template <int STAGES, int SETS>
+__device__ __forceinline__ bool mbar_wait_set(uint64_t *empty, uint64_t *full, uint32_t ph, volatile int *abort_flag, int *status, int code)
+{
+    static_assert(SETS <= STAGES, "a set's k-block before this one is at most one round back");
+    if constexpr (STAGES % SETS == 0) return mbar_wait(full, ph, abort_flag, status, code);
+    const bool free = mbar_try(empty, ph ^ 1), there = mbar_try(full, ph);  // (in this order)
+    if (free && there) return true;
+    if (!free && !mbar_wait(empty, ph ^ 1, abort_flag, status, code)) return false;
+    return mbar_wait(full, ph, abort_flag, status, code);
+}
 
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar)
 {
