@@ -116,3 +116,20 @@ def test_more_sequences_than_a_grid_dimension_holds(built_lib, oracle, T):
         model.close()
     rms = float(np.sqrt(np.mean(ref.astype(np.float64) ** 2)))
     assert np.abs(got - ref[pick]).max() < 2e-2 * rms  # fp16 operands, as in the tests above
+
+
+# o and down cut along K with their slices left to the next norm: 16 slices, and the largest numbers that o and down of 896 columns
+# take; slices of the CTA-pair kernel; more than eight row tiles of the tensor-memory kernel on a K above 4096.
+@pytest.mark.parametrize("C,heads,I,n", [(256, 4, 4992, 340), (896, 14, 4992, 256), (896, 14, 4992, 600), (1024, 16, 8192, 1300), (896, 14, 4992, 1100)])
+def test_slices_that_the_norm_adds(built_lib, oracle, C, heads, I, n):
+    cfg = synthetic.QwenShape(256, 1, heads, 2, C, I)
+    G = synthetic.random_qwen_gptq(cfg, seed=15, std=0.05)
+    tokens = np.random.default_rng(n).integers(0, cfg.vocab_size, n).astype(np.uint32)
+    ref = oracle.qwen_forward_ref(_ocfg(oracle, cfg), _dense_from_gptq(oracle, G), tokens, 1, n, threads=oracle.max_threads())
+    rms = float(np.sqrt(np.mean(ref.astype(np.float64) ** 2)))
+    with Gpu(0, weight_bytes=96 << 20, act_bytes=512 << 20) as gpu:
+        model = QwenGpt(gpu, cfg, max_t=n, kv_dtype="f16")
+        model.upload_gptq_model(G, fuse=True)
+        for got in (model.read_tensor(model.forward(tokens, 1, n)), model.read_tensor(model.prefill(tokens))):
+            assert oracle.check_tolerance(got.reshape(n, -1), ref, 1e-2 * rms, 2e-2).ok
+        model.close()

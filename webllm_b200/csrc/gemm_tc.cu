@@ -768,12 +768,26 @@ static bool persist_enabled()
     return on;
 }
 
+// Microseconds that S K slices cost behind the product: the reduce launch, which moves slices + 1 copies of the output. Slices that
+// the next norm adds (`kept`) cost next to nothing while they lie in the L2: the norm has rows enough under way to read them beside the
+// residual (prefill layers of 896, 1536 and 2048 columns, 129 to 2048 rows, every number of slices: no cost that a fit shows, up to
+// some 30 MB written and read). With the launch in the estimate nevertheless, o and down ran unsplit, or on row tiles of gemm_thin.cu
+// that are slower. A layer, us, before -> after: 896 -> 896, 256 rows 52.6 -> 51.0, 340 60.5 -> 59.9, 378 62.1 -> 60.9, 512 67.3 -> 65.9;
+// 8960 -> 1536, 900 rows 145.3 -> 141.6, 2048 262 -> 257; 11008 -> 2048, 704 rows 164 -> 159. Up to 128 rows gemm_thin.cu is ahead by more
+// than the estimates tell apart (896 columns, 64 rows 37.0 -> 37.8), and they stay as they were.
+static double slices_cost(int64_t M, int64_t N, int S, bool kept)
+{
+    if (S <= 1) return 0.;
+    if (!kept) return 1.5 + (S + 1) * (double)M * N * 4. / 5e6;
+    return 0.2 + std::max(0., (S - 1) * (double)M * N * 8. - 30e6) / 10e6;
+}
+
 // Tile (mt tokens x 128 * nh output columns) and number of K slices, by a small cost model in microseconds whose
 // constants are measurements: the time of one 64-k block of a tile (the unpack of the weight tile bounds it, so it
 // depends on the columns far more than on the tokens), a fixed time per tile (pipeline fill, TMEM drain and stores),
-// and for split-K the reduce launch, which moves slices + 1 copies of the output.
+// and what the K slices cost (slices_cost).
 // WEBLLM_B200_GEMM_MT / _NH / _SPLIT pin one of the three for experiments.
-static double pick_plan(int64_t M, int64_t N, int kblocks, int sms, int force_split, double t_remote, int *mt_out, int *nh_out, int *s_out)
+static double pick_plan(int64_t M, int64_t N, int kblocks, int sms, int force_split, bool kept, double t_remote, int *mt_out, int *nh_out, int *s_out)
 {
     static const int force_mt = env_int("WEBLLM_B200_GEMM_MT"), force_nh = env_int("WEBLLM_B200_GEMM_NH"),
                      env_split = env_int("WEBLLM_B200_GEMM_SPLIT");
@@ -807,7 +821,7 @@ static double pick_plan(int64_t M, int64_t N, int kblocks, int sms, int force_sp
                 // a column-sharded call also stores the result into the peers: under the next tile's MMAs in the
                 // persistent loop, at the end of every CTA (on top of the arithmetic) otherwise
                 if (t_remote > 0.) t = persist ? (t > t_remote ? t : t_remote) : t + t_remote;
-                if (S > 1) t += 1.5 + (S + 1) * (double)M * N * 4. / 5e6;
+                t += slices_cost(M, N, S, kept);
                 if (best < 0. || t < best) best = t, *mt_out = mt, *nh_out = nh, *s_out = S;
             }
         }
@@ -817,7 +831,7 @@ static double pick_plan(int64_t M, int64_t N, int kblocks, int sms, int force_sp
 
 // The same model for the CTA-pair kernel (gemm_pair.cu): work items of mt tokens x 256 columns x one K slice, walked by
 // sms / 2 persistent pairs; fill, drain and stores are paid once per pair.
-static double pick_plan_pair(int64_t M, int64_t N, int kblocks, int sms, int force_split, bool tail_ok, int *mt_out, int *s_out)
+static double pick_plan_pair(int64_t M, int64_t N, int kblocks, int sms, int force_split, bool kept, bool tail_ok, int *mt_out, int *s_out)
 {
     static const int force_mt = env_int("WEBLLM_B200_GEMM_MT"), env_split = env_int("WEBLLM_B200_GEMM_SPLIT");
     if (force_split <= 0) force_split = env_split;
@@ -841,7 +855,7 @@ static double pick_plan_pair(int64_t M, int64_t N, int kblocks, int sms, int for
             int tr, trem, tst, tper;
             if (S == 1 && tail_ok && pair_tail_plan(tiles, pairs, kblocks, &tr, &trem, &tst, &tper))  // the last round cut along K
                 t = 3.3 + t_tile + tr * (per * t_kb + kPairItem) + (tper * t_kb + kPairItem) + 3.0;
-            if (S > 1) t += 1.5 + (S + 1) * (double)M * N * 4. / 5e6;
+            t += slices_cost(M, N, S, kept);
             if (best < 0. || t < best) best = t, *mt_out = mt, *s_out = S;
         }
     }
@@ -858,7 +872,8 @@ int plan_gemm_tc(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int
     int mt, nh, S;
     // microseconds that the stores to the peers of a column-sharded call take at ~700 GB/s per direction
     const double t_remote = ctx->place.n_dst > 1 ? (double)(ctx->place.n_dst - 1) * M * w.N * ctx->place.elem_bytes / 700e3 : 0.;
-    const double t_one = pick_plan(M, w.N, kblocks, ctx->sm_count, ctx->force_split, t_remote, &mt, &nh, &S);
+    const bool kept = ctx->keep_slices && M > 128 && ctx->place.n_dst == 0 && w.N % 4 == 0;  // (as launch_gemm_tc keeps them)
+    const double t_one = pick_plan(M, w.N, kblocks, ctx->sm_count, ctx->force_split, kept, t_remote, &mt, &nh, &S);
     wb_plan thin = *plan;
     double t_thin = 0.;
     const bool thin_ok = pair_mode == 1 && plan_gemm_thin(ctx, w, M, act_dtype, &thin, &t_thin) && t_thin < t_one;
@@ -868,7 +883,7 @@ int plan_gemm_tc(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int
     if (pair_mode == 2 && !pair_ok) return WB_OK;
     if (pair_ok) {
         int pmt, pS;
-        double t_pair = pick_plan_pair(M, w.N, kblocks, ctx->sm_count, ctx->force_split, ctx->place.n_dst == 0, &pmt, &pS);
+        double t_pair = pick_plan_pair(M, w.N, kblocks, ctx->sm_count, ctx->force_split, kept, ctx->place.n_dst == 0, &pmt, &pS);
         if (t_remote > 0. && pS == 1 && t_pair < t_remote) t_pair = t_remote;  // the stores to the peers run under the MMAs
         if (pair_mode == 2 || (t_pair > 0. && t_pair < t_one && !(thin_ok && t_thin < t_pair))) {
             plan->kernel = WB_KERNEL_GEMM_TC_PAIR;
