@@ -97,3 +97,17 @@ def test_several_row_tiles(gpu, oracle, K, N, M):
                 assert_close(oracle, run_linear(gpu, h, xin, M, N, hb, act=act, out=out), ref, 1e-3, f"{K}x{N} M={M} {act} split {split}")
         finally:
             gpu.plan_override(0, 0)
+
+
+@pytest.mark.parametrize("M,split", [(1100, 2), (1280, 2), (2300, 1), (2368, 1)])
+def test_long_k_and_many_rows_by_themselves(gpu, oracle, M, split):
+    """Slices of 128-row tiles while two fit, one slice where the tiles fill four fifths of the SMs."""
+    K, N = 4864, 896
+    t = synthetic.random_gptq(K, N, 128, seed=4, zeros="any")
+    h = register(gpu, f"thl_{M}", t)
+    x16 = np.random.default_rng(M).standard_normal((M, K)).astype(np.float16)
+    p = gpu.plan(h, M, "f16")
+    assert p["block"] == BLOCK and p["tile_m"] <= 128 and p["split_k"] == split, p
+    rows = [0, 127, 128, 700, M - 1]
+    got = run_linear(gpu, h, x16, M, N, act="f16", out="f32").reshape(M, N)
+    assert_close(oracle, got[rows].ravel(), _reference(oracle, t, x16[rows], len(rows), N, K), 1e-3, f"{M}")

@@ -466,13 +466,16 @@ bool plan_gemm_thin(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, 
         const int nt = thin_rows(M, most);
         const int64_t rows = thin_tiles(M, most), tiles = cols * rows;
         if (rows > 1 && tiles > sms) continue;  // every CTA sets itself up and drains: larger products go to persistent ones
-        // Long products of a long K: as a call by itself these stay with the pairs, whose plan cuts K, as it is asked to
-        // (4864 -> 896, 2048 rows: 25.5 us, 17.3 here). A caller that would add the slices itself gets the whole result from here.
-        if (rows > 8 && chunks > 32 && !ctx->keep_slices) continue;
         for (int S = 1; S <= 8 && S <= chunks; S++) {
             if (ctx->force_split > 0 && S != std::min(ctx->force_split, chunks)) continue;
             const int per = (chunks + S - 1) / S, at_once = thin_clusters(S, sms);
             if ((chunks + per - 1) / per != S || (S > 1 && tiles > at_once)) continue;
+            // A long K of nine row tiles or more is cut while a fifth of the SMs would have no tile: of a call by itself a plan
+            // promises that, and here it is the slower choice, by a third. Uncut and cut, us: 4864 -> 896 at 1500 rows 18.2, 21.1 (three
+            // slices of 256-row tiles), 2048 rows 18.2, 24.5 (two); 6144 -> 1200 at 1280 21.0, 27.5; 18944 -> 512 at 2048 63, 42.
+            // With fewer SMs idle, or cut in slices of 128-row tiles, nothing holds it back: 4864 -> 896 at 2500 rows 30.4 -> 19.5, at
+            // 1100 19.8 -> 14.2; 11008 -> 2048 at 1100 54 -> 41. A caller that adds the slices itself has the uncut one everywhere.
+            if (S == 1 && rows > 8 && chunks > 32 && tiles * 5 < sms * 4 && !ctx->keep_slices) continue;
             const int64_t rounds = S > 1 ? 1 : (tiles + sms - 1) / sms;
             const double chunk = nt > kRows ? 0.66 : 0.27 + 0.07 * std::min<double>(1., (double)tiles * S / sms);
             const double t = 1.6 + 0.022 * nt + rounds * per * chunk + (S > 1 ? 1.3 : 0.);
