@@ -1,5 +1,11 @@
 """GPU parity of the int4 GEMM with its weights in tensor memory (up to 128 rows): row counts around its tiles, columns and K that do not
 fill theirs, groups smaller and larger than its chunks, every number of slices, both activation and result types."""
+import json
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -111,3 +117,20 @@ def test_long_k_and_many_rows_by_themselves(gpu, oracle, M, split):
     rows = [0, 127, 128, 700, M - 1]
     got = run_linear(gpu, h, x16, M, N, act="f16", out="f32").reshape(M, N)
     assert_close(oracle, got[rows].ravel(), _reference(oracle, t, x16[rows], len(rows), N, K), 1e-3, f"{M}")
+
+
+@pytest.mark.parametrize("var,value,key,want", [("MT", 192, "tile_m", 192), ("NH", 2, "tile_n", 256), ("SPLIT", 3, "split_k", 3), ("THIN", 0, None, None)])
+def test_pins_hold_where_this_kernel_would_be_taken(gpu, var, value, key, want):
+    """The switches are read once per process, so a child asks for the plan."""
+    h = register(gpu, f"thp_{var}", synthetic.random_gptq(896, 1152, 128, seed=2))
+    assert gpu.plan(h, 404, "f16")["block"] == BLOCK
+    code = ("import json; from webllm_b200 import Gpu, synthetic\n"
+            "with Gpu(0, weight_bytes=16 << 20, act_bytes=16 << 20) as g:\n"
+            "    t = synthetic.random_gptq(896, 1152, 128, seed=2)\n"
+            "    h = g.gptq_register('w', t.qweight, t.qzeros, t.scales, 896, 1152, 128)\n"
+            "    print(json.dumps(g.plan(h, 404, 'f16')))\n")
+    r = subprocess.run([sys.executable, "-c", code], env={**os.environ, f"WEBLLM_B200_GEMM_{var}": str(value)}, capture_output=True, text=True,
+                       cwd=Path(__file__).resolve().parent.parent, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    p = json.loads(r.stdout.splitlines()[-1])
+    assert p["block"] != BLOCK and (key is None or p[key] == want), p

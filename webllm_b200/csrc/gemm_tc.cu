@@ -863,11 +863,13 @@ static double pick_plan_pair(int64_t M, int64_t N, int kblocks, int sms, int for
 }
 
 // pair_mode: 0 = one-CTA kernels only, 1 = whichever the cost model prefers, 2 = the CTA-pair kernel or nothing
-// (plan->kernel stays 0 when the shape does not qualify).
+// (plan->kernel stays 0 when the shape does not qualify). A pinned tile or number of slices (pick_plan) is one of these kernels': the
+// small-batch and the tensor-memory kernel, which have neither, step back.
 int plan_gemm_tc(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int exact, int pair_mode, wb_plan *plan)
 {
     (void)exact;
-    if (pair_mode == 1 && plan_gemm_small(ctx, w, M, plan)) return WB_OK;
+    static const bool pinned = env_int("WEBLLM_B200_GEMM_MT") || env_int("WEBLLM_B200_GEMM_NH") || env_int("WEBLLM_B200_GEMM_SPLIT");
+    if (pair_mode == 1 && !pinned && plan_gemm_small(ctx, w, M, plan)) return WB_OK;
     const int kblocks = (int)(w.K / 64);
     int mt, nh, S;
     // microseconds that the stores to the peers of a column-sharded call take at ~700 GB/s per direction
@@ -876,7 +878,7 @@ int plan_gemm_tc(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int
     const double t_one = pick_plan(M, w.N, kblocks, ctx->sm_count, ctx->force_split, kept, t_remote, &mt, &nh, &S);
     wb_plan thin = *plan;
     double t_thin = 0.;
-    const bool thin_ok = pair_mode == 1 && plan_gemm_thin(ctx, w, M, act_dtype, &thin, &t_thin) && t_thin < t_one;
+    const bool thin_ok = pair_mode == 1 && !pinned && plan_gemm_thin(ctx, w, M, act_dtype, &thin, &t_thin) && t_thin < t_one;
     // Stores into peers' slabs stay with the one-CTA kernels: a two-GPU run of the pair kernel with peer destinations
     // (7B-class shards at M = 4096) ended in a launch failure whose cause reading has not shown, so it is not launched so.
     const bool pair_ok = pair_mode > 0 && ctx->place.n_dst <= 1 && gemm_pair_supports(w, M) && ctx->sm_count >= 2;
