@@ -8,7 +8,9 @@
 // key, 32 lines touched per load, took the L1 8000 cycles an SM); scores are taken four dims at a time from 16-byte pieces. One CTA per single row, as the scalar kernel (qwen_ops.cu) has it, reads every
 // key 32 times as often and leaves a warp's lanes one multiply per load. 4 x 101 rows, 14 heads: 57 -> 22 us with
 // one group, whose chain of key blocks it was, 17 with four, 14 with rows read as they lie. Bound by the multiply-adds and the loads
-// that feed them on the SMs that have two long tiles.
+// that feed them on the SMs that have two long tiles. Two CTAs an SM leave a thread 64 registers, and 44 bytes are spilled. With one of 128
+// registers nothing is, and a layer of 1 x 384 tokens takes 74 us instead of 82, of 4 x 101 67.4 instead of 68.1, but of 6 x 50 61.7
+// instead of 61.0.
 #include <algorithm>
 
 #include "qwen_ops.cuh"
@@ -163,9 +165,9 @@ __global__ void __launch_bounds__(kThreads, 2) attention_f32_kernel(const float 
 constexpr int kSequences = 65535;
 
 // Sequences of more than 8 rows, 16-byte aligned heads of 64 dims. A tile has 32 rows and keys whatever the sequence has, and the
-// scalar kernel's work goes with the rows times the keys. Whole layers of 14 heads, us, scalar and tiled, one sequence / 64 / 256:
-// T = 4 29.6, 31.5 / 49.4, 61.0 / 78.8, 122; T = 8 36.9, 37.8 / 60.7, 65.8 / 118, 138 (2 to 16 sequences 0.7 the other way);
-// T = 10 36.3, 34.9 / 69.0, 69.8 / 148, 153; T = 16 38.7, 35.8 / 89.6, 76.9 / 227, 178.
+// scalar kernel's work goes with the rows times the keys. Whole layers of 14 heads, us, scalar and tiled, one sequence / 4 / 64 / 256:
+// T = 4 34.0, 35.2 / 36.2, 35.0 / 55.9, 65.8 / 99, 139; T = 8 41.2, 41.6 / 37.9, 35.2 / 72.6, 75.8 / 153, 168; T = 9 37.5, 34.3 / 39.7, 36.3 /
+// 77.7, 78.1 / 166, 173; T = 10 38.0, 34.4 / 39.8, 36.7 / 81.3, 80.0 / 183, 182; T = 16 39.4, 34.8 / 43.4, 39.0 / 110, 94 / 287, 233.
 bool op_attention_f32_supported(int T, int D, int ldq, int kv_ld) { return T > 8 && D == kD && ldq % 4 == 0 && kv_ld % 4 == 0; }
 
 int op_attention_f32(wb_context *ctx, const float *q, const void *kmem, const void *vmem, int kv_f16, float *out, int M, int H, int KVH, int T,

@@ -204,7 +204,7 @@ bool gemm_small_takes(wb_context *ctx, const Weight &w, int64_t M);
 bool plan_gemm_small(wb_context *ctx, const Weight &w, int64_t M, wb_plan *plan);
 int launch_gemm_small(wb_context *ctx, const Weight &w, const void *A, void *C, const float *bias, int64_t M, int act_dtype, int out_dtype,
                       const wb_plan &plan);
-// gemm_thin.cu: the tensor-core GEMM with its weight operand in tensor memory, up to 128 rows; likewise with this block size
+// gemm_thin.cu: the tensor-core GEMM with its weight operand in tensor memory, tiles of up to 256 rows; likewise with this block size
 constexpr int kThinBlock = 896;
 inline bool is_thin_plan(const wb_plan &plan) { return plan.kernel == WB_KERNEL_GEMM_TC && plan.block == kThinBlock; }
 bool plan_gemm_thin(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, wb_plan *plan, double *t_out);

@@ -15,7 +15,9 @@
 //   * The K slices of a column tile meet in the workspace: the last one to arrive adds them in slice order. No second launch.
 // Measured, f32 activations, M = 16, tcgen05 kernel with its two extra launches -> this: 3584 -> 18944 24.4 -> 17.3 us, 18944 -> 3584
 // 28.1 -> 24.4, 3584 -> 3584 11.6 -> 8.9; M = 9 alike. It is bound by its fixed parts (staging, the slices' meeting), not by
-// HBM (5.2 us) or the MMAs. A version for 24 and 32 rows was no faster than the tcgen05 kernel (three and four row blocks leave no
+// HBM (5.2 us) or the MMAs. gemm_thin.cu is faster (16 fp16 rows: 16.1 and 12.0, 23.3 and 15.8, 8.3 and 6.5 us on the three), but these rows
+// stay: here the nibbles are multiplied as they are and f32 sums are scaled, there each weight times its scale is rounded to fp16. Against
+// 64 bits, with the same activations, 1.5e-6 and 1.8e-4 of the result (2-norm). A version for 24 and 32 rows was no faster than the tcgen05 kernel (three and four row blocks leave no
 // registers for loads under way), nor were slices as clusters with one CTA of 16 warps an SM.
 #include <stdlib.h>
 

@@ -1109,11 +1109,10 @@ int launch_gemm_tc(wb_context *ctx, const Weight &w, const void *A, void *C, con
 }
 
 // gate | up with silu as one kernel from 129 rows on wherever the product runs unsplit on CTA pairs (in the tile that it would have there),
-// also where the plain product would rather be one of the other kernels and a launch for silu: whole layers, separate and fused, us, K = 896 (I = 4864): 256 rows 60.1, 59.2; 512 75.6, 74.3; 1024 108, 103; 2048 152, 147; K = 2048
-// (11008): 256 rows 109, 106; 1024 229, 217; 2048 454, 430; K = 3584 (18944): 192 rows 157, 152; 1024 545, 529; 2048 1105, 1051. At no
-// size measured (128 to 2048 rows, K = 896, 1536, 2048 and 3584) was it slower. Against the persistent one-CTA kernel and silu (257 to
-// 384 rows) or the tensor-memory one and silu (129 to 256), twelve layers of K = 896, us: 144 rows 557, 550; 256 634, 631; 258 698, 674;
-// 300 724, 697; 384 776, 745. Up to 128 rows a tile would be half empty.
+// also where the plain product would rather be one of the other kernels and a launch for silu. A prefill layer, us, separate and fused, K = 896
+// (I = 4864): 129 rows 45.9, 45.5; 192 49.3, 48.8; 224 50.8, 51.0; 256 51.6, 51.1; 300 60.0, 58.4; 512 69.8, 65.8; 1024 95.1, 87.8; 2048 139, 124;
+// K = 1536 (8960): 129 rows 63.2, 61.5; 256 73.7, 71.7; 1024 158, 143; K = 2048 (11008): 129 rows 87.5, 84.7; 256 99.7, 95.2; 1024 215, 192; 2048
+// 412, 373. At no other size measured (13 row counts) was it slower. Up to 128 rows a tile would be half empty.
 int launch_gate_up_silu(wb_context *ctx, const Weight &w, const __half *A, __half *act, int64_t M, bool *done)
 {
     *done = false;

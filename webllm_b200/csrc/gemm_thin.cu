@@ -1,5 +1,5 @@
 // int4 GEMM on the 5th-generation tensor cores with the weight operand taken from tensor memory, for products that are one round of tiles
-// of 128 columns x up to 128 rows: served batches, short prompts, and the narrow projections of long ones. Same contract as
+// of 128 columns x up to 128 or 256 rows: served batches, short prompts, and the narrow projections of long ones. Same contract as
 // gemm_tc.cu: fp16 operands, the weight rounded to fp16 once, f32 accumulation, f32 activations rounded to fp16
 // (gemm_nt_f16_from_f32.wgsl:58-62).
 //
@@ -23,8 +23,9 @@
 // Measured, gemm_tc.cu -> this, fp16 activations, us at 20 and 128 rows: 3584 -> 18944 20.4 -> 12.2, 23.2 -> 14.9; 18944 -> 3584 23.6 ->
 // 16.1, 27.5 -> 19.2; 3584 -> 3584 9.2 -> 6.8, 11.5 -> 9.5; 3584 -> 512 6.9 -> 4.3, 8.4 -> 7.2; 896 -> 4864 6.9 -> 4.2, 8.6 -> 6.6; 4864 -> 896
 // 7.6 -> 4.9, 9.2 -> 7.8; 896 -> 896 5.2 -> 4.1, 6.5 -> 6.4; at 512 and 2048 rows (against the CTA pairs where they were taken): 896 -> 1152
-// 8.7 -> 6.6, 9.2 -> 7.9; 4864 -> 896 12.6 -> 10.5, 25.5 -> 17.4; 3584 -> 3584 at 512 and 1024 22.8 -> 14.3, 27.8 -> 22.6; 3584 -> 18944
-// at 256 29.7 -> 23.3. Built and slower: weights straight into registers (a use waits for the youngest load),
+// 8.7 -> 6.6, 9.2 -> 7.9; 4864 -> 896 12.6 -> 10.5, 26.3 -> 18.2 (uncut, as a caller that adds slices itself has it; a layer of a prefill
+// 125.9 -> 123.2, since the norm added the slices of the pair kernel at hardly any cost); 3584 -> 3584 at 512 and 1024 22.8 -> 14.3, 27.8 -> 22.6;
+// 3584 -> 18944 at 256 29.7 -> 23.3. Built and slower: weights straight into registers (a use waits for the youngest load),
 // cp.async for all of them (130 cycles each to issue), activations rounded by warps of this kernel, the next chunk's words read under
 // this one's arithmetic, two CTAs of half the size per SM, and shares of several tiles per CTA (the code for that alone cost a
 // fifth: the roles' code does not fit the instruction caches side by side).
