@@ -133,3 +133,20 @@ def test_slices_that_the_norm_adds(built_lib, oracle, C, heads, I, n):
         for got in (model.read_tensor(model.forward(tokens, 1, n)), model.read_tensor(model.prefill(tokens))):
             assert oracle.check_tolerance(got.reshape(n, -1), ref, 1e-2 * rms, 2e-2).ok
         model.close()
+
+
+def test_rounded_activations_and_kept_slices_share_the_workspace(built_lib):
+    """A long prompt through separate projections, whose f32 activations are rounded into the workspace: 57 MB for down, beside which 46 MB of
+    K slices would not fit. Against the same model with fused projections."""
+    cfg, n = synthetic.QwenShape(256, 1, 14, 2, 896, 8960), 3200
+    G = synthetic.random_qwen_gptq(cfg, seed=16, std=0.05)
+    tokens = np.random.default_rng(n).integers(0, cfg.vocab_size, n).astype(np.uint32)
+    got = []
+    for fuse in (True, False):
+        with Gpu(0, weight_bytes=64 << 20, act_bytes=1 << 30) as gpu:
+            model = QwenGpt(gpu, cfg, max_t=n, kv_dtype="f16")
+            model.upload_gptq_model(G, fuse=fuse)
+            got.append(model.read_tensor(model.prefill(tokens)).astype(np.float64))
+            model.close()
+    rms = float(np.sqrt(np.mean(got[0] ** 2)))
+    assert np.abs(got[1] - got[0]).max() < 3e-2 * rms

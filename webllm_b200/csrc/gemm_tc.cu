@@ -768,6 +768,8 @@ static bool persist_enabled()
     return on;
 }
 
+constexpr double kPartialBytes = 64e6;  // of the workspace, at most, for the partial sums of K slices
+
 // Microseconds that S K slices cost behind the product: the reduce launch, which moves slices + 1 copies of the output. Slices that
 // the next norm adds (`kept`) cost next to nothing while they lie in the L2: the norm has rows enough under way to read them beside the
 // residual (prefill layers of 896, 1536 and 2048 columns, 129 to 2048 rows, every number of slices: no cost that a fit shows, up to
@@ -812,7 +814,7 @@ static double pick_plan(int64_t M, int64_t N, int kblocks, int sms, int force_sp
                 if (force_split > 0 ? S != (force_split < kblocks ? force_split : kblocks) : (S > 1 && kblocks / S < min_per)) continue;
                 const int per = (kblocks + S - 1) / S;
                 if ((kblocks + per - 1) / per != S) continue;  // would leave an empty slice
-                if (S > 1 && (double)S * M * N * 4. > 64e6) continue;  // partial sums must fit the workspace
+                if (S > 1 && (double)S * M * N * 4. > kPartialBytes) continue;  // partial sums must fit the workspace
                 const int64_t waves = (tiles * S + sms - 1) / sms;
                 double t = 2.0 + waves * (per * t_kb + t_tile);
                 // persistent CTAs (where TMEM holds two accumulator sets): fill, drain and stores are paid once
@@ -849,7 +851,7 @@ static double pick_plan_pair(int64_t M, int64_t N, int kblocks, int sms, int for
             if (force_split > 0 ? S != (force_split < kblocks ? force_split : kblocks) : (S > 1 && kblocks / S < min_per)) continue;
             const int per = (kblocks + S - 1) / S;
             if ((kblocks + per - 1) / per != S) continue;
-            if (S > 1 && (double)S * M * N * 4. > 64e6) continue;
+            if (S > 1 && (double)S * M * N * 4. > kPartialBytes) continue;
             const int64_t rounds = (tiles * S + pairs - 1) / pairs;
             double t = 3.3 + t_tile + rounds * (per * t_kb + kPairItem);
             int tr, trem, tst, tper;
@@ -874,7 +876,9 @@ int plan_gemm_tc(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int
     int mt, nh, S;
     // microseconds that the stores to the peers of a column-sharded call take at ~700 GB/s per direction
     const double t_remote = ctx->place.n_dst > 1 ? (double)(ctx->place.n_dst - 1) * M * w.N * ctx->place.elem_bytes / 700e3 : 0.;
-    const bool kept = ctx->keep_slices && M > 128 && ctx->place.n_dst == 0 && w.N % 4 == 0;  // (as launch_gemm_tc keeps them)
+    const uint64_t stage_bytes = act_dtype == WB_F32 ? align_up((uint64_t)M * w.K * 2) : 0;
+    // (as launch_gemm_tc keeps them; and where the rounded activations leave them no room, the estimate is not to ask for them)
+    const bool kept = ctx->keep_slices && M > 128 && ctx->place.n_dst == 0 && w.N % 4 == 0 && stage_bytes + (uint64_t)kPartialBytes <= kWorkspaceBytes;
     const double t_one = pick_plan(M, w.N, kblocks, ctx->sm_count, ctx->force_split, kept, t_remote, &mt, &nh, &S);
     wb_plan thin = *plan;
     double t_thin = 0.;
@@ -912,7 +916,6 @@ int plan_gemm_tc(wb_context *ctx, const Weight &w, int64_t M, int act_dtype, int
         plan->tile_m = mt;
         plan->tile_n = 128 * nh;
     }
-    const uint64_t stage_bytes = act_dtype == WB_F32 ? align_up((uint64_t)M * w.K * 2) : 0;
     // a pair launch that cuts its last round along K (PairTail, gemm_pair.cu) parks one partial tile per pair and adds a launch
     int tr, trem, tst, tper;
     const bool pair_tail = plan->kernel == WB_KERNEL_GEMM_TC_PAIR && S == 1 && ctx->place.n_dst == 0 &&
