@@ -93,8 +93,8 @@ __device__ __forceinline__ bool mbar_wait_idle(uint64_t *bar, uint32_t parity, v
 // and the parity of a barrier two phases back is the same: with the boxes of the stage's previous k-block still under way (two sets
 // can be done with later ones by then) the wait would be over at once, the set would unpack what is not there, and its arrivals would
 // be taken for the other set's. So it first waits until that k-block's MMAs are done, which the TMA producer waits for too. That
-// answer can not be taken for another: the MMAs two rounds back are done, since the set has had a k-block whose boxes were asked for
-// after them, and this round's can not be, without the set. Both are asked at once; the first has nearly always come long before.
+// answer can not be taken for another: the stage's MMAs before those are done, since the set has had a k-block whose boxes were asked for
+// after them, and its own k-block's can not be, without the set. Both are asked at once; the first has nearly always come long before.
 // (Two barriers a stage, for even and odd rounds, are as sound and measured the same: a layer of 2048 rows 124.3 us, 124.5.)
 template <int STAGES, int SETS>
 __device__ __forceinline__ bool mbar_wait_set(uint64_t *empty, uint64_t *full, uint32_t ph, volatile int *abort_flag, int *status, int code)
