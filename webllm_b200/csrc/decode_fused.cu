@@ -8,7 +8,10 @@
 //     keep two to three blocks in flight, across phase, layer and token boundaries;
 //   * activations are handed over WITHOUT a barrier: every f32 value is stored together with the step's epoch in one 64-bit
 //     word (as in NCCL's LL protocol), and a reader polls the very words that it needs. A hand-over is one store and one load through L2, about
-//     0.9 us from all CTAs to all, against a store, a fence, an atomic and a second round trip for a grid barrier. All layers
+//     0.4 us at best from all CTAs to all, against a store, a fence, an atomic and a second round trip for a grid barrier. A store
+//     covers whole 32-byte sectors: one that covers half of a sector which other SMs poll took 1.6 us longer to be seen (16-byte
+//     stores of some gate|up results, of the splits' maxima and of the argmax candidates: a step of 298 us became 263 us when each
+//     had a sector for itself). All layers
 //     use the same words, with an epoch of their own: while each layer had its own, a poll's first try missed L2 (the weights
 //     had pushed the words out since the step before) and came back from HBM a microsecond later, empty. Writing them over is
 //     safe because a CTA gets to write a vector of layer l + 1 only through down of l, which needs the gate|up of every CTA of
@@ -16,20 +19,22 @@
 //     by gate|up of l + 1 and by q|k|v of l + 1;
 //   * every CTA keeps the residual stream itself, so the norms need no hand-over of their own.
 // A layer is five such hand-overs: q|k|v, attention, o, gate|up (with silu * up at the producer), down.
-// Measured on the 0.5B shapes: 0.49 -> 0.31 ms per token at short contexts (0.34 at 400 keys; 0.315 and 0.40 with an f32 cache), of
-// which about 0.13 are the CTA's own arithmetic and latencies, 0.03 lm_head beyond what its first slots hide, and the rest
-// hand-overs.
+// Measured on the 0.5B shapes: 0.26 ms per token at short contexts, 0.295 at 500 keys (one kernel per operation: 0.49). HBM's 0.07 is
+// hidden; a layer is 8.6 us of hand-overs (4 x 0.8 us and attention's) and of each CTA's own chain between them: staging, products,
+// sums over warps, barriers.
 //
-// Arithmetic. A CTA owns whole output columns in tiles of 8. One m16n8k16 MMA multiplies 256 weights: rows 0-7 of the weight
-// operand are half of the positions of a tile's 8 columns, rows 8-15 the other half, and the activation operand holds the first
-// half in columns 0 (fp16 value) and 1 (fp16 remainder) and the second in columns 2 and 3, so f32 activations keep
-// ~22 bits as in the int4 GEMV; weights are exact integers q - z, f32 accumulation, one f32 scale per 128-row group.
+// Arithmetic. A CTA owns whole output columns in tiles of 8. Weights are exact integers q with a scale and a zero point per group of 128
+// rows; the f32 activations of a group become 30-bit integers of one power-of-two scale, cut into four signed bytes, and one int8
+// m16n8k32 MMA multiplies 512 weights with all four bytes exactly: two instructions a unit of 8 columns x 128 rows. (With fp16
+// value and remainder, 22 bits, it was four of m16n8k16, 8 cycles each like the int8 one, and 20 instructions to put nibbles in place
+// where it is 8 now. Logits of two layers against 64 bits: 4e-6 to 1e-5 then, 3e-7 to 1e-6 now.)
 //
 // All CTAs have to be resident at once, hence the cooperative launch. Every poll is bounded in time; one that gives up sets
 // the context's status word and lets all later polls of its CTA through, so the kernel drains its copies and ends.
 #include <stdlib.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "qwen_internal.cuh"
 
@@ -37,9 +42,9 @@ namespace wb {
 namespace fd {
 
 constexpr int kThreads = 256, kWarps = 8;
-constexpr int kUnitBytes = 576;   // 8 columns x 128 rows: 512 of nibbles, then scale * 2^24 and scale * zero point of every column
+constexpr int kUnitBytes = 576;   // 8 columns x 128 rows: 512 of nibbles, then scale and scale * zero point of every column
 constexpr int kSplitMax = 8;      // CTAs that share the keys of one head
-constexpr int kPartWords = 66;    // one split's partial attention result: 64 sums, max, sum of weights
+constexpr int kPartWords = 72;    // one split's partial attention result: 64 sums, max, sum of weights (twice: a whole sector), and up to a sector's end
 constexpr int kLmRows = 32;       // lm_head rows per slot of the weight ring
 constexpr int kMaxC = 1024;       // hidden size: four values per thread, four 16-byte pieces of an lm_head row per lane
 constexpr int kMaxI = 8192;
@@ -48,9 +53,10 @@ constexpr int kStatusHandover = 41, kStatusRing = 42;
 
 typedef unsigned long long u64;
 
-// Shared memory: Head | ring of weight slots | planes [4][pitch] | red | attention floats | x [C] f32 | small words
+// Shared memory: Head | ring of weight slots | staged groups of C | staged groups of the MLP's activations, or the attention's V tiles |
+// red | attention floats | x [C] f32 | small words
 struct Smem {
-    int ring, planes, red, att, xs, sums, small, total;
+    int ring, act_c, act_i, red, att, xs, small, total;
 };
 struct Params {
     const char *blobs;      // [layer][cta] blocks of blob_stride bytes
@@ -87,8 +93,20 @@ __host__ __device__ inline int deal_count(const Deal &d, int cta, int n)
 __host__ __device__ inline int deal_tile(const Deal &d, int cta, int n, int i) { return (cta - d.off % n + n) % n + i * n; }
 __host__ __device__ inline Deal deal_qkv(int C, int KV) { return {(C + 2 * KV) / 8, 0}; }
 __host__ __device__ inline Deal deal_o(int C, int n) { return {C / 8, n - (C / 8) % n}; }
-__host__ __device__ inline Deal deal_gu(int I) { return {I / 8, 0}; }  // pairs of a gate and an up tile
 __host__ __device__ inline Deal deal_down(int C, int n) { return {C / 8, n - (C / 8) % n}; }
+// gate | up has tiles of four gate columns and the four up columns that go with them. Eight neighbouring tiles make a line (32 results,
+// 128 bytes), which one CTA computes and stores at once; lines that do not go round are dealt by tiles.
+struct DealLines {
+    int lines, loose;  // lines of a CTA; tiles that are dealt singly
+};
+__host__ __device__ inline DealLines deal_gu(int I, int n) { return {I / 32 / n, I / 32 % n * 8}; }
+__host__ __device__ inline int deal_count(const DealLines &d, int cta, int n) { return d.lines * 8 + (cta < d.loose ? (d.loose - cta + n - 1) / n : 0); }
+__host__ __device__ inline int deal_tile(const DealLines &d, int cta, int n, int i)
+{
+    return i < d.lines * 8 ? (cta + (i >> 3) * n) * 8 + (i & 7) : d.lines * n * 8 + cta + (i - d.lines * 8) * n;
+}
+// Where the hand-over word of a column lies: a tile's eight words, two sectors, have a 128-byte line of their own.
+__host__ __device__ inline int word_at(int column) { return (column >> 3) * 16 + (column & 7); }
 
 // ---------------------------------------------------------------------------------------------------- device helpers
 __device__ __forceinline__ uint32_t s32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -195,6 +213,7 @@ __device__ __forceinline__ float2 ll_get2(const u64 *p, uint32_t ep, Head *hd)
 // every step). Scaled by 2^-15 a value below 65536 leaves that bit clear and keeps all of its own bits; from there on the fp16 pair
 // that the reader stages is no number, and neither is it for the word that stands for all of those and for NaN.
 constexpr uint32_t kActParity = 1u << 30, kActTooLarge = kActParity - 1;
+constexpr float kActLimit = 65520.f;  // rounds to no fp16 number
 __device__ __forceinline__ void act_put(uint32_t *p, float v, uint32_t ep)
 {
     v *= 1.f / 32768.f;
@@ -221,43 +240,52 @@ __device__ __forceinline__ float warp_sum(float v)
     return v;
 }
 
-// ---- staging: f32 values -> the four planes of the activation operand ----
-// Plane 0/1: fp16 value / remainder of the positions 0, 1, 4, 5 of every 8, plane 2/3 of 2, 3, 6, 7. The weights' nibbles are laid
-// out to match (lay_out_kernel), so that four neighbouring values are four 32-bit stores. Inside a group of 128 positions the
-// 8-byte pieces (one per plane and packed row) are ordered by row % 4, then row / 4: what a lane needs for the four k-steps of a
-// unit is 32 bytes in a row.
-__host__ __device__ inline int plane_pitch(int K) { return K + 16; }  // bytes, K a multiple of 128: conflict-free 16-byte reads
+// ---- staging: f32 values -> signed bytes, group by group of 128 positions ----
+// A group's values become 30-bit integers of one scale, the power of two that puts the group's largest magnitude into [2^29, 2^30),
+// and these four signed bytes ("digits", base 256) each. A digit of four neighbouring positions is one word; the 32 words of a digit
+// are ordered as the MMA's lanes take them (half of the group, lane % 4, word), so that a lane reads its 16 bytes of a group at
+// once: [half][digit][lane % 4][4 words]. Between the halves stand the scale taken back and the sum of the values.
+constexpr int kGroupBytes = 576, kHalfAt = 320, kScaleAt = 256;  // (an offset of 320: the halves' stores hit different banks)
 __device__ __forceinline__ uint32_t half2_bits(__half2 h) { return *reinterpret_cast<const uint32_t *>(&h); }
-__device__ __forceinline__ void stage4(char *planes, int pitch, int k, float4 v)  // positions k (a multiple of 4) to k + 3
+__device__ __forceinline__ uint32_t abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+// The four bytes of an integer below 2^31 - 2^23 in balanced base 256: byte i holds the digit i.
+__device__ __forceinline__ uint32_t digits(float v)
 {
-    char *at = planes + (k & ~127) + ((k & 24) << 2) + ((k & 96) >> 2) + (k & 4);
-    const __half2 e = __floats2half2_rn(v.x, v.y), o = __floats2half2_rn(v.z, v.w);
-    const float2 fe = __half22float2(e), fo = __half22float2(o);
-    *reinterpret_cast<uint32_t *>(at) = half2_bits(e);
-    *reinterpret_cast<uint32_t *>(at + pitch) = half2_bits(__floats2half2_rn(v.x - fe.x, v.y - fe.y));
-    *reinterpret_cast<uint32_t *>(at + 2 * pitch) = half2_bits(o);
-    *reinterpret_cast<uint32_t *>(at + 3 * pitch) = half2_bits(__floats2half2_rn(v.z - fo.x, v.w - fo.y));
+    constexpr uint32_t kCarry = 0x00808080u;
+    return ((uint32_t)__float2int_rn(v) + kCarry) ^ kCarry;
+}
+// One warp, one group: positions 4 lane to 4 lane + 3. A magnitude of `limit` or more makes the whole group NaN.
+__device__ __forceinline__ void stage_group(char *group, float4 v, int lane, float limit = INFINITY)
+{
+    const uint32_t top = __reduce_max_sync(0xffffffffu, max(max(abs_bits(v.x), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w))));
+    const uint32_t e = (uint32_t)min(283 - (int)(top >> 23), 253);  // biased exponent; the scale and its inverse are normal numbers
+    const float up = __uint_as_float(e << 23);
+    const uint32_t a = digits(v.x * up), b = digits(v.y * up), c = digits(v.z * up), d = digits(v.w * up);
+    const uint32_t ab = __byte_perm(a, b, 0x5140), cd = __byte_perm(c, d, 0x5140), AB = __byte_perm(a, b, 0x7362), CD = __byte_perm(c, d, 0x7362);
+    uint32_t *at = reinterpret_cast<uint32_t *>(group + (lane >> 4) * kHalfAt + (lane & 3) * 16 + ((lane >> 2) & 3) * 4);
+    at[0] = __byte_perm(ab, cd, 0x5410), at[16] = __byte_perm(ab, cd, 0x7632);
+    at[32] = __byte_perm(AB, CD, 0x5410), at[48] = __byte_perm(AB, CD, 0x7632);
+    if (lane == 0) *reinterpret_cast<float *>(group + kScaleAt) = top >= __float_as_uint(limit) ? __uint_as_float(0x7fffffffu) : __uint_as_float((254 - e) << 23);
 }
 
-// A nibble masked in place is the fp16 subnormal q * 2^-24 (or 16 q * 2^-24), which the MMA multiplies exactly; the zero point
-// comes off through the group's activation sum (as in gemv_core.cuh).
-__device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b)
+// One m16n8k32 MMA takes 512 weights: rows 0 to 7 of its weight operand are the 8 columns of a tile with the first half of the
+// group's positions, rows 8 to 15 the same columns with the second half, times 16 as their nibbles lie; the columns of the
+// activation operand are the four digits of the first half, then of the second. Integers: every product and sum is exact. Lane
+// (c, t) of the result uses two of its four sums: digits 2 (t % 2) and the next one of half t / 2, and the four lanes of a column
+// add up to the dot product. The zero point comes off through the group's sum.
+__device__ __forceinline__ void mma8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
 {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y));
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void mma_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b)
+__device__ __forceinline__ void mma8_first(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
 {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y), "f"(0.f));
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
-// Units are worked on B at a time without a branch between them, so that their chains (load, mask, four MMAs, one shuffle)
-// overlap: five units of a warp take 500 cycles together, and 1340 with a condition around each. Results of units that are not
-// there are computed from whatever lies behind and not stored. Five is what divides the long projections of the 0.5B model
-// (ten tiles of gate|up and five groups of down per warp).
-constexpr int kBurst = 5;
+constexpr int kBurst = 5;  // units of a warp that are worked on side by side, without a branch between them (down: five groups per warp in the 0.5B model)
 struct Unit {  // weights in registers, requested before the activations are there
     uint4 q;
     float2 s;
@@ -267,42 +295,42 @@ struct Unit {  // weights in registers, requested before the activations are the
         s = *reinterpret_cast<const float2 *>(ub + 512 + (lane >> 2) * 8);
     }
 };
-// This lane's part of a group's staged activations: the four k-steps of its plane.
-struct Acts {
-    uint2 b[4];
-    // (lanes 16 to 31 hold columns of the product that nobody reads)
-    __device__ __forceinline__ void load(const char *xu)
+// What a lane knows about its two digits.
+struct Lane {
+    int at;            // its bytes of a staged group
+    bool second;       // half of the positions
+    float digit, fac;  // 1 or 2^16; the same, with the second half's 16 taken back
+    __device__ __forceinline__ explicit Lane(int lane)
+        : at(lane * 16 + (lane >> 4) * (kHalfAt - 256)), second(lane & 2), digit((lane & 1) ? 65536.f : 1.f), fac((lane & 2) ? digit * 0.0625f : digit)
     {
-        const uint4 p = *reinterpret_cast<const uint4 *>(xu), q = *reinterpret_cast<const uint4 *>(xu + 16);
-        b[0] = make_uint2(p.x, p.y), b[1] = make_uint2(p.z, p.w), b[2] = make_uint2(q.x, q.y), b[3] = make_uint2(q.z, q.w);
     }
-    // Sum of the positions whose products this lane holds (lane % 4 = 0: the first half, 1: the second), by the same instruction
-    // with a weight operand of ones: no reduction over the warp that staged them.
-    __device__ __forceinline__ float sum() const
-    {
-        constexpr uint32_t kOnes = 0x3c003c00u;
-        float d[4];
-        mma_first(d, kOnes, kOnes, kOnes, kOnes, b[0]);
-#pragma unroll
-        for (int i = 1; i < 4; i++) mma(d, kOnes, kOnes, kOnes, kOnes, b[i]);
-        return d[0] + d[1];
-    }
+    __device__ __forceinline__ float value(const int (&d)[4]) const { return (float)((second ? d[3] : d[1]) * 256 + (second ? d[2] : d[0])); }
 };
-// Product of the two before the halves are added: lanes 4c and 4c + 1 hold column c's.
-__device__ __forceinline__ float unit_half(const Unit &u, const Acts &x, float sum, int lane)
+__device__ __forceinline__ void unit_dot(int (&d)[4], const uint4 &q, const uint4 &b)
 {
-    const uint32_t qv[4] = {u.q.x, u.q.y, u.q.z, u.q.w};
-    float d[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const uint32_t w8 = qv[i] >> 8;
-        if (i == 0) mma_first(d, qv[i] & 0x000f000fu, qv[i] & 0x00f000f0u, w8 & 0x000f000fu, w8 & 0x00f000f0u, x.b[i]);
-        else mma(d, qv[i] & 0x000f000fu, qv[i] & 0x00f000f0u, w8 & 0x000f000fu, w8 & 0x00f000f0u, x.b[i]);
-    }
-    const float v = (lane & 1) == 0 ? d[0] + d[1] : (d[2] + d[3]) * 0.0625f;
-    return fmaf(u.s.x, v, -u.s.y * sum);
+    constexpr uint32_t kLow = 0x0f0f0f0fu, kHigh = 0xf0f0f0f0u;
+    mma8_first(d, q.x & kLow, q.x & kHigh, q.y & kLow, q.y & kHigh, b.x, b.y);
+    mma8(d, q.z & kLow, q.z & kHigh, q.w & kLow, q.w & kHigh, b.z, b.w);
 }
-__device__ __forceinline__ float halves(float v) { return v + __shfl_xor_sync(0xffffffffu, v, 1); }
+// Sums of the digits, by the same instruction with a weight operand of ones.
+__device__ __forceinline__ void digit_sums(int (&d)[4], const uint4 &b)
+{
+    constexpr uint32_t kOnes = 0x01010101u;
+    mma8_first(d, kOnes, kOnes, kOnes, kOnes, b.x, b.y);
+    mma8(d, kOnes, kOnes, kOnes, kOnes, b.z, b.w);
+}
+__device__ __forceinline__ float quad_sum(float a)  // over the four lanes of a column
+{
+    a += __shfl_xor_sync(0xffffffffu, a, 1);
+    return a + __shfl_xor_sync(0xffffffffu, a, 2);
+}
+// fp16 MMA of the attention.
+__device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y));
+}
 
 // ---------------------------------------------------------------------------------------------------- attention
 // One CTA per (head, split of the keys), 16 keys per warp and pass. A lane takes 16 consecutive dims of two keys (K rows as they lie
@@ -533,7 +561,7 @@ struct Attend {
         rows.load_v(tile, vbase + (size_t)first * ld, ld, nk_mem - first, lane);
     }
     // one: the only split of its head: the result is final
-    __device__ __forceinline__ void run(const KV *kbase, const KV *vbase, int ld, int nk, bool own_new, float *sm, char *tile, u64 *out, bool one,
+    __device__ __forceinline__ void run(const KV *kbase, const KV *vbase, int ld, int nk, bool own_new, float *sm, char *tile, u64 *out, int copy, bool one,
                                         uint32_t ep, int warp, int lane)
     {
         float *wm = sm + kAttMax, *wl = wm + kWarps, *wa = wl + kWarps;
@@ -578,37 +606,32 @@ struct Attend {
             if (warp < 2) {
 #pragma unroll
                 for (int i = 0; i < kWarps; i++) r = fmaf(wa[i * 64 + warp * 32 + lane], __shfl_sync(0xffffffffu, ew, i), r);
-                ll_put(out + warp * 32 + lane, one ? r / den : r, ep);
-            } else if (lane < 2) {
-                ll_put(out + 64 + lane, lane == 0 ? M : den, ep);
+                if (one) r /= den;
+                ll_put(out + warp * 32 + lane, r, ep), ll_put(out + copy + warp * 32 + lane, r, ep);
+            } else if (lane < 4) {
+                const float v = lane & 1 ? den : M;
+                ll_put(out + 64 + lane, v, ep), ll_put(out + copy + 64 + lane, v, ep);
             }
         }
     }
 };
 
 // ---------------------------------------------------------------------------------------------------- the kernel
-inline Smem smem_layout(int slots, int slot_bytes, int C, int I, int red_units)
+inline Smem smem_layout(int slots, int slot_bytes, int C, int I, int KV, int n)
 {
     Smem s;
-    // (the V tiles of the attention lie behind the planes of C)
-    const int planes = 4 * plane_pitch(padded(I)), tiles = 4 * plane_pitch(C) + kWarps * 2048;
+    const int G = C / 128, most = ((C + 2 * KV) / 8 + n - 1) / n, most_c = (C / 8 + n - 1) / n;  // tiles of a CTA
+    const int staged = padded(I) / 128 * kGroupBytes, tiles = kWarps * 2048, r1 = (most > most_c ? most : most_c) * G, r2 = most_c * kWarps, r3 = kWarps + (deal_count(deal_gu(I, n), 0, n) + 3) / 4;
+    const int r12 = r1 > r2 ? r1 : r2;
     s.ring = 128;
-    s.planes = s.ring + slots * slot_bytes;
-    s.red = s.planes + (planes > tiles ? planes : tiles);
-    s.att = s.red + red_units * 32;
+    s.act_c = s.ring + slots * slot_bytes;
+    s.act_i = s.act_c + (G * kGroupBytes + 127) / 128 * 128;
+    s.red = s.act_i + (staged > tiles ? staged : tiles);
+    s.att = s.red + (r12 > r3 ? r12 : r3) * 128;
     s.xs = s.att + kAttFloats * 4;
-    s.sums = s.xs + C * 4;
-    s.small = s.sums + (padded(I) / 128 * 4 + 15) / 16 * 16;
+    s.small = s.xs + C * 4;
     s.total = s.small + 2 * kWarps * 4;
     return s;
-}
-inline int max_units(int C, int I, int KV, int n)
-{
-    const int G = C / 128, GI = I / 128;
-    const int a = (((C + 2 * KV) / 8 + n - 1) / n) * G, b = ((C / 8 + n - 1) / n) * G;
-    const int c = ((I / 8 + n - 1) / n) * 2 * G, d = ((C / 8 + n - 1) / n) * GI;
-    const int m1 = a > b ? a : b, m2 = c > d ? c : d;
-    return m1 > m2 ? m1 : m2;
 }
 
 template <typename KV>
@@ -617,14 +640,15 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     extern __shared__ __align__(128) char smem[];
     const int cta = blockIdx.x, n = gridDim.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int C = p.C, I = p.I, KVd = p.KV, QKV = C + 2 * KVd, G = C / 128, GI = I / 128, L = p.n_layer;
-    const Deal dq = deal_qkv(C, KVd), dow = deal_o(C, n), dg = deal_gu(I), dd = deal_down(C, n);
+    const Deal dq = deal_qkv(C, KVd), dow = deal_o(C, n), dd = deal_down(C, n);
+    const DealLines dg = deal_gu(I, n);
     const int nq = deal_count(dq, cta, n), no = deal_count(dow, cta, n), ng = deal_count(dg, cta, n), nd = deal_count(dd, cta, n);
-    const int fq = deal_tile(dq, cta, n, 0), fo = deal_tile(dow, cta, n, 0), fg = deal_tile(dg, cta, n, 0), fdn = deal_tile(dd, cta, n, 0);
-    const int uq = nq * G, uo = no * G, ug = ng * 2 * G, ud = nd * GI;
+    const int fq = deal_tile(dq, cta, n, 0), fo = deal_tile(dow, cta, n, 0), fdn = deal_tile(dd, cta, n, 0);
+    const int uq = nq * G, uo = no * G, ug = ng * G, ud = nd * GI;
     const Smem &so = p.sm;
-    char *planes = smem + so.planes;
+    char *act_c = smem + so.act_c, *act_i = smem + so.act_i;
     float *red = reinterpret_cast<float *>(smem + so.red), *att = reinterpret_cast<float *>(smem + so.att);
-    float *xs = reinterpret_cast<float *>(smem + so.xs), *sums = reinterpret_cast<float *>(smem + so.sums);
+    float *xs = reinterpret_cast<float *>(smem + so.xs);
     float *ssq = reinterpret_cast<float *>(smem + so.small);  // [16]
     int *widx = reinterpret_cast<int *>(ssq + kWarps);        // [16]
     Head *hd = reinterpret_cast<Head *>(smem);
@@ -643,11 +667,13 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     __syncthreads();
 
     // The ring of weight slots: the fills of a step are its layers' blocks, then the lm_head rows, and the next step's follow.
-    // One thread of the last warp (the one with the least other work) refills a slot as soon as a barrier has told it that every
-    // warp is done with it.
+    // One thread of the last warp (the one with the least other work) refills a slot after a barrier has told it that every warp is
+    // done with it: the first half while attention runs, the second under gate | up. All CTAs do so at about the same time, and the
+    // 9 MB of a layer take 1.4 us in which a hand-over takes twice as long (refilled at the end of the layer, in front of the hand-over
+    // of down, a step took 295 us at 8 keys and 349 at 500; under gate | up 278 and 328, in halves 272 and 328).
     const bool feeder = tid == kThreads - 32;
     const uint32_t block_bytes = (uint32_t)(uq + uo + ug + ud) * kUnitBytes;
-    auto fill = [&]() {
+    auto fill = [&](int halves = 3) {  // bit 0: the first half, bit 1: the second, and the fill is done
         if (hd->fill_left == 0 || hd->ring_lost) return;
         const int i = hd->fill_i, at = hd->fill_slot;
         const char *src;
@@ -658,8 +684,10 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
             const int r = row0 + (i - L) * kLmRows;
             src = reinterpret_cast<const char *>(p.embed + (size_t)r * C), bytes = (uint32_t)min(kLmRows, row1 - r) * C * 2;
         }
-        mbar_expect(&full[at], bytes);
-        if (bytes) bulk_load(ring + at * p.slot_bytes, src, bytes, &full[at]);
+        const uint32_t cut = bytes / 32 * 16, first = halves & 1 ? 0u : cut, end = halves & 2 ? bytes : cut;
+        if (halves & 1) mbar_expect(&full[at], bytes);
+        if (end > first) bulk_load(ring + at * p.slot_bytes + first, src + first, end - first, &full[at]);
+        if (!(halves & 2)) return;
         hd->fills++;
         hd->fill_slot = at + 1 == p.slots ? 0 : at + 1;
         if (i + 1 == L + lm_fills) hd->fill_i = 0, hd->fill_left--;
@@ -675,93 +703,126 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     };
 
     const int H = p.H, hpk = H / p.KVH;
-    const int pitch_c = plane_pitch(C), pitch_i = plane_pitch(padded(I)), c4 = 4 * tid;
+    const int c4 = 4 * tid;
     const bool has4 = c4 < C;
     const float inv_c = 1.f / (float)C;
-    const int w_o = QKV, w_act = w_o + C, w_down = w_act + I / 2, w_att = w_down + C;  // words of a layer; q | k | v first
+    const int w_o = 2 * QKV, w_act = w_o + 2 * C, w_down = w_act + I / 2 + 2 * dg.loose, w_att = w_down + 2 * C;  // words of a layer; q | k | v first
+    const int att_words = H * kSplitMax * kPartWords;
     u64 *const ll = p.ll, *const cand = ll + p.ll_layer;
     uint32_t *const act = reinterpret_cast<uint32_t *>(ll + w_act);
+    const int first_loose = dg.lines * n * 32;
+    auto act_at = [&](int k) { return k < first_loose ? k : 2 * k - first_loose; };  // a loose tile's four words have a sector for themselves
     uint32_t token = p.first_token;
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);  // this thread's part of the residual stream
     // Projections from C: a warp stays with one group of 128 rows (its activations are loaded once) and takes the CTA's tiles in
     // turn; where there are fewer groups than half the warps, several warps share a group's tiles.
     const int wpg = kWarps / G, grp = warp % G, sub = warp / G;
     const int t_first = sub < wpg ? sub : 1 << 16;  // (no tiles for the warps that are left over)
-    const char *xp_c = planes + ((lane >> 2) & 3) * pitch_c + (lane & 3) * 32 + grp * 128, *xp_i = planes + ((lane >> 2) & 3) * pitch_i + (lane & 3) * 32;
-    const int part = lane & 3, red_at = part * 8 + (lane >> 2);
-    float *red_c = red + grp * 8 + (lane >> 2), *red_i = red + (lane >> 2);
-    char *tile = planes + 4 * pitch_c + warp * 2048;
+    const Lane ln(lane);
+    const int part = lane & 3;
+    char *tile = act_i + warp * 2048;
 
-    // rmsnorm of the residual stream (rmsNormRef, src/reference/qwen-ref.ts:12-29)
-    auto norm = [&](float4 w) {
-        const float ss = warp_sum(fmaf(x.x, x.x, x.y * x.y) + fmaf(x.z, x.z, x.w * x.w));
-        if (lane == 0) ssq[warp] = ss;
-        __syncthreads();
+    // rmsnorm of the residual stream (rmsNormRef, src/reference/qwen-ref.ts:12-29). A projection takes x * weight as it is, and its
+    // results are multiplied by the reciprocal root mean square: it is known behind the same barrier as the staged values.
+    auto inv_rms = [&]() {
         const float4 a = reinterpret_cast<const float4 *>(ssq)[0], b = reinterpret_cast<const float4 *>(ssq)[1];
-        const float rstd = rsqrtf((((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) * inv_c + p.eps);
-        return make_float4(x.x * rstd * w.x, x.y * rstd * w.y, x.z * rstd * w.z, x.w * rstd * w.w);
+        return rsqrtf((((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) * inv_c + p.eps);
+    };
+    auto squares = [&]() { return fmaf(x.x, x.x, x.y * x.y) + fmaf(x.z, x.z, x.w * x.w); };
+    auto norm_stage = [&](float4 w) {
+        const float4 y = make_float4(x.x * w.x, x.y * w.y, x.z * w.z, x.w * w.w);
+        if (has4) stage_group(act_c + warp * kGroupBytes, y, lane);
+        float ss = squares(), sum = (y.x + y.y) + (y.z + y.w);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o), sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) {
+            ssq[warp] = ss;
+            if (has4) *reinterpret_cast<float *>(act_c + warp * kGroupBytes + kScaleAt + 4) = sum;
+        }
+        __syncthreads();
     };
     auto load4 = [&](const float *a) { return has4 ? __ldg(reinterpret_cast<const float4 *>(a) + tid) : make_float4(0.f, 0.f, 0.f, 0.f); };
     auto add_residual = [&](const u64 *a, uint32_t ep) {
         if (!has4) return;
         ulonglong2 v[2];
-        ll_get(v, a + c4, 2, ep, hd);
+        ll_get(v, a + word_at(c4), 2, ep, hd);
         const float2 f = ll_vals(v[0]), g = ll_vals(v[1]);
         x.x += f.x, x.y += f.y, x.z += g.x, x.w += g.y;
     };
-    Unit u[kBurst];
-    const int tile_step = wpg * G * kUnitBytes;
-    auto load_tiles = [&](const char *w, int i) {  // this warp's tiles from i on (the block's end is not the ring's: no bounds)
-        w += (i * G + grp) * kUnitBytes;
-#pragma unroll
-        for (int j = 0; j < kBurst; j++) u[j].load(w + j * tile_step, lane);
-    };
+    // q | k | v and o: a CTA has few tiles; a warp takes one group of 128 rows of each, the sums over the groups go through shared memory.
+    Unit u[8];
     auto load_one = [&](const char *w) { u[0].load(w + (t_first * G + grp) * kUnitBytes, lane); };
-    auto run_tiles = [&](const char *w, int tiles) {  // from load_tiles
-        Acts xa;
-        xa.load(xp_c);
-        const float sum = xa.sum();
-#pragma unroll 1
-        for (int i = t_first; i < tiles; i += kBurst * wpg) {
-            float v[kBurst];
-#pragma unroll
-            for (int j = 0; j < kBurst; j++) v[j] = unit_half(u[j], xa, sum, lane);
-            if (i + kBurst * wpg < tiles) load_tiles(w, i + kBurst * wpg);
-#pragma unroll
-            for (int j = 0; j < kBurst; j++) v[j] = halves(v[j]);
-#pragma unroll
-            for (int j = 0; j < kBurst; j++)
-                if (part == 0 && i + j * wpg < tiles) red_c[(i + j * wpg) * G * 8] = v[j];
-        }
-    };
-    auto run_short = [&](const char *w, int tiles) {  // a projection of few tiles per CTA, from load_one
-        Acts xa;
-        xa.load(xp_c);
-        const float sum = xa.sum();
+    auto run_short = [&](const char *w, int tiles) {  // from load_one
+        const char *group = act_c + grp * kGroupBytes;
+        const uint4 b = *reinterpret_cast<const uint4 *>(group + ln.at);
+        const float scale = *reinterpret_cast<const float *>(group + kScaleAt), gx = scale * ln.fac;
+        int ds[4];
+        digit_sums(ds, b);
+        const float sum = ln.value(ds) * (scale * ln.digit);
 #pragma unroll 1
         for (int i = t_first; i < tiles; i += wpg) {
             if (i > t_first) u[0].load(w + (i * G + grp) * kUnitBytes, lane);
-            const float v = halves(unit_half(u[0], xa, sum, lane));
-            if (part == 0) red_c[i * G * 8] = v;
+            int d[4];
+            unit_dot(d, u[0].q, b);
+            red[(i * G + grp) * 32 + lane] = fmaf(u[0].s.x, ln.value(d) * gx, -u[0].s.y * sum);
         }
     };
-    // sum over the groups of one tile: four lanes per column; r: the tile's results
-    auto column_sum_c = [&](const float *r) {  // up to 8 groups (C <= 1024)
-        float a = part < G ? r[red_at] : 0.f;
-        if (part + 4 < G) a += r[red_at + 32];
-        a += __shfl_xor_sync(0xffffffffu, a, 1);
-        return a + __shfl_xor_sync(0xffffffffu, a, 2);
+    auto column_sum = [&](int first, int n_sums) {  // of up to 8 rows of red
+        float a[2] = {};
+#pragma unroll
+        for (int g = 0; g < 8; g++)
+            if (g < n_sums) a[g & 1] += red[(first + g) * 32 + lane];
+        return quad_sum(a[0] + a[1]);
     };
-    auto column_sum_i = [&](const float *r) {
-        float a = 0.f, b = 0.f;
-        r += red_at;
-        int g = part;
-#pragma unroll 2
-        for (; g + 4 < GI; g += 8, r += 64) a += r[0], b += r[32];
-        if (g < GI) a += r[0];
-        a += b;
-        a += __shfl_xor_sync(0xffffffffu, a, 1);
-        return a + __shfl_xor_sync(0xffffffffu, a, 2);
+    // gate | up: a warp takes whole tiles, all groups of them (the activations of all groups lie in registers). Loose tiles, if they are
+    // no more than a unit per warp, are dealt by units and added up through shared memory: 32 CTAs of the 0.5B model have a ninth
+    // tile, and for a warp that took it alone everybody waited 0.8 us.
+    const int loose = ng - dg.lines * 8, spread = loose * G <= kWarps ? loose : 0, whole = ng - spread;
+    const int my_extra = warp < spread * G ? warp : 0;
+    auto load_tile = [&](const char *w) {
+#pragma unroll
+        for (int g = 0; g < 8; g++) u[g].load(w + min(g, G - 1) * kUnitBytes, lane);
+    };
+    float *line = red + kWarps * 32;
+    auto run_tiles = [&](const char *w) {  // from load_tile
+        uint4 b[8];
+        float gx[8], sum[8];
+#pragma unroll
+        for (int g = 0; g < 8; g++) {  // (groups that are not there: the last one's, times 0)
+            const char *group = act_c + min(g, G - 1) * kGroupBytes;
+            b[g] = *reinterpret_cast<const uint4 *>(group + ln.at);
+            const float2 s2 = *reinterpret_cast<const float2 *>(group + kScaleAt);
+            gx[g] = g < G ? s2.x * ln.fac : 0.f, sum[g] = g < G && part == 0 ? s2.y : 0.f;
+        }
+        if (spread) {
+            Unit e;
+            e.load(w + (whole * G + my_extra) * kUnitBytes, lane);
+            const char *group = act_c + my_extra % G * kGroupBytes;
+            const float2 s2 = *reinterpret_cast<const float2 *>(group + kScaleAt);
+            int d[4];
+            unit_dot(d, e.q, *reinterpret_cast<const uint4 *>(group + ln.at));
+            red[warp * 32 + lane] = fmaf(e.s.x, ln.value(d) * (s2.x * ln.fac), part == 0 ? -e.s.y * s2.y : 0.f);
+        }
+#pragma unroll 1
+        for (int i = warp; i < whole; i += kWarps) {
+            if (i > warp) load_tile(w + i * G * kUnitBytes);
+            float a[2] = {};
+            auto four = [&](auto first) {
+                constexpr int g0 = decltype(first)::value;
+                int d[4][4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) unit_dot(d[j], u[g0 + j].q, b[g0 + j]);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    a[0] = fmaf(u[g0 + j].s.x, ln.value(d[j]) * gx[g0 + j], a[0]);
+                    a[1] = fmaf(u[g0 + j].s.y, sum[g0 + j], a[1]);
+                }
+            };
+            four(std::integral_constant<int, 0>());
+            if (G > 4) four(std::integral_constant<int, 4>());
+            const float r = quad_sum(a[0] - a[1]);
+            if (part == 0) line[i * 8 + (lane >> 2)] = r;
+        }
     };
 
     if (feeder) ring_wait(hd, 0, 0);
@@ -801,23 +862,23 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
             const KV *vc = reinterpret_cast<const KV *>(p.v_cache + (size_t)l * p.kv_layer_bytes) + (size_t)k0 * KVd + kvh * 64;
             if (is_att) at.load(kc, vc, KVd, warp * 16, own_new ? nk - 1 : nk, tile, lane);
             if (l > 0) add_residual(ll + w_down, ep - 1);
-            float4 y = norm(nw);
-            if (has4) stage4(planes, pitch_c, c4, y);
-            __syncthreads();
+            norm_stage(nw);
+            float rstd = inv_rms();
             run_short(wb, nq);
             wb += uq * kUnitBytes;
             if (nq > 0) __syncthreads();
             if (warp < nq) {
-                const float a = column_sum_c(red + warp * G * 8) + bias;
-                if (part == 0) ll_put(ll + (fq + warp * n) * 8 + (lane >> 2), a, ep);
+                const float a = fmaf(column_sum(warp * G, G), rstd, bias);
+                if (part == 0) ll_put(ll + word_at((fq + warp * n) * 8 + (lane >> 2)), a, ep);
             }
+            if (feeder && l > 0) fill(1);
 
             // -- attention: rotary embedding of q and the new k (ropeHalfRef, src/reference/qwen-ref.ts:35-64), cache append
             if (is_att) {
                 if (warp < 3 && (warp == 0 || own_new)) {
                     // a lane reads the pair (2i, 2i + 1), the rotation needs (i, i + 32)
                     const float2 cs = __ldg(reinterpret_cast<const float2 *>(p.cs_table) + (size_t)pos * 32 + lane);
-                    const float2 a = ll_get2(ll + (warp == 0 ? h * 64 : warp == 1 ? C + kvh * 64 : C + KVd + kvh * 64) + 2 * lane, ep ^ p.miss, hd);
+                    const float2 a = ll_get2(ll + word_at((warp == 0 ? h * 64 : warp == 1 ? C + kvh * 64 : C + KVd + kvh * 64) + 2 * lane), ep ^ p.miss, hd);
                     float *dst = att + (warp == 0 ? kAttQ : warp * 64 - 64);
                     *reinterpret_cast<float2 *>(dst + 2 * lane) = a;
                     __syncwarp();
@@ -840,14 +901,14 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
                     }
                 }
                 __syncthreads();
-                at.run(kc, vc, KVd, nk, own_new, att, tile, ll + w_att + (h * S + sp) * kPartWords, S == 1, ep, warp, lane);
+                at.run(kc, vc, KVd, nk, own_new, att, tile, ll + w_att + (h * S + sp) * kPartWords, att_words, S == 1, ep, warp, lane);
             }
 
             // -- o: merge the splits of every head while staging
             if (no > 0) {
                 if (sub < wpg) load_one(wb);
                 if (has4) {
-                    const u64 *src = ll + w_att + (c4 >> 6) * S * kPartWords, *mine = src + (c4 & 63);
+                    const u64 *src = ll + w_att + (cta & 1) * att_words + (c4 >> 6) * S * kPartWords, *mine = src + (c4 & 63);
                     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (S == 1) {
                         ulonglong2 w[2];
@@ -902,37 +963,46 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
                         const float inv = 1.f / den;
                         a.x *= inv, a.y *= inv, a.z *= inv, a.w *= inv;
                     }
-                    stage4(planes, pitch_c, c4, a);
+                    stage_group(act_c + warp * kGroupBytes, a, lane);
                 }
                 __syncthreads();
                 run_short(wb, no);
                 wb += uo * kUnitBytes;
                 __syncthreads();
                 if (warp < no) {
-                    const float a = column_sum_c(red + warp * G * 8);
-                    if (part == 0) ll_put(ll + w_o + (fo + warp * n) * 8 + (lane >> 2), a, ep);
+                    const float a = column_sum(warp * G, G);
+                    if (part == 0) ll_put(ll + w_o + word_at((fo + warp * n) * 8 + (lane >> 2)), a, ep);
                 }
             }
 
             // -- gate | up, silu * up
-            if (sub < wpg) load_tiles(wb, t_first);
+            load_tile(wb + min(warp, ng - 1) * G * kUnitBytes);
             nw = load4(aux + C);
             add_residual(ll + w_o, ep);
-            y = norm(nw);
-            if (has4) stage4(planes, pitch_c, c4, y);
+            norm_stage(nw);
+            rstd = inv_rms();
+            if (feeder && l > 0) fill(2);
+            run_tiles(wb);
             __syncthreads();
-            run_tiles(wb, 2 * ng);
+            auto silu_up = [&](float gate, float up) { return gate / (1.f + expf(-gate)) * up; };
+            auto loose_word = [&](int i) { return act + act_at(deal_tile(dg, cta, n, i) * 4) + part * 4 + (lane >> 2); };  // (a sector, both halves)
+#pragma unroll 1
+            for (int i = warp; i < dg.lines; i += kWarps) {
+                const float *r = line + i * 64 + (lane >> 2) * 8 + (lane & 3);
+                act_put(act + (cta + i * n) * 32 + lane, silu_up(r[0] * rstd, r[4] * rstd), ep);
+            }
+            if (const int i = kWarps - 1 - warp; i < spread) {
+                const float a = column_sum(i * G, G) * rstd, up = __shfl_xor_sync(0xffffffffu, a, 16);
+                if (lane < 16 && part < 2) act_put(loose_word(whole + i), silu_up(a, up), ep);
+            }
+#pragma unroll 1
+            for (int i = dg.lines * 8 + warp; i < whole; i += kWarps)
+                if (lane < 16 && part < 2) act_put(loose_word(i), silu_up(line[i * 8 + (lane >> 2)] * rstd, line[i * 8 + 4 + (lane >> 2)] * rstd), ep);
             wb += ug * kUnitBytes;
             if (nd == 0) {
                 next_slot();
                 if (feeder && l + 1 < L) ring_wait(hd, slot, par);
-            }
-            __syncthreads();
-#pragma unroll 1
-            for (int i = warp; i < ng; i += kWarps) {
-                const float *r = red + i * 2 * G * 8;
-                const float gate = column_sum_c(r), up = column_sum_c(r + G * 8);
-                if (part == 0) act_put(act + (fg + i * n) * 8 + (lane >> 2), gate / (1.f + expf(-gate)) * up, ep);
+                __syncthreads();
             }
 
             // -- down
@@ -944,13 +1014,11 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
                 load_groups(wb);
 #pragma unroll 1
                 for (int k = c4; k < I; k += kBatch * 4 * kThreads) {
-                    // (fours beyond I are those at its end once more, staged behind everything that is used)
+                    // (beyond I zeros, staged behind everything that is used)
                     uint4 w[kBatch];
-                    const uint32_t *src[kBatch];
+                    const uint32_t none = ep & 1 ? kActParity : 0u;
 #pragma unroll
-                    for (int i = 0; i < kBatch; i++) src[i] = act + min(k + i * 4 * kThreads, I - 128 + 4 * lane);
-#pragma unroll
-                    for (int i = 0; i < kBatch; i++) w[i] = act_load4(src[i]);
+                    for (int i = 0; i < kBatch; i++) w[i] = k + i * 4 * kThreads < I ? act_load4(act + act_at(k + i * 4 * kThreads)) : make_uint4(none, none, none, none);
 #pragma unroll 1
                     for (uint32_t it = 1;; it++) {
                         bool ok = true;
@@ -959,62 +1027,56 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
                         if (ll_done(ok, it, hd)) break;
 #pragma unroll
                         for (int i = 0; i < kBatch; i++)
-                            if (!act_ok(w[i], ep)) w[i] = act_load4(src[i]);
+                            if (!act_ok(w[i], ep)) w[i] = act_load4(act + act_at(k + i * 4 * kThreads));
                     }
-                    // a warp's 128 values are one group: its sum, all of the batch's reductions side by side
-                    float g[kBatch];
+                    // a warp's 128 values are one group
 #pragma unroll
-                    for (int i = 0; i < kBatch; i++) {
-                        const float4 f = act_vals(w[i]);
-                        stage4(planes, pitch_i, k + i * 4 * kThreads, f);
-                        g[i] = (f.x + f.y) + (f.z + f.w);
-                    }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                        for (int i = 0; i < kBatch; i++) g[i] += __shfl_xor_sync(0xffffffffu, g[i], o);
-                    if (lane == 0)
-#pragma unroll
-                        for (int i = 0; i < kBatch; i++) sums[(k >> 7) + i * kWarps] = g[i];
+                    for (int i = 0; i < kBatch; i++) stage_group(act_i + ((k >> 7) + i * kWarps) * kGroupBytes, act_vals(w[i]), lane, kActLimit);
                 }
                 __syncthreads();
 #pragma unroll 1
                 for (int t = 0; t < nd; t++) {
+                    float a = 0.f;
 #pragma unroll 1
                     for (int i = warp; i < GI; i += kBurst * kWarps) {
                         if (t > 0 || i > warp) load_groups(wb + (t * GI + i - warp) * kUnitBytes);
-                        float v[kBurst];
-                        Acts xa[kBurst];
-#pragma unroll
-                        for (int j = 0; j < kBurst; j++) xa[j].load(xp_i + (i + j * kWarps) * 128);
+                        int d[kBurst][4], ds[kBurst][4];
+                        float scale[kBurst];
 #pragma unroll
                         for (int j = 0; j < kBurst; j++) {
-                            const float g = sums[i + j * kWarps];  // comes off once, in the lane of the first half
-                            v[j] = unit_half(u[j], xa[j], (lane & 1) == 0 ? g : 0.f, lane);
+                            const char *group = act_i + (i + j * kWarps) * kGroupBytes;
+                            const uint4 b = *reinterpret_cast<const uint4 *>(group + ln.at);
+                            scale[j] = *reinterpret_cast<const float *>(group + kScaleAt);
+                            unit_dot(d[j], u[j].q, b);
+                            digit_sums(ds[j], b);
                         }
 #pragma unroll
-                        for (int j = 0; j < kBurst; j++) v[j] = halves(v[j]);
-#pragma unroll
-                        for (int j = 0; j < kBurst; j++)
-                            if (part == 0 && i + j * kWarps < GI) red_i[(t * GI + i + j * kWarps) * 8] = v[j];
+                        for (int j = 0; j < kBurst; j++) {
+                            const float v = fmaf(u[j].s.x, ln.value(d[j]) * (scale[j] * ln.fac), -u[j].s.y * (ln.value(ds[j]) * (scale[j] * ln.digit)));
+                            if (i + j * kWarps < GI) a += v;
+                        }
                     }
+                    red[(t * kWarps + warp) * 32 + lane] = a;
                 }
                 next_slot();
                 if (feeder && l + 1 < L) ring_wait(hd, slot, par);
                 __syncthreads();
                 if (warp < nd) {
-                    const float a = column_sum_i(red + warp * GI * 8);
-                    if (part == 0) ll_put(ll + w_down + (fdn + warp * n) * 8 + (lane >> 2), a, ep);
+                    const float a = column_sum(warp * kWarps, kWarps);
+                    if (part == 0) ll_put(ll + w_down + word_at((fdn + warp * n) * 8 + (lane >> 2)), a, ep);
                 }
             }
-            if (feeder) fill();  // every warp is past the barrier behind its last unit
         }
+        if (feeder) fill();  // every warp is past the barrier behind its last unit
 
         // -- final norm, tied lm_head (f32 activations, fp16 rows), argmax
         const float4 w_final = load4(p.final_norm);
         add_residual(ll + w_down, --ep);  // the last layer's epoch is the step's
-        const float4 y = norm(w_final);
-        if (has4) *reinterpret_cast<float4 *>(xs + c4) = y;
+        const float ss = warp_sum(squares());
+        if (lane == 0) ssq[warp] = ss;
+        __syncthreads();
+        const float rstd = inv_rms();
+        if (has4) *reinterpret_cast<float4 *>(xs + c4) = make_float4(x.x * rstd * w_final.x, x.y * rstd * w_final.y, x.z * rstd * w_final.z, x.w * rstd * w_final.w);
         __syncthreads();
         const bool last = s + 1 == p.n_steps;
         float best = -INFINITY;
@@ -1082,7 +1144,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
         if (lane == 0) ssq[warp] = best, widx[warp] = best_i;
         __threadfence();  // the cache rows of this step, before the words that let other CTAs go on to the next
         __syncthreads();
-        u64 *cd = cand + (size_t)(s & 1) * 2 * n;  // two sets: a CTA may be a step ahead of one that still reads its candidates
+        u64 *cd = cand + (size_t)(s & 1) * 4 * n;  // two sets: a CTA may be a step ahead of one that still reads its candidates
         auto better = [&](float v, int i) {
             if (v > best || (v == best && i < best_i)) best = v, best_i = i;
         };
@@ -1090,13 +1152,13 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
             best = lane < kWarps ? ssq[lane] : -INFINITY, best_i = lane < kWarps ? widx[lane] : 0x7fffffff;
 #pragma unroll
             for (int o = kWarps / 2; o > 0; o >>= 1) better(__shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, best_i, o));
-            if (lane == 0) ll_put(cd + 2 * cta, best, ep), ll_put(cd + 2 * cta + 1, __int_as_float(best_i), ep);
+            if (lane < 4) ll_put(cd + 4 * cta + lane, lane & 1 ? __int_as_float(best_i) : best, ep);  // (twice: a whole sector)
         }
         __syncthreads();
         if (last && cta != 0) break;
         best = -INFINITY, best_i = 0x7fffffff;
         if (warp * 32 < n) {
-            const float2 c = ll_get2(cd + 2 * min(tid, n - 1), ep, hd);
+            const float2 c = ll_get2(cd + 4 * min(tid, n - 1), ep, hd);
             best = c.x, best_i = __float_as_int(c.y);
         }
 #pragma unroll
@@ -1129,45 +1191,46 @@ __global__ void __launch_bounds__(256) lay_out_kernel(const Source *__restrict__
                                                       int blob_stride)
 {
     const int QKV = C + 2 * KV, G = C / 128, GI = I / 128, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int uq = QKV / 8 * G, uo = C / 8 * G, ug = I / 8 * 2 * G, ud = C / 8 * GI;
+    const int uq = QKV / 8 * G, uo = C / 8 * G, ug = I / 4 * G, ud = C / 8 * GI;
     int u = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (u >= uq + uo + ug + ud) return;
     const Source &s = src[blockIdx.y];
-    int proj, N, groups, tile, group, col0, at;  // at: unit index inside the CTA's block
-    Deal d;
-    const Deal dq = deal_qkv(C, KV), dow = deal_o(C, n), dg = deal_gu(I), dd = deal_down(C, n);
+    int proj, N, groups, at;  // at: unit index inside the CTA's block
+    Deal d = {0, 0};
+    const Deal dq = deal_qkv(C, KV), dow = deal_o(C, n), dd = deal_down(C, n);
+    const DealLines dg = deal_gu(I, n);
     if (u < uq) proj = 0, N = QKV, groups = G, d = dq;
     else if ((u -= uq) < uo) proj = 1, N = C, groups = G, d = dow;
-    else if ((u -= uo) < ug) proj = 2, N = 2 * I, groups = G, d = dg;
+    else if ((u -= uo) < ug) proj = 2, N = 2 * I, groups = G;
     else u -= ug, proj = 3, N = C, groups = GI, d = dd;
-    group = u % groups, tile = u / groups;
-    int half = 0;
-    if (proj == 2) half = tile & 1, tile >>= 1;
-    col0 = half * I + tile * 8;
-    const int cta = (tile % n + d.off) % n, local = tile / n;
-    at = (proj == 2 ? local * 2 + half : local) * groups + group;
+    const int group = u % groups, tile = u / groups;
+    auto column = [&](int c) { return proj == 2 ? (c >> 2) * I + tile * 4 + (c & 3) : tile * 8 + c; };
+    int cta = (tile % n + d.off) % n, local = tile / n;
+    if (proj == 2) {
+        const int line = tile >> 3, single = tile - dg.lines * n * 8;
+        cta = single < 0 ? line % n : single % n, local = single < 0 ? line / n * 8 + (tile & 7) : dg.lines * 8 + single / n;
+    }
+    at = local * groups + group;
     if (proj > 0) at += deal_count(dq, cta, n) * G;
     if (proj > 1) at += deal_count(dow, cta, n) * G;
-    if (proj > 2) at += deal_count(dg, cta, n) * 2 * G;
+    if (proj > 2) at += deal_count(dg, cta, n) * G;
     char *out = blobs + ((size_t)blockIdx.y * n + cta) * blob_stride + (size_t)at * kUnitBytes;
-    // a word's nibbles in the order of stage4's planes: masks 0x000f000f, 0x00f000f0 (shifted by 0 and 8) pick the positions
-    // 0 1 | 2 3 and 4 5 | 6 7
-    auto order = [](uint32_t q) {
-        constexpr int kNibble[8] = {0, 2, 4, 6, 1, 3, 5, 7};  // position held by nibble i
-        uint32_t r = 0;
+    // Byte b of word m: the nibble of position 16 m + 4 t + b, and in its upper half that of the position 64 further on.
+    const uint32_t *q = s.qw[proj] + (size_t)(group * 16 + (t >> 1)) * N + column(g);
+    uint32_t w[4];
 #pragma unroll
-        for (int i = 0; i < 8; i++) r |= ((q >> (4 * kNibble[i])) & 15u) << (4 * i);
-        return r;
-    };
-    uint4 w;
-    const uint32_t *q = s.qw[proj] + (size_t)(group * 16 + t) * N + col0 + g;
-    w.x = order(q[0]), w.y = order(q[(size_t)4 * N]), w.z = order(q[(size_t)8 * N]), w.w = order(q[(size_t)12 * N]);
-    *reinterpret_cast<uint4 *>(out + lane * 16) = w;
+    for (int m = 0; m < 4; m++) {
+        const uint32_t lo = q[(size_t)(2 * m) * N] >> (16 * (t & 1)), hi = q[(size_t)(2 * m + 8) * N] >> (16 * (t & 1));
+        w[m] = 0;
+#pragma unroll
+        for (int b = 0; b < 4; b++) w[m] |= (((lo >> (4 * b)) & 15u) | (((hi >> (4 * b)) & 15u) << 4)) << (8 * b);
+    }
+    *reinterpret_cast<uint4 *>(out + lane * 16) = make_uint4(w[0], w[1], w[2], w[3]);
     if (lane < 8) {
-        const int c = col0 + lane;
+        const int c = column(lane);
         const uint32_t z = s.qz[proj] ? ((s.qz[proj][(size_t)group * ((N + 7) / 8) + (c >> 3)] >> ((c & 7) * 4)) & 15u) + 1u : 8u;
         const float sc = __half2float(s.sc[proj][(size_t)group * N + c]);
-        *reinterpret_cast<float2 *>(out + 512 + lane * 8) = make_float2(sc * 16777216.f, sc * (float)z);
+        *reinterpret_cast<float2 *>(out + 512 + lane * 8) = make_float2(sc, sc * (float)z);
     }
 }
 
@@ -1204,12 +1267,12 @@ static bool fused_shape(const wb_qwen *m, int n, int *blob, int *slot, int *slot
     int units = 0;
     for (int c = 0; c < n; c++)
         units = std::max(units, deal_count(deal_qkv(C, KV), c, n) * (C / 128) + deal_count(deal_o(C, n), c, n) * (C / 128) +
-                                    deal_count(deal_gu(I), c, n) * 2 * (C / 128) + deal_count(deal_down(C, n), c, n) * (I / 128));
+                                    deal_count(deal_gu(I, n), c, n) * (C / 128) + deal_count(deal_down(C, n), c, n) * (I / 128));
     if (deal_count(deal_qkv(C, KV), 0, n) > kWarps || (C / 8 + n - 1) / n > kWarps) return false;  // one warp per tile of a sum
     *blob = (units * kUnitBytes + 127) / 128 * 128;
     *slot = std::max(*blob, kLmRows * C * 2);
     for (*slots = kSlotsMax; *slots >= 2; --*slots) {
-        *smem = smem_layout(*slots, *slot, C, I, max_units(C, I, KV, n)).total;
+        *smem = smem_layout(*slots, *slot, C, I, KV, n).total;
         if (*smem <= 227 * 1024) return true;
     }
     return false;
@@ -1244,9 +1307,9 @@ static int fused_setup(wb_qwen *m)
     const int n = fused_ctas(m), C = m->C, I = m->I, KV = m->KV, QKV = C + 2 * KV, L = m->cfg.n_layer;
     int blob, slot, slots, smem;
     if (!fused_shape(m, n, &blob, &slot, &slots, &smem)) return WB_OK;
-    const size_t ll_layer = (size_t)QKV + 2 * C + I / 2 + (size_t)m->H * kSplitMax * kPartWords;
+    const size_t ll_layer = 2 * (size_t)QKV + 4 * C + I / 2 + 2 * deal_gu(I, n).loose + 2 * (size_t)m->H * kSplitMax * kPartWords;
     const size_t blob_bytes = align_up((size_t)L * n * blob), aux_bytes = align_up((size_t)L * (2 * C + QKV) * 4);
-    const size_t ll_bytes = align_up((ll_layer + 4 * (size_t)n) * 8), src_bytes = align_up(L * sizeof(Source));
+    const size_t ll_bytes = align_up((ll_layer + 8 * (size_t)n) * 8), src_bytes = align_up(L * sizeof(Source));
     char *mem = nullptr;
     if (cudaMalloc(&mem, blob_bytes + aux_bytes + ll_bytes + src_bytes) != cudaSuccess) {
         cudaGetLastError();  // no room for the second layout of the weights: the model keeps one kernel per projection
@@ -1278,7 +1341,7 @@ static int fused_setup(wb_qwen *m)
     const bool kv16 = m->cfg.kv_dtype == WB_F16;
     p.kv_layer_bytes = (size_t)m->cfg.max_t * KV * (kv16 ? 2 : 4), p.ll_layer = ll_layer;
     p.n_cta = n, p.n_layer = L, p.C = C, p.H = m->H, p.KVH = m->KVH, p.I = I, p.V = m->V, p.KV = KV;
-    p.sm = smem_layout(slots, slot, C, I, max_units(C, I, KV, n));
+    p.sm = smem_layout(slots, slot, C, I, KV, n);
     p.slots = slots, p.slot_bytes = slot, p.blob_stride = blob, p.eps = m->cfg.rms_eps;
     WB_CHECK(fused_lay_out(m, p));
     WB_CUDA(cudaFuncSetAttribute(kv16 ? (const void *)decode_fused_kernel<__half> : (const void *)decode_fused_kernel<float>,
@@ -1302,7 +1365,7 @@ int decode_fused_run(wb_qwen *m, uint32_t token, int64_t n_steps, float *logits,
     if (m->fused_writes != ctx->weight_writes) WB_CHECK(fused_lay_out(m, p));
     const uint64_t epochs = (uint64_t)n_steps * p.n_layer;
     if (m->fused_epoch + epochs > 0xfffffff0u) {  // epochs do not wrap: start again on zeroed words
-        WB_CUDA(cudaMemsetAsync(p.ll, 0, (p.ll_layer + 4 * (size_t)p.n_cta) * 8, ctx->stream));
+        WB_CUDA(cudaMemsetAsync(p.ll, 0, (p.ll_layer + 8 * (size_t)p.n_cta) * 8, ctx->stream));
         m->fused_epoch = 1;
     }
     p.epoch = m->fused_epoch, p.first_token = token, p.pos0 = (int)m->cache_len, p.n_steps = (int)n_steps;
