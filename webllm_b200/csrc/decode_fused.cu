@@ -129,10 +129,10 @@ __device__ __forceinline__ bool mbar_poll(uint64_t *b, uint32_t parity, uint32_t
     }
     return false;
 }
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)  // (shared addresses)
 {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(s32(dst)), "l"(src),
-                 "r"(bytes), "r"(s32(bar))
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+                 "r"(bytes), "r"(bar)
                  : "memory");
 }
 
@@ -143,6 +143,12 @@ __device__ __forceinline__ void ll_put(u64 *p, float v, uint32_t ep)
 {
     const u64 w = ((u64)ep << 32) | __float_as_uint(v);
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+__device__ __forceinline__ u64 ll_load(const u64 *p)
+{
+    u64 v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
 }
 __device__ __forceinline__ ulonglong2 ll_load2(const u64 *p)
 {
@@ -162,6 +168,8 @@ struct Head {
     volatile uint32_t token;
     int fill_i, fill_slot, fill_left;  // the feeder's: next fill of the ring (its index in the step, its slot), steps left
     uint32_t fills, ring_polls;        // ... fills so far
+    uint32_t rest_bytes, rest_dst, rest_bar;  // ... what is left of a fill that was begun
+    const char *rest_src;
     volatile int ring_lost;            // a wait for a slot has given up
 };
 static_assert(sizeof(Head) <= 128, "the ring begins behind it");
@@ -202,6 +210,17 @@ __device__ __forceinline__ void ll_get(ulonglong2 (&v)[N], const u64 *p, int str
             if (!ll_ok(v[i], ep)) v[i] = ll_load2(p + i * stride);
     }
 }
+__device__ __forceinline__ void ll_get_pair(float &a, float &b, const u64 *pa, const u64 *pb, uint32_t ep, Head *hd)
+{
+    u64 va = ll_load(pa), vb = ll_load(pb);
+#pragma unroll 1
+    for (uint32_t it = 1;; it++) {
+        if (ll_done((uint32_t)(va >> 32) == ep && (uint32_t)(vb >> 32) == ep, it, hd)) break;
+        if ((uint32_t)(va >> 32) != ep) va = ll_load(pa);
+        if ((uint32_t)(vb >> 32) != ep) vb = ll_load(pb);
+    }
+    a = __uint_as_float((uint32_t)va), b = __uint_as_float((uint32_t)vb);
+}
 __device__ __forceinline__ float2 ll_get2(const u64 *p, uint32_t ep, Head *hd)
 {
     ulonglong2 v[1];
@@ -233,6 +252,12 @@ __device__ __forceinline__ bool act_ok(const uint4 &v, uint32_t ep)
 __device__ __forceinline__ float act_val(uint32_t w) { return __uint_as_float(w & ~kActParity) * 32768.f; }
 __device__ __forceinline__ float4 act_vals(const uint4 &v) { return make_float4(act_val(v.x), act_val(v.y), act_val(v.z), act_val(v.w)); }
 
+// Largest value of a warp (-0 counts as less than 0; NaN as larger or smaller than all, by its sign: what comes of it is NaN anyhow).
+__device__ __forceinline__ float warp_max(float v)
+{
+    const int b = __float_as_int(v), m = __reduce_max_sync(0xffffffffu, b ^ ((b >> 31) & 0x7fffffff));
+    return __int_as_float(m ^ ((m >> 31) & 0x7fffffff));
+}
 __device__ __forceinline__ float warp_sum(float v)
 {
 #pragma unroll
@@ -244,7 +269,8 @@ __device__ __forceinline__ float warp_sum(float v)
 // A group's values become 30-bit integers of one scale, the power of two that puts the group's largest magnitude into [2^29, 2^30),
 // and these four signed bytes ("digits", base 256) each. A digit of four neighbouring positions is one word; the 32 words of a digit
 // are ordered as the MMA's lanes take them (half of the group, lane % 4, word), so that a lane reads its 16 bytes of a group at
-// once: [half][digit][lane % 4][4 words]. Between the halves stand the scale taken back and the sum of the values.
+// once: [half][digit][lane % 4][4 words]. Between the halves stands the scale taken back, four times, each with a quarter of the sum of the
+// values behind it (where sums are staged).
 constexpr int kGroupBytes = 576, kHalfAt = 320, kScaleAt = 256;  // (an offset of 320: the halves' stores hit different banks)
 __device__ __forceinline__ uint32_t half2_bits(__half2 h) { return *reinterpret_cast<const uint32_t *>(&h); }
 __device__ __forceinline__ uint32_t abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
@@ -254,18 +280,24 @@ __device__ __forceinline__ uint32_t digits(float v)
     constexpr uint32_t kCarry = 0x00808080u;
     return ((uint32_t)__float2int_rn(v) + kCarry) ^ kCarry;
 }
-// One warp, one group: positions 4 lane to 4 lane + 3. A magnitude of `limit` or more makes the whole group NaN.
-__device__ __forceinline__ void stage_group(char *group, float4 v, int lane, float limit = INFINITY)
+// One warp, a group: positions 4 lane to 4 lane + 3.
+__device__ __forceinline__ uint32_t group_top(const float4 &v)  // largest magnitude, its bits
 {
-    const uint32_t top = __reduce_max_sync(0xffffffffu, max(max(abs_bits(v.x), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w))));
-    const uint32_t e = (uint32_t)min(283 - (int)(top >> 23), 253);  // biased exponent; the scale and its inverse are normal numbers
-    const float up = __uint_as_float(e << 23);
+    return __reduce_max_sync(0xffffffffu, max(max(abs_bits(v.x), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w))));
+}
+__device__ __forceinline__ uint32_t scale_exponent(uint32_t top) { return (uint32_t)min(283 - (int)(top >> 23), 253); }  // biased; the scale and its inverse are normal numbers
+__device__ __forceinline__ float scale_back(uint32_t top, float limit = INFINITY)  // a magnitude of `limit` or more makes the whole group NaN
+{
+    return top >= __float_as_uint(limit) ? __uint_as_float(0x7fffffffu) : __uint_as_float((254 - scale_exponent(top)) << 23);
+}
+__device__ __forceinline__ void stage_digits(char *group, const float4 &v, uint32_t top, int lane)
+{
+    const float up = __uint_as_float(scale_exponent(top) << 23);
     const uint32_t a = digits(v.x * up), b = digits(v.y * up), c = digits(v.z * up), d = digits(v.w * up);
     const uint32_t ab = __byte_perm(a, b, 0x5140), cd = __byte_perm(c, d, 0x5140), AB = __byte_perm(a, b, 0x7362), CD = __byte_perm(c, d, 0x7362);
     uint32_t *at = reinterpret_cast<uint32_t *>(group + (lane >> 4) * kHalfAt + (lane & 3) * 16 + ((lane >> 2) & 3) * 4);
     at[0] = __byte_perm(ab, cd, 0x5410), at[16] = __byte_perm(ab, cd, 0x7632);
     at[32] = __byte_perm(AB, CD, 0x5410), at[48] = __byte_perm(AB, CD, 0x7632);
-    if (lane == 0) *reinterpret_cast<float *>(group + kScaleAt) = top >= __float_as_uint(limit) ? __uint_as_float(0x7fffffffu) : __uint_as_float((254 - e) << 23);
 }
 
 // One m16n8k32 MMA takes 512 weights: rows 0 to 7 of its weight operand are the 8 columns of a tile with the first half of the
@@ -418,7 +450,7 @@ struct Rows<__half> {
             const uint32_t w = take2(r0, r1);
             qp[64 * i + lane] = (uint16_t)w, qp[64 * i + 32 + lane] = (uint16_t)(w >> 16);
         }
-        if (lane == 0) att[kAttScale] = __uint_as_float((254 - e) << 23);
+        att[kAttScale] = __uint_as_float((254 - e) << 23);
     }
     __device__ __forceinline__ void begin(const float *att, int g, int t)
     {
@@ -581,10 +613,7 @@ struct Attend {
             float2 s = rows.scores();
             if (t != 0 || first + g >= nk) s.x = -INFINITY;
             if (t != 0 || first + g + 8 >= nk) s.y = -INFINITY;
-            float mn = fmaxf(s.x, s.y);
-#pragma unroll
-            for (int o = 4; o <= 16; o <<= 1) mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-            mn = fmaxf(m, __shfl_sync(0xffffffffu, mn, 0));
+            const float mn = fmaxf(m, warp_max(fmaxf(s.x, s.y)));
             const float corr = expf(m - mn), p0 = expf(s.x - mn), p1 = expf(s.y - mn);
             m = mn, l = l * corr + (p0 + p1);
             rows.add(tile, p0, p1, corr, g, t, lane);
@@ -592,23 +621,28 @@ struct Attend {
 #pragma unroll
         for (int o = 4; o <= 16; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
         rows.put_sums(wa + warp * 64, g, t, lane);
-        if (lane == 0) wm[warp] = m, wl[warp] = l;
+        wm[warp] = m, wl[warp] = l;
         __syncthreads();
-        if (warp < 3) {  // warps 0 and 1: 32 sums each; warp 2: max and sum of weights
-            const float mw = wm[lane & (kWarps - 1)], lw = wl[lane & (kWarps - 1)];
-            float M = mw;
+        if (warp < 2) {  // 32 sums each, and warp 0 the max and the sum of weights
+            float mw[kWarps], lw[kWarps], r[kWarps];
 #pragma unroll
-            for (int o = kWarps / 2; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-            const float ew = mw == -INFINITY ? 0.f : expf(mw - M);
-            float den = lw * ew, r = 0.f;
+            for (int i = 0; i < kWarps; i += 4) {
+                *reinterpret_cast<float4 *>(&mw[i]) = *reinterpret_cast<const float4 *>(wm + i);
+                *reinterpret_cast<float4 *>(&lw[i]) = *reinterpret_cast<const float4 *>(wl + i);
+            }
 #pragma unroll
-            for (int o = kWarps / 2; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
-            if (warp < 2) {
+            for (int i = 0; i < kWarps; i++) r[i] = wa[i * 64 + warp * 32 + lane];
+            float M = mw[0], den = 0.f, sum = 0.f;
 #pragma unroll
-                for (int i = 0; i < kWarps; i++) r = fmaf(wa[i * 64 + warp * 32 + lane], __shfl_sync(0xffffffffu, ew, i), r);
-                if (one) r /= den;
-                ll_put(out + warp * 32 + lane, r, ep), ll_put(out + copy + warp * 32 + lane, r, ep);
-            } else if (lane < 4) {
+            for (int i = 1; i < kWarps; i++) M = fmaxf(M, mw[i]);
+#pragma unroll
+            for (int i = 0; i < kWarps; i++) {
+                const float e = mw[i] == -INFINITY ? 0.f : expf(mw[i] - M);  // (a warp without keys)
+                den = fmaf(lw[i], e, den), sum = fmaf(r[i], e, sum);
+            }
+            if (one) sum /= den;
+            ll_put(out + warp * 32 + lane, sum, ep), ll_put(out + copy + warp * 32 + lane, sum, ep);
+            if (warp == 0 && lane < 4) {
                 const float v = lane & 1 ? den : M;
                 ll_put(out + 64 + lane, v, ep), ll_put(out + copy + 64 + lane, v, ep);
             }
@@ -630,16 +664,19 @@ inline Smem smem_layout(int slots, int slot_bytes, int C, int I, int KV, int n)
     s.att = s.red + (r12 > r3 ? r12 : r3) * 128;
     s.xs = s.att + kAttFloats * 4;
     s.small = s.xs + C * 4;
-    s.total = s.small + 2 * kWarps * 4;
+    s.total = s.small + 5 * kWarps * 4;
     return s;
 }
 
-template <typename KV>
+// G: groups of 128 of the hidden size. It is known when this is compiled, so that the staged groups' and the units' offsets are.
+template <typename KV, int G>
 __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params p)
 {
     extern __shared__ __align__(128) char smem[];
-    const int cta = blockIdx.x, n = gridDim.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int C = p.C, I = p.I, KVd = p.KV, QKV = C + 2 * KVd, G = C / 128, GI = I / 128, L = p.n_layer;
+    const int cta = blockIdx.x, n = gridDim.x, tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (the same for the whole warp, and known to be)
+    constexpr int C = G * 128;
+    const int I = p.I, KVd = p.KV, QKV = C + 2 * KVd, GI = I / 128, L = p.n_layer;
     const Deal dq = deal_qkv(C, KVd), dow = deal_o(C, n), dd = deal_down(C, n);
     const DealLines dg = deal_gu(I, n);
     const int nq = deal_count(dq, cta, n), no = deal_count(dow, cta, n), ng = deal_count(dg, cta, n), nd = deal_count(dd, cta, n);
@@ -649,8 +686,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     char *act_c = smem + so.act_c, *act_i = smem + so.act_i;
     float *red = reinterpret_cast<float *>(smem + so.red), *att = reinterpret_cast<float *>(smem + so.att);
     float *xs = reinterpret_cast<float *>(smem + so.xs);
-    float *ssq = reinterpret_cast<float *>(smem + so.small);  // [16]
-    int *widx = reinterpret_cast<int *>(ssq + kWarps);        // [16]
+    float *ssq = reinterpret_cast<float *>(smem + so.small);  // [4 kWarps]
+    int *widx = reinterpret_cast<int *>(ssq + 4 * kWarps);    // [kWarps]
     Head *hd = reinterpret_cast<Head *>(smem);
     uint64_t *full = hd->full;
     char *ring = smem + so.ring;
@@ -660,7 +697,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     if (tid == 0) {
         for (int i = 0; i < p.slots; i++) mbar_init(&full[i], 1);
         hd->gave_up = 0, hd->status = p.status, hd->polls = p.polls;
-        hd->fills = 0, hd->ring_lost = 0, hd->ring_polls = p.ring_polls;
+        hd->fills = 0, hd->rest_bytes = 0, hd->ring_lost = 0, hd->ring_polls = p.ring_polls;
         hd->fill_i = 0, hd->fill_slot = 0, hd->fill_left = p.n_steps;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -673,7 +710,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     // of down, a step took 295 us at 8 keys and 349 at 500; under gate | up 278 and 328, in halves 272 and 328).
     const bool feeder = tid == kThreads - 32;
     const uint32_t block_bytes = (uint32_t)(uq + uo + ug + ud) * kUnitBytes;
-    auto fill = [&](int halves = 3) {  // bit 0: the first half, bit 1: the second, and the fill is done
+    auto fill = [&](bool half = false) {  // half: the first half now, the rest by fill_rest
         if (hd->fill_left == 0 || hd->ring_lost) return;
         const int i = hd->fill_i, at = hd->fill_slot;
         const char *src;
@@ -684,14 +721,19 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
             const int r = row0 + (i - L) * kLmRows;
             src = reinterpret_cast<const char *>(p.embed + (size_t)r * C), bytes = (uint32_t)min(kLmRows, row1 - r) * C * 2;
         }
-        const uint32_t cut = bytes / 32 * 16, first = halves & 1 ? 0u : cut, end = halves & 2 ? bytes : cut;
-        if (halves & 1) mbar_expect(&full[at], bytes);
-        if (end > first) bulk_load(ring + at * p.slot_bytes + first, src + first, end - first, &full[at]);
-        if (!(halves & 2)) return;
+        const uint32_t now = half ? bytes / 32 * 16 : bytes;
+        char *dst = ring + at * p.slot_bytes;
+        mbar_expect(&full[at], bytes);
+        if (now) bulk_load(s32(dst), src, now, s32(&full[at]));
+        hd->rest_src = src + now, hd->rest_dst = s32(dst) + now, hd->rest_bar = s32(&full[at]), hd->rest_bytes = bytes - now;
         hd->fills++;
         hd->fill_slot = at + 1 == p.slots ? 0 : at + 1;
         if (i + 1 == L + lm_fills) hd->fill_i = 0, hd->fill_left--;
         else hd->fill_i = i + 1;
+    };
+    auto fill_rest = [&]() {  // (under gate | up, where every warp is busy: little to do)
+        if (hd->rest_bytes) bulk_load(hd->rest_dst, hd->rest_src, hd->rest_bytes, hd->rest_bar);
+        hd->rest_bytes = 0;
     };
     if (feeder)
 #pragma unroll 1
@@ -704,8 +746,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
 
     const int H = p.H, hpk = H / p.KVH;
     const int c4 = 4 * tid;
-    const bool has4 = c4 < C;
-    const float inv_c = 1.f / (float)C;
+    const bool has4 = warp < G;  // 4 tid < C
+    constexpr float inv_c = 1.f / (float)C;
     const int w_o = 2 * QKV, w_act = w_o + 2 * C, w_down = w_act + I / 2 + 2 * dg.loose, w_att = w_down + 2 * C;  // words of a layer; q | k | v first
     const int att_words = H * kSplitMax * kPartWords;
     u64 *const ll = p.ll, *const cand = ll + p.ll_layer;
@@ -716,7 +758,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);  // this thread's part of the residual stream
     // Projections from C: a warp stays with one group of 128 rows (its activations are loaded once) and takes the CTA's tiles in
     // turn; where there are fewer groups than half the warps, several warps share a group's tiles.
-    const int wpg = kWarps / G, grp = warp % G, sub = warp / G;
+    constexpr int wpg = kWarps / G;
+    const int grp = warp % G, sub = warp / G;
     const int t_first = sub < wpg ? sub : 1 << 16;  // (no tiles for the warps that are left over)
     const Lane ln(lane);
     const int part = lane & 3;
@@ -725,20 +768,28 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     // rmsnorm of the residual stream (rmsNormRef, src/reference/qwen-ref.ts:12-29). A projection takes x * weight as it is, and its
     // results are multiplied by the reciprocal root mean square: it is known behind the same barrier as the staged values.
     auto inv_rms = [&]() {
-        const float4 a = reinterpret_cast<const float4 *>(ssq)[0], b = reinterpret_cast<const float4 *>(ssq)[1];
-        return rsqrtf((((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) * inv_c + p.eps);
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) {
+            const float4 b = reinterpret_cast<const float4 *>(ssq)[w];
+            a.x += b.x, a.y += b.y, a.z += b.z, a.w += b.w;
+        }
+        return rsqrtf(((a.x + a.y) + (a.z + a.w)) * inv_c + p.eps);
     };
     auto squares = [&]() { return fmaf(x.x, x.x, x.y * x.y) + fmaf(x.z, x.z, x.w * x.w); };
+    // (sums over eight lanes each: who needs them adds up the four; the steps stand between those of the staging because a warp issues in order)
     auto norm_stage = [&](float4 w) {
         const float4 y = make_float4(x.x * w.x, x.y * w.y, x.z * w.z, x.w * w.w);
-        if (has4) stage_group(act_c + warp * kGroupBytes, y, lane);
+        uint32_t top = 0;
+        if (has4) top = group_top(y);
         float ss = squares(), sum = (y.x + y.y) + (y.z + y.w);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 16), sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+        if (has4) stage_digits(act_c + warp * kGroupBytes, y, top, lane);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o), sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (lane == 0) {
-            ssq[warp] = ss;
-            if (has4) *reinterpret_cast<float *>(act_c + warp * kGroupBytes + kScaleAt + 4) = sum;
-        }
+        for (int o = 8; o >= 4; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o), sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        // (lanes of the same part have the same sums: all of them store, a branch for four takes 0.1 us)
+        ssq[warp * 4 + part] = ss;
+        if (has4) *reinterpret_cast<float2 *>(act_c + warp * kGroupBytes + kScaleAt + part * 8) = make_float2(scale_back(top), sum);
         __syncthreads();
     };
     auto load4 = [&](const float *a) { return has4 ? __ldg(reinterpret_cast<const float4 *>(a) + tid) : make_float4(0.f, 0.f, 0.f, 0.f); };
@@ -751,6 +802,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     };
     // q | k | v and o: a CTA has few tiles; a warp takes one group of 128 rows of each, the sums over the groups go through shared memory.
     Unit u[8];
+    constexpr std::integral_constant<int, G> groups{};
     auto load_one = [&](const char *w) { u[0].load(w + (t_first * G + grp) * kUnitBytes, lane); };
     auto run_short = [&](const char *w, int tiles) {  // from load_one
         const char *group = act_c + grp * kGroupBytes;
@@ -767,11 +819,10 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
             red[(i * G + grp) * 32 + lane] = fmaf(u[0].s.x, ln.value(d) * gx, -u[0].s.y * sum);
         }
     };
-    auto column_sum = [&](int first, int n_sums) {  // of up to 8 rows of red
+    auto column_sum = [&](int first, auto rows) {  // of rows of red
         float a[2] = {};
 #pragma unroll
-        for (int g = 0; g < 8; g++)
-            if (g < n_sums) a[g & 1] += red[(first + g) * 32 + lane];
+        for (int g = 0; g < decltype(rows)::value; g++) a[g & 1] += red[(first + g) * 32 + lane];
         return quad_sum(a[0] + a[1]);
     };
     // gate | up: a warp takes whole tiles, all groups of them (the activations of all groups lie in registers). Loose tiles, if they are
@@ -781,45 +832,40 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     const int my_extra = warp < spread * G ? warp : 0;
     auto load_tile = [&](const char *w) {
 #pragma unroll
-        for (int g = 0; g < 8; g++) u[g].load(w + min(g, G - 1) * kUnitBytes, lane);
+        for (int g = 0; g < G; g++) u[g].load(w + g * kUnitBytes, lane);
     };
     float *line = red + kWarps * 32;
     auto run_tiles = [&](const char *w) {  // from load_tile
-        uint4 b[8];
-        float gx[8], sum[8];
+        uint4 b[G];
+        float gx[G], sum[G];
 #pragma unroll
-        for (int g = 0; g < 8; g++) {  // (groups that are not there: the last one's, times 0)
-            const char *group = act_c + min(g, G - 1) * kGroupBytes;
+        for (int g = 0; g < G; g++) {
+            const char *group = act_c + g * kGroupBytes;
             b[g] = *reinterpret_cast<const uint4 *>(group + ln.at);
-            const float2 s2 = *reinterpret_cast<const float2 *>(group + kScaleAt);
-            gx[g] = g < G ? s2.x * ln.fac : 0.f, sum[g] = g < G && part == 0 ? s2.y : 0.f;
+            const float2 s2 = *reinterpret_cast<const float2 *>(group + kScaleAt + part * 8);
+            gx[g] = s2.x * ln.fac, sum[g] = s2.y;
         }
         if (spread) {
             Unit e;
             e.load(w + (whole * G + my_extra) * kUnitBytes, lane);
             const char *group = act_c + my_extra % G * kGroupBytes;
-            const float2 s2 = *reinterpret_cast<const float2 *>(group + kScaleAt);
+            const float2 s2 = *reinterpret_cast<const float2 *>(group + kScaleAt + part * 8);
             int d[4];
             unit_dot(d, e.q, *reinterpret_cast<const uint4 *>(group + ln.at));
-            red[warp * 32 + lane] = fmaf(e.s.x, ln.value(d) * (s2.x * ln.fac), part == 0 ? -e.s.y * s2.y : 0.f);
+            red[warp * 32 + lane] = fmaf(e.s.x, ln.value(d) * (s2.x * ln.fac), -e.s.y * s2.y);
         }
 #pragma unroll 1
         for (int i = warp; i < whole; i += kWarps) {
             if (i > warp) load_tile(w + i * G * kUnitBytes);
             float a[2] = {};
-            auto four = [&](auto first) {
-                constexpr int g0 = decltype(first)::value;
-                int d[4][4];
+            int d[G][4];
 #pragma unroll
-                for (int j = 0; j < 4; j++) unit_dot(d[j], u[g0 + j].q, b[g0 + j]);
+            for (int g = 0; g < G; g++) unit_dot(d[g], u[g].q, b[g]);
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    a[0] = fmaf(u[g0 + j].s.x, ln.value(d[j]) * gx[g0 + j], a[0]);
-                    a[1] = fmaf(u[g0 + j].s.y, sum[g0 + j], a[1]);
-                }
-            };
-            four(std::integral_constant<int, 0>());
-            if (G > 4) four(std::integral_constant<int, 4>());
+            for (int g = 0; g < G; g++) {
+                a[0] = fmaf(u[g].s.x, ln.value(d[g]) * gx[g], a[0]);
+                a[1] = fmaf(u[g].s.y, sum[g], a[1]);
+            }
             const float r = quad_sum(a[0] - a[1]);
             if (part == 0) line[i * 8 + (lane >> 2)] = r;
         }
@@ -863,27 +909,24 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
             if (is_att) at.load(kc, vc, KVd, warp * 16, own_new ? nk - 1 : nk, tile, lane);
             if (l > 0) add_residual(ll + w_down, ep - 1);
             norm_stage(nw);
-            float rstd = inv_rms();
             run_short(wb, nq);
             wb += uq * kUnitBytes;
+            float rstd = warp < nq ? inv_rms() : 0.f;
             if (nq > 0) __syncthreads();
             if (warp < nq) {
-                const float a = fmaf(column_sum(warp * G, G), rstd, bias);
+                const float a = fmaf(column_sum(warp * G, groups), rstd, bias);
                 if (part == 0) ll_put(ll + word_at((fq + warp * n) * 8 + (lane >> 2)), a, ep);
             }
-            if (feeder && l > 0) fill(1);
+            if (feeder && l > 0) fill(true);
 
             // -- attention: rotary embedding of q and the new k (ropeHalfRef, src/reference/qwen-ref.ts:35-64), cache append
             if (is_att) {
                 if (warp < 3 && (warp == 0 || own_new)) {
-                    // a lane reads the pair (2i, 2i + 1), the rotation needs (i, i + 32)
                     const float2 cs = __ldg(reinterpret_cast<const float2 *>(p.cs_table) + (size_t)pos * 32 + lane);
-                    const float2 a = ll_get2(ll + word_at((warp == 0 ? h * 64 : warp == 1 ? C + kvh * 64 : C + KVd + kvh * 64) + 2 * lane), ep ^ p.miss, hd);
+                    const u64 *src = ll + word_at((warp == 0 ? h * 64 : warp == 1 ? C + kvh * 64 : C + KVd + kvh * 64) + lane);
+                    float r0, r1;
+                    ll_get_pair(r0, r1, src, src + word_at(32), ep ^ p.miss, hd);
                     float *dst = att + (warp == 0 ? kAttQ : warp * 64 - 64);
-                    *reinterpret_cast<float2 *>(dst + 2 * lane) = a;
-                    __syncwarp();
-                    float r0 = dst[lane], r1 = dst[lane + 32];
-                    __syncwarp();
                     if (warp < 2) {
                         const float t0 = r0 * cs.x - r1 * cs.y, t1 = r0 * cs.y + r1 * cs.x;
                         r0 = t0, r1 = t1;
@@ -963,14 +1006,16 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
                         const float inv = 1.f / den;
                         a.x *= inv, a.y *= inv, a.z *= inv, a.w *= inv;
                     }
-                    stage_group(act_c + warp * kGroupBytes, a, lane);
+                    const uint32_t top = group_top(a);
+                    stage_digits(act_c + warp * kGroupBytes, a, top, lane);
+                    *reinterpret_cast<float *>(act_c + warp * kGroupBytes + kScaleAt) = scale_back(top);
                 }
                 __syncthreads();
                 run_short(wb, no);
                 wb += uo * kUnitBytes;
                 __syncthreads();
                 if (warp < no) {
-                    const float a = column_sum(warp * G, G);
+                    const float a = column_sum(warp * G, groups);
                     if (part == 0) ll_put(ll + w_o + word_at((fo + warp * n) * 8 + (lane >> 2)), a, ep);
                 }
             }
@@ -980,9 +1025,9 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
             nw = load4(aux + C);
             add_residual(ll + w_o, ep);
             norm_stage(nw);
-            rstd = inv_rms();
-            if (feeder && l > 0) fill(2);
+            if (feeder && l > 0) fill_rest();
             run_tiles(wb);
+            rstd = inv_rms();
             __syncthreads();
             auto silu_up = [&](float gate, float up) { return gate / (1.f + expf(-gate)) * up; };
             auto loose_word = [&](int i) { return act + act_at(deal_tile(dg, cta, n, i) * 4) + part * 4 + (lane >> 2); };  // (a sector, both halves)
@@ -992,7 +1037,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
                 act_put(act + (cta + i * n) * 32 + lane, silu_up(r[0] * rstd, r[4] * rstd), ep);
             }
             if (const int i = kWarps - 1 - warp; i < spread) {
-                const float a = column_sum(i * G, G) * rstd, up = __shfl_xor_sync(0xffffffffu, a, 16);
+                const float a = column_sum(i * G, groups) * rstd, up = __shfl_xor_sync(0xffffffffu, a, 16);
                 if (lane < 16 && part < 2) act_put(loose_word(whole + i), silu_up(a, up), ep);
             }
 #pragma unroll 1
@@ -1030,8 +1075,15 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
                             if (!act_ok(w[i], ep)) w[i] = act_load4(act + act_at(k + i * 4 * kThreads));
                     }
                     // a warp's 128 values are one group
+                    uint32_t top[kBatch];
 #pragma unroll
-                    for (int i = 0; i < kBatch; i++) stage_group(act_i + ((k >> 7) + i * kWarps) * kGroupBytes, act_vals(w[i]), lane, kActLimit);
+                    for (int i = 0; i < kBatch; i++) top[i] = group_top(act_vals(w[i]));
+#pragma unroll
+                    for (int i = 0; i < kBatch; i++) {
+                        char *group = act_i + ((k >> 7) + i * kWarps) * kGroupBytes;
+                        stage_digits(group, act_vals(w[i]), top[i], lane);
+                        *reinterpret_cast<float *>(group + kScaleAt) = scale_back(top[i], kActLimit);
+                    }
                 }
                 __syncthreads();
 #pragma unroll 1
@@ -1062,7 +1114,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
                 if (feeder && l + 1 < L) ring_wait(hd, slot, par);
                 __syncthreads();
                 if (warp < nd) {
-                    const float a = column_sum(warp * kWarps, kWarps);
+                    const float a = column_sum(warp * kWarps, std::integral_constant<int, kWarps>());
                     if (part == 0) ll_put(ll + w_down + word_at((fdn + warp * n) * 8 + (lane >> 2)), a, ep);
                 }
             }
@@ -1073,7 +1125,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
         const float4 w_final = load4(p.final_norm);
         add_residual(ll + w_down, --ep);  // the last layer's epoch is the step's
         const float ss = warp_sum(squares());
-        if (lane == 0) ssq[warp] = ss;
+        if (lane < 4) ssq[warp * 4 + lane] = lane == 0 ? ss : 0.f;
         __syncthreads();
         const float rstd = inv_rms();
         if (has4) *reinterpret_cast<float4 *>(xs + c4) = make_float4(x.x * rstd * w_final.x, x.y * rstd * w_final.y, x.z * rstd * w_final.z, x.w * rstd * w_final.w);
@@ -1299,6 +1351,25 @@ static int fused_lay_out(wb_qwen *m, const fd::Params &p)
     return WB_OK;
 }
 
+static const void *fused_kernel(const wb_qwen *m)
+{
+    using namespace fd;
+    auto pick = [&](auto g) {
+        constexpr int G = decltype(g)::value;
+        return m->cfg.kv_dtype == WB_F16 ? (const void *)decode_fused_kernel<__half, G> : (const void *)decode_fused_kernel<float, G>;
+    };
+    switch (m->C / 128) {
+    case 1: return pick(std::integral_constant<int, 1>());
+    case 2: return pick(std::integral_constant<int, 2>());
+    case 3: return pick(std::integral_constant<int, 3>());
+    case 4: return pick(std::integral_constant<int, 4>());
+    case 5: return pick(std::integral_constant<int, 5>());
+    case 6: return pick(std::integral_constant<int, 6>());
+    case 7: return pick(std::integral_constant<int, 7>());
+    default: return pick(std::integral_constant<int, kMaxC / 128>());
+    }
+}
+
 static int fused_setup(wb_qwen *m)
 {
     using namespace fd;
@@ -1344,8 +1415,7 @@ static int fused_setup(wb_qwen *m)
     p.sm = smem_layout(slots, slot, C, I, KV, n);
     p.slots = slots, p.slot_bytes = slot, p.blob_stride = blob, p.eps = m->cfg.rms_eps;
     WB_CHECK(fused_lay_out(m, p));
-    WB_CUDA(cudaFuncSetAttribute(kv16 ? (const void *)decode_fused_kernel<__half> : (const void *)decode_fused_kernel<float>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    WB_CUDA(cudaFuncSetAttribute(fused_kernel(m), cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     static_assert(sizeof(Params) <= sizeof(m->fused_params), "room for the parameters in the model object");
     memcpy(m->fused_params, &p, sizeof p);
     m->fused_smem = smem, m->fused_epoch = 1, m->fused_state = 1;
@@ -1375,8 +1445,7 @@ int decode_fused_run(wb_qwen *m, uint32_t token, int64_t n_steps, float *logits,
     static const int give_up = [] { const char *e = getenv("WEBLLM_B200_DECODE_GIVE_UP"); return e ? atoi(e) : 0; }();
     p.miss = give_up == 1 ? 0x80000000u : 0u, p.polls = give_up == 1 ? kPollsTest : kPolls, p.ring_polls = give_up == 2 ? 0u : kRingPolls;
     void *args[] = {&p};
-    const void *kern = m->cfg.kv_dtype == WB_F16 ? (const void *)decode_fused_kernel<__half> : (const void *)decode_fused_kernel<float>;
-    WB_CUDA(cudaLaunchCooperativeKernel(kern, dim3(p.n_cta), dim3(kThreads), args, (size_t)m->fused_smem, ctx->stream));
+    WB_CUDA(cudaLaunchCooperativeKernel(fused_kernel(m), dim3(p.n_cta), dim3(kThreads), args, (size_t)m->fused_smem, ctx->stream));
     m->fused_epoch += (uint32_t)epochs;
     ctx->launches++;
     *ran = true;
