@@ -19,8 +19,8 @@
 //     by gate|up of l + 1 and by q|k|v of l + 1;
 //   * every CTA keeps the residual stream itself, so the norms need no hand-over of their own.
 // A layer is five such hand-overs: q|k|v, attention, o, gate|up (with silu * up at the producer), down.
-// Measured on the 0.5B shapes: 0.26 ms per token at short contexts, 0.295 at 500 keys (one kernel per operation: 0.49). HBM's 0.07 is
-// hidden; a layer is 8.6 us of hand-overs (4 x 0.8 us and attention's) and of each CTA's own chain between them: staging, products,
+// Measured on the 0.5B shapes: 0.232 ms per token at short contexts, 0.263 at 500 keys (one kernel per operation: 0.49). HBM's 0.07 is
+// hidden; a layer is 7.9 us, of which 2 are five hand-overs and the rest is attention and each CTA's own chain between them: staging, products,
 // sums over warps, barriers.
 //
 // Arithmetic. A CTA owns whole output columns in tiles of 8. Weights are exact integers q with a scale and a zero point per group of 128
@@ -301,10 +301,11 @@ __device__ __forceinline__ void stage_digits(char *group, const float4 &v, uint3
 }
 
 // One m16n8k32 MMA takes 512 weights: rows 0 to 7 of its weight operand are the 8 columns of a tile with the first half of the
-// group's positions, rows 8 to 15 the same columns with the second half, times 16 as their nibbles lie; the columns of the
-// activation operand are the four digits of the first half, then of the second. Integers: every product and sum is exact. Lane
-// (c, t) of the result uses two of its four sums: digits 2 (t % 2) and the next one of half t / 2, and the four lanes of a column
-// add up to the dot product. The zero point comes off through the group's sum.
+// group's positions, rows 8 to 15 the same columns with whole bytes, which are the first half's nibbles and 16 times the second's;
+// the columns of the activation operand are the four digits of the first half, then of the second. Integers: every product and sum
+// is exact. Lane (c, t) of the result has the sums of digits 2 (t % 2) and the next one of half t / 2: the first half's are in the
+// upper row, the second's are the lower row's less the upper's (a subtraction for four masks). The four lanes of a column add up to
+// the dot product. The zero point comes off through the group's sum.
 __device__ __forceinline__ void mma8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
 {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -330,19 +331,20 @@ struct Unit {  // weights in registers, requested before the activations are the
 // What a lane knows about its two digits.
 struct Lane {
     int at;            // its bytes of a staged group
-    bool second;       // half of the positions
+    int m0, m2;        // weights of the sums of its column's two rows
     float digit, fac;  // 1 or 2^16; the same, with the second half's 16 taken back
     __device__ __forceinline__ explicit Lane(int lane)
-        : at(lane * 16 + (lane >> 4) * (kHalfAt - 256)), second(lane & 2), digit((lane & 1) ? 65536.f : 1.f), fac((lane & 2) ? digit * 0.0625f : digit)
+        : at(lane * 16 + (lane >> 4) * (kHalfAt - 256)), m0((lane & 2) ? -1 : 1), m2((lane >> 1) & 1), digit((lane & 1) ? 65536.f : 1.f), fac((lane & 2) ? digit * 0.0625f : digit)
     {
     }
-    __device__ __forceinline__ float value(const int (&d)[4]) const { return (float)((second ? d[3] : d[1]) * 256 + (second ? d[2] : d[0])); }
+    __device__ __forceinline__ float value(const int (&d)[4]) const { return (float)(d[0] * m0 + d[2] * m2 + 256 * (d[1] * m0 + d[3] * m2)); }
+    __device__ __forceinline__ float sum(const int (&d)[4]) const { return (float)(d[1] * 256 + d[0]); }  // of digit_sums
 };
 __device__ __forceinline__ void unit_dot(int (&d)[4], const uint4 &q, const uint4 &b)
 {
-    constexpr uint32_t kLow = 0x0f0f0f0fu, kHigh = 0xf0f0f0f0u;
-    mma8_first(d, q.x & kLow, q.x & kHigh, q.y & kLow, q.y & kHigh, b.x, b.y);
-    mma8(d, q.z & kLow, q.z & kHigh, q.w & kLow, q.w & kHigh, b.z, b.w);
+    constexpr uint32_t kLow = 0x0f0f0f0fu;
+    mma8_first(d, q.x & kLow, q.x, q.y & kLow, q.y, b.x, b.y);
+    mma8(d, q.z & kLow, q.z, q.w & kLow, q.w, b.z, b.w);
 }
 // Sums of the digits, by the same instruction with a weight operand of ones.
 __device__ __forceinline__ void digit_sums(int (&d)[4], const uint4 &b)
@@ -380,7 +382,10 @@ __device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uin
 // warp's 16 keys. A step at 8, 120 and 510 keys: 315, 350, 376 us; with MMAs of two fp16 parts 327, 369, 386 (22 bits, and infinite
 // from 65504 on), of three bf16 parts 345, 388, 403.
 constexpr int kPassKeys = kWarps * 16;
-constexpr int kSplitKeys = 2 * kPassKeys;  // a head gets one more CTA per so many keys: a pass costs less than merging one more split
+// A head gets a CTA per pass up to four, then one per two passes: a second pass costs what merging two more splits does (a step at 300
+// keys 263 us with two CTAs a head, 255 with three; at 420 266 and 261, f32 cache at 460 306 and 273; at 600 269 with three, 274 with
+// four or five; at 1100 286 with five, 302 with three, 292 with eight).
+constexpr int kOnePassKeys = 4 * kPassKeys;
 
 // shared memory, in floats: new k [64], new v [64], the query [64] or its parts (fp16) [3][64], max [8], sum [8], sums [8][64], the
 // query's scale taken back [4]
@@ -755,6 +760,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     const int first_loose = dg.lines * n * 32;
     auto act_at = [&](int k) { return k < first_loose ? k : 2 * k - first_loose; };  // a loose tile's four words have a sector for themselves
     uint32_t token = p.first_token;
+    int asks = 0;  // the CTA that asks for a layer's constants
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);  // this thread's part of the residual stream
     // Projections from C: a warp stays with one group of 128 rows (its activations are loaded once) and takes the CTA's tiles in
     // turn; where there are fewer groups than half the warps, several warps share a group's tiles.
@@ -762,7 +768,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     const int grp = warp % G, sub = warp / G;
     const int t_first = sub < wpg ? sub : 1 << 16;  // (no tiles for the warps that are left over)
     const Lane ln(lane);
-    const int part = lane & 3;
+    const int part = lane & 3, mine = kWarps - 1 - warp;  // the tile (of few) that a warp finishes: the last warps have less to multiply
     char *tile = act_i + warp * 2048;
 
     // rmsnorm of the residual stream (rmsNormRef, src/reference/qwen-ref.ts:12-29). A projection takes x * weight as it is, and its
@@ -810,7 +816,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
         const float scale = *reinterpret_cast<const float *>(group + kScaleAt), gx = scale * ln.fac;
         int ds[4];
         digit_sums(ds, b);
-        const float sum = ln.value(ds) * (scale * ln.digit);
+        const float sum = ln.sum(ds) * (scale * ln.digit);
 #pragma unroll 1
         for (int i = t_first; i < tiles; i += wpg) {
             if (i > t_first) u[0].load(w + (i * G + grp) * kUnitBytes, lane);
@@ -877,7 +883,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
     for (int s = 0; s < p.n_steps; s++) {
         uint32_t ep = p.epoch + (uint32_t)(s * L);  // of this step's first layer; one more per layer
         const int pos = p.pos0 + s, n_keys = pos + 1;
-        const int S = max(1, min(min(kSplitMax, n / H), (n_keys + kSplitKeys - 1) / kSplitKeys));
+        const int split_keys = n_keys <= kOnePassKeys ? kPassKeys : 2 * kPassKeys;
+        const int S = max(1, min(min(kSplitMax, n / H), (n_keys + split_keys - 1) / split_keys));
         const int chunk = (n_keys + S - 1) / S;
         const bool is_att = cta < H * S;
         const int h = is_att ? cta / S : 0, sp = cta - h * S, kvh = h / hpk;
@@ -898,11 +905,12 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
             // -- q | k | v
             if (sub < wpg) load_one(wb);
             float4 nw = load4(aux);
-            const float bias = warp < nq ? __ldg(aux + 2 * C + (fq + warp * n) * 8 + (lane >> 2)) : 0.f;
+            const float bias = mine < nq ? __ldg(aux + 2 * C + (fq + mine * n) * 8 + (lane >> 2)) : 0.f;
             // the rest of the layer's constants comes from HBM too (the weight stream pushes it out of L2): one CTA asks L2 for
             // the next layer's norm weights and biases, and the attention CTAs request their cache rows here
-            if (l + 1 < L && cta == l % n)
+            if (l + 1 < L && cta == asks)
                 for (int i = tid * 32; i < 2 * C + QKV; i += kThreads * 32) prefetch_l2(aux + 2 * C + QKV + i);
+            asks = asks + 1 == n ? 0 : asks + 1;
             Attend<KV> at;
             const KV *kc = reinterpret_cast<const KV *>(p.k_cache + (size_t)l * p.kv_layer_bytes) + (size_t)k0 * KVd + kvh * 64;
             const KV *vc = reinterpret_cast<const KV *>(p.v_cache + (size_t)l * p.kv_layer_bytes) + (size_t)k0 * KVd + kvh * 64;
@@ -911,11 +919,11 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
             norm_stage(nw);
             run_short(wb, nq);
             wb += uq * kUnitBytes;
-            float rstd = warp < nq ? inv_rms() : 0.f;
+            float rstd = mine < nq ? inv_rms() : 0.f;
             if (nq > 0) __syncthreads();
-            if (warp < nq) {
-                const float a = fmaf(column_sum(warp * G, groups), rstd, bias);
-                if (part == 0) ll_put(ll + word_at((fq + warp * n) * 8 + (lane >> 2)), a, ep);
+            if (mine < nq) {
+                const float a = fmaf(column_sum(mine * G, groups), rstd, bias);
+                if (part == 0) ll_put(ll + word_at((fq + mine * n) * 8 + (lane >> 2)), a, ep);
             }
             if (feeder && l > 0) fill(true);
 
@@ -1014,9 +1022,9 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
                 run_short(wb, no);
                 wb += uo * kUnitBytes;
                 __syncthreads();
-                if (warp < no) {
-                    const float a = column_sum(warp * G, groups);
-                    if (part == 0) ll_put(ll + w_o + word_at((fo + warp * n) * 8 + (lane >> 2)), a, ep);
+                if (mine < no) {
+                    const float a = column_sum(mine * G, groups);
+                    if (part == 0) ll_put(ll + w_o + word_at((fo + mine * n) * 8 + (lane >> 2)), a, ep);
                 }
             }
 
@@ -1027,16 +1035,16 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
             norm_stage(nw);
             if (feeder && l > 0) fill_rest();
             run_tiles(wb);
-            rstd = inv_rms();
+            if (mine < dg.lines || warp < spread || whole > dg.lines * 8) rstd = inv_rms();
             __syncthreads();
             auto silu_up = [&](float gate, float up) { return gate / (1.f + expf(-gate)) * up; };
             auto loose_word = [&](int i) { return act + act_at(deal_tile(dg, cta, n, i) * 4) + part * 4 + (lane >> 2); };  // (a sector, both halves)
 #pragma unroll 1
-            for (int i = warp; i < dg.lines; i += kWarps) {
+            for (int i = mine; i < dg.lines; i += kWarps) {
                 const float *r = line + i * 64 + (lane >> 2) * 8 + (lane & 3);
                 act_put(act + (cta + i * n) * 32 + lane, silu_up(r[0] * rstd, r[4] * rstd), ep);
             }
-            if (const int i = kWarps - 1 - warp; i < spread) {
+            if (const int i = warp; i < spread) {
                 const float a = column_sum(i * G, groups) * rstd, up = __shfl_xor_sync(0xffffffffu, a, 16);
                 if (lane < 16 && part < 2) act_put(loose_word(whole + i), silu_up(a, up), ep);
             }
@@ -1104,7 +1112,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_fused_kernel(const Params 
                         }
 #pragma unroll
                         for (int j = 0; j < kBurst; j++) {
-                            const float v = fmaf(u[j].s.x, ln.value(d[j]) * (scale[j] * ln.fac), -u[j].s.y * (ln.value(ds[j]) * (scale[j] * ln.digit)));
+                            const float v = fmaf(u[j].s.x, ln.value(d[j]) * (scale[j] * ln.fac), -u[j].s.y * (ln.sum(ds[j]) * (scale[j] * ln.digit)));
                             if (i + j * kWarps < GI) a += v;
                         }
                     }
