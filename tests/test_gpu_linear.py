@@ -237,6 +237,32 @@ def test_streaming_kernel_matches_oracle(gpu, oracle, K, N, S, M, zeros):
         gpu.plan_override(0, 0)
 
 
+@pytest.mark.parametrize("K,N,S,group", [(2688, 38016, 1, 128), (5376, 96, 2, 256), (2560, 64, 1, 128)])
+@pytest.mark.parametrize("spread", [False, True])
+def test_one_row_streaming_kernel(gpu, oracle, K, N, S, group, spread):
+    """The streaming kernel's form for one row: an odd number of chunks (a last group of 128 that is staged twice), more tiles per CTA
+    than a round of four holds, a group of two chunks; activations of one magnitude, and of eight decades within a group. Its
+    integers have 30 bits of a group's largest value, so the f32 bar stands for both."""
+    t = synthetic.random_gptq(K, N, group, seed=K + N, zeros="any")
+    W = oracle_weight(oracle, t)
+    h = register(gpu, f"onerow_{K}x{N}_{spread}", t)
+    rng = np.random.default_rng(K)
+    x = _x(1, K, K)
+    if spread:
+        x *= 10.0 ** rng.integers(-5, 4, x.shape)
+    x[0, 128:256] = 0  # a group of zeros
+    try:
+        gpu.plan_override(_lib.WB_KERNEL_GEMV_STREAM, S)
+        ref = oracle.gemm_nt_ref(x, W, 1, N, K, threads=oracle.max_threads())
+        assert_close(oracle, run_linear(gpu, h, x, 1, N), ref, F32_RTOL, f"one row K={K} N={N}")
+        x16 = x.astype(np.float16)
+        ref16 = oracle.gemm_nt_ref(x16.astype(np.float32), W, 1, N, K, threads=oracle.max_threads())
+        assert_close(oracle, run_linear(gpu, h, x16, 1, N), ref16, F16_RTOL, f"one row K={K} N={N} f16")
+    finally:
+        gpu.plan_override(0, 0)
+        gpu.weight_pop()
+
+
 @pytest.mark.parametrize("K,N", [(3584, 18944), (3584, 37888)])
 def test_7b_gate_up_decode_takes_the_streaming_kernel(gpu, oracle, K, N):
     """The 7B-class gate / up projection (3584 -> 18944) and gate|up as one matrix (3584 -> 37888), the shapes behind

@@ -36,10 +36,13 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "digits.cuh"
 #include "qwen_internal.cuh"
 
 namespace wb {
 namespace fd {
+
+using namespace dg;
 
 constexpr int kThreads = 256, kWarps = 8;
 constexpr int kUnitBytes = 576;   // 8 columns x 128 rows: 512 of nibbles, then scale and scale * zero point of every column
@@ -265,58 +268,16 @@ __device__ __forceinline__ float warp_sum(float v)
     return v;
 }
 
-// ---- staging: f32 values -> signed bytes, group by group of 128 positions ----
-// A group's values become 30-bit integers of one scale, the power of two that puts the group's largest magnitude into [2^29, 2^30),
-// and these four signed bytes ("digits", base 256) each. A digit of four neighbouring positions is one word; the 32 words of a digit
-// are ordered as the MMA's lanes take them (half of the group, lane % 4, word), so that a lane reads its 16 bytes of a group at
-// once: [half][digit][lane % 4][4 words]. Between the halves stands the scale taken back, four times, each with a quarter of the sum of the
-// values behind it (where sums are staged).
-constexpr int kGroupBytes = 576, kHalfAt = 320, kScaleAt = 256;  // (an offset of 320: the halves' stores hit different banks)
 __device__ __forceinline__ uint32_t half2_bits(__half2 h) { return *reinterpret_cast<const uint32_t *>(&h); }
-__device__ __forceinline__ uint32_t abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
-// The four bytes of an integer below 2^31 - 2^23 in balanced base 256: byte i holds the digit i.
-__device__ __forceinline__ uint32_t digits(float v)
-{
-    constexpr uint32_t kCarry = 0x00808080u;
-    return ((uint32_t)__float2int_rn(v) + kCarry) ^ kCarry;
-}
-// One warp, a group: positions 4 lane to 4 lane + 3.
+// Staging (digits.cuh): one warp, a group; positions 4 lane to 4 lane + 3.
 __device__ __forceinline__ uint32_t group_top(const float4 &v)  // largest magnitude, its bits
 {
     return __reduce_max_sync(0xffffffffu, max(max(abs_bits(v.x), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w))));
 }
-__device__ __forceinline__ uint32_t scale_exponent(uint32_t top) { return (uint32_t)min(283 - (int)(top >> 23), 253); }  // biased; the scale and its inverse are normal numbers
-__device__ __forceinline__ float scale_back(uint32_t top, float limit = INFINITY)  // a magnitude of `limit` or more makes the whole group NaN
-{
-    return top >= __float_as_uint(limit) ? __uint_as_float(0x7fffffffu) : __uint_as_float((254 - scale_exponent(top)) << 23);
-}
 __device__ __forceinline__ void stage_digits(char *group, const float4 &v, uint32_t top, int lane)
 {
-    const float up = __uint_as_float(scale_exponent(top) << 23);
-    const uint32_t a = digits(v.x * up), b = digits(v.y * up), c = digits(v.z * up), d = digits(v.w * up);
-    const uint32_t ab = __byte_perm(a, b, 0x5140), cd = __byte_perm(c, d, 0x5140), AB = __byte_perm(a, b, 0x7362), CD = __byte_perm(c, d, 0x7362);
-    uint32_t *at = reinterpret_cast<uint32_t *>(group + (lane >> 4) * kHalfAt + (lane & 3) * 16 + ((lane >> 2) & 3) * 4);
-    at[0] = __byte_perm(ab, cd, 0x5410), at[16] = __byte_perm(ab, cd, 0x7632);
-    at[32] = __byte_perm(AB, CD, 0x5410), at[48] = __byte_perm(AB, CD, 0x7632);
-}
-
-// One m16n8k32 MMA takes 512 weights: rows 0 to 7 of its weight operand are the 8 columns of a tile with the first half of the
-// group's positions, rows 8 to 15 the same columns with whole bytes, which are the first half's nibbles and 16 times the second's;
-// the columns of the activation operand are the four digits of the first half, then of the second. Integers: every product and sum
-// is exact. Lane (c, t) of the result has the sums of digits 2 (t % 2) and the next one of half t / 2: the first half's are in the
-// upper row, the second's are the lower row's less the upper's (a subtraction for four masks). The four lanes of a column add up to
-// the dot product. The zero point comes off through the group's sum.
-__device__ __forceinline__ void mma8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
-{
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma8_first(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
-{
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+    put_digits(reinterpret_cast<uint32_t *>(group + (lane >> 4) * kHalfAt + (lane & 3) * 16 + ((lane >> 2) & 3) * 4), v.x, v.y, v.z, v.w,
+               __uint_as_float(scale_exponent(top) << 23));
 }
 constexpr int kBurst = 5;  // units of a warp that are worked on side by side, without a branch between them (down: five groups per warp in the 0.5B model)
 struct Unit {  // weights in registers, requested before the activations are there
@@ -328,36 +289,6 @@ struct Unit {  // weights in registers, requested before the activations are the
         s = *reinterpret_cast<const float2 *>(ub + 512 + (lane >> 2) * 8);
     }
 };
-// What a lane knows about its two digits.
-struct Lane {
-    int at;            // its bytes of a staged group
-    int m0, m2;        // weights of the sums of its column's two rows
-    float digit, fac;  // 1 or 2^16; the same, with the second half's 16 taken back
-    __device__ __forceinline__ explicit Lane(int lane)
-        : at(lane * 16 + (lane >> 4) * (kHalfAt - 256)), m0((lane & 2) ? -1 : 1), m2((lane >> 1) & 1), digit((lane & 1) ? 65536.f : 1.f), fac((lane & 2) ? digit * 0.0625f : digit)
-    {
-    }
-    __device__ __forceinline__ float value(const int (&d)[4]) const { return (float)(d[0] * m0 + d[2] * m2 + 256 * (d[1] * m0 + d[3] * m2)); }
-    __device__ __forceinline__ float sum(const int (&d)[4]) const { return (float)(d[1] * 256 + d[0]); }  // of digit_sums
-};
-__device__ __forceinline__ void unit_dot(int (&d)[4], const uint4 &q, const uint4 &b)
-{
-    constexpr uint32_t kLow = 0x0f0f0f0fu;
-    mma8_first(d, q.x & kLow, q.x, q.y & kLow, q.y, b.x, b.y);
-    mma8(d, q.z & kLow, q.z, q.w & kLow, q.w, b.z, b.w);
-}
-// Sums of the digits, by the same instruction with a weight operand of ones.
-__device__ __forceinline__ void digit_sums(int (&d)[4], const uint4 &b)
-{
-    constexpr uint32_t kOnes = 0x01010101u;
-    mma8_first(d, kOnes, kOnes, kOnes, kOnes, b.x, b.y);
-    mma8(d, kOnes, kOnes, kOnes, kOnes, b.z, b.w);
-}
-__device__ __forceinline__ float quad_sum(float a)  // over the four lanes of a column
-{
-    a += __shfl_xor_sync(0xffffffffu, a, 1);
-    return a + __shfl_xor_sync(0xffffffffu, a, 2);
-}
 // fp16 MMA of the attention.
 __device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b)
 {

@@ -1,0 +1,90 @@
+// Exact products of int4 weights with f32 activations on the int8 tensor instruction (decode_fused.cu, gemv_stream.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+#include <math.h>
+#include <stdint.h>
+
+namespace wb {
+namespace dg {
+
+// ---- staging: f32 values -> signed bytes, group by group of 128 positions ----
+// Which positions are a group's two halves follows from how the weights lie: a word's low nibbles and its high ones.
+// A group's values become 30-bit integers of one scale, the power of two that puts the group's largest magnitude into [2^29, 2^30),
+// and these four signed bytes ("digits", base 256) each. A digit of four neighbouring positions is one word; the 32 words of a digit
+// are ordered as the MMA's lanes take them (half of the group, lane % 4, word), so that a lane reads its 16 bytes of a group at
+// once: [half][digit][lane % 4][4 words]. Between the halves stands the scale taken back, four times, each with a quarter of the sum of the
+// values behind it (where sums are staged).
+constexpr int kGroupBytes = 576, kHalfAt = 320, kScaleAt = 256;  // (an offset of 320: the halves' stores hit different banks)
+__device__ __forceinline__ uint32_t abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+// The four bytes of an integer below 2^31 - 2^23 in balanced base 256: byte i holds the digit i.
+__device__ __forceinline__ uint32_t digits(float v)
+{
+    constexpr uint32_t kCarry = 0x00808080u;
+    return ((uint32_t)__float2int_rn(v) + kCarry) ^ kCarry;
+}
+__device__ __forceinline__ uint32_t scale_exponent(uint32_t top) { return (uint32_t)min(283 - (int)(top >> 23), 253); }  // biased; the scale and its inverse are normal numbers
+__device__ __forceinline__ float scale_back(uint32_t top, float limit = INFINITY)  // a magnitude of `limit` or more makes the whole group NaN
+{
+    return top >= __float_as_uint(limit) ? __uint_as_float(0x7fffffffu) : __uint_as_float((254 - scale_exponent(top)) << 23);
+}
+// Four positions of a half, `at` their words: digit k goes to at[16 k].
+__device__ __forceinline__ void put_digits(uint32_t *at, float x, float y, float z, float w, float up)
+{
+    const uint32_t a = digits(x * up), b = digits(y * up), c = digits(z * up), d = digits(w * up);
+    const uint32_t ab = __byte_perm(a, b, 0x5140), cd = __byte_perm(c, d, 0x5140), AB = __byte_perm(a, b, 0x7362), CD = __byte_perm(c, d, 0x7362);
+    at[0] = __byte_perm(ab, cd, 0x5410), at[16] = __byte_perm(ab, cd, 0x7632);
+    at[32] = __byte_perm(AB, CD, 0x5410), at[48] = __byte_perm(AB, CD, 0x7632);
+}
+
+// One m16n8k32 MMA takes 512 weights: rows 0 to 7 of its weight operand are the 8 columns of a tile with the first half of the
+// group's positions, rows 8 to 15 the same columns with whole bytes, which are the first half's nibbles and 16 times the second's;
+// the columns of the activation operand are the four digits of the first half, then of the second. Integers: every product and sum
+// is exact. Lane (c, t) of the result has the sums of digits 2 (t % 2) and the next one of half t / 2: the first half's are in the
+// upper row, the second's are the lower row's less the upper's (a subtraction for four masks). The four lanes of a column add up to
+// the dot product. The zero point comes off through the group's sum.
+__device__ __forceinline__ void mma8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
+{
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma8_first(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
+{
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+}
+// What a lane knows about its two digits.
+struct Lane {
+    int at;            // its bytes of a staged group
+    int m0, m2;        // weights of the sums of its column's two rows
+    float digit, fac;  // 1 or 2^16; the same, with the second half's 16 taken back
+    __device__ __forceinline__ explicit Lane(int lane)
+        : at(lane * 16 + (lane >> 4) * (kHalfAt - 256)), m0((lane & 2) ? -1 : 1), m2((lane >> 1) & 1), digit((lane & 1) ? 65536.f : 1.f), fac((lane & 2) ? digit * 0.0625f : digit)
+    {
+    }
+    __device__ __forceinline__ float value(const int (&d)[4]) const { return (float)(d[0] * m0 + d[2] * m2 + 256 * (d[1] * m0 + d[3] * m2)); }
+    __device__ __forceinline__ float sum(const int (&d)[4]) const { return (float)(d[1] * 256 + d[0]); }  // of digit_sums
+};
+__device__ __forceinline__ void unit_dot(int (&d)[4], const uint4 &q, const uint4 &b)
+{
+    constexpr uint32_t kLow = 0x0f0f0f0fu;
+    mma8_first(d, q.x & kLow, q.x, q.y & kLow, q.y, b.x, b.y);
+    mma8(d, q.z & kLow, q.z, q.w & kLow, q.w, b.z, b.w);
+}
+// Sums of the digits, by the same instruction with a weight operand of ones.
+__device__ __forceinline__ void digit_sums(int (&d)[4], const uint4 &b)
+{
+    constexpr uint32_t kOnes = 0x01010101u;
+    mma8_first(d, kOnes, kOnes, kOnes, kOnes, b.x, b.y);
+    mma8(d, kOnes, kOnes, kOnes, kOnes, b.z, b.w);
+}
+__device__ __forceinline__ float quad_sum(float a)  // over the four lanes of a column
+{
+    a += __shfl_xor_sync(0xffffffffu, a, 1);
+    return a + __shfl_xor_sync(0xffffffffu, a, 2);
+}
+
+}  // namespace dg
+}  // namespace wb

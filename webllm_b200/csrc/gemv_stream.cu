@@ -15,12 +15,14 @@
 //     outputs a thread owns, not sixteen;
 //   * CTAs are persistent over column tiles (two CTAs per SM, one wave): the activations are staged once per CTA and the
 //     register prefetch runs on across tile boundaries, so the loads never drain between tiles.
+// One row goes to a kernel of its own (gptq_gemv_digits_kernel).
 // A TMA-fed variant of this kernel (one elected thread copying [16 rows x 32 columns] boxes into a ring of shared-memory
 // slots, persistent over column tiles) was built and measured slower (16.7 us against 14.0 us on K = 3584, N = 18944),
 // so the loads stay per thread.
 // 80 registers and two buffers, so that a third CTA (of this launch or of the next one) fits an SM, were no faster either: a
 // 7B-class layer of seven projections at M = 1 36.6 -> 37.4 us, at M = 4 with f32 activations 48.4 -> 55.6.
 #include "common.cuh"
+#include "digits.cuh"
 #include "gemv_core.cuh"
 
 namespace wb {
@@ -36,6 +38,8 @@ __device__ __forceinline__ void mma_16816_zero(float (&d)[4], uint32_t a0, uint3
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
+
+constexpr int kRoundTiles = 4, kDepth = 4;
 
 struct StreamRegs {
     uint4 w[4];  // packed words: rows 4 * st + t of the chunk, columns c .. c + 3
@@ -274,6 +278,180 @@ __global__ void __launch_bounds__(256, 2) gptq_gemv_stream_kernel(const GemvPara
     }
 }
 
+// One row, with int8 MMAs (digits.cuh): the activations as 30-bit integers of one scale per 128 rows, a chunk's packed words as they
+// lie, one mask a word and 8 MMAs a chunk of 128 rows x 32 columns where the fp16 form has four masks a word and 16. What it is bound
+// by is bytes in flight, and by the idle time of HBM between launches: 128 registers hold four chunks a warp, two CTAs fill an SM.
+// A 7B-class layer (seven projections, fp16, weights from HBM in every pass): 50.1 us with the fp16 form; with 2 buffers in 80 registers,
+// three CTAs an SM, so that the next launch's requests start early, 48.9; 3 buffers 42.9; 4 buffers 41.2; 5 (which spill) 43.8; 8 buffers
+// in one CTA an SM 46.5. Two rows would need their own MMAs for each: 56.0 us, the fp16 form, which has room for four rows in one
+// MMA, 54.9.
+__global__ void __launch_bounds__(256, 2) gptq_gemv_digits_kernel(const GemvParams p)
+{
+    using namespace dg;
+    extern __shared__ __align__(16) char smem[];
+    const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int ch_begin = blockIdx.y * p.chunks_per_split, chunks_cta = min(p.chunks, ch_begin + p.chunks_per_split) - ch_begin;
+    const int col_tiles = p.N >> 5;
+    const int tiles_cta = (int)blockIdx.x < col_tiles ? (col_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+    char *staged = smem;                                                               // [chunks_cta] groups
+    float *red = reinterpret_cast<float *>(smem + p.chunks_per_split * kGroupBytes);   // [tiles of a round][8 warps][32 lanes][4]
+    __shared__ int is_last[kRoundTiles];
+
+    // A round is up to kRoundTiles column tiles; its (tile, chunk) items are dealt to the warps in turn, so that a warp comes to every
+    // tile of it (a slice has at least 8 chunks), and its sums wait in shared memory for the round's end: one barrier a round.
+    // Offsets are 32 bits wide (the host checks), which is what leaves the registers for the buffers.
+    struct Pos {
+        int j, ch;  // tile, chunk
+    };
+    auto round_of = [&](int j) { return min((j / kRoundTiles + 1) * kRoundTiles, tiles_cta); };  // its last tile + 1
+    auto advance = [&](Pos &q) {                                                                 // true: another tile
+        q.ch += 8;
+        if (q.ch < chunks_cta) return false;
+        q.ch -= chunks_cta, q.j++;
+        if (q.j % kRoundTiles == 0) q.ch = warp;
+        return true;
+    };
+    struct Buf {
+        uint4 w[4];
+        uint2 s;
+        uint32_t z;
+    };
+    const uint32_t N = (uint32_t)p.N;
+    Pos next = {0, warp};
+    uint32_t wo, so, zo;
+    auto point = [&]() {
+        const uint32_t ch = (uint32_t)(ch_begin + next.ch), c = ((uint32_t)blockIdx.x + (uint32_t)next.j * gridDim.x) * 32 + 4 * g;
+        const uint32_t G = p.group_chunks == 1 ? ch : ch / (uint32_t)p.group_chunks;
+        wo = (ch * 16 + t) * N + c, so = G * N + c, zo = G * (uint32_t)p.zcols + (c >> 3);
+    };
+    auto fetch = [&](Buf &v) {
+        if (next.j >= tiles_cta) return;
+#pragma unroll
+        for (int st = 0; st < 4; st++) v.w[st] = ldg_stream_v4(p.qw + (wo + st * 4 * N));
+        v.s = *reinterpret_cast<const uint2 *>(p.sc + so);
+        v.z = p.qz ? p.qz[zo] : 0x77777777u;
+        if (advance(next) || p.group_chunks != 1) point();
+        else wo += 128 * N, so += 8 * N, zo += 8 * (uint32_t)p.zcols;
+    };
+    point();
+    Buf buf[kDepth];
+#pragma unroll
+    for (int u = 0; u < kDepth; u++) fetch(buf[u]);
+    pdl_sync();
+
+    // ---- the activations, two groups a warp at a time: a lane has one packed row's 8 positions ----
+#pragma unroll 1
+    for (int i0 = 2 * warp; i0 < chunks_cta; i0 += 16) {
+        const int gi = min(i0 + (lane >> 4), chunks_cta - 1), r = lane & 15;  // (an odd last group twice)
+        const int k0 = (ch_begin + gi) * 128 + r * 8;
+        float v[8];
+        if (p.x_f16) {
+            const uint4 raw = *reinterpret_cast<const uint4 *>((const __half *)p.x + k0);
+            const __half2 *h = reinterpret_cast<const __half2 *>(&raw);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float2 f = __half22float2(h[j]);
+                v[2 * j] = f.x, v[2 * j + 1] = f.y;
+            }
+        } else {
+            const float4 a = reinterpret_cast<const float4 *>((const float *)p.x + k0)[0], b = reinterpret_cast<const float4 *>((const float *)p.x + k0)[1];
+            v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+        }
+        uint32_t top = 0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) top = max(top, abs_bits(v[j]));
+        float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        sum += __shfl_xor_sync(0xffffffffu, sum, 8), top = max(top, __shfl_xor_sync(0xffffffffu, top, 8));
+        sum += __shfl_xor_sync(0xffffffffu, sum, 4), top = max(top, __shfl_xor_sync(0xffffffffu, top, 4));
+        top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
+        top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
+        const float up = __uint_as_float(scale_exponent(top) << 23);
+        char *group = staged + gi * kGroupBytes;
+        uint32_t *at = reinterpret_cast<uint32_t *>(group) + (r & 3) * 4 + (r >> 2);
+        put_digits(at, v[0], v[2], v[4], v[6], up);
+        put_digits(at + kHalfAt / 4, v[1], v[3], v[5], v[7], up);
+        *reinterpret_cast<float2 *>(group + kScaleAt + (r & 3) * 8) = make_float2(scale_back(top), sum);
+    }
+    __syncthreads();
+
+    const Lane ln(lane);
+    const int zshift = ((4 * g) & 7) * 4;
+    float tot[4] = {};
+    auto chunk_step = [&](const Buf &v, int ch) {
+        const char *group = staged + ch * kGroupBytes;
+        const uint4 b = *reinterpret_cast<const uint4 *>(group + ln.at);
+        const float2 s2 = *reinterpret_cast<const float2 *>(group + kScaleAt + t * 8);
+        const float gx = s2.x * ln.fac;
+        const uint32_t zw = v.z >> zshift;
+        const float2 s01 = __half22float2(u32_as_h2(v.s.x)), s23 = __half22float2(u32_as_h2(v.s.y));
+        const float scale[4] = {s01.x, s01.y, s23.x, s23.y};
+        int d[4][4];
+        unit_dot(d[0], make_uint4(v.w[0].x, v.w[1].x, v.w[2].x, v.w[3].x), b);
+        unit_dot(d[1], make_uint4(v.w[0].y, v.w[1].y, v.w[2].y, v.w[3].y), b);
+        unit_dot(d[2], make_uint4(v.w[0].z, v.w[1].z, v.w[2].z, v.w[3].z), b);
+        unit_dot(d[3], make_uint4(v.w[0].w, v.w[1].w, v.w[2].w, v.w[3].w), b);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float zero = __uint_as_float(0x4b000000u | ((zw >> (4 * i)) & 15u)) - 8388607.f;  // stored nibble + 1
+            tot[i] = fmaf(scale[i], fmaf(-zero, s2.y, ln.value(d[i]) * gx), tot[i]);
+        }
+    };
+    // End of a round: the sums over the warps (in their order) and over the four lanes of a column, then out or, where K is split, to the
+    // workspace; the last slice to arrive for a tile adds the slices in their order and the bias once.
+    auto round_end = [&](int first, int tiles) {
+        __syncthreads();
+        auto store = [&](int n, float v) {
+            if (p.bias) v += p.bias[n];
+            if (p.out_f16) ((__half *)p.out)[n] = __float2half_rn(v);
+            else ((float *)p.out)[n] = v;
+        };
+        for (int idx = tid; idx < tiles * 128; idx += 256) {
+            const int slot = idx >> 7, c = (idx & 127) >> 2, src = ((c >> 2) * 4 + (idx & 3)) * 4 + (c & 3);
+            float v = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; w++) v += red[(slot * 8 + w) * 128 + src];
+            v = quad_sum(v);
+            const int n = ((int)blockIdx.x + (first + slot) * (int)gridDim.x) * 32 + c;
+            if ((idx & 3) == 0) {
+                if (p.S == 1) store(n, v);
+                else p.partial[(int64_t)blockIdx.y * p.N + n] = v;
+            }
+        }
+        if (p.S > 1) {
+            __threadfence();
+            __syncthreads();
+            if (tid < tiles) is_last[tid] = atomicAdd(&p.counters[(int)blockIdx.x + (first + tid) * (int)gridDim.x], 1u) == (unsigned)(p.S - 1);
+            __syncthreads();
+            __threadfence();
+            if (tid < tiles * 32 && is_last[tid >> 5]) {
+                const int tile = (int)blockIdx.x + (first + (tid >> 5)) * (int)gridDim.x, n = tile * 32 + (tid & 31);
+                float v = 0.f;
+                for (int s = 0; s < p.S; s++) v += __ldcg(&p.partial[(int64_t)s * p.N + n]);
+                store(n, v);
+                if ((tid & 31) == 0) p.counters[tile] = 0u;
+            }
+        }
+        __syncthreads();  // red and is_last are the next round's
+    };
+
+    Pos at = {0, warp};
+    while (at.j < tiles_cta) {
+#pragma unroll
+        for (int u = 0; u < kDepth; u++) {
+            if (at.j >= tiles_cta) break;
+            chunk_step(buf[u], at.ch);
+            fetch(buf[u]);
+            const int j = at.j;
+            if (advance(at)) {
+                reinterpret_cast<float4 *>(red)[(j % kRoundTiles * 8 + warp) * 32 + lane] = make_float4(tot[0], tot[1], tot[2], tot[3]);
+                tot[0] = tot[1] = tot[2] = tot[3] = 0.f;
+                if (j + 1 == round_of(j)) round_end(j / kRoundTiles * kRoundTiles, j % kRoundTiles + 1);
+            }
+        }
+    }
+}
+
 // ---- host side -------------------------------------------------------------------------------------------------
 // Dynamic shared memory of one CTA: the staged operand rows (hi, lo for f32 activations, one row of zeros), the
 // per-chunk activation sums and the cross-warp reduction buffer.
@@ -306,6 +484,8 @@ int gemv_stream_grid_x(int sm_count, int64_t N, int S)
     return (col_tiles + waves - 1) / waves;
 }
 
+static size_t gemv_digits_smem(int cps) { return (size_t)cps * dg::kGroupBytes + (size_t)kRoundTiles * 4096; }
+
 int launch_gemv_stream(wb_context *ctx, const Weight &w, const GemvParams &gp, bool has_lo)
 {
     GemvParams p = gp;
@@ -316,7 +496,10 @@ int launch_gemv_stream(wb_context *ctx, const Weight &w, const GemvParams &gp, b
     const size_t smem = gemv_stream_smem(p.M, cps, has_lo);
     dim3 grid((unsigned)gemv_stream_grid_x(ctx->sm_count, w.N, p.S), (unsigned)p.S);
     cudaError_t e;
-    if (has_lo) {
+    if (p.M == 1 && w.K / 8 * w.N < (int64_t)1 << 31) {
+        e = smem_limit_once<gptq_gemv_digits_kernel>(200 * 1024);
+        if (e == cudaSuccess) e = launch_pdl(gptq_gemv_digits_kernel, grid, dim3(256), gemv_digits_smem(cps), ctx->stream, p);
+    } else if (has_lo) {
         e = smem_limit_once<gptq_gemv_stream_kernel<true>>(100 * 1024);
         if (e == cudaSuccess) e = launch_pdl(gptq_gemv_stream_kernel<true>, grid, dim3(256), smem, ctx->stream, p);
     } else {
