@@ -53,6 +53,18 @@ def test_fused_decode_matches_oracle(built_lib, oracle, C, H, KVH, I, V, prompt,
         model.close()
 
 
+@pytest.mark.parametrize("C,H,KVH,I,V,prompt,kv", [
+    (384, 6, 2, 8192, 700, 20, "f32"),
+    (512, 8, 2, 6400, 700, 20, "f16"),
+    (768, 12, 3, 5120, 700, 450, "f16"),
+])
+def test_fused_decode_shares_of_the_mlp(built_lib, oracle, C, H, KVH, I, V, prompt, kv):
+    """The hidden sizes that the cases above leave out, with MLPs of more lines of 32 results than CTAs: the rest of the lines dealt by
+    tiles, five or six of a CTA (8192), two or three (6400: two are shared out by units, three are not), one of some CTAs (5120); and
+    a context that crosses 512 keys, where the splits of a head change from one pass each to two."""
+    test_fused_decode_matches_oracle(built_lib, oracle, C, H, KVH, I, V, prompt, kv)
+
+
 @pytest.mark.parametrize("kv", ["f16", "f32"])
 @pytest.mark.parametrize("prompt", [3, 140])
 def test_attention_takes_values_beyond_fp16(built_lib, oracle, kv, prompt):
