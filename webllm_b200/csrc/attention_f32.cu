@@ -8,10 +8,9 @@
 // key, 32 lines touched per load, took the L1 8000 cycles an SM); scores are taken four dims at a time from 16-byte pieces. One CTA per single row, as the scalar kernel (qwen_ops.cu) has it, reads every
 // key 32 times as often and leaves a warp's lanes one multiply per load. 4 x 101 rows, 14 heads: 57 -> 22 us with
 // one group, whose chain of key blocks it was, 17 with four, 14 with rows read as they lie. Bound by the multiply-adds and the loads
-// that feed them on the SMs that have two long tiles. Two CTAs an SM leave a thread 64 registers, and 44 bytes are spilled. With one of 128
-// registers nothing is, and a layer of 1 x 384 tokens takes 74 us instead of 82, of 4 x 101 67.4 instead of 68.1, but of 6 x 50 61.7
-// instead of 61.0.
+// that feed them on the SMs that have two long tiles.
 #include <algorithm>
+#include <type_traits>
 
 #include "qwen_ops.cuh"
 
@@ -41,8 +40,9 @@ __device__ __forceinline__ float4 load4(const __half *p)
 }
 
 // Rows i of sequence b (row b * T + i of q and out) see keys 0 .. past + i, row b * key_rows + key of kmem / vmem.
-template <typename KV>
-__global__ void __launch_bounds__(kThreads, 2) attention_f32_kernel(const float *__restrict__ q, const KV *__restrict__ kmem,
+// CTAS: of an SM (see op_attention_f32).
+template <typename KV, int CTAS>
+__global__ void __launch_bounds__(kThreads, CTAS) attention_f32_kernel(const float *__restrict__ q, const KV *__restrict__ kmem,
                                                                  const KV *__restrict__ vmem, float *__restrict__ out, __half *__restrict__ out16, int H, int KVH, int T,
                                                                  const int *__restrict__ past_ptr, int past_imm, int key_rows, int ldq,
                                                                  int kv_ld, float scale)
@@ -175,24 +175,33 @@ int op_attention_f32(wb_context *ctx, const float *q, const void *kmem, const vo
 {
     const float scale = 1.0f / sqrtf((float)kD);
     const int key_rows = use_cache ? 0 : T;  // (one sequence with a cache)
-    if (const cudaError_t e = kv_f16 ? smem_limit_once<attention_f32_kernel<__half>>((int)sizeof(Smem)) : smem_limit_once<attention_f32_kernel<float>>((int)sizeof(Smem));
-        e != cudaSuccess)
-        WB_CUDA(e);
+    // Two CTAs an SM leave a thread 64 registers, and 44 bytes are spilled; one has 118 and spills nothing. It is taken where every SM gets
+    // one at most, or two whose lengths even out because a sequence has several tiles (forward passes of 24 layers, 14 heads, us, two and
+    // one: 2 x 100 tokens 1404, 1300; 1 x 250 1576, 1459; 4 x 64 1335, 1265; 1 x 384 2005, 1834; 2 x 190 1798, 1630; 3 x 130 1780, 1704; 4 x 101
+    // 1695, 1678; 5 x 80 1642, 1627; 1 x 32 885, 867; 8 x 16 1186, 1158; but 6 x 66 1633, 1654; 6 x 60 1550, 1557). With more than two for every SM it is two as before.
+    constexpr int kSeveralTiles = 73;  // tokens: two tiles and more than a quarter of a third
     const int B = M / T;
-    for (int b = 0; b < B; b += kSequences) {
-        const dim3 grid((unsigned)H, (unsigned)((T + kRows - 1) / kRows), (unsigned)std::min(B - b, kSequences));
-        const int64_t row = (int64_t)b * T, at = row * H * kD, key = (int64_t)b * key_rows * kv_ld;
-        const float *qb = q + row * ldq;
-        float *ob = out ? out + at : nullptr;
-        __half *o16 = out16 ? out16 + at : nullptr;
-        const cudaError_t e =
-            kv_f16 ? launch_pdl(attention_f32_kernel<__half>, grid, dim3(kThreads), sizeof(Smem), ctx->stream, qb, (const __half *)kmem + key,
-                                (const __half *)vmem + key, ob, o16, H, KVH, T, past_ptr, past_imm, key_rows, ldq, kv_ld, scale)
-                   : launch_pdl(attention_f32_kernel<float>, grid, dim3(kThreads), sizeof(Smem), ctx->stream, qb, (const float *)kmem + key,
-                                (const float *)vmem + key, ob, o16, H, KVH, T, past_ptr, past_imm, key_rows, ldq, kv_ld, scale);
-        ctx->launches++;
-        WB_CUDA(e);
-    }
+    const int64_t ctas = (int64_t)H * ((T + kRows - 1) / kRows) * B, sms = ctx->sm_count;
+    const bool one = ctas <= sms || (ctas <= 2 * sms && T >= kSeveralTiles);
+    auto run = [&](auto kern, cudaError_t limit, auto kv) -> cudaError_t {  // kern's launches, kv: a null pointer of the keys' type
+        if (limit != cudaSuccess) return limit;
+        using KV = std::remove_pointer_t<decltype(kv)>;
+        for (int b = 0; b < B; b += kSequences) {
+            const dim3 grid((unsigned)H, (unsigned)((T + kRows - 1) / kRows), (unsigned)std::min(B - b, kSequences));
+            const int64_t row = (int64_t)b * T, at = row * H * kD, key = (int64_t)b * key_rows * kv_ld;
+            const cudaError_t e = launch_pdl(kern, grid, dim3(kThreads), sizeof(Smem), ctx->stream, q + row * ldq, (const KV *)kmem + key, (const KV *)vmem + key,
+                                             out ? out + at : nullptr, out16 ? out16 + at : nullptr, H, KVH, T, past_ptr, past_imm, key_rows, ldq, kv_ld, scale);
+            ctx->launches++;
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    };
+    auto pick = [&](auto kv) {
+        using KV = std::remove_pointer_t<decltype(kv)>;
+        return one ? run(attention_f32_kernel<KV, 1>, smem_limit_once<attention_f32_kernel<KV, 1>>((int)sizeof(Smem)), kv)
+                   : run(attention_f32_kernel<KV, 2>, smem_limit_once<attention_f32_kernel<KV, 2>>((int)sizeof(Smem)), kv);
+    };
+    WB_CUDA(kv_f16 ? pick((__half *)nullptr) : pick((float *)nullptr));
     return WB_OK;
 }
 
