@@ -62,8 +62,8 @@ CONFIG = {"workload": WORKLOAD,
           "l2": "each step streams 458 MB of weights (> 126 MB L2); no flush needed"}
 
 # dram__bytes_read.sum + dram__bytes_write.sum per step of decode_fused_kernel, from an ncu capture of a launch of two steps of
-# the 24-layer model at 18 keys (956.2 MB). Algorithmic bytes: int4 tensors + fp16 lm_head, 458 171 392 a step.
-NCU_TRAFFIC_BYTES_PER_STEP = 478115384
+# the 24-layer model at 18 keys (953.8 MB). Algorithmic bytes: int4 tensors + fp16 lm_head, 458 171 392 a step.
+NCU_TRAFFIC_BYTES_PER_STEP = 476906240
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of gptq_gemv_mma_kernel, mean over the four projections
 # of a layer, from an ncu capture of a 2-layer model of the same shapes (one pass per launch, caches flushed between
