@@ -34,9 +34,9 @@ def test_f32_attention_tiles(built_lib, oracle, small, B, T):
         model.close()
 
 
-@pytest.mark.parametrize("B,T", [(10, 97), (25, 73), (25, 72), (80, 33)])
+@pytest.mark.parametrize("B,T", [(11, 128), (11, 127), (80, 33)])
 def test_f32_attention_ctas(built_lib, oracle, small, B, T):
-    """More tiles of 32 rows than SMs: from 73 tokens on up to two an SM go to the kernel's form of one CTA an SM, fewer tokens (72) and
+    """More tiles of 32 rows than SMs: from 128 tokens on up to two an SM go to the kernel's form of one CTA an SM, fewer tokens (127) and
     more tiles (640) to the one of two."""
     test_f32_attention_tiles(built_lib, oracle, small, B, T)
 

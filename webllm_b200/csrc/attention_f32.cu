@@ -176,10 +176,10 @@ int op_attention_f32(wb_context *ctx, const float *q, const void *kmem, const vo
     const float scale = 1.0f / sqrtf((float)kD);
     const int key_rows = use_cache ? 0 : T;  // (one sequence with a cache)
     // Two CTAs an SM leave a thread 64 registers, and 44 bytes are spilled; one has 118 and spills nothing. It is taken where every SM gets
-    // one at most, or two whose lengths even out because a sequence has several tiles (forward passes of 24 layers, 14 heads, us, two and
-    // one: 2 x 100 tokens 1404, 1300; 1 x 250 1576, 1459; 4 x 64 1335, 1265; 1 x 384 2005, 1834; 2 x 190 1798, 1630; 3 x 130 1780, 1704; 4 x 101
-    // 1695, 1678; 5 x 80 1642, 1627; 1 x 32 885, 867; 8 x 16 1186, 1158; but 6 x 66 1633, 1654; 6 x 60 1550, 1557). With more than two for every SM it is two as before.
-    constexpr int kSeveralTiles = 73;  // tokens: two tiles and more than a quarter of a third
+    // one at most, or two whose lengths even out because a sequence has four tiles and more (forward passes of 24 layers, 14 heads, us, two
+    // and one: 1 x 128 tokens 687, 645; 1 x 250 998, 920; 2 x 100 894, 864; 4 x 64 858, 843; 1 x 384 1645, 1456; 2 x 190 1384, 1330; 3 x 130 1280,
+    // 1255; but 4 x 101 1239, 1248, and, at lower clocks, 6 x 66 1633, 1654). With more than two for every SM it is two as before.
+    constexpr int kSeveralTiles = 4 * kRows;  // tokens
     const int B = M / T;
     const int64_t ctas = (int64_t)H * ((T + kRows - 1) / kRows) * B, sms = ctx->sm_count;
     const bool one = ctas <= sms || (ctas <= 2 * sms && T >= kSeveralTiles);
