@@ -68,7 +68,7 @@ struct Params {
     const __half *embed;
     const float *cs_table;
     char *k_cache, *v_cache;
-    u64 *ll;                // hand-over words of a layer (ll_layer), then two sets of 2 per CTA for the argmax candidates
+    u64 *ll;                // hand-over words of a layer (ll_layer), then two sets of 4 per CTA for the argmax candidates
     float *logits;
     uint32_t *history;      // nullable; pinned host memory
     int *status;
